@@ -298,7 +298,8 @@ __device__ __forceinline__ void group_reduce_ff(const Group& g, const GroupSmem&
 __device__ inline void stage_chain_f64(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                        const MovedInfo& mi, int lane) {
   for (int i = lane; i < mi.len; i += 32) {
-    const double2 bl = blend64(P.sig[mi.atom0 + i], P.eps[mi.atom0 + i]);
+    const int a0 = mi.atom0 + i;
+    const double2 bl = P.blend ? P.blend[a0] : blend64(P.sig[a0], P.eps[a0]);
     s.sd[i] = bl.x;
     s.ed[i] = bl.y;
     s.qd[i] = P.q[mi.atom0 + i];
@@ -311,37 +312,15 @@ __device__ inline void stage_chain_f64(const Pool& P, const ChainHdr& H, const G
 
 __device__ __forceinline__ void batch_chain64(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                               const MovedInfo& mi, const int* rj, int head,
-                                              int count, int lane, int T, double& eo, double& en) {
-  const int tm = lane / T, tl = lane - tm * T, nteams = 32 / T;
-  for (int e0 = 0; e0 < count; e0 += nteams) {
-    const int e = e0 + tm;
-    int f = 0, b0 = 0, lenj = 0;
-    uint4 Aj = make_uint4(0u, 0u, 0u, 0u);
-    if (e < count) {
-      const int jf = rj[(head + e) & (kRing - 1)];
-      const int j = jf >> 4;
-      f = jf & 15;
-      b0 = P.mstart[j];
-      lenj = P.mlen[j] & 255;
-      Aj = P.mfix[j];
-    }
-    double so = 0.0, sn = 0.0;
-    for (int b = b0 + tl; b < b0 + lenj; b += T) {
-      const double3 xb = chain_pos3(Aj, P.aoff[b], H);
-      const double2 bl = P.blend ? P.blend[b] : blend64(P.sig[b], P.eps[b]);
-      const double sb = bl.x, eb = bl.y, qb = P.q[b];
-      if (f & kInOld) so += sum_moved64(s, false, mi.len, xb.x, xb.y, xb.z, sb, eb, qb, H);
-      if (f & kInNew) sn += sum_moved64(s, true, mi.len, xb.x, xb.y, xb.z, sb, eb, qb, H);
-    }
-    for (int off = T >> 1; off > 0; off >>= 1) {
-      so += __shfl_xor_sync(~0u, so, off);
-      sn += __shfl_xor_sync(~0u, sn, off);
-    }
-    if (tl == 0 && f) {
-      if (f & kInOld) eo += so;
-      if (f & kInNew) en += sn;
-    }
-  }
+                                              int count, int lane, double& eo, double& en,
+                                              long long& np) {
+  batch_items64(P, H, s, mi, rj, head, count, lane, eo, en, np,
+                [&](int j, int b, double& x, double& y, double& z) {
+                  const double3 p = chain_pos3(P.mfix[j], P.aoff[b], H);
+                  x = p.x;
+                  y = p.y;
+                  z = p.z;
+                });
 }
 
 // The FP64 re-take's screen: the reference's test for every primary pair
@@ -351,8 +330,8 @@ __device__ __forceinline__ void batch_chain64(const Pool& P, const ChainHdr& H, 
 // every nw-th entry per warp as in warp_eval_chain.
 __device__ inline void warp_eval_chain64(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                   const MovedInfo& mi, const float4* pcache, int c_begin,
-                                  int c_end, int w, int nw, int lane, int T, double& eo,
-                                  double& en, const int* cand = nullptr) {
+                                  int c_end, int w, int nw, int lane, double& eo,
+                                  double& en, long long& np, const int* cand = nullptr) {
   int* rj = s.lj + w * kRing;
   int head = 0, tail = 0;
   const unsigned lt = lanemask_lt();
@@ -382,18 +361,18 @@ __device__ inline void warp_eval_chain64(const Pool& P, const ChainHdr& H, const
         q0 = P.ppos[P.mpi[j].x];
       f = screen_chain(P, H, s, mi, j, q0);
     }
-  const unsigned bal = __ballot_sync(~0u, f != 0);
+    const unsigned bal = __ballot_sync(~0u, f != 0);
     if (f) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 4) | f;
     tail += __popc(bal);
     if (tail - head >= 32) {
       __syncwarp();
-      batch_chain64(P, H, s, mi, rj, head, 32, lane, T, eo, en);
+      batch_chain64(P, H, s, mi, rj, head, 32, lane, eo, en, np);
       head += 32;
       __syncwarp();
     }
   }
   __syncwarp();
-  if (tail > head) batch_chain64(P, H, s, mi, rj, head, tail - head, lane, T, eo, en);
+  if (tail > head) batch_chain64(P, H, s, mi, rj, head, tail - head, lane, eo, en, np);
   __syncwarp();
 }
 

@@ -428,15 +428,15 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     }
     __syncthreads();
     const int mol = prop.mol, m = H.mol0 + mol;
-    double eo = 0.0, en = 0.0, ab = 0.0;
+    double eo = 0.0, en = 0.0;
     long long np = 0;
     if (!intra) {
       // old and new placement in one pass (k_move_energies on one CTA)
       if (w == 0) stage(P, H, m, &prop, s, lane);
       grp.sync();
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, ab, np);
-      group_reduce(grp, s, eo, en, ab, np);
+      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, np);
+      group_reduce(grp, s, eo, en, np);
       if (tid == 0) {
         const double de = en - eo;
         flag = loop_accept(st.rng, de, kT);
@@ -459,8 +459,8 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     grp.sync();
     {
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, ab, np);
-      group_reduce(grp, s, eo, en, ab, np);
+      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, np);
+      group_reduce(grp, s, eo, en, np);
     }
     const double e_old = eo + ei_old;
     long long pairs = np;
@@ -546,12 +546,12 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     const double ei_new = have_cur ? cur : intra_energy(P, R, H, mol, red);
     if (w == 0) stage(P, H, m, nullptr, s, lane);
     grp.sync();
-    eo = en = ab = 0.0;
+    eo = en = 0.0;
     np = 0;
     {
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, ab, np);
-      group_reduce(grp, s, eo, en, ab, np);
+      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, np);
+      group_reduce(grp, s, eo, en, np);
     }
     if (tid == 0) {
       const double de = (eo + ei_new) - e_old;

@@ -62,10 +62,10 @@ __global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr,
   const int chunk = ((n_cand + gridDim.x - 1) / gridDim.x + 31) & ~31;
   const int cb = H.mol0 + start + blockIdx.x * chunk;
   const int ce = min(cb + chunk, H.mol0 + H.n_mol);
-  double eo = 0.0, en = 0.0, ab = 0.0;
+  double eo = 0.0, en = 0.0;
   long long np = 0;
-  if (cb < ce) warp_eval<F64>(P, H, s, mi, cb, ce, w, nw, lane, H.tpm, eo, en, ab, np);
-  group_reduce(g, s, eo, en, ab, np);
+  if (cb < ce) warp_eval<F64>(P, H, s, mi, cb, ce, w, nw, lane, H.tpm, eo, en, np);
+  group_reduce(g, s, eo, en, np);
   if (threadIdx.x == 0) {
     if (pairs) atomicAdd((unsigned long long*)pairs, (unsigned long long)np);
     partials[blockIdx.x] = eo;
@@ -99,10 +99,10 @@ __global__ void __launch_bounds__(256) k_move_energies(Pool P, int chain, int mo
   const int chunk = ((H.n_mol + gridDim.x - 1) / gridDim.x + 31) & ~31;
   const int cb = H.mol0 + blockIdx.x * chunk;
   const int ce = min(cb + chunk, H.mol0 + H.n_mol);
-  double eo = 0.0, en = 0.0, ab = 0.0;
+  double eo = 0.0, en = 0.0;
   long long np = 0;
-  if (cb < ce) warp_eval<F64>(P, H, s, mi, cb, ce, w, nw, lane, H.tpm, eo, en, ab, np);
-  group_reduce(g, s, eo, en, ab, np);
+  if (cb < ce) warp_eval<F64>(P, H, s, mi, cb, ce, w, nw, lane, H.tpm, eo, en, np);
+  group_reduce(g, s, eo, en, np);
   __shared__ int last;
   if (threadIdx.x == 0) {
     if (pairs) atomicAdd((unsigned long long*)pairs, (unsigned long long)np);
@@ -183,10 +183,10 @@ __global__ void __launch_bounds__(256) k_mol_pair_sums(Pool P, const int* mol_ch
   if (w == 0) stage(P, H, m, nullptr, s, lane);
   g.sync();
   const MovedInfo mi = load_moved(s);
-  double eo = 0.0, en = 0.0, ab = 0.0;
+  double eo = 0.0, en = 0.0;
   long long np = 0;
-  warp_eval<F64>(P, H, s, mi, m + 1, H.mol0 + H.n_mol, w, nw, lane, H.tpm, eo, en, ab, np);
-  group_reduce(g, s, eo, en, ab, np);
+  warp_eval<F64>(P, H, s, mi, m + 1, H.mol0 + H.n_mol, w, nw, lane, H.tpm, eo, en, np);
+  group_reduce(g, s, eo, en, np);
   if (threadIdx.x == 0) {
     emol[m] = eo;
     if (pairs) pairs[m] = np;
@@ -413,15 +413,15 @@ __device__ __forceinline__ void chain_steps(Pool P, int n_steps, unsigned* queue
       if (tie) {
         if (w == 0) stage_chain_f64(P, H, ss, mi, lane);
         g.sync();
-        double eo = 0.0, en = 0.0, ab2 = 0.0;
+        double eo = 0.0, en = 0.0;
         long long np2 = 0;
         if (use_list)
-          warp_eval_chain64(P, H, ss, mi, pcache, 0, P.nl_cnt[mi.mol], w, nw, lane, T, eo, en,
+          warp_eval_chain64(P, H, ss, mi, pcache, 0, P.nl_cnt[mi.mol], w, nw, lane, eo, en, np2,
                             P.nl + (size_t)mi.mol * P.nl_stride);
         else
-          warp_eval_chain64(P, H, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, w, nw, lane, T, eo,
-                            en);
-        group_reduce(g, ss, eo, en, ab2, np2, st & 1);
+          warp_eval_chain64(P, H, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, w, nw, lane, eo,
+                            en, np2);
+        group_reduce(g, ss, eo, en, np2, st & 1);
         e_old = eo;
         e_new = en;
         const double d64 = e_new - e_old;

@@ -104,7 +104,7 @@ __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Prop
   for (int i = lane; i < len; i += 32) {
     int a = a0 + i;
     s.ox[i] = P.x[a]; s.oy[i] = P.y[a]; s.oz[i] = P.z[a];
-    const double2 bl = blend64(P.sig[a], P.eps[a]);
+    const double2 bl = P.blend ? P.blend[a] : blend64(P.sig[a], P.eps[a]);
     s.sd[i] = bl.x; s.ed[i] = bl.y; s.qd[i] = P.q[a];
     const float4 o = P.aoff[a];
     const float2 q = P.aeq[a];
@@ -522,65 +522,169 @@ __device__ __forceinline__ void batch_u1(const Pool& P, const ChainHdr& H, const
   acc.ab += sa;
 }
 
-// FP64 pair terms from the master rows, the reference's per-pair minimum
-// image and dummy-site rule (BruteForceStep.cpp:61-76); sb, eb: the
-// neighbour atom's blending factors (blend64), the moved atoms' staged in
-// s.sd / s.ed.
-__device__ __forceinline__ double sum_moved64(const GroupSmem& s, bool use_new, int len, double xb,
-                                              double yb, double zb, double sb, double eb, double qb,
-                                              const ChainHdr& H) {
-  const double* xs = use_new ? s.nx : s.ox;
-  const double* ys = use_new ? s.ny : s.oy;
-  const double* zs = use_new ? s.nz : s.oz;
+// ---- FP64 pair batches -------------------------------------------------------
+//
+// GB300 issues FP64 at 1/64 of the FP32 rate: one warp instruction per 16
+// cycles on an SM whatever its active lanes, so an FP64 batch is bound by its
+// count of FP64 warp instructions.  Hence
+//   * the items of a batch (placement, neighbour atom) fill the lanes of the
+//     warp without gaps (a team of lanes per neighbour left 1 of 4 lanes idle
+//     on 3-site and 7 of 16 on 9-site molecules);
+//   * no FP64 comparison on a pair's path: the image, r = 0 and skipped-site
+//     tests read the operands' high words on the integer pipe;
+//   * the LJ term is formed only where its sigma and epsilon products are not
+//     zero (water: 1 pair of 9), and r^2 by fused multiply-adds.
+// 17 FP64 instructions a Coulomb pair and 25 with LJ, 43 before.
+
+// sigma factor of a skipped site (blend64).
+__device__ __forceinline__ bool blend_skipped(double sa) {
+  return __double2hiint(sa) == (int)0xBFF00000;
+}
+__device__ __forceinline__ bool bits_nonzero(double v) {
+  return (__double2hiint(v) | __double2loint(v)) != 0;
+}
+__device__ __forceinline__ int hi_abs(double v) { return __double2hiint(v) & 0x7fffffff; }
+
+// make_periodic with its comparisons on the high words; half = the high word
+// of L / 2 (equal high words take the FP64 comparisons).
+__device__ __forceinline__ double image64(double d, double L, int half) {
+  const int h = hi_abs(d);
+  if (h < half) return d;
+  if (h > half) return __dadd_rn(d, copysign(L, -d));
+  return make_periodic(d, L);
+}
+
+// Sum over the moved molecule's atoms (rows xs, ys, zs) of the FP64 pair
+// terms with neighbour atom b: the reference's minimum image of every pair
+// and its rule for skipped sites (BruteForceStep.cpp:61-76).  b is shifted
+// once to its image nearest the moved molecule's first atom; a pair that
+// still lies beyond half an edge (molecules straddling it, or rows outside
+// the box) takes the reference's own image from the unshifted rows.
+// (sb, eb): b's blending factors, qb its charge; the moved atoms' factors
+// are staged in s.sd / s.ed.
+__device__ __forceinline__ double sum_moved64(const GroupSmem& s, const double* xs,
+                                              const double* ys, const double* zs, int len,
+                                              double xb, double yb, double zb, double sb,
+                                              double eb, double qb, const ChainHdr& H) {
+  if (blend_skipped(sb)) return 0.0;
+  const double Lx = H.L[0], Ly = H.L[1], Lz = H.L[2];
+  const int hx = __double2hiint(0.5 * Lx), hy = __double2hiint(0.5 * Ly),
+            hz = __double2hiint(0.5 * Lz);
+  const double tx = xb - xs[0], ty = yb - ys[0], tz = zb - zs[0];
+  const double bx = hi_abs(tx) >= hx ? xb - copysign(Lx, tx) : xb;
+  const double by = hi_abs(ty) >= hy ? yb - copysign(Ly, ty) : yb;
+  const double bz = hi_abs(tz) >= hz ? zb - copysign(Lz, tz) : zb;
+  const bool lj_b = bits_nonzero(sb) && bits_nonzero(eb);
+  const double qk = qb * kCoulomb, e4 = 4.0 * eb;
   double acc = 0.0;
-  if (sb < 0) return acc;
+#pragma unroll 3
   for (int i = 0; i < len; i++) {
     const double sa = s.sd[i], ea = s.ed[i];
-    if (sa < 0) continue;
-    const double dx = make_periodic(xb - xs[i], H.L[0]);
-    const double dy = make_periodic(yb - ys[i], H.L[1]);
-    const double dz = make_periodic(zb - zs[i], H.L[2]);
-    const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    acc += pair64(r2, sa, sb, ea, eb, s.qd[i], qb);
+    if (blend_skipped(sa)) continue;
+    double dx = bx - xs[i], dy = by - ys[i], dz = bz - zs[i];
+    if (hi_abs(dx) >= hx || hi_abs(dy) >= hy || hi_abs(dz) >= hz) {
+      dx = image64(xb - xs[i], Lx, hx);
+      dy = image64(yb - ys[i], Ly, hy);
+      dz = image64(zb - zs[i], Lz, hz);
+    }
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    if (!bits_nonzero(r2)) continue;   // coincident: skipped (BruteForceStep.cpp:68-69)
+    const double ri = rsqrt(r2);
+    acc = fma(s.qd[i] * qk, ri, acc);
+    if (lj_b && bits_nonzero(sa) && bits_nonzero(ea)) {
+      const double t = (sa * sb) * ri;
+      const double t2 = t * t, s6 = t2 * t2 * t2;
+      const double e = ea * e4;
+      acc = fma(s6, fma(e, s6, -e), acc);
+    }
   }
   return acc;
 }
 
+// FP64 pair batch of `count` (1..32) ring entries from `head`: the items
+// (placement, entry, neighbour atom) are dealt to the lanes in order, old
+// placements first.  A uniform chain's items run atom by atom over the
+// entries, so the lanes of a round share the neighbour atom's kind and agree
+// on the LJ term; else an item's entry is found in the prefix sums of the
+// entries' lengths.  atom(j, b, x, y, z) gives the FP64 position of atom b of
+// neighbour j.
+template <class AtomPos>
+__device__ __forceinline__ void batch_items64(const Pool& P, const ChainHdr& H,
+                                              const GroupSmem& s, const MovedInfo& mi,
+                                              const int* rj, int head, int count, int lane,
+                                              double& eo, double& en, long long& np,
+                                              AtomPos atom) {
+  const int two = mi.states == 3 ? 2 : 1;
+  int pref = 0, total;
+  const bool uni = H.uniform != 0;
+  if (uni) {
+    total = count * H.ulen;
+    if (lane < count) {
+      const int f = rj[(head + lane) & (kRing - 1)] & 15;
+      np += (long long)__popc(f & (kInOld | kInNew)) * (mi.act * H.uact);
+    }
+  } else {
+    int len = 0;
+    if (lane < count) {
+      const int jf = rj[(head + lane) & (kRing - 1)];
+      const int lw = P.mlen[jf >> 4];
+      len = lw & 255;
+      np += (long long)__popc(jf & (kInOld | kInNew)) * (mi.act * (lw >> 8));
+    }
+    pref = len;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(~0u, pref, off);
+      if (lane >= off) pref += v;
+    }
+    total = __shfl_sync(~0u, pref, 31);
+    pref -= len;
+  }
+  const int items = total * two;
+  for (int base = 0; base < items; base += 32) {
+    const int it = base + lane;
+    const bool second = it >= total;
+    const int local = second ? it - total : it;
+    int e, k;
+    if (uni) {
+      k = local / count;
+      e = local - k * count;
+    } else {
+      e = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int at = e + step;
+        const int v = __shfl_sync(~0u, pref, at & 31);
+        if (at < count && v <= local) e = at;
+      }
+      k = local - __shfl_sync(~0u, pref, e);
+    }
+    if (it >= items) continue;
+    const int jf = rj[(head + e) & (kRing - 1)];
+    const bool use_new = second || mi.states == 2;
+    if (!(jf & (use_new ? kInNew : kInOld))) continue;
+    const int j = jf >> 4;
+    const int b = (uni ? H.atom0 + (j - H.mol0) * H.ulen : P.mstart[j]) + k;
+    double xb, yb, zb;
+    atom(j, b, xb, yb, zb);
+    const double2 bl = P.blend ? P.blend[b] : blend64(P.sig[b], P.eps[b]);
+    const double v = sum_moved64(s, use_new ? s.nx : s.ox, use_new ? s.ny : s.oy,
+                                 use_new ? s.nz : s.oz, mi.len, xb, yb, zb, bl.x, bl.y, P.q[b],
+                                 H);
+    if (use_new) en += v; else eo += v;
+  }
+}
+
+// The batch on the master rows (plain path).
 __device__ __forceinline__ void batch_f64(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                           const MovedInfo& mi, const int* rj, int head, int count,
-                                          int lane, int T, double& eo, double& en, double& ab,
-                                          long long& np) {
-  const int tm = lane / T, tl = lane - tm * T, nteams = 32 / T;
-  for (int e0 = 0; e0 < count; e0 += nteams) {
-    const int e = e0 + tm;
-    int f = 0, b0 = 0, lenj = 0, actj = 0;
-    if (e < count) {
-      const int jf = rj[(head + e) & (kRing - 1)];
-      const int j = jf >> 4;
-      f = jf & 15;
-      b0 = P.mstart[j];
-      const int lw = P.mlen[j];
-      lenj = lw & 255;
-      actj = lw >> 8;
-    }
-    double so = 0.0, sn = 0.0;
-    for (int b = b0 + tl; b < b0 + lenj; b += T) {
-      const double xb = P.x[b], yb = P.y[b], zb = P.z[b];
-      const double2 bl = P.blend[b];
-      const double qb = P.q[b];
-      if (f & kInOld) so += sum_moved64(s, false, mi.len, xb, yb, zb, bl.x, bl.y, qb, H);
-      if (f & kInNew) sn += sum_moved64(s, true, mi.len, xb, yb, zb, bl.x, bl.y, qb, H);
-    }
-    for (int off = T >> 1; off > 0; off >>= 1) {
-      so += __shfl_xor_sync(~0u, so, off);
-      sn += __shfl_xor_sync(~0u, sn, off);
-    }
-    if (tl == 0 && f) {
-      if (f & kInOld) { eo += so; np += (long long)mi.act * actj; }
-      if (f & kInNew) { en += sn; np += (long long)mi.act * actj; }
-      ab += fabs(so) + fabs(sn);
-    }
-  }
+                                          int lane, double& eo, double& en, long long& np) {
+  batch_items64(P, H, s, mi, rj, head, count, lane, eo, en, np,
+                [&](int, int b, double& x, double& y, double& z) {
+                  x = P.x[b];
+                  y = P.y[b];
+                  z = P.z[b];
+                });
 }
 
 // One warp screens candidates [c_begin, c_end) in warp-strided rounds of 32
@@ -590,7 +694,7 @@ __device__ __forceinline__ void batch_f64(const Pool& P, const ChainHdr& H, cons
 template <bool F64>
 __device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSmem& s, const MovedInfo& mi,
                           int c_begin, int c_end, int w, int nw, int lane, int T, double& eo,
-                          double& en, double& ab, long long& np) {
+                          double& en, long long& np) {
   int* rj = s.lj + w * kRing;
   int head = 0, tail = 0;
   const unsigned lt = lanemask_lt();
@@ -607,7 +711,7 @@ __device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSm
     if (tail - head >= 32) {
       __syncwarp();
       if (F64)
-        batch_f64(P, H, s, mi, rj, head, 32, lane, T, eo, en, ab, np);
+        batch_f64(P, H, s, mi, rj, head, 32, lane, eo, en, np);
       else if (H.precise)
         batch_ff<true, true>(P, H, s, mi, rj, head, 32, lane, T, acc);
       else
@@ -619,7 +723,7 @@ __device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSm
   __syncwarp();
   if (tail > head) {
     if (F64)
-      batch_f64(P, H, s, mi, rj, head, tail - head, lane, T, eo, en, ab, np);
+      batch_f64(P, H, s, mi, rj, head, tail - head, lane, eo, en, np);
     else if (H.precise)
       batch_ff<true, true>(P, H, s, mi, rj, head, tail - head, lane, T, acc);
     else
@@ -629,42 +733,44 @@ __device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSm
   if (!F64) {
     eo += (double)acc.oh + (double)acc.ol;
     en += (double)acc.nh + (double)acc.nl;
-    ab += (double)acc.ab;
     np += acc.np;
   }
 }
 
-// Group-wide deterministic sum of (a, b, d, c): warp shuffles, then every
-// thread adds the per-warp values in warp order.  Two calls must be
-// separated by a group barrier (the scratch is reused).
+// Warp sum of 64-bit counts (each below 2^48), in every lane: two integer
+// reductions of 24-bit halves.
+__device__ __forceinline__ long long warp_count(long long c) {
+  const unsigned lo = __reduce_add_sync(~0u, (unsigned)(c & 0xffffff));
+  const unsigned hi = __reduce_add_sync(~0u, (unsigned)(c >> 24));
+  return ((long long)hi << 24) + (long long)lo;
+}
+
+// Group-wide deterministic sum of (a, b, c), the same in every thread.  The
+// two halves of a warp take one sum each after the first exchange, and the
+// warps' values are added by a second butterfly over the lanes: 10 FP64
+// instructions a warp (adding the warps one by one in every thread took 15 +
+// 3 per warp, and FP64 issues once in 16 cycles per SM).  At most 16 warps.
+// Two calls must be separated by a group barrier (the scratch is reused).
 __device__ __forceinline__ void group_reduce(const Group& g, const GroupSmem& s, double& a,
-                                             double& b, double& d, long long& c, int par = 0) {
-  for (int off = 16; off > 0; off >>= 1) {
-    a += __shfl_xor_sync(~0u, a, off);
-    b += __shfl_xor_sync(~0u, b, off);
-    d += __shfl_xor_sync(~0u, d, off);
-    c += __shfl_xor_sync(~0u, c, off);
-  }
+                                             double& b, long long& c, int par = 0) {
+  const int lane = g.tid & 31, half = lane >> 4, k = lane & 15;
+  double x = (half ? b : a) + __shfl_xor_sync(~0u, half ? a : b, 16);
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) x += __shfl_xor_sync(~0u, x, off);
+  const long long n = warp_count(c);
   const int nw = g.nwarps();
   double* red = s.red + par * 3 * nw;   // buffer `par` of two
   long long* redl = s.redl + par * nw;
-  if ((g.tid & 31) == 0) {
-    red[g.warp()] = a;
-    red[nw + g.warp()] = b;
-    red[2 * nw + g.warp()] = d;
-    redl[g.warp()] = c;
-  }
+  if (k == 0) red[half * nw + g.warp()] = x;
+  if (lane == 0) redl[g.warp()] = n;
   g.sync();
-  a = 0.0;
-  b = 0.0;
-  d = 0.0;
-  c = 0;
-  for (int w = 0; w < nw; w++) {
-    a += red[w];
-    b += red[nw + w];
-    d += red[2 * nw + w];
-    c += redl[w];
-  }
+  x = k < nw ? red[half * nw + k] : 0.0;
+  c = (half == 0 && k < nw) ? redl[k] : 0;
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) x += __shfl_xor_sync(~0u, x, off);
+  a = __shfl_sync(~0u, x, 0);
+  b = __shfl_sync(~0u, x, 16);
+  c = warp_count(c);
 }
 
 // Writes the staged new placement of the moved molecule to the pool

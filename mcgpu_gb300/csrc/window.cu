@@ -208,14 +208,14 @@ __device__ void window_eval(const Pool& P, const ChainHdr& H, const Group& g, co
   if (tie) {
     if (w == 0) stage_chain_f64(P, H, ss, mi, lane);
     g.sync();
-    double eo = 0.0, en = 0.0, ab2 = 0.0;
+    double eo = 0.0, en = 0.0;
     long long np2 = 0;
     if (use_list)
-      warp_eval_chain64(P, H, ss, mi, pcache, 0, P.nl_cnt[mi.mol], w, nw, lane, T, eo, en,
+      warp_eval_chain64(P, H, ss, mi, pcache, 0, P.nl_cnt[mi.mol], w, nw, lane, eo, en, np2,
                         P.nl + (size_t)mi.mol * P.nl_stride);
     else
-      warp_eval_chain64(P, H, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, w, nw, lane, T, eo, en);
-    group_reduce(g, ss, eo, en, ab2, np2, nred++ & 1);
+      warp_eval_chain64(P, H, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, w, nw, lane, eo, en, np2);
+    group_reduce(g, ss, eo, en, np2, nred++ & 1);
     x.eo = eo;
     x.en = en;
   }
