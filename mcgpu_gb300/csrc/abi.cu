@@ -314,7 +314,6 @@ int upload_pool(mcgpu_ctx* ctx, HostPool& hp, DevPool& dp) {
   dp.mol_chain = dalloc<int>(nm, &e);
   dp.atom_mol = dalloc<int>(na, &e);
   dp.emol = dalloc<double>(nm, &e);
-  dp.pairs = dalloc<long long>(nm, &e);
   dp.esum = dalloc<double>(nc, &e);
   if (e != cudaSuccess) {
     dp.release();
@@ -340,6 +339,9 @@ int upload_pool(mcgpu_ctx* ctx, HostPool& hp, DevPool& dp) {
   dp.mlen.assign(hp.mlen.begin(), hp.mlen.end());
   return MCGPU_OK;
 }
+
+// Warps of a CTA of the FP32 system-energy kernel.
+static constexpr int kEnergyWarps = 4;
 
 SmemShape shape_for(int max_len, int nwarps, int cache_n) {
   SmemShape s;
@@ -443,16 +445,8 @@ int pool_nl_rebuild(mcgpu_ctx* ctx, DevPool& dp, cudaStream_t st) {
 
 // Full system energy of every chain of the pool into dp.esum (device).
 int pool_system_energy(mcgpu_ctx* ctx, DevPool& dp, bool f64, cudaStream_t st) {
-  const int nw = 4;
-  SmemShape sh = shape_for(dp.max_len, nw);
-  const int bytes = sh.bytes();
-  // split the grid to keep launches moderate
-  const int chunk = 1 << 20;
-  for (int m0 = 0; m0 < dp.n_mol; m0 += chunk) {
-    int n = std::min(chunk, dp.n_mol - m0);
-    (void)bytes;
-    CK(ctx, launch_mol_pair_sums(f64, n, nw * 32, sh, st, dp.P, dp.mol_chain, m0, dp.emol, dp.pairs));
-  }
+  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, shape_for(dp.max_len, kEnergyWarps), st, dp.P,
+                               dp.mol_chain, dp.emol));
   k_chain_sums<<<dp.n_chains, 256, 0, st>>>(dp.P, dp.emol, dp.esum);
   CK(ctx, cudaGetLastError());
   return MCGPU_OK;
@@ -546,7 +540,6 @@ struct mcgpu_box {
   bool rows_stale = false;   // FP64 rows lag the chain state (export before use)
   std::unique_ptr<IntraHost> intra;  // bond / angle rows (flexible molecules)
   bool intra_on = false;             // ENABLE_INTRA for this box
-  PlainLoop* dloop = nullptr;        // state of mcgpu_run_plain_device
   int window = 1;                    // steps per window of mcgpu_chain_run (cluster CTAs)
 };
 
@@ -645,7 +638,6 @@ extern "C" int mcgpu_box_destroy(mcgpu_box* b) {
   if (b->dout) cudaFree(b->dout);
   if (b->hout) cudaFreeHost(b->hout);
   if (b->dpairs) cudaFree(b->dpairs);
-  if (b->dloop) cudaFree(b->dloop);
   if (b->dtrace) cudaFree(b->dtrace);
   if (b->queue) cudaFree(b->queue);
   if (b->order) cudaFree(b->order);
@@ -785,13 +777,9 @@ extern "C" int mcgpu_system_energy(mcgpu_box* b, double* out) {
     // calcSystemEnergy with ENABLE_INTRA: molecule m adds E(m, j > m) and its
     // intramolecular energy (SimulationStep.cpp:40-71 over :15-18)
     DevPool& dp = b->pool;
-    const int nw = 4;
-    SmemShape sh = shape_for(dp.max_len, nw);
-    const int chunk = 1 << 20;
-    for (int m0 = 0; m0 < dp.n_mol; m0 += chunk)
-      CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64,
-                                   std::min(chunk, dp.n_mol - m0), nw * 32, sh, ctx->stream,
-                                   dp.P, dp.mol_chain, m0, dp.emol, dp.pairs));
+    CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64, dp.n_mol,
+                                 shape_for(dp.max_len, kEnergyWarps), ctx->stream, dp.P,
+                                 dp.mol_chain, dp.emol));
     CK(ctx, launch_intra_add(dp.P, b->intra->R, dp.n_mol, dp.emol, ctx->stream));
     k_chain_sums<<<dp.n_chains, 256, 0, ctx->stream>>>(dp.P, dp.emol, dp.esum);
     CK(ctx, cudaGetLastError());
@@ -900,39 +888,58 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
   if (!b0) return set_err(nullptr, MCGPU_ERR_INVALID, "null box");
   mcgpu_ctx* ctx = b0->ctx;
   if (n_steps < 0) return set_err(ctx, MCGPU_ERR_INVALID, "negative step count");
-  int max_len = 0;
+  int max_len = 0, max_mol = 0, max_groups = 0;
+  bool intra = false;
   for (int i = 0; i < n_boxes; i++) {
     mcgpu_box* b = boxes[i];
     if (!b) return set_err(ctx, MCGPU_ERR_INVALID, "null box %d", i);
     if (b->ctx != ctx) return set_err(ctx, MCGPU_ERR_INVALID, "box %d: another context", i);
     if (b->precision != b0->precision)
       return set_err(ctx, MCGPU_ERR_INVALID, "box %d: another pair precision", i);
-    for (int j = 0; j < i; j++)
-      if (boxes[j] == b) return set_err(ctx, MCGPU_ERR_INVALID, "box %d given twice", i);
     if (b->intra_on && b->intra->max_intra_moves > kLoopSel)
       return set_err(ctx, MCGPU_ERR_UNSUPPORTED, "box %d: max_intra_moves %d above %d", i,
                      b->intra->max_intra_moves, kLoopSel);
     max_len = std::max(max_len, b->pool.max_len);
+    max_mol = std::max(max_mol, b->pool.n_mol);
+    max_groups = std::max(max_groups, pair_sum_groups(b->pool.n_mol));
+    intra = intra || b->intra_on;
   }
+  {
+    std::vector<mcgpu_box*> sorted(boxes, boxes + n_boxes);
+    std::sort(sorted.begin(), sorted.end());
+    const auto twin = std::adjacent_find(sorted.begin(), sorted.end());
+    if (twin != sorted.end()) {
+      // the second place of the first box given twice, as a walk meets it
+      for (int i = 0; i < n_boxes; i++)
+        if (std::find(boxes, boxes + i, boxes[i]) != boxes + i)
+          return set_err(ctx, MCGPU_ERR_INVALID, "box %d given twice", i);
+    }
+  }
+  // the tasks, then the loop states, in one device buffer
   std::vector<LoopTask> tasks(n_boxes);
   std::vector<PlainLoop> loops(n_boxes);
+  char* dbuf = nullptr;
+  const size_t task_bytes = (sizeof(LoopTask) * (size_t)n_boxes + 255) & ~(size_t)255;
+  CK(ctx, cudaMalloc((void**)&dbuf, task_bytes + sizeof(PlainLoop) * n_boxes));
+  LoopTask* dt = (LoopTask*)dbuf;
+  PlainLoop* dl = (PlainLoop*)(dbuf + task_bytes);
   for (int i = 0; i < n_boxes; i++) {
     mcgpu_box* b = boxes[i];
-    mcgpu_plain_stats& o = out[i];
-    std::memset(&o, 0, sizeof(o));
-    double e = 0.0;
-    int rc = mcgpu_system_energy(b, &e);
-    if (rc) return rc;
-    o.energy0 = e;
-    if (!b->dloop) CK(ctx, cudaMalloc((void**)&b->dloop, sizeof(PlainLoop)));
+    std::memset(&out[i], 0, sizeof(out[i]));
+    int rc = box_rows(b);
+    if (rc) {
+      cudaFree(dbuf);
+      return rc;
+    }
     PlainLoop& L = loops[i];
     std::memset(&L, 0, sizeof(L));
     crand_seed(L.rng, seeds[i]);
-    L.energy = e;
     LoopTask& T = tasks[i];
     std::memset(&T, 0, sizeof(T));
     T.P = b->pool.P;
-    T.L = b->dloop;
+    T.L = dl + i;
+    T.emol = b->pool.emol;
+    T.n_mol = b->pool.n_mol;
     T.intra = b->intra_on ? 1 : 0;
     if (b->intra_on) {
       IntraHost& I = *b->intra;
@@ -946,21 +953,25 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
       L.angle_accepted = I.angle_accepted;
       L.max_intra_moves = I.max_intra_moves;
     }
-    CK(ctx, cudaMemcpyAsync(b->dloop, &L, sizeof(L), cudaMemcpyHostToDevice, ctx->stream));
   }
-  LoopTask* dt = nullptr;
-  CK(ctx, cudaMalloc((void**)&dt, sizeof(LoopTask) * n_boxes));
+  const bool f64 = b0->precision == MCGPU_PREC_FP64;
   cudaError_t e = cudaMemcpyAsync(dt, tasks.data(), sizeof(LoopTask) * n_boxes,
                                   cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(dl, loops.data(), sizeof(PlainLoop) * n_boxes, cudaMemcpyHostToDevice,
+                        ctx->stream);
+  if (e == cudaSuccess)
+    e = launch_box_energies(f64, dt, n_boxes, max_mol, max_groups, intra,
+                            shape_for(max_len, kEnergyWarps), ctx->stream);
   SmemShape sh = shape_for(max_len, 8);
   for (int done = 0; e == cudaSuccess && done < n_steps; done += kDeviceLoopSteps)
-    e = launch_plain_steps(b0->precision == MCGPU_PREC_FP64, dt, n_boxes,
-                           std::min(kDeviceLoopSteps, n_steps - done), sh, ctx->stream);
-  for (int i = 0; e == cudaSuccess && i < n_boxes; i++)
-    e = cudaMemcpyAsync(&loops[i], boxes[i]->dloop, sizeof(PlainLoop), cudaMemcpyDeviceToHost,
+    e = launch_plain_steps(f64, dt, n_boxes, std::min(kDeviceLoopSteps, n_steps - done), sh,
+                           ctx->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(loops.data(), dl, sizeof(PlainLoop) * n_boxes, cudaMemcpyDeviceToHost,
                         ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(dt);
+  cudaFree(dbuf);
   if (e != cudaSuccess)
     return set_err(ctx, MCGPU_ERR_CUDA, "device loop failed: %s", cudaGetErrorString(e));
   for (int i = 0; i < n_boxes; i++) {
@@ -981,6 +992,7 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
       I.angle_moves = L.angle_moves;
       I.angle_accepted = L.angle_accepted;
     }
+    out[i].energy0 = L.energy0;
     out[i].energy = L.energy;
     out[i].accepted = L.accepted;
     out[i].rejected = L.rejected;

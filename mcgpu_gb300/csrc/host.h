@@ -30,7 +30,6 @@ __global__ void k_chain_steps_wide(Pool P, int n_steps, unsigned* queue, const i
                                    int n_tasks, int gwarps, SmemShape shape, mcgpu_trace* trace,
                                    int trace_off, int trace_stride, int lanes_cap);
 __global__ void k_chain_init(Pool P, const int* mol_chain, int m_begin, int m_end);
-__global__ void k_chain_energy1(Pool P, int c, const double* emol);
 __global__ void k_nl_config(Pool P, const NlCfg* cfg);
 cudaError_t launch_nl_rebuild(Pool P, const int* mol_chain, int n_mol, int max_cells,
                               cudaStream_t st);
@@ -42,9 +41,9 @@ cudaError_t launch_mol_energy(bool f64, int grid, int threads, SmemShape sh, cud
 cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
                                  Pool P, int chain, int mol, Proposal prop, double* partials,
                                  unsigned* counter, double* out, long long* pairs = nullptr);
-cudaError_t launch_mol_pair_sums(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
-                                 Pool P, const int* mol_chain, int m_begin, double* emol,
-                                 long long* pairs);
+// emol[m] with the sum over the chains' molecules of E(m, j > m).
+cudaError_t launch_mol_pair_sums(bool f64, int n_mol, SmemShape sh, cudaStream_t st,
+                                 const Pool& P, const int* mol_chain, double* emol);
 // One volume phase of the chains in act (all when act has no ranges) on
 // stream st: proposals, cell grids, FP32 / FP64 totals, decisions, the
 // double-float and FP64 re-takes; vlist holds 3 * (chains) + 3 ints.
@@ -160,7 +159,6 @@ struct DevPool {
   int* mol_chain = nullptr;
   int* atom_mol = nullptr;
   double* emol = nullptr;
-  long long* pairs = nullptr;
   double* esum = nullptr;
   std::vector<ChainHdr> hdr;  // host copy of the headers at upload
   std::vector<int> mstart, mlen;  // host copies (pool-absolute)
@@ -173,14 +171,13 @@ struct DevPool {
                     P.mfix, P.mrad, P.mq, P.atpl, P.pidx, P.ppos, P.hdr, P.rb, P.trace,
                     P.nl, P.nl_cnt, P.pbuild, P.mcell, P.cell_cnt, P.cell_start, P.cell_mol,
                     P.vc_cnt, P.vc_start, P.vc_mol, P.vc_of,
-                    mol_chain, atom_mol, emol, pairs, esum};
+                    mol_chain, atom_mol, emol, esum};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     P = Pool{};
     mol_chain = nullptr;
     atom_mol = nullptr;
     emol = nullptr;
-    pairs = nullptr;
     esum = nullptr;
   }
 };

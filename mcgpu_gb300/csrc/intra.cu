@@ -145,12 +145,23 @@ __global__ void __launch_bounds__(kIntraThreads) k_intra_energy(Pool P, IntraRow
   if (threadIdx.x == 0) out[0] = e;
 }
 
-__global__ void __launch_bounds__(kIntraThreads) k_intra_add(Pool P, IntraRows R, double* emol) {
-  __shared__ double red[3 * (kIntraThreads / 32)];
+// One warp per molecule: a molecule's pairs are a few rounds of 32, and the
+// block sum costs FP64 instructions in every warp.
+__global__ void __launch_bounds__(32) k_intra_add(Pool P, IntraRows R, double* emol) {
+  __shared__ double red[3];
   const ChainHdr& H = P.hdr[0];
   const int mol = blockIdx.x;
   const double e = intra_energy(P, R, H, mol, red);
   if (threadIdx.x == 0) emol[H.mol0 + mol] += e;
+}
+
+__global__ void __launch_bounds__(32) k_intra_add_boxes(const LoopTask* tasks) {
+  __shared__ double red[3];
+  const LoopTask& T = tasks[blockIdx.y];
+  const int mol = blockIdx.x;
+  if (!T.intra || mol >= T.n_mol) return;
+  const double e = intra_energy(T.P, T.R, T.P.hdr[0], mol, red);
+  if (threadIdx.x == 0) T.emol[mol] += e;
 }
 
 // One SimCalcs::stretchBond (kind 0, SimulationStep.cpp:257-315) or
@@ -768,7 +779,13 @@ cudaError_t launch_plain_steps(bool f64, const LoopTask* tasks, int n_tasks, int
 cudaError_t launch_intra_add(const Pool& P, const IntraRows& R, int n_mol, double* emol,
                              cudaStream_t st) {
   if (n_mol <= 0) return cudaSuccess;
-  k_intra_add<<<n_mol, kIntraThreads, 0, st>>>(P, R, emol);
+  k_intra_add<<<n_mol, 32, 0, st>>>(P, R, emol);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_intra_add_boxes(const LoopTask* tasks, int n_tasks, int max_mol,
+                                   cudaStream_t st) {
+  k_intra_add_boxes<<<dim3(max_mol, n_tasks), 32, 0, st>>>(tasks);
   return cudaGetLastError();
 }
 

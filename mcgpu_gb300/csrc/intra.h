@@ -98,7 +98,7 @@ constexpr int kLoopSel = 64;
 // kLoopDrawCap draws (the loop stops).
 struct PlainLoop {
   CRand rng;
-  double energy;
+  double energy, energy0;   // running and at the start
   long long accepted, rejected, pairs;
   long long step;
   double max_bond_delta, max_angle_delta;
@@ -107,13 +107,25 @@ struct PlainLoop {
 };
 
 // One box of a device loop launch: its pool (chain 0), bond / angle rows
-// (when intra != 0) and loop state.
+// (when intra != 0), loop state and scratch of its system energy (n_mol).
 struct LoopTask {
   Pool P;
   IntraRows R;
   PlainLoop* L;
-  int intra, pad;
+  double* emol;
+  int intra, n_mol;
 };
+
+// The system energies of n_tasks boxes (max_mol molecules and max_groups
+// groups of the FP64 kernel the largest) into their loop states; intra: some
+// box has intramolecular moves on.
+cudaError_t launch_box_energies(bool f64, const LoopTask* tasks, int n_tasks, int max_mol,
+                                int max_groups, bool intra, SmemShape sh, cudaStream_t st);
+// CTAs of the FP64 system-energy kernel for a box of n_mol molecules.
+int pair_sum_groups(int n_mol);
+// emol[m] += calcIntraMolecularEnergy(m) for the boxes with intra != 0.
+cudaError_t launch_intra_add_boxes(const LoopTask* tasks, int n_tasks, int max_mol,
+                                   cudaStream_t st);
 
 // n_steps of Simulation::run's loop for each of n_tasks boxes, one CTA per
 // box, the draws from each L->rng; intra != 0: with the intramolecular term

@@ -6,12 +6,16 @@
 //   k_move_energies<F64>   old energy + move + new energy in one launch
 //   k_change_molecule      the move alone (saves the rollback copy)
 //   k_rollback             restores the rollback copy
-//   k_mol_pair_sums<F64>   E(m, j>m) per molecule of every chain
+//   k_pair_sums64          E(m, j>m) of groups of molecules, FP64 pairs
+//   k_pair_sums32          E(m, j>m) per molecule, FP32 pairs
 //   k_chain_sums           per-chain ordered sum of the above
+//   k_box_energies         the same for many boxes, into their loop states
 //   k_chain_steps          persistent Metropolis steps of many chains:
 //                          Philox proposal, staging, screen, pairs, FP64
 //                          dE, decision and commit without leaving the GPU
 #include "chain.cuh"
+#include "intra.h"
+#include "pairsum.cuh"
 
 namespace mcgpu {
 
@@ -168,15 +172,145 @@ __global__ void k_rollback(Pool P, int chain, int mol) {
   refresh_molecule(P, H, m, lane, 32);
 }
 
-// E(m, j > m) for pool molecule m = blockIdx.x + m_begin: one term of
-// SimulationStep::calcSystemEnergy (SimulationStep.cpp:47-48).
-template <bool F64>
-__global__ void __launch_bounds__(256) k_mol_pair_sums(Pool P, const int* mol_chain, int m_begin,
-                                                       SmemShape shape, double* emol,
-                                                       long long* pairs) {
+// The pool of a launch: P0, or with tasks that of box blockIdx.y, copied to
+// shared memory by the whole block.
+__device__ __forceinline__ void load_pool(Pool& SP, const Pool& P0, const LoopTask* tasks) {
+  static_assert(sizeof(Pool) % 4 == 0, "Pool words");
+  if (tasks) {
+    const int* src = (const int*)&tasks[blockIdx.y].P;
+    for (int i = threadIdx.x; i < (int)(sizeof(Pool) / 4); i += blockDim.x) ((int*)&SP)[i] = src[i];
+  } else if (threadIdx.x == 0) {
+    SP = P0;
+  }
+  __syncthreads();
+}
+
+// The pool's rows as ps_items reads them.
+struct PoolRows {
+  const Pool& P;
+  __device__ __forceinline__ int len(int j) const { return P.mlen[j] & 255; }
+  __device__ __forceinline__ int start(int j) const { return P.mstart[j]; }
+  __device__ __forceinline__ void atom(int b, double& x, double& y, double& z, double& sb,
+                                       double& eb, double& qb) const {
+    x = P.x[b];
+    y = P.y[b];
+    z = P.z[b];
+    const double2 bl = P.blend ? P.blend[b] : blend64(P.sig[b], P.eps[b]);
+    sb = bl.x;
+    eb = bl.y;
+    qb = P.q[b];
+  }
+};
+
+// E(m, j > m) of SimulationStep::calcSystemEnergy (SimulationStep.cpp:47-48)
+// with FP64 pairs, ps_group consecutive molecules per CTA (a group that spans
+// chains is taken chain by chain): emol[first molecule] holds the sum over
+// the group's molecules of the chain, the others 0.  The in-range set is the
+// FP64 test's (the FP32 screen decides outside its guard band).  32,768
+// waters (rc 12 A, 35.6 M pairs): 5.84 ms with a CTA per molecule, which
+// screened at one candidate load per test, see pairsum.cuh.
+__global__ void __launch_bounds__(kPsThreads, 4)
+    k_pair_sums64(Pool P0, const LoopTask* tasks, const int* mol_chain, int m_begin, int m_end,
+                  double* emol) {
+  __shared__ Pool SP;
+  __shared__ PsGroup G;
+  __shared__ float4 pp[kPsGroup][kMaxP];
+  __shared__ int pslot[kPsGroup][kMaxP], pnum[kPsGroup];
+  load_pool(SP, P0, tasks);
+  const Pool& P = SP;
+  if (tasks) {
+    m_end = tasks[blockIdx.y].n_mol;
+    emol = tasks[blockIdx.y].emol;
+  }
+  const int group = ps_group(m_end - m_begin);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = lanemask_lt();
+  int m0 = m_begin + (int)blockIdx.x * group;
+  const int mg = min(m0 + group, m_end);
+  while (m0 < mg) {
+    const int c = tasks ? 0 : mol_chain[m0];
+    const ChainHdr& H = P.hdr[c];
+    const int m1 = min(mg, H.mol0 + H.n_mol), n = m1 - m0;
+    for (int g = 0; g < n; g++) {
+      const int m = m0 + g, a0 = P.mstart[m], len = P.mlen[m] & 255;
+      const int2 pi = P.mpi[m];
+      for (int i = threadIdx.x; i < len; i += kPsThreads) {
+        const int o = g * kPsPitch + i;
+        PoolRows{P}.atom(a0 + i, G.x[o], G.y[o], G.z[o], G.sd[o], G.ed[o], G.qd[o]);
+      }
+      for (int k = threadIdx.x; k < pi.y; k += kPsThreads) {
+        pp[g][k] = P.ppos[pi.x + k];
+        pslot[g][k] = g * kPsPitch + P.pidx[pi.x + k] - a0;
+      }
+      if (threadIdx.x == 0) {
+        G.len[g] = len;
+        pnum[g] = pi.y;
+      }
+    }
+    __syncthreads();
+    int* rj = G.ring[w];
+    int head = 0, tail = 0;
+    double acc = 0.0;
+    const int end = H.mol0 + H.n_mol;
+    const bool simple = H.simple_prim != 0;
+    for (int base = m0 + 1 + w * 32; base < end; base += kPsThreads) {
+      const int j = base + lane;
+      int2 pj = make_int2(0, 0);
+      float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j < end) {
+        pj = simple ? make_int2(H.pidx0 + (j - H.mol0), 1) : P.mpi[j];
+        q0 = P.ppos[pj.x];
+      }
+      for (int g = 0; g < n; g++) {
+        bool in = false;
+        if (j > m0 + g)
+          for (int k2 = 0; k2 < pj.y && !in; k2++) {
+            const float4 q = k2 == 0 ? q0 : P.ppos[pj.x + k2];
+            for (int k1 = 0; k1 < pnum[g] && !in; k1++) {
+              const float r2 = r2_screen(pp[g][k1], q, H);
+              if (r2 <= H.cut2_lo) {
+                in = true;
+              } else if (r2 <= H.cut2_hi) {
+                const int o = pslot[g][k1];
+                in = in_range64(G.x[o], G.y[o], G.z[o], P.pidx[pj.x + k2], P, H);
+              }
+            }
+          }
+        const unsigned bal = __ballot_sync(~0u, in);
+        if (in) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 3) | g;
+        tail += __popc(bal);
+        if (tail - head >= 32) {
+          __syncwarp();
+          acc += ps_items<true>(G, PoolRows{P}, rj, head, 32, lane, H.L[0], H.L[1], H.L[2]);
+          head += 32;
+          __syncwarp();
+        }
+      }
+    }
+    __syncwarp();
+    if (tail > head)
+      acc += ps_items<true>(G, PoolRows{P}, rj, head, tail - head, lane, H.L[0], H.L[1], H.L[2]);
+    const double sum = ps_block_sum(G, acc);
+    if ((int)threadIdx.x < n) emol[m0 + threadIdx.x] = threadIdx.x == 0 ? sum : 0.0;
+    m0 = m1;
+    __syncthreads();   // the next chain's molecules overwrite the stage
+  }
+}
+
+// The same with FP32 pairs, one molecule m = m_begin + blockIdx.x per CTA.
+__global__ void __launch_bounds__(256) k_pair_sums32(Pool P0, const LoopTask* tasks,
+                                                     const int* mol_chain, int m_begin,
+                                                     SmemShape shape, double* emol) {
   extern __shared__ __align__(16) char smem[];
+  __shared__ Pool SP;
+  load_pool(SP, P0, tasks);
+  const Pool& P = SP;
   const int m = m_begin + blockIdx.x;
-  const ChainHdr& H = P.hdr[mol_chain[m]];
+  if (tasks) {
+    if (m >= tasks[blockIdx.y].n_mol) return;
+    emol = tasks[blockIdx.y].emol;
+  }
+  const ChainHdr& H = P.hdr[tasks ? 0 : mol_chain[m]];
   Group g{(int)threadIdx.x, (int)blockDim.x, 1};
   GroupSmem s = shape.carve(smem);
   const int lane = threadIdx.x & 31, w = g.warp(), nw = g.nwarps();
@@ -185,50 +319,49 @@ __global__ void __launch_bounds__(256) k_mol_pair_sums(Pool P, const int* mol_ch
   const MovedInfo mi = load_moved(s);
   double eo = 0.0, en = 0.0;
   long long np = 0;
-  warp_eval<F64>(P, H, s, mi, m + 1, H.mol0 + H.n_mol, w, nw, lane, H.tpm, eo, en, np);
+  warp_eval<false>(P, H, s, mi, m + 1, H.mol0 + H.n_mol, w, nw, lane, H.tpm, eo, en, np);
   group_reduce(g, s, eo, en, np);
-  if (threadIdx.x == 0) {
-    emol[m] = eo;
-    if (pairs) pairs[m] = np;
-  }
+  if (threadIdx.x == 0) emol[m] = eo;
 }
 
-// Ordered per-chain sum of emol: thread t adds every blockDim-th term from
-// t, then a fixed tree; one CTA per chain.
-__global__ void k_chain_sums(Pool P, const double* emol, double* out) {
-  __shared__ double red[256];
-  const ChainHdr& H = P.hdr[blockIdx.x];
+// Ordered sum of n terms: thread t adds every blockDim-th term from t, then
+// a fixed tree; the total in thread 0 (one CTA of at most 256 threads).
+__device__ __forceinline__ double ordered_sum(const double* v, int n, double* red) {
   double acc = 0.0;
-  for (int i = threadIdx.x; i < H.n_mol; i += blockDim.x) acc += emol[H.mol0 + i];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += v[i];
   red[threadIdx.x] = acc;
   __syncthreads();
   for (int off = blockDim.x >> 1; off > 0; off >>= 1) {
     if ((int)threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+  return red[0];
+}
+
+// Ordered per-chain sum of emol; one CTA per chain.
+__global__ void k_chain_sums(Pool P, const double* emol, double* out) {
+  __shared__ double red[256];
+  const ChainHdr& H = P.hdr[blockIdx.x];
+  const double e = ordered_sum(emol + H.mol0, H.n_mol, red);
+  if (threadIdx.x == 0) out[blockIdx.x] = e;
+}
+
+// The boxes' system energies from their emol rows, as the start of their
+// loops; one CTA per box.
+__global__ void k_box_energies(const LoopTask* tasks) {
+  __shared__ double red[256];
+  const LoopTask& T = tasks[blockIdx.x];
+  const double e = ordered_sum(T.emol, T.n_mol, red);
+  if (threadIdx.x == 0) {
+    T.L->energy = e;
+    T.L->energy0 = e;
+  }
 }
 
 // Sets every chain's running energy from out[] (the start of a run).
 __global__ void k_set_energy(Pool P, const double* e) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < P.n_chains) P.hdr[c].energy = e[c];
-}
-
-// Running energy of chain c from its emol terms: the ordered sum of
-// k_chain_sums for one chain (a served job entering the pool).
-__global__ void k_chain_energy1(Pool P, int c, const double* emol) {
-  __shared__ double red[256];
-  ChainHdr& H = P.hdr[c];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < H.n_mol; i += blockDim.x) acc += emol[H.mol0 + i];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int off = blockDim.x >> 1; off > 0; off >>= 1) {
-    if ((int)threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) H.energy = red[0];
 }
 
 // ---- device-resident Metropolis -------------------------------------------
@@ -543,15 +676,40 @@ cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_mol_pair_sums(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
-                                 Pool P, const int* mol_chain, int m_begin, double* emol,
-                                 long long* pairs) {
-  if (f64)
-    k_mol_pair_sums<true><<<grid, threads, sh.bytes(), st>>>(P, mol_chain, m_begin, sh, emol, pairs);
-  else
-    k_mol_pair_sums<false><<<grid, threads, sh.bytes(), st>>>(P, mol_chain, m_begin, sh, emol,
-                                                              pairs);
+int pair_sum_groups(int n_mol) { return (n_mol + ps_group(n_mol) - 1) / ps_group(n_mol); }
+
+cudaError_t launch_mol_pair_sums(bool f64, int n_mol, SmemShape sh, cudaStream_t st,
+                                 const Pool& P, const int* mol_chain, double* emol) {
+  if (f64) {
+    k_pair_sums64<<<pair_sum_groups(n_mol), kPsThreads, 0, st>>>(P, nullptr, mol_chain, 0, n_mol,
+                                                             emol);
+  } else {
+    k_pair_sums32<<<n_mol, sh.nwarps * 32, sh.bytes(), st>>>(P, nullptr, mol_chain, 0, sh, emol);
+  }
   return cudaGetLastError();
+}
+
+cudaError_t launch_box_energies(bool f64, const LoopTask* tasks, int n_tasks, int max_mol,
+                                int max_groups, bool intra, SmemShape sh, cudaStream_t st) {
+  // grid.y holds at most 65,535 boxes
+  for (int t0 = 0; t0 < n_tasks; t0 += 65535) {
+    const int nt = n_tasks - t0 < 65535 ? n_tasks - t0 : 65535;
+    const LoopTask* T = tasks + t0;
+    if (f64) {
+      k_pair_sums64<<<dim3(max_groups, nt), kPsThreads, 0, st>>>(Pool{}, T, nullptr, 0, 0,
+                                                                 nullptr);
+    } else {
+      k_pair_sums32<<<dim3(max_mol, nt), sh.nwarps * 32, sh.bytes(), st>>>(Pool{}, T, nullptr, 0,
+                                                                           sh, nullptr);
+    }
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && intra) e = launch_intra_add_boxes(T, nt, max_mol, st);
+    if (e != cudaSuccess) return e;
+    k_box_energies<<<nt, 256, 0, st>>>(T);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace mcgpu

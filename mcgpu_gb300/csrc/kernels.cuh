@@ -550,24 +550,25 @@ __device__ __forceinline__ int hi_abs(double v) { return __double2hiint(v) & 0x7
 __device__ __forceinline__ double image64(double d, double L, int half) {
   const int h = hi_abs(d);
   if (h < half) return d;
-  if (h > half) return __dadd_rn(d, copysign(L, -d));
+  if (h > half && half >= 0) return __dadd_rn(d, copysign(L, -d));
   return make_periodic(d, L);
 }
 
-// Sum over the moved molecule's atoms (rows xs, ys, zs) of the FP64 pair
-// terms with neighbour atom b: the reference's minimum image of every pair
-// and its rule for skipped sites (BruteForceStep.cpp:61-76).  b is shifted
-// once to its image nearest the moved molecule's first atom; a pair that
-// still lies beyond half an edge (molecules straddling it, or rows outside
-// the box) takes the reference's own image from the unshifted rows.
-// (sb, eb): b's blending factors, qb its charge; the moved atoms' factors
-// are staged in s.sd / s.ed.
-__device__ __forceinline__ double sum_moved64(const GroupSmem& s, const double* xs,
-                                              const double* ys, const double* zs, int len,
-                                              double xb, double yb, double zb, double sb,
-                                              double eb, double qb, const ChainHdr& H) {
+// Sum over the atoms of one molecule (rows xs, ys, zs) of the FP64 pair terms
+// with atom b of another: the reference's minimum image of every pair and its
+// rule for skipped sites (BruteForceStep.cpp:61-76).  b is shifted once to
+// its image nearest the molecule's first atom; a pair that still lies beyond
+// half an edge (molecules straddling it, or rows outside the box) takes the
+// reference's own image from the unshifted rows.
+// (sb, eb): b's factors, qb its charge; sd, ed, qd the molecule's: sqrt(eps)
+// and, with ROOT, sqrt(sigma), else sigma itself (sigma_ab^2 = s_a s_b).
+template <bool ROOT>
+__device__ __forceinline__ double pair_sum64(const double* xs, const double* ys, const double* zs,
+                                             const double* sd, const double* ed, const double* qd,
+                                             int len, double xb, double yb, double zb, double sb,
+                                             double eb, double qb, double Lx, double Ly,
+                                             double Lz) {
   if (blend_skipped(sb)) return 0.0;
-  const double Lx = H.L[0], Ly = H.L[1], Lz = H.L[2];
   const int hx = __double2hiint(0.5 * Lx), hy = __double2hiint(0.5 * Ly),
             hz = __double2hiint(0.5 * Lz);
   const double tx = xb - xs[0], ty = yb - ys[0], tz = zb - zs[0];
@@ -579,7 +580,7 @@ __device__ __forceinline__ double sum_moved64(const GroupSmem& s, const double* 
   double acc = 0.0;
 #pragma unroll 3
   for (int i = 0; i < len; i++) {
-    const double sa = s.sd[i], ea = s.ed[i];
+    const double sa = sd[i], ea = ed[i];
     if (blend_skipped(sa)) continue;
     double dx = bx - xs[i], dy = by - ys[i], dz = bz - zs[i];
     if (hi_abs(dx) >= hx || hi_abs(dy) >= hy || hi_abs(dz) >= hz) {
@@ -590,10 +591,16 @@ __device__ __forceinline__ double sum_moved64(const GroupSmem& s, const double* 
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
     if (!bits_nonzero(r2)) continue;   // coincident: skipped (BruteForceStep.cpp:68-69)
     const double ri = rsqrt(r2);
-    acc = fma(s.qd[i] * qk, ri, acc);
+    acc = fma(qd[i] * qk, ri, acc);
     if (lj_b && bits_nonzero(sa) && bits_nonzero(ea)) {
-      const double t = (sa * sb) * ri;
-      const double t2 = t * t, s6 = t2 * t2 * t2;
+      double t2;
+      if (ROOT) {
+        const double t = (sa * sb) * ri;
+        t2 = t * t;
+      } else {
+        t2 = (sa * sb) * (ri * ri);
+      }
+      const double s6 = t2 * t2 * t2;
       const double e = ea * e4;
       acc = fma(s6, fma(e, s6, -e), acc);
     }
@@ -668,9 +675,9 @@ __device__ __forceinline__ void batch_items64(const Pool& P, const ChainHdr& H,
     double xb, yb, zb;
     atom(j, b, xb, yb, zb);
     const double2 bl = P.blend ? P.blend[b] : blend64(P.sig[b], P.eps[b]);
-    const double v = sum_moved64(s, use_new ? s.nx : s.ox, use_new ? s.ny : s.oy,
-                                 use_new ? s.nz : s.oz, mi.len, xb, yb, zb, bl.x, bl.y, P.q[b],
-                                 H);
+    const double v = pair_sum64<true>(use_new ? s.nx : s.ox, use_new ? s.ny : s.oy,
+                                      use_new ? s.nz : s.oz, s.sd, s.ed, s.qd, mi.len, xb, yb,
+                                      zb, bl.x, bl.y, P.q[b], H.L[0], H.L[1], H.L[2]);
     if (use_new) en += v; else eo += v;
   }
 }

@@ -153,7 +153,6 @@ int server_alloc(mcgpu_server* s) {
   dp.mol_chain = dalloc<int>(nm, &e);
   dp.atom_mol = dalloc<int>(na, &e);
   dp.emol = dalloc<double>(nm, &e);
-  dp.pairs = dalloc<long long>(nm, &e);
   dp.esum = dalloc<double>(nc, &e);
   dp.n_chains = nc;
   dp.n_atom = (int)na;

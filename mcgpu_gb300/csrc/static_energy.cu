@@ -9,8 +9,7 @@
 // application whose device memory is owned by another allocator (a
 // framework's caching allocator, a fixed arena of a long-running service)
 // and forbids allocations from third-party code.  They pass device pointers
-// to their rows and to one output double; the per-molecule partial energies
-// live in a fixed file-scope device array instead of a cudaMalloc'd buffer.
+// to their rows and to one output double; the partial energies live in a fixed file-scope device array instead of a cudaMalloc'd buffer.
 //
 // Limits and sharing: at most kStaticMaxMol molecules per call (larger boxes
 // are rejected with MCGPU_ERR_UNSUPPORTED).  Every GPU that loads the
@@ -30,7 +29,7 @@
 #include <cstdio>
 #include <mutex>
 
-#include "../../include/mcgpu_gb300.h"
+#include "pairsum.cuh"
 #include "static_scratch_cache.h"
 
 namespace mcgpu {
@@ -42,8 +41,9 @@ constexpr int kStaticMaxMol = 32768;
 constexpr int kMaxDevices = 64;
 }  // namespace
 
-// The scratch: E(m, j > m) for every molecule m of the box, one copy per
-// device, never cleared (every entry a call reads, it wrote first).
+// The scratch: one partial sum of E(m, j > m) per CTA (at most one per
+// molecule of the box), one copy per device, never cleared (every entry a
+// call reads, it wrote first).
 static __device__ __align__(256) double g_static_emol[kStaticMaxMol];
 
 namespace {
@@ -55,18 +55,11 @@ struct Rows {
   double L[3], cutoff;
 };
 
-// SimCalcs::makePeriodic (SimulationStep.cpp:377-385).
-__device__ __forceinline__ double periodic(double x, double L) {
-  if (x < -0.5 * L) x = __dadd_rn(x, L);
-  if (x > 0.5 * L) x = __dadd_rn(x, -L);
-  return x;
-}
-
 // SimCalcs::calcAtomDistSquared (SimulationStep.cpp:332-342), a2 - a1.
 __device__ __forceinline__ double dist2(const Rows& r, int a1, int a2) {
-  const double dx = periodic(r.x[a2] - r.x[a1], r.L[0]);
-  const double dy = periodic(r.y[a2] - r.y[a1], r.L[1]);
-  const double dz = periodic(r.z[a2] - r.z[a1], r.L[2]);
+  const double dx = mcgpu::make_periodic(r.x[a2] - r.x[a1], r.L[0]);
+  const double dy = mcgpu::make_periodic(r.y[a2] - r.y[a1], r.L[1]);
+  const double dz = mcgpu::make_periodic(r.z[a2] - r.z[a1], r.L[2]);
   return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
 
@@ -78,60 +71,152 @@ __device__ __forceinline__ bool valid_mol(const Rows& r, int m) {
   return s >= 0 && n >= 1 && s + n <= r.n_atom && ps >= 0 && pc >= 0 && ps + pc <= r.n_pidx;
 }
 
-// E(m, j > m) per CTA m: threads stride over candidates j; the reference's
-// primary-pair cutoff (SimulationStep.cpp:317-330) and FP64 pair terms
-// (BruteForceStep.cpp:48-79, SimulationStep.cpp:344-375).  A molecule with
-// out-of-range rows makes the partial NaN instead of reading past them.
-__global__ void k_static_pair_sums(Rows r, double* emol) {
-  const int m = blockIdx.x;
-  __shared__ double red[256];
-  double acc = 0.0;
-  bool bad = !valid_mol(r, m);
-  if (!bad) {
-    const int s1 = r.mstart[m], e1 = s1 + r.mlen[m];
-    const int p1s = r.mps[m], p1e = p1s + r.mpc[m];
-    for (int j = m + 1 + (int)threadIdx.x; j < r.n_mol; j += blockDim.x) {
-      if (!valid_mol(r, j)) {
-        bad = true;
-        continue;
-      }
-      bool in = false;
-      for (int p1 = p1s; p1 < p1e && !in; p1++)
-        for (int p2 = r.mps[j]; p2 < r.mps[j] + r.mpc[j] && !in; p2++) {
-          const int a1 = r.pidx[p1], a2 = r.pidx[p2];
-          if (a1 < 0 || a1 >= r.n_atom || a2 < 0 || a2 >= r.n_atom) {
-            bad = true;
-            break;
-          }
-          in = dist2(r, a1, a2) <= __dmul_rn(r.cutoff, r.cutoff);
-        }
-      if (!in) continue;
-      const int s2 = r.mstart[j], e2 = s2 + r.mlen[j];
-      double e = 0.0;
-      for (int i = s1; i < e1; i++)
-        for (int k = s2; k < e2; k++) {
-          const double si = r.sig[i], sk = r.sig[k], ei = r.eps[i], ek = r.eps[k];
-          if (!(si >= 0 && sk >= 0 && ei >= 0 && ek >= 0)) continue;
-          const double r2 = dist2(r, i, k);
-          if (r2 == 0.0) continue;
-          const double ss = si * sk, ee = ei * ek;
-          const double sigma = sqrt(ss >= 0 ? ss : -ss);
-          const double eps = sqrt(ee >= 0 ? ee : -ee);
-          const double s2r2 = (sigma * sigma) / r2;
-          const double s6 = s2r2 * s2r2 * s2r2;
-          e += 4.0 * eps * (s6 * s6 - s6);
-          e += (r.q[i] * r.q[k] * 332.06) / sqrt(r2);
-        }
-      acc += e;
+// The caller's rows as ps_items reads them: sigma as it is, sqrt(eps), -1 for
+// a skipped site (a negative sigma or epsilon, BruteForceStep.cpp:64-65).
+struct StaticRows {
+  const Rows& r;
+  __device__ __forceinline__ int len(int j) const { return r.mlen[j]; }
+  __device__ __forceinline__ int start(int j) const { return r.mstart[j]; }
+  __device__ __forceinline__ void atom(int b, double& x, double& y, double& z, double& sb,
+                                       double& eb, double& qb) const {
+    x = r.x[b];
+    y = r.y[b];
+    z = r.z[b];
+    const double sg = r.sig[b], ep = r.eps[b];
+    const bool real = sg >= 0 && ep >= 0;
+    sb = real ? sg : -1.0;
+    eb = real && mcgpu::bits_nonzero(ep) ? sqrt(ep) : 0.0;
+    qb = r.q[b];
+  }
+};
+
+// FP32 primary screen of the rows: distances decided outright below lo and
+// above hi (squared), by the FP64 test between; rows farther than `far` from
+// the origin along an axis always by the FP64 test.
+struct StaticScreen {
+  float L[3], lo, hi, far;
+};
+
+// Minimum-image distance squared as makePeriodic's single shift gives it.
+__device__ __forceinline__ float screen2(float3 a, float3 b, const float* L) {
+  float d[3] = {fabsf(b.x - a.x), fabsf(b.y - a.y), fabsf(b.z - a.z)};
+#pragma unroll
+  for (int k = 0; k < 3; k++) d[k] = d[k] > 0.5f * L[k] ? fabsf(d[k] - L[k]) : d[k];
+  return fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
+}
+
+// E(m, j > m) of the molecules [blockIdx.x * group, ...) of a CTA into
+// emol[blockIdx.x]: the reference's primary-pair cutoff
+// (SimulationStep.cpp:317-330; FP32 outside the guard band) and FP64 pair
+// terms (BruteForceStep.cpp:48-79, SimulationStep.cpp:344-375), as pairsum.cuh
+// describes; molecules of more than kMaxA atoms pass by in chunks of their
+// atoms.  A molecule with out-of-range rows makes the partial NaN instead of
+// reading past them.  1,999 molecules of 16 atoms (rc 12 A, 11.5 M pairs):
+// 11.9 ms when each thread took a whole in-range candidate, its square root
+// and division per pair included.
+__global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
+    k_static_pair_sums(Rows r, StaticScreen sc, int group, double* emol) {
+  using namespace mcgpu;
+  __shared__ PsGroup G;
+  __shared__ int ms[kPsGroup], ml[kPsGroup], p0[kPsGroup], pc[kPsGroup], pa[kPsGroup];
+  __shared__ float3 pf[kPsGroup];
+  __shared__ int near[kPsGroup];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = lanemask_lt();
+  const int m0 = (int)blockIdx.x * group, n = min(group, r.n_mol - m0);
+  bool bad = false;
+  if ((int)threadIdx.x < n) {
+    const int g = threadIdx.x, m = m0 + g;
+    const bool ok = valid_mol(r, m);
+    bad = !ok;
+    ms[g] = ok ? r.mstart[m] : 0;
+    ml[g] = ok ? r.mlen[m] : 0;
+    p0[g] = ok ? r.mps[m] : 0;
+    pc[g] = ok ? r.mpc[m] : 0;
+    const int a = pc[g] > 0 ? r.pidx[p0[g]] : -1;
+    pa[g] = a;
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    bool nr = false;
+    if (a >= 0 && a < r.n_atom) {
+      f = make_float3((float)r.x[a], (float)r.y[a], (float)r.z[a]);
+      nr = fabsf(f.x) <= sc.far && fabsf(f.y) <= sc.far && fabsf(f.z) <= sc.far;
     }
+    pf[g] = f;
+    near[g] = nr;
   }
-  red[threadIdx.x] = bad ? __longlong_as_double(0x7ff8000000000000LL) : acc;
   __syncthreads();
-  for (int off = blockDim.x >> 1; off > 0; off >>= 1) {
-    if ((int)threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
+  int longest = 0;
+  for (int g = 0; g < n; g++) longest = max(longest, ml[g]);
+  const double rc2 = __dmul_rn(r.cutoff, r.cutoff);
+  int* rj = G.ring[w];
+  double acc = 0.0;
+  for (int c0 = 0; c0 < longest; c0 += kMaxA) {
+    for (int g = 0; g < n; g++) {
+      const int len = max(0, min(kMaxA, ml[g] - c0));
+      for (int i = threadIdx.x; i < len; i += kPsThreads) {
+        const int o = g * kPsPitch + i;
+        StaticRows{r}.atom(ms[g] + c0 + i, G.x[o], G.y[o], G.z[o], G.sd[o], G.ed[o], G.qd[o]);
+      }
+      if (threadIdx.x == 0) G.len[g] = len;
+    }
     __syncthreads();
+    int head = 0, tail = 0;
+    for (int base = m0 + 1 + w * 32; base < r.n_mol; base += kPsThreads) {
+      const int j = base + lane;
+      int q0 = 0, qc = 0, qa = -1;
+      float3 f = make_float3(0.f, 0.f, 0.f);
+      bool nr = false;
+      if (j < r.n_mol) {
+        if (valid_mol(r, j)) {
+          q0 = r.mps[j];
+          qc = r.mpc[j];
+          qa = qc > 0 ? r.pidx[q0] : -1;
+          if (qa >= 0 && qa < r.n_atom) {
+            f = make_float3((float)r.x[qa], (float)r.y[qa], (float)r.z[qa]);
+            nr = fabsf(f.x) <= sc.far && fabsf(f.y) <= sc.far && fabsf(f.z) <= sc.far;
+          }
+        } else {
+          bad = true;
+        }
+      }
+      for (int g = 0; g < n; g++) {
+        bool in = false;
+        if (j > m0 + g && G.len[g] > 0)
+          for (int k1 = 0; k1 < pc[g] && !in; k1++)
+            for (int k2 = 0; k2 < qc && !in; k2++) {
+              const int a1 = k1 == 0 ? pa[g] : r.pidx[p0[g] + k1];
+              const int a2 = k2 == 0 ? qa : r.pidx[q0 + k2];
+              if (a1 < 0 || a1 >= r.n_atom || a2 < 0 || a2 >= r.n_atom) {
+                bad = true;
+                break;
+              }
+              bool exact = true;
+              if (k1 == 0 && k2 == 0 && nr && near[g]) {
+                const float r2 = screen2(pf[g], f, sc.L);
+                in = r2 <= sc.lo;
+                exact = !in && r2 <= sc.hi;
+              }
+              if (exact) in = dist2(r, a1, a2) <= rc2;
+            }
+        const unsigned bal = __ballot_sync(~0u, in);
+        if (in) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 3) | g;
+        tail += __popc(bal);
+        if (tail - head >= 32) {
+          __syncwarp();
+          acc += ps_items<false>(G, StaticRows{r}, rj, head, 32, lane, r.L[0], r.L[1], r.L[2]);
+          head += 32;
+          __syncwarp();
+        }
+      }
+    }
+    __syncwarp();
+    if (tail > head)
+      acc += ps_items<false>(G, StaticRows{r}, rj, head, tail - head, lane, r.L[0], r.L[1],
+                             r.L[2]);
+    __syncthreads();   // the next atoms overwrite the stage
   }
-  if (threadIdx.x == 0) emol[m] = red[0];
+  const double sum = ps_block_sum(G, bad ? __longlong_as_double(0x7ff8000000000000LL) : acc);
+  if (threadIdx.x == 0) emol[blockIdx.x] = sum;
 }
 
 // Ordered sum of the partials into *out (thread t adds every blockDim-th
@@ -222,10 +307,26 @@ extern "C" int mcgpu_system_energy_static(const mcgpu_box_desc* rows, double* ou
     const cudaError_t e = prior == cudaSuccess ? cudaGetLastError() : cudaPeekAtLastError();
     return e == prior ? cudaSuccess : e;
   };
-  k_static_pair_sums<<<r.n_mol, 256, 0, st>>>(r, emol);
+  // FP32 coordinates within 2 edges of the origin carry at most 2 L 2^-24
+  // each; with the difference's and the image's rounding at most 10 L 2^-24
+  // along an axis; the band around rc^2 is four times what that makes of r^2
+  StaticScreen sc;
+  double Lmax = 0;
+  for (int k = 0; k < 3; k++) {
+    sc.L[k] = (float)r.L[k];
+    Lmax = std::fmax(Lmax, std::fabs(r.L[k]));
+  }
+  const double err = 10.0 * std::ldexp(Lmax, -24);
+  const double band = 4.0 * (2.0 * 1.7320508075688772 * std::fabs(r.cutoff) * err + 3.0 * err * err +
+                             4.0 * std::ldexp(r.cutoff * r.cutoff, -24)) + 1e-6;
+  sc.lo = (float)(r.cutoff * r.cutoff - band);
+  sc.hi = (float)(r.cutoff * r.cutoff + band);
+  sc.far = (float)(2.0 * Lmax);
+  const int group = mcgpu::ps_group(r.n_mol), grid = (r.n_mol + group - 1) / group;
+  k_static_pair_sums<<<grid, mcgpu::kPsThreads, 0, st>>>(r, sc, group, emol);
   cudaError_t e = launch_error();
   if (e == cudaSuccess) {
-    k_static_sum<<<1, 256, 0, st>>>(emol, r.n_mol, out);
+    k_static_sum<<<1, 256, 0, st>>>(emol, grid, out);
     e = launch_error();
   }
   if (e != cudaSuccess) {

@@ -1,4 +1,5 @@
-"""The FP64 pair batches (batch_items64, sum_moved64) where their item
+"""The FP64 pair batches (batch_items64, pair_sum64) and the grouped system
+energies (k_pair_sums64, k_static_pair_sums) where their item
 mapping and image choice can go wrong: molecules of 1 to 64 atoms in one
 box (items found in prefix sums), one species (items by atom), partial and
 full batches, several primaries, skipped sites, sites without LJ or charge,
@@ -135,3 +136,102 @@ def test_fp64_chains(ctx, name):
         assert abs(t.de - r.de) <= 1e-9 * max(1.0, abs(r.e_old) + abs(r.e_new))
     assert np.array_equal(np.stack(bt.download(0), 1), oc.coords())
     bt.close()
+
+
+def device_energy(box: BoxData) -> float:
+    """mcgpu_system_energy_static over the box's rows in device memory."""
+    import ctypes as C
+    import torch
+    from mcgpu_gb300 import _abi
+    d, keep = _abi.BoxDesc(), []
+    d.n_mol, d.n_atom, d.n_pidx = box.n_mol, box.n_atom, box.n_pidx
+    for k in ("x", "y", "z", "sigma", "epsilon", "charge", "mol_start", "mol_len",
+              "mol_pidx_start", "mol_pidx_count", "pidx"):
+        t = torch.from_numpy(getattr(box, k).copy()).cuda()
+        keep.append(t)
+        kind = _abi._dp if t.dtype == torch.float64 else _abi._ip
+        setattr(d, k, C.cast(C.c_void_p(t.data_ptr()), kind))
+    for k in range(3):
+        d.size[k] = float(box.size[k])
+    d.cutoff = float(box.cutoff)
+    out = torch.full((1,), float("nan"), dtype=torch.float64, device="cuda")
+    _abi.check(_abi.lib().mcgpu_system_energy_static(
+        C.byref(d), C.c_void_p(out.data_ptr()),
+        C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return float(out.item())
+
+
+def unwrapped(box: BoxData) -> BoxData:
+    """The box with whole molecules moved by up to three edges (the reference
+    then takes its single shift of the raw difference)."""
+    b = box.copy()
+    rng = np.random.default_rng(11)
+    for k, v in enumerate((b.x, b.y, b.z)):
+        v += np.repeat(rng.integers(-3, 4, b.n_mol) * b.size[k], b.mol_len)
+    return b
+
+
+STATIC = {
+    # molecules of more atoms than one stage holds, alone and beside short ones
+    "long_molecules": lambda: mixed_box(6, 11, [70, 130, 3, 64], (22.0, 22.0, 22.0), 10.0),
+    "unwrapped": lambda: unwrapped(mixed_box(7, 60, [3, 9, 1], (24.0, 24.0, 24.0), 9.0)),
+    "one_molecule": lambda: mixed_box(8, 1, [4], (20.0, 20.0, 20.0), 9.0),
+    "nine_molecules": lambda: mixed_box(9, 9, [5, 2], (20.0, 20.0, 20.0), 9.9),
+}
+
+
+@pytest.mark.parametrize("name", sorted(STATIC))
+def test_static_rows(ctx, name):
+    box = STATIC[name]()
+    o = OracleBox(box)
+    ref = o.system_energy()
+    scale = sum(o.mol_energy_abs(m, m) for m in range(box.n_mol))
+    assert abs(device_energy(box) - ref) <= tol64(ref, scale)
+
+
+@pytest.mark.parametrize("n_mol", [2433, 2500, 9729])
+def test_groups_of_molecules(ctx, n_mol):
+    """Sizes at which a CTA takes 2 and 8 molecules (the last group short)."""
+    from mcgpu_gb300.workloads import water_box
+    box = water_box(n_mol, seed=n_mol)
+    o = OracleBox(box)
+    ref = o.system_energy()
+    scale = sum(o.mol_energy_abs(m, m) for m in range(0, n_mol, 37)) * 37
+    g = GpuBox(ctx, box, PREC_FP64)
+    assert abs(g.system_energy() - ref) <= tol64(ref, scale)
+    assert abs(device_energy(box) - ref) <= tol64(ref, scale)
+    g.close()
+
+
+def test_groups_that_span_chains(ctx):
+    """A batch of many small chains: groups of molecules from several."""
+    from mcgpu_gb300.workloads import WATER_DENSITY, water_box
+    boxes = []
+    for c in range(600):
+        n = 8 + c % 7
+        L = (n / WATER_DENSITY) ** (1 / 3)
+        boxes.append(water_box(n, L=L, cutoff=L / 2, seed=c, dmin=2.0))
+    bt = ChainBatch(ctx, boxes, list(range(600)), rotation=ROT_AXIS)
+    e = bt.system_energies()
+    for c in range(0, 600, 7):
+        b = boxes[c].copy()
+        b.x, b.y, b.z = bt.download(c)
+        o = OracleBox(b)
+        scale = sum(o.mol_energy_abs(m, m) for m in range(b.n_mol))
+        assert abs(e[c] - o.system_energy()) <= tol64(o.system_energy(), scale), c
+    bt.close()
+
+
+@pytest.mark.parametrize("prec", [PREC_FP64, 1])
+def test_many_boxes_start_energies(ctx, prec):
+    """The device loop's start energies of boxes of uneven sizes, all in one
+    launch: each the box's own system energy."""
+    from mcgpu_gb300 import run_plain_device_many
+    boxes = [GpuBox(ctx, one_primary(mixed_box(20 + i, 2 + 9 * i, [3, 5], (21.0, 21.0, 21.0), 9.0)),
+                    prec) for i in range(5)]
+    own = [b.system_energy() for b in boxes]
+    st = run_plain_device_many(boxes, range(5), 0)
+    for e, s in zip(own, st):
+        assert s.energy0 == e and s.energy == e
+    for b in boxes:
+        b.close()
