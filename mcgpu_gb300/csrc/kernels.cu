@@ -207,8 +207,8 @@ struct PoolRows {
 // chains is taken chain by chain): emol[first molecule] holds the sum over
 // the group's molecules of the chain, the others 0.  The in-range set is the
 // FP64 test's (the FP32 screen decides outside its guard band).  32,768
-// waters (rc 12 A, 35.6 M pairs): 5.84 ms with a CTA per molecule, which
-// screened at one candidate load per test, see pairsum.cuh.
+// waters (rc 12 A, 35.6 M pairs): 1.84 ms, bound by the issue of the N^2 / 2
+// screen beside the FP64 pipe (58 % busy); 5.84 ms with a CTA per molecule.
 __global__ void __launch_bounds__(kPsThreads, 4)
     k_pair_sums64(Pool P0, const LoopTask* tasks, const int* mol_chain, int m_begin, int m_end,
                   double* emol) {
@@ -253,6 +253,9 @@ __global__ void __launch_bounds__(kPsThreads, 4)
     double acc = 0.0;
     const int end = H.mol0 + H.n_mol;
     const bool simple = H.simple_prim != 0;
+    // the screen's constants in registers (the header is global memory, and
+    // the ring's stores would have it read again for every test)
+    const float Lx = H.Lf[0], Ly = H.Lf[1], Lz = H.Lf[2], lo = H.cut2_lo, hi = H.cut2_hi;
     for (int base = m0 + 1 + w * 32; base < end; base += kPsThreads) {
       const int j = base + lane;
       int2 pj = make_int2(0, 0);
@@ -263,7 +266,19 @@ __global__ void __launch_bounds__(kPsThreads, 4)
       }
       for (int g = 0; g < n; g++) {
         bool in = false;
-        if (j > m0 + g)
+        if (simple) {
+          // one primary each: a straight line (r2_screen's arithmetic)
+          const float4 a = pp[g][0];
+          const float dx = wrapf(q0.x - a.x, Lx), dy = wrapf(q0.y - a.y, Ly),
+                      dz = wrapf(q0.z - a.z, Lz);
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          const bool mine = j > m0 + g && j < end;
+          in = mine && r2 <= lo;
+          if (mine && !in && r2 <= hi) {
+            const int o = pslot[g][0];
+            in = in_range64(G.x[o], G.y[o], G.z[o], P.pidx[pj.x], P, H);
+          }
+        } else if (j > m0 + g)
           for (int k2 = 0; k2 < pj.y && !in; k2++) {
             const float4 q = k2 == 0 ? q0 : P.ppos[pj.x + k2];
             for (int k1 = 0; k1 < pnum[g] && !in; k1++) {
@@ -277,6 +292,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
             }
           }
         const unsigned bal = __ballot_sync(~0u, in);
+        if (bal == 0) continue;
         if (in) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 3) | g;
         tail += __popc(bal);
         if (tail - head >= 32) {

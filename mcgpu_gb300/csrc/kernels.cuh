@@ -577,22 +577,31 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
   const double bz = hi_abs(tz) >= hz ? zb - copysign(Lz, tz) : zb;
   const bool lj_b = bits_nonzero(sb) && bits_nonzero(eb);
   const double qk = qb * kCoulomb, e4 = 4.0 * eb;
+  const unsigned am = __activemask();
   double acc = 0.0;
 #pragma unroll 3
   for (int i = 0; i < len; i++) {
     const double sa = sd[i], ea = ed[i];
     if (blend_skipped(sa)) continue;
     double dx = bx - xs[i], dy = by - ys[i], dz = bz - zs[i];
-    if (hi_abs(dx) >= hx || hi_abs(dy) >= hy || hi_abs(dz) >= hz) {
-      dx = image64(xb - xs[i], Lx, hx);
-      dy = image64(yb - ys[i], Ly, hy);
-      dz = image64(zb - zs[i], Lz, hz);
+    const bool far = hi_abs(dx) >= hx || hi_abs(dy) >= hy || hi_abs(dz) >= hz;
+    if (__any_sync(am, far)) {
+      __syncwarp(am);
+      if (far) {
+        dx = image64(xb - xs[i], Lx, hx);
+        dy = image64(yb - ys[i], Ly, hy);
+        dz = image64(zb - zs[i], Lz, hz);
+      }
+      __syncwarp(am);
     }
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    if (!bits_nonzero(r2)) continue;   // coincident: skipped (BruteForceStep.cpp:68-69)
+    const bool apart = bits_nonzero(r2);  // coincident: skipped (BruteForceStep.cpp:68-69)
     const double ri = rsqrt(r2);
-    acc = fma(qd[i] * qk, ri, acc);
-    if (lj_b && bits_nonzero(sa) && bits_nonzero(ea)) {
+    const double q = qd[i] * qk;
+    acc = fma(apart ? q : 0.0, apart ? ri : 0.0, acc);
+    const bool lj = apart && lj_b && bits_nonzero(sa) && bits_nonzero(ea);
+    if (__any_sync(am, lj)) {
+      __syncwarp(am);
       double t2;
       if (ROOT) {
         const double t = (sa * sb) * ri;
@@ -602,7 +611,8 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
       }
       const double s6 = t2 * t2 * t2;
       const double e = ea * e4;
-      acc = fma(s6, fma(e, s6, -e), acc);
+      if (lj) acc = fma(s6, fma(e, s6, -e), acc);
+      __syncwarp(am);
     }
   }
   return acc;

@@ -95,11 +95,12 @@ __device__ __forceinline__ double ps_block_sum(PsGroup& G, double acc) {
   return sum;
 }
 
-// Molecules per CTA for a box of n: at least 256 CTAs (more than one per SM of
-// the 152), more molecules per candidate load above that.  It depends on the
-// box alone, so a box's sum is the same alone and among others.
+// Molecules per CTA for a box of n: as many as leave eight CTAs for each of the
+// 152 SMs (their shares of the in-range pairs are uneven; 286 CTAs of 7 of
+// 1,999 16-atom molecules left the busiest SM 1.6 times the mean).  It
+// depends on the box alone, so a box's sum is the same alone and among others.
 __host__ __device__ inline int ps_group(int n) {
-  const int g = n / 256;
+  const int g = n / (152 * 8);
   return g < 1 ? 1 : g > kPsGroup ? kPsGroup : g;
 }
 

