@@ -9,13 +9,21 @@
 // s0 + r against the state at the window's start (FP32 pair terms, the FP64
 // re-take inside the guard band -- the one-group kernel's step) and stores
 // what it found in every CTA's shared memory (distributed shared memory).
-// Every CTA then walks the window in step order.  Step j's result stands
+// Every CTA then takes the decisions in step order.  Step j's result stands
 // unless an earlier accepted step i of the window moved the same molecule,
 // or moved a molecule whose primaries, before or after step i, come within
 // the screen's outer guard radius of step j's molecule at either of its
 // placements (the screen of step j could have seen that move).  Such a step
 // is staged again if needed and re-evaluated on the current state by every
-// CTA alike.  Decisions, coordinates and counters are therefore those of
+// CTA alike.
+//
+// The decisions of a window are taken side by side: lane j of every warp
+// decides step j on its record, warp j has found the steps step j depends on
+// (once the moves are staged, before the evaluation), and the first step that
+// depends on an accepted one is a vote away.  The steps before it stand and
+// are committed by one warp each.  Walking the steps one by one, every warp
+// committing each, took 2 to 2.5 us a step and most of a window: 28 us per
+// window of 8 on 32,768 waters where a step's evaluation takes 10.  Decisions, coordinates and counters are therefore those of
 // the one-group kernel on the same draws; the FP32 pair sums are the
 // one-group kernel's too when the CTA has as many warps (same split of the
 // candidates over the warps).
@@ -111,11 +119,13 @@ struct WinSmem {
   WinRec* rec;        // [2][K]: the records of the window (two windows in rotation)
   unsigned* flag;     // [K]: barrier count CTA q reached, stored by CTA q
   unsigned* ok;       // [2]: outcome of this CTA's last waits
+  unsigned* dep;      // [K]: steps of the window step j depends on: the same
+                      // molecule (bits 16 + i) or one in range (bits i)
   char* slots;        // [2][K] staging slots (two windows in rotation)
 };
 
 __host__ __device__ inline int win_extra_bytes(const SmemShape& sh, int K) {
-  return SmemShape::align16(2 * K * (int)sizeof(WinRec)) + SmemShape::align16(K * 4) + 16 +
+  return SmemShape::align16(2 * K * (int)sizeof(WinRec)) + 2 * SmemShape::align16(K * 4) + 16 +
          2 * K * sh.ahead_bytes();
 }
 
@@ -156,20 +166,36 @@ __device__ bool win_wait(const Group& g, const WinSmem& ws, unsigned K, unsigned
   return ws.ok[n & 1] != 0;
 }
 
-// Step i (slot a, accepted) moved a molecule that step j's screen (slot b)
-// could see: a primary pair within the guard band's outer radius for any
-// of the four placement pairs, with the screen's own FP32 distance (same
-// operands, same order).  The same answer in every lane.
-__device__ bool window_near(const StageSlot& a, const StageSlot& b, const ChainHdr& H, int lane) {
+// Whether step i (slot a), once accepted, has moved a molecule that step j's
+// screen (slot b) could see: a primary pair within the guard band's outer
+// radius for any of the four placement pairs, with the screen's own FP32
+// distance (same operands, same order).  One thread.
+__device__ bool window_near(const StageSlot& a, const StageSlot& b, const ChainHdr& H) {
   const int na = a.misc[3], nb = b.misc[3];
-  bool near = false;
-  for (int t = lane; t < na * nb; t += 32) {
-    const int ka = t / nb, kb = t - ka * nb;
-    const float4 ao = a.p_old[ka], an = a.p_new[ka], bo = b.p_old[kb], bn = b.p_new[kb];
-    near = near || r2_screen(bo, ao, H) <= H.cut2_hi || r2_screen(bn, ao, H) <= H.cut2_hi ||
-           r2_screen(bo, an, H) <= H.cut2_hi || r2_screen(bn, an, H) <= H.cut2_hi;
+  for (int ka = 0; ka < na; ka++) {
+    const float4 ao = a.p_old[ka], an = a.p_new[ka];
+    for (int kb = 0; kb < nb; kb++) {
+      const float4 bo = b.p_old[kb], bn = b.p_new[kb];
+      if (r2_screen(bo, ao, H) <= H.cut2_hi || r2_screen(bn, ao, H) <= H.cut2_hi ||
+          r2_screen(bo, an, H) <= H.cut2_hi || r2_screen(bn, an, H) <= H.cut2_hi)
+        return true;
+    }
   }
-  return __any_sync(~0u, near);
+  return false;
+}
+
+// The decision on a record: on the FP64 totals where it holds them, else on
+// the FP32 ones; bound gets the rounding bound of the FP32 difference.
+__device__ __forceinline__ bool window_accept(const WinRec& x, float u, const ChainHdr& H,
+                                              float& bound) {
+  const float de_f = __fadd_rn(__fsub_rn(x.nh, x.oh), __fsub_rn(x.nl, x.ol));
+  bound = (float)kTieRel * x.ab + 2.4e-7f * (fabsf(x.nh) + fabsf(x.oh)) + 1e-9f;
+  if (x.tie) {
+    const double d64 = x.en - x.eo;
+    return (d64 < 0) || (exp(-d64 / H.kT) >= (double)u);
+  }
+  const float pf = expf(-fmaxf(de_f, 0.f) * H.kTinvf);
+  return (de_f < 0.f) || (pf >= u);
 }
 
 // The one-group kernel's step evaluation (chain_steps in kernels.cu): FP32
@@ -244,6 +270,8 @@ __global__ void __launch_bounds__(512, 1)
     p += SmemShape::align16(K * 4);
     ws.ok = (unsigned*)p;
     p += 16;
+    ws.dep = (unsigned*)p;
+    p += SmemShape::align16(K * 4);
     ws.slots = p;
   }
   const int sbytes = shape.ahead_bytes();
@@ -264,7 +292,9 @@ __global__ void __launch_bounds__(512, 1)
       for (int i = g.tid; i < H.ulen; i += g.nthreads) s.teq[i] = P.aeq[H.atom0 + i];
     g.sync();
     if (g.tid == 0) Hp->ljmask = uniform_lj_mask(P, H, s.teq);  // the same value in every CTA
-    const bool lead = rank == 0 && g.tid == 0;
+    // warp 0 of the first CTA keeps the chain's sums and counters, one step
+    // of the window per lane
+    const bool lead = rank == 0 && w == 0;
     int full_scans = 0, ties = 0, redo = 0;
     float de_h = 0.f, de_l = 0.f, err_h = 0.f, err_l = 0.f;
     long long acc_n = 0, npairs = 0;
@@ -279,6 +309,7 @@ __global__ void __launch_bounds__(512, 1)
     int nred = 0;
     for (int s0 = 0; s0 < my_steps; s0 += (int)K) {
       const int nst = min((int)K, my_steps - s0), par = (s0 / (int)K) & 1;
+      WinRec* recs = ws.rec + par * (int)K;
       // draws 32 steps at a time (K divides 32, so a window never straddles)
       if ((s0 & 31) == 0) {
         if (w == 0) {
@@ -290,10 +321,19 @@ __global__ void __launch_bounds__(512, 1)
         }
         g.sync();
       }
-      // warp j stages step s0 + j (slots of the other parity may still be
-      // read by warps finishing the previous window)
+      // warp j stages step s0 + j, then finds the steps it depends on
       if (w < nst) stage_chain(P, H, props[(s0 + w) & 31], slot(par, w), pcache, lane);
       g.sync();
+      if (w < nst) {
+        bool same = false, near = false;
+        if (lane < w) {
+          const StageSlot ti = slot(par, lane), tj = slot(par, w);
+          same = ti.misc[0] == tj.misc[0];
+          near = same || window_near(ti, tj, H);
+        }
+        const unsigned d = __ballot_sync(~0u, near) | (__ballot_sync(~0u, same) << 16);
+        if (lane == 0) ws.dep[w] = d;
+      }
       const bool nl_ok0 = nl_ok;
       WinRec x = {};
       if ((int)rank < nst) {
@@ -306,106 +346,133 @@ __global__ void __launch_bounds__(512, 1)
         alive = false;
         break;
       }
-      unsigned accm = 0;
-      for (int j = 0; j < nst; j++) {
-        const StageSlot tj = slot(par, j);
+      // lane j: step j's decision on its record, dependences, and whether its
+      // trial placement leaves the Verlet list valid
+      unsigned dep = 0;
+      bool ok = false, trial_near = true, listed = false;
+      if (lane < nst) {
+        const StageSlot tj = slot(par, lane);
+        float bound;
+        ok = window_accept(recs[lane], __int_as_float(tj.misc[kMiscU]), H, bound);
+        trial_near = tj.misc[kMiscNlTrial] != 0;
+        listed = nl_ok0 && trial_near;
+        dep = ws.dep[lane];
+      }
+      unsigned okm = __ballot_sync(~0u, ok);
+      for (int cur = 0;;) {
+        // the first undecided step that depends on an accepted earlier one
+        const unsigned conf = __ballot_sync(
+            ~0u, lane >= cur && lane < nst && (dep & okm & ((1u << lane) - 1u)) != 0);
+        const int jx = conf ? __ffs(conf) - 1 : nst;
+        // the steps before it stand: warp j commits step j if accepted
+        if (w >= cur && w < jx && ((okm >> w) & 1u)) {
+          const GroupSmem ss = with_slot(s, slot(par, w));
+          commit_chain(P, H, ss, load_moved(ss), pcache, lane);
+        }
+        if (__any_sync(~0u, lane >= cur && lane < jx && ok && !trial_near)) nl_ok = false;
+        if (jx == nst) break;
+        g.sync();  // the commits, before the state is read again
+        const StageSlot tj = slot(par, jx);
         const GroupSmem ss = with_slot(s, tj);
-        MovedInfo mi = load_moved(ss);
-        bool same = false, near = false;
-        for (int i = 0; i < j; i++) {
-          if (!((accm >> i) & 1u)) continue;
-          const StageSlot ti = slot(par, i);
-          if (ti.misc[0] == mi.mol)
-            same = true;
-          else if (!near)
-            near = window_near(ti, tj, H, lane);
+        const unsigned dj = __shfl_sync(~0u, dep, jx);
+        if ((dj >> 16) & okm & ((1u << jx) - 1u)) {
+          // staged from rows an earlier step of the window changed: stage it
+          // again, and look which later steps its new placements reach
+          if (w == 0) stage_chain(P, H, props[(s0 + jx) & 31], tj, pcache, lane);
+          g.sync();
+          if (lane > jx && lane < nst) {
+            const StageSlot tk = slot(par, lane);
+            const bool near = tk.misc[0] == tj.misc[0] || window_near(tj, tk, H);
+            dep = (dep & ~(1u << jx)) | ((near ? 1u : 0u) << jx);
+          }
         }
+        const bool near_j = ss.misc[kMiscNlTrial] != 0;
+        const bool listed_j = nl_ok && near_j;
+        const float uj = __int_as_float(ss.misc[kMiscU]);
         WinRec xj;
-        bool listed;
-        if (same || near) {
-          if (same) {
-            // the move was staged from rows an earlier step of the window
-            // changed: stage it again once every warp is done reading it
-            g.sync();
-            if (w == 0) stage_chain(P, H, props[(s0 + j) & 31], tj, pcache, lane);
-            g.sync();
-            mi = load_moved(ss);
-          }
-          listed = nl_ok && ss.misc[kMiscNlTrial] != 0;
-          window_eval(P, H, g, ss, mi, pcache, listed, T, __int_as_float(ss.misc[kMiscU]), nred,
-                      xj);
-          // nobody commits step j (or a later one) while a CTA still reads
-          // the state for it
-          if (!win_wait(g, ws, K, rank, ++nbar, nullptr, 0)) {
-            alive = false;
-            break;
-          }
-          redo++;
-        } else {
-          xj = ws.rec[par * (int)K + j];
-          listed = nl_ok0 && ss.misc[kMiscNlTrial] != 0;
+        window_eval(P, H, g, ss, load_moved(ss), pcache, listed_j, T, uj, nred, xj);
+        // nobody commits step j (or a later one) while a CTA still reads the
+        // state for it
+        if (!win_wait(g, ws, K, rank, ++nbar, nullptr, 0)) {
+          alive = false;
+          break;
         }
-        const float u = __int_as_float(ss.misc[kMiscU]);
-        const float de_f = __fadd_rn(__fsub_rn(xj.nh, xj.oh), __fsub_rn(xj.nl, xj.ol));
-        const float bound =
-            (float)kTieRel * xj.ab + 2.4e-7f * (fabsf(xj.nh) + fabsf(xj.oh)) + 1e-9f;
-        int ok;
-        if (xj.tie) {
-          const double d64 = xj.en - xj.eo;
-          ok = (d64 < 0) || (exp(-d64 / H.kT) >= (double)u);
-        } else {
-          const float pf = expf(-fmaxf(de_f, 0.f) * H.kTinvf);
-          ok = (de_f < 0.f) || (pf >= u);
+        float bound;
+        const bool okj = window_accept(xj, uj, H, bound);
+        okm = (okm & ~(1u << jx)) | ((okj ? 1u : 0u) << jx);
+        if (lane == jx) {
+          ok = okj;
+          trial_near = near_j;
+          listed = listed_j;
+          if (lead) recs[jx] = xj;
         }
-        if (ok) {
-          commit_chain(P, H, ss, mi, pcache, lane);
-          accm |= 1u << j;
-        }
+        if (okj && w == jx) commit_chain(P, H, ss, load_moved(ss), pcache, lane);
+        if (okj && !near_j) nl_ok = false;
+        redo++;
+        cur = jx + 1;
+      }
+      if (!alive) break;
+      if (lead) {
         __syncwarp();
-        if (ok && !ss.misc[kMiscNlTrial]) nl_ok = false;
-        if (lead) {
+        float vh = 0.f, vl = 0.f, ve = 0.f;
+        long long np = 0;
+        int tie = 0;
+        if (lane < nst) {
+          const WinRec r = recs[lane];
+          tie = r.tie;
+          np = r.np;
           if (ok) {
-            if (xj.tie) {
-              const double d64 = xj.en - xj.eo;
-              const float dh = (float)d64;
-              ff_add2(de_h, de_l, dh, (float)(d64 - (double)dh));
-              ff_add(err_h, err_l, 1e-12f * xj.ab);
+            if (r.tie) {
+              const double d64 = r.en - r.eo;
+              vh = (float)d64;
+              vl = (float)(d64 - (double)vh);
+              ve = 1e-12f * r.ab;
             } else {
-              ff_add2(de_h, de_l, xj.nh, xj.nl);
-              ff_add2(de_h, de_l, -xj.oh, -xj.ol);
-              ff_add(err_h, err_l, bound);
+              vh = r.nh;
+              vl = r.nl;
+              ff_add2(vh, vl, -r.oh, -r.ol);
+              ve = (float)kTieRel * r.ab + 2.4e-7f * (fabsf(r.nh) + fabsf(r.oh)) + 1e-9f;
             }
-            acc_n++;
           }
-          if (H.nl_on && !listed) full_scans++;
-          npairs += xj.np;
-          ties += xj.tie;
           if (trace) {
-            double e_old = xj.eo, e_new = xj.en;
-            if (!xj.tie) {
-              e_old = (double)xj.oh + (double)xj.ol;
-              e_new = (double)xj.nh + (double)xj.nl;
+            const StageSlot tj = slot(par, lane);
+            double e_old = r.eo, e_new = r.en;
+            if (!r.tie) {
+              e_old = (double)r.oh + (double)r.ol;
+              e_new = (double)r.nh + (double)r.nl;
             }
             mcgpu_trace t;
-            t.mol = mi.mol - H.mol0;
-            t.accepted = ok;
+            t.mol = tj.misc[0] - H.mol0;
+            t.accepted = ok ? 1 : 0;
             t.e_old = e_old;
             t.e_new = e_new;
             t.de = e_new - e_old;
-            t.u = (double)u;
-            t.fp64 = xj.tie;
+            t.u = (double)__int_as_float(tj.misc[kMiscU]);
+            t.fp64 = r.tie;
             t.pad0 = 0;
-            trace[(size_t)c * trace_stride + trace_off + s0 + j] = t;
+            trace[(size_t)c * trace_stride + trace_off + s0 + lane] = t;
           }
         }
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) {
+          const float oh = __shfl_xor_sync(~0u, vh, off), ol = __shfl_xor_sync(~0u, vl, off);
+          ff_add2(vh, vl, oh, ol);
+          ve += __shfl_xor_sync(~0u, ve, off);
+        }
+        ff_add2(de_h, de_l, vh, vl);   // lane 0's is the window's
+        ff_add(err_h, err_l, ve);
+        acc_n += __popc(okm);
+        npairs += warp_count(np);
+        ties += __popc(__ballot_sync(~0u, tie != 0));
+        full_scans += __popc(__ballot_sync(~0u, H.nl_on && lane < nst && !listed));
       }
-      if (!alive) break;
+      g.sync();  // the commits, before the next moves are staged
     }
     if (!alive) {
       if (g.tid == 0) Hp->error = kErrWindowSync;
       break;
     }
-    if (lead) {
+    if (lead && lane == 0) {
       Hp->energy = H.energy + ((double)de_h + (double)de_l);
       Hp->run_err += (double)err_h + (double)err_l;
       Hp->step = step0 + my_steps;
