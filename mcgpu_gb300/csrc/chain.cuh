@@ -164,15 +164,14 @@ __device__ __forceinline__ int screen_chain(const Pool& P, const ChainHdr& H, co
   return f;
 }
 
-// The single-lane pair batch for the chain's molecule length (inner atom
-// loop unrolled for 3-site molecules).
+// The single-lane pair batch for the chain's molecule length.
 __device__ __forceinline__ void batch_u1_any(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                              const MovedInfo& mi, const int* rj, int head,
                                              int count, int w, int lane, AccFF& acc) {
   if (H.ulen == 3)
-    batch_u1<3>(P, H, s, mi, rj, head, count, w, lane, acc, H.ljmask);
+    batch_u3(P, H, s, mi, rj, head, count, lane, acc, H.ljmask);
   else
-    batch_u1<0>(P, H, s, mi, rj, head, count, w, lane, acc, ~0u);
+    batch_u1(P, H, s, mi, rj, head, count, w, lane, acc);
 }
 
 // Bits 4k + i: the LJ term between atoms i and k of a uniform chain's
@@ -206,6 +205,13 @@ __device__ inline void warp_eval_chain(const Pool& P, const ChainHdr& H, const G
   // gets its share of the in-range neighbours
   const int rounds = cand ? (c_end - c_begin + 32 * nw - 1) / (32 * nw) : 0;
   const bool u1 = H.uniform && T == 1 && H.ulen <= 4 && !H.precise;
+  // one primary each (the common chain): the moved molecule's two placements
+  // and the screen's constants in registers -- the header is global memory,
+  // and the ring's stores would have it read again every round
+  const bool single = H.simple_prim && mi.npidx == 1;
+  const float Lx = H.Lf[0], Ly = H.Lf[1], Lz = H.Lf[2], lo = H.cut2_lo, hi = H.cut2_hi;
+  const float4 po = s.p_old[0], pn = s.p_new[0];
+  const int mol0 = H.mol0, pidx0 = H.pidx0;
   for (int it = 0;; it++) {
     int idx;
     if (cand) {
@@ -219,14 +225,22 @@ __device__ inline void warp_eval_chain(const Pool& P, const ChainHdr& H, const G
     const int j = (cand && idx < c_end) ? cand[idx] : idx;
     int f = 0;
     if (idx < c_end && j != mi.mol) {
-      float4 q0;
-      if (pcache)
-        q0 = pcache[j - H.mol0];
-      else if (H.simple_prim)
-        q0 = P.ppos[H.pidx0 + (j - H.mol0)];
-      else
-        q0 = P.ppos[P.mpi[j].x];
-      f = screen_chain(P, H, s, mi, j, q0);
+      if (single) {
+        const float4 q0 = pcache ? pcache[j - mol0] : P.ppos[pidx0 + (j - mol0)];
+        const float ox = wrapf(q0.x - po.x, Lx), oy = wrapf(q0.y - po.y, Ly),
+                    oz = wrapf(q0.z - po.z, Lz);
+        const float nx = wrapf(q0.x - pn.x, Lx), ny = wrapf(q0.y - pn.y, Ly),
+                    nz = wrapf(q0.z - pn.z, Lz);
+        const float ro = fmaf(ox, ox, fmaf(oy, oy, oz * oz));
+        const float rn = fmaf(nx, nx, fmaf(ny, ny, nz * nz));
+        f = (ro <= lo ? kInOld : 0) | (rn <= lo ? kInNew : 0);
+        if ((ro > lo && ro <= hi) || (rn > lo && rn <= hi))
+          f = screen_chain(P, H, s, mi, j, q0);   // inside the guard band
+      } else {
+        const float4 q0 = pcache ? pcache[j - mol0]
+                                 : P.ppos[H.simple_prim ? pidx0 + (j - mol0) : P.mpi[j].x];
+        f = screen_chain(P, H, s, mi, j, q0);
+      }
     }
     const unsigned bal = __ballot_sync(~0u, f != 0);
     if (f) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 4) | f;
@@ -255,39 +269,58 @@ __device__ inline void warp_eval_chain(const Pool& P, const ChainHdr& H, const G
   __syncwarp();
 }
 
-// Group-wide deterministic double-float sum: warp butterflies, then every
-// thread adds the per-warp values in warp order.
+// Group-wide deterministic double-float sum, the same in every thread.  After
+// the first exchange the lower half of a warp carries the old placement's sum
+// and the upper half the new one's, and the warps' values are added by a
+// second butterfly over the lanes: a third of the instructions of reducing
+// both sums in every lane and adding the warps one by one (a step of the 512
+// water chains spent 1,250 of its 12,500 warp instructions there).
 __device__ __forceinline__ void group_reduce_ff(const Group& g, const GroupSmem& s, AccFF& a,
                                                 int par = 0) {
-  for (int off = 16; off > 0; off >>= 1) {
-    const float oh = __shfl_xor_sync(~0u, a.oh, off), ol = __shfl_xor_sync(~0u, a.ol, off);
-    const float nh = __shfl_xor_sync(~0u, a.nh, off), nl = __shfl_xor_sync(~0u, a.nl, off);
-    ff_add2(a.oh, a.ol, oh, ol);
-    ff_add2(a.nh, a.nl, nh, nl);
-    a.ab += __shfl_xor_sync(~0u, a.ab, off);
-    a.np += __shfl_xor_sync(~0u, a.np, off);
+  const int lane = g.tid & 31, half = lane >> 4, k = lane & 15;
+  float h = half ? a.nh : a.oh, l = half ? a.nl : a.ol;
+  {
+    const float oh = __shfl_xor_sync(~0u, half ? a.oh : a.nh, 16);
+    const float ol = __shfl_xor_sync(~0u, half ? a.ol : a.nl, 16);
+    ff_add2(h, l, oh, ol);
   }
+  float ab = a.ab + __shfl_xor_sync(~0u, a.ab, 16);
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) {
+    const float oh = __shfl_xor_sync(~0u, h, off), ol = __shfl_xor_sync(~0u, l, off);
+    ff_add2(h, l, oh, ol);
+    ab += __shfl_xor_sync(~0u, ab, off);
+  }
+  const long long n = warp_count(a.np);
   const int nw = g.nwarps();
   // buffer `par` of two; 5 floats per warp fit the 3 doubles reserved per warp
   float* red = (float*)(s.red + par * 3 * nw);
   long long* redl = s.redl + par * nw;
-  if ((g.tid & 31) == 0) {
-    red[5 * g.warp() + 0] = a.oh;
-    red[5 * g.warp() + 1] = a.ol;
-    red[5 * g.warp() + 2] = a.nh;
-    red[5 * g.warp() + 3] = a.nl;
-    red[5 * g.warp() + 4] = a.ab;
-    redl[g.warp()] = a.np;
+  if (k == 0) {
+    red[5 * g.warp() + 2 * half] = h;
+    red[5 * g.warp() + 2 * half + 1] = l;
+  }
+  if (lane == 0) {
+    red[5 * g.warp() + 4] = ab;
+    redl[g.warp()] = n;
   }
   g.sync();
-  a.oh = a.ol = a.nh = a.nl = a.ab = 0.f;
-  a.np = 0;
-  for (int w = 0; w < nw; w++) {
-    ff_add2(a.oh, a.ol, red[5 * w + 0], red[5 * w + 1]);
-    ff_add2(a.nh, a.nl, red[5 * w + 2], red[5 * w + 3]);
-    a.ab += red[5 * w + 4];
-    a.np += redl[w];
+  const bool on = k < nw;
+  h = on ? red[5 * k + 2 * half] : 0.f;
+  l = on ? red[5 * k + 2 * half + 1] : 0.f;
+  ab = on ? red[5 * k + 4] : 0.f;
+  a.np = warp_count(on && half == 0 ? redl[k] : 0);
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) {
+    const float oh = __shfl_xor_sync(~0u, h, off), ol = __shfl_xor_sync(~0u, l, off);
+    ff_add2(h, l, oh, ol);
+    ab += __shfl_xor_sync(~0u, ab, off);
   }
+  a.oh = __shfl_sync(~0u, h, 0);
+  a.ol = __shfl_sync(~0u, l, 0);
+  a.nh = __shfl_sync(~0u, h, 16);
+  a.nl = __shfl_sync(~0u, l, 16);
+  a.ab = ab;
 }
 
 // FP64 re-take of a step near the decision threshold: FP64 pair terms

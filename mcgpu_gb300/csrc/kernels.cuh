@@ -471,21 +471,16 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // copies into its own shared-memory slot (one round trip to L2 instead of
 // one per atom, no registers held), and the pair factors come from the
 // chain's per-slot template.  Each placement's sum is batch_ff's bit for bit.
-//
-// ULEN > 0: molecules of ULEN atoms (the inner atom loop unrolls); ljmask
-// bits 4k..4k+3: the LJ terms of neighbour atom k with moved atoms 0..3 that
-// are not exactly zero (the same in every lane: the chain is uniform).  Both
-// placements run through one copy of the pair code (a rolled loop), which
-// keeps the step loop's code small enough for the instruction cache.
-template <int ULEN>
+// Both placements run through one copy of the pair code (a rolled loop),
+// which keeps the step loop's code small enough for the instruction cache.
 __device__ __forceinline__ void batch_u1(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                          const MovedInfo& mi, const int* rj, int head, int count,
-                                         int w, int lane, AccFF& acc, unsigned ljmask) {
+                                         int w, int lane, AccFF& acc) {
   if (lane >= count) return;  // lanes are independent: no shuffles below
   const int jf = rj[(head + lane) & (kRing - 1)];
   const int j = jf >> 4;
   const int f = jf & 15;
-  const int lenj = ULEN > 0 ? ULEN : H.ulen;
+  const int lenj = H.ulen;
   const int b0 = H.atom0 + (j - H.mol0) * lenj;
   float4* nb = s.nbuf + (w * 32 + lane) * 5;
   cp_async16(nb + 4, P.mfix + j);
@@ -506,12 +501,10 @@ __device__ __forceinline__ void batch_u1(const Pool& P, const ChainHdr& H, const
     for (int k = 0; k < lenj; k++) {
       const float4 ob = nb[k];
       const float2 qb = s.teq[k];
-      const unsigned lm = (ljmask >> (4 * k)) & 15u;
       const float3 bh = make_float3(D.x + ob.x, D.y + ob.y, D.z + ob.z);
-      sp += wrap ? sum_moved32_wrap<false, ULEN>(o, s.l_old, s.eq, mi.len, bh, z3, ob.w, qb, H,
-                                                 sa, lm)
-                 : sum_moved32_cf<false, ULEN>(o, s.l_old, s.eq, mi.len, p != 0, bh, z3, ob.w, qb,
-                                               mi.qm, sa, lm);
+      sp += wrap ? sum_moved32_wrap<false>(o, s.l_old, s.eq, mi.len, bh, z3, ob.w, qb, H, sa)
+                 : sum_moved32_cf<false>(o, s.l_old, s.eq, mi.len, p != 0, bh, z3, ob.w, qb,
+                                         mi.qm, sa);
     }
     if (p)
       ff_add(acc.nh, acc.nl, sp);
@@ -520,6 +513,72 @@ __device__ __forceinline__ void batch_u1(const Pool& P, const ChainHdr& H, const
     acc.np += (long long)mi.act * H.uact;
   }
   acc.ab += sa;
+}
+
+// batch_u1 for molecules of 3 atoms, one lane per (entry, placement): a batch
+// of at most 16 entries then takes one round of 9 pair terms instead of 18
+// (a warp's share of the in-range neighbours is about 15 to 20, so a lane per
+// entry left half the lanes idle for twice the time).  The header's scales
+// and the moved atoms go to registers once per round, the neighbour's rows
+// come with four independent loads (one round trip).  ljmask bits 4k + i: the
+// LJ term of neighbour atom k with moved atom i is not exactly zero (the same
+// in every lane: the chain is uniform).  Each placement's sum is batch_ff's
+// bit for bit.
+__device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const GroupSmem& s,
+                                         const MovedInfo& mi, const int* rj, int head, int count,
+                                         int lane, AccFF& acc, unsigned ljmask) {
+  const int atom0 = H.atom0, mol0 = H.mol0;
+  const float sx = H.fxs[0], sy = H.fxs[1], sz = H.fxs[2];
+  const float Lx = H.Lf[0], Ly = H.Lf[1], Lz = H.Lf[2];
+  const float rr = mi.rad + H.umrad;
+  const int pairs = mi.act * H.uact;
+#pragma unroll 1
+  for (int base = 0; base < 2 * count; base += 32) {
+    const int it = base + lane;
+    const bool p = it >= count;
+    if (it >= 2 * count) continue;   // lanes are independent: no shuffles below
+    const int jf = rj[(head + (p ? it - count : it)) & (kRing - 1)];
+    if (!(jf & (p ? kInNew : kInOld))) continue;
+    const int j = jf >> 4;
+    const int b0 = atom0 + (j - mol0) * 3;
+    const uint4 fj = P.mfix[j];
+    float4 ob[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) ob[k] = P.aoff[b0 + k];
+    const float4* o = p ? s.o_new : s.o_old;
+    const uint4 fm = p ? mi.fx_new : mi.fx_old;
+    const float3 D = make_float3((float)(int)(fj.x - fm.x) * sx, (float)(int)(fj.y - fm.y) * sy,
+                                 (float)(int)(fj.z - fm.z) * sz);
+    // some pair may need its own periodic image (needs_wrap)
+    const bool wrap = fabsf(D.x) + rr > 0.5f * Lx - 1e-3f ||
+                      fabsf(D.y) + rr > 0.5f * Ly - 1e-3f || fabsf(D.z) + rr > 0.5f * Lz - 1e-3f;
+    float sp = 0.f, sa = 0.f;
+    if (wrap) {
+#pragma unroll 1
+      for (int k = 0; k < 3; k++) {
+        const float4 b = k == 0 ? ob[0] : k == 1 ? ob[1] : ob[2];
+        sp += sum_moved32_wrap<false, 3>(o, s.l_old, s.eq, 3,
+                                         make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
+                                         make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], H, sa,
+                                         (ljmask >> (4 * k)) & 15u);
+      }
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < 3; k++) {
+        const float4 b = k == 0 ? ob[0] : k == 1 ? ob[1] : ob[2];
+        sp += sum_moved32_cf<false, 3>(o, s.l_old, s.eq, 3, p,
+                                       make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
+                                       make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], mi.qm, sa,
+                                       (ljmask >> (4 * k)) & 15u);
+      }
+    }
+    if (p)
+      ff_add(acc.nh, acc.nl, sp);
+    else
+      ff_add(acc.oh, acc.ol, sp);
+    acc.ab += sa;
+    acc.np += pairs;
+  }
 }
 
 // ---- FP64 pair batches -------------------------------------------------------
