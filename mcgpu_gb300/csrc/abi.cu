@@ -613,12 +613,12 @@ extern "C" int mcgpu_box_upload(mcgpu_ctx* ctx, const mcgpu_box_desc* desc, int 
   b->counter = dalloc<unsigned>(2, &e);
   b->dout = dalloc<double>(4, &e);
   b->queue = dalloc<unsigned>(1, &e);
-  b->order = dalloc<int>(1, &e);
+  b->order = dalloc<int>(2, &e);   // chain 0, and a zero for its size
   if (e == cudaSuccess) e = cudaMallocHost((void**)&b->hout, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMemsetAsync(b->counter, 0, 2 * sizeof(unsigned), ctx->stream);
   if (e == cudaSuccess) b->dpairs = dalloc<long long>(1, &e);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->dpairs, 0, sizeof(long long), ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->order, 0, sizeof(int), ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->order, 0, 2 * sizeof(int), ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
     mcgpu_box_destroy(b);
@@ -1438,12 +1438,15 @@ extern "C" int mcgpu_chain_run(mcgpu_box* b, uint64_t seed, uint32_t chain_id, i
     if (K > 1)
       CK(ctx, launch_chain_window(K, 1, nw * 32, wsmem, st, P, k, b->order, 1, sh,
                                   trace ? b->dtrace : nullptr, done, 0, 0));
-    else if (nw > 8)
-      k_chain_steps_wide<<<1, nw * 32, sh.bytes(), st>>>(P, k, b->queue, b->order, 1, nw, sh,
-                                                         trace ? b->dtrace : nullptr, done, 0, 0);
-    else
-      k_chain_steps<<<1, nw * 32, sh.bytes(), st>>>(P, k, b->queue, b->order, 1, nw, sh,
-                                                    trace ? b->dtrace : nullptr, done, 0, 0);
+    else {
+      ChainLaunch A{k, k, 1, nw, b->queue, b->order, b->order + 1, sh};
+      A.trace = trace ? b->dtrace : nullptr;
+      A.trace_off = done;
+      if (nw > 8)
+        k_chain_steps_wide<<<1, nw * 32, sh.bytes(), st>>>(P, A);
+      else
+        k_chain_steps<<<1, nw * 32, sh.bytes(), st>>>(P, A);
+    }
     CK(ctx, cudaGetLastError());
     b->rows_stale = true;
   }
@@ -1476,8 +1479,8 @@ extern "C" int mcgpu_chain_run(mcgpu_box* b, uint64_t seed, uint32_t chain_id, i
 struct mcgpu_batch {
   mcgpu_ctx* ctx = nullptr;
   DevPool pool;
-  unsigned* queue = nullptr;   // one counter per launch slot of a graph
-  int* order = nullptr;
+  unsigned* sched = nullptr;   // steps each chain has taken in a launch (n_chains)
+  int* order = nullptr;        // chains by descending cost, then their molecule counts
   int threads = 128, cpc = 1, spl = 16;  // CTA threads, chains per CTA, steps per launch
   int lanes = 0;                          // lanes per neighbour molecule cap (0 = per chain)
   int cache_n = 0;                        // shared-memory screen cache per group
@@ -1518,7 +1521,10 @@ static int batch_grid(mcgpu_batch* bt, int* smem_out) {
   return std::max(1, std::min(need, per_sm * bt->ctx->sm_count));
 }
 
-static int batch_launch(mcgpu_batch* bt, int steps, unsigned* q, cudaStream_t st,
+// One launch of `steps` steps of every chain, each chain spl steps at a time on
+// a group (the running energy takes a chain's dE sum once per spl steps, so a
+// batch's energies do not depend on how its steps are split into launches).
+static int batch_launch(mcgpu_batch* bt, int steps, cudaStream_t st,
                         mcgpu_trace* trace = nullptr, int trace_off = 0, int trace_stride = 0) {
   mcgpu_ctx* ctx = bt->ctx;
   int smem = 0;
@@ -1528,7 +1534,6 @@ static int batch_launch(mcgpu_batch* bt, int steps, unsigned* q, cudaStream_t st
   bt->rows_stale = true;
   int rc = pool_nl_rebuild(ctx, bt->pool, st);
   if (rc) return rc;
-  CK(ctx, cudaMemsetAsync(q, 0, sizeof(unsigned), st));
   if (bt->window > 1) {
     const int K = bt->window, wsmem = window_smem_bytes(sh, K);
     const int n_cl = std::max(1, std::min(bt->pool.n_chains,
@@ -1537,14 +1542,15 @@ static int batch_launch(mcgpu_batch* bt, int steps, unsigned* q, cudaStream_t st
                                 bt->pool.n_chains, sh, trace, trace_off, trace_stride, bt->lanes));
     return MCGPU_OK;
   }
+  const int seg = std::min(steps, bt->spl);
+  CK(ctx, cudaMemsetAsync(bt->sched, 0, sizeof(unsigned) * bt->pool.n_chains, st));
+  const int n = bt->pool.n_chains;
+  const ChainLaunch A{steps, seg, n, gw, bt->sched, bt->order, bt->order + n, sh, trace,
+                      trace_off, trace_stride, bt->lanes};
   if (bt->threads > 256)
-    k_chain_steps_wide<<<grid, bt->threads, smem, st>>>(bt->pool.P, steps, q, bt->order,
-                                                        bt->pool.n_chains, gw, sh, trace,
-                                                        trace_off, trace_stride, bt->lanes);
+    k_chain_steps_wide<<<grid, bt->threads, smem, st>>>(bt->pool.P, A);
   else
-    k_chain_steps<<<grid, bt->threads, smem, st>>>(bt->pool.P, steps, q, bt->order,
-                                                   bt->pool.n_chains, gw, sh, trace, trace_off,
-                                                   trace_stride, bt->lanes);
+    k_chain_steps<<<grid, bt->threads, smem, st>>>(bt->pool.P, A);
   CK(ctx, cudaGetLastError());
   return MCGPU_OK;
 }
@@ -1576,11 +1582,12 @@ extern "C" int mcgpu_batch_create(mcgpu_ctx* ctx, int n_chains, const mcgpu_box_
   });
   bt->max_slots = 64;
   cudaError_t e = cudaSuccess;
-  bt->queue = dalloc<unsigned>(bt->max_slots, &e);
-  bt->order = dalloc<int>(n_chains, &e);
+  bt->sched = dalloc<unsigned>(n_chains, &e);
+  bt->order = dalloc<int>(2 * (size_t)n_chains, &e);
+  for (int c = 0; c < n_chains; c++) order.push_back(hp.hdr[order[c]].n_mol);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(bt->order, order.data(), sizeof(int) * n_chains, cudaMemcpyHostToDevice,
-                        ctx->stream);
+    e = cudaMemcpyAsync(bt->order, order.data(), sizeof(int) * order.size(),
+                        cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) {
     mcgpu_batch_destroy(bt);
     return set_err(ctx, MCGPU_ERR_NOMEM, "batch allocation failed: %s", cudaGetErrorString(e));
@@ -1635,7 +1642,7 @@ extern "C" int mcgpu_batch_destroy(mcgpu_batch* bt) {
   cudaStreamSynchronize(bt->ctx->stream);
   batch_drop_graph(bt);
   bt->pool.release();
-  if (bt->queue) cudaFree(bt->queue);
+  if (bt->sched) cudaFree(bt->sched);
   if (bt->order) cudaFree(bt->order);
   if (bt->vm) cudaFree(bt->vm);
   if (bt->emol2) cudaFree(bt->emol2);
@@ -1734,8 +1741,7 @@ extern "C" int mcgpu_batch_get_tile(mcgpu_batch* bt, int* threads, int* cpc, int
   return MCGPU_OK;
 }
 
-// Captures `launches` launches of spl steps each into a graph (one queue
-// counter per launch, reset by a memset node).  With interval > 0 the graph
+// Captures `launches` launches of spl steps each into a graph.  With interval > 0 the graph
 // is one NPT interval instead: launches covering `interval` steps, then the
 // volume phase.
 static int batch_build_graph(mcgpu_batch* bt, int launches, int interval) {
@@ -1747,9 +1753,9 @@ static int batch_build_graph(mcgpu_batch* bt, int launches, int interval) {
   int rc = MCGPU_OK;
   if (interval > 0) {
     int done = 0;
-    for (int l = 0; done < interval && rc == MCGPU_OK; l++) {
+    while (done < interval && rc == MCGPU_OK) {
       const int k = std::min(bt->spl, interval - done);
-      rc = batch_launch(bt, k, bt->queue + l, st);
+      rc = batch_launch(bt, k, st);
       done += k;
     }
     if (rc == MCGPU_OK) {
@@ -1760,7 +1766,7 @@ static int batch_build_graph(mcgpu_batch* bt, int launches, int interval) {
       if (e != cudaSuccess) rc = set_err(ctx, MCGPU_ERR_CUDA, "volume phase launch: %s", cudaGetErrorString(e));
     }
   } else {
-    for (int l = 0; l < launches && rc == MCGPU_OK; l++) rc = batch_launch(bt, bt->spl, bt->queue + l, st);
+    for (int l = 0; l < launches && rc == MCGPU_OK; l++) rc = batch_launch(bt, bt->spl, st);
   }
   cudaError_t e = cudaStreamEndCapture(st, &g);
   if (rc) {
@@ -1788,14 +1794,13 @@ static bool batch_graph_matches(const mcgpu_batch* bt, int launches, int interva
          bt->graph_window == bt->window;
 }
 
-// Steps n_steps with direct launches of at most spl steps (recording steps
+// Steps n_steps with direct launches of at most `most` steps (recording steps
 // at trace[c * trace_stride + trace_off + s] when trace is non-null).
-static int batch_steps_direct(mcgpu_batch* bt, int n_steps, mcgpu_trace* trace, int trace_off,
-                              int trace_stride) {
+static int batch_steps_direct(mcgpu_batch* bt, int n_steps, int most, mcgpu_trace* trace,
+                              int trace_off, int trace_stride) {
   for (int done = 0; done < n_steps;) {
-    const int k = std::min(bt->spl, n_steps - done);
-    int rc = batch_launch(bt, k, bt->queue + ((done / bt->spl) % bt->max_slots), bt->ctx->stream,
-                          trace, trace_off + done, trace_stride);
+    const int k = std::min(most, n_steps - done);
+    int rc = batch_launch(bt, k, bt->ctx->stream, trace, trace_off + done, trace_stride);
     if (rc) return rc;
     done += k;
   }
@@ -1817,7 +1822,11 @@ static int batch_advance(mcgpu_batch* bt, int n_steps, mcgpu_trace* trace, int t
     const int full = n_steps / spl;
     const int per_graph = std::min(bt->max_slots, 32);
     int done = 0;
-    if (!trace && full >= per_graph) {
+    // nothing to do between the launches of a one-step NVT batch without
+    // lists: one launch takes the steps of 32, the chains spl steps at a time
+    const bool merged = bt->window == 1 && !bt->pool.nl_on;
+    const int most = merged ? (int)std::min(32LL * spl, 1LL << 30) : spl;
+    if (!merged && !trace && full >= per_graph) {
       if (!batch_graph_matches(bt, per_graph, 0)) {
         int rc = batch_build_graph(bt, per_graph, 0);
         if (rc) return rc;
@@ -1827,7 +1836,7 @@ static int batch_advance(mcgpu_batch* bt, int n_steps, mcgpu_trace* trace, int t
         done += per_graph;
       }
     }
-    int rc = batch_steps_direct(bt, n_steps - done * spl, trace, done * spl, trace_stride);
+    int rc = batch_steps_direct(bt, n_steps - done * spl, most, trace, done * spl, trace_stride);
     if (rc) return rc;
     bt->steps_done += n_steps;
     return MCGPU_OK;
@@ -1848,7 +1857,7 @@ static int batch_advance(mcgpu_batch* bt, int n_steps, mcgpu_trace* trace, int t
       continue;
     }
     const int seg = std::min(n_steps - done, iv - phase);
-    int rc = batch_steps_direct(bt, seg, trace, done, trace_stride);
+    int rc = batch_steps_direct(bt, seg, spl, trace, done, trace_stride);
     if (rc) return rc;
     done += seg;
     bt->steps_done += seg;
@@ -2276,21 +2285,19 @@ extern "C" int mcgpu_batch_autotune(mcgpu_batch* bt, int trial_steps) {
     bt->steps_done = steps0;
     r = mcgpu_batch_run(bt, T.spl, 0);
     if (r) return r;
-    const int n = std::max(trial_steps, 2 * T.spl);
+    // runs of four segments of a chain, in one launch where a run is one: the
+    // groups pass the chains on between segments
+    const int n = std::max(trial_steps, 4 * T.spl);
     for (int rep = 0; rep < 3; rep++) {
-      float total = 0;
-      for (int done = 0; done < n; done += T.spl) {
-        if (flush) CK(ctx, cudaMemsetAsync(flush, rep + 1, flush_bytes, ctx->stream));
-        CK(ctx, cudaEventRecord(e0, ctx->stream));
-        r = mcgpu_batch_run(bt, std::min(T.spl, n - done), 0);
-        if (r) return r;
-        CK(ctx, cudaEventRecord(e1, ctx->stream));
-        CK(ctx, cudaEventSynchronize(e1));
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        total += ms;
-      }
-      *out = std::min(*out, total * (float)trial_steps / (float)n);
+      if (flush) CK(ctx, cudaMemsetAsync(flush, rep + 1, flush_bytes, ctx->stream));
+      CK(ctx, cudaEventRecord(e0, ctx->stream));
+      r = mcgpu_batch_run(bt, n, 0);
+      if (r) return r;
+      CK(ctx, cudaEventRecord(e1, ctx->stream));
+      CK(ctx, cudaEventSynchronize(e1));
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      *out = std::min(*out, ms * (float)trial_steps / (float)n);
     }
     return MCGPU_OK;
   };

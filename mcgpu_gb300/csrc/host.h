@@ -23,12 +23,20 @@ __global__ void k_change_molecule(Pool P, int chain, int mol, Proposal prop, Sme
 __global__ void k_rollback(Pool P, int chain, int mol);
 __global__ void k_chain_sums(Pool P, const double* emol, double* out);
 __global__ void k_set_energy(Pool P, const double* e);
-__global__ void k_chain_steps(Pool P, int n_steps, unsigned* queue, const int* order, int n_tasks,
-                              int gwarps, SmemShape shape, mcgpu_trace* trace, int trace_off,
-                              int trace_stride, int lanes_cap);
-__global__ void k_chain_steps_wide(Pool P, int n_steps, unsigned* queue, const int* order,
-                                   int n_tasks, int gwarps, SmemShape shape, mcgpu_trace* trace,
-                                   int trace_off, int trace_stride, int lanes_cap);
+// One launch of the one-step chain kernels: n_steps steps of each task (task k
+// runs chain order[k] of sizes[k] molecules), seg at a time on a group of
+// gwarps warps; sched: n_tasks zeroed words.  trace: as mcgpu_batch_run_traced;
+// lanes_cap > 0 caps the lanes per neighbour molecule.
+struct ChainLaunch {
+  int n_steps, seg, n_tasks, gwarps;
+  unsigned* sched;
+  const int *order, *sizes;
+  SmemShape shape;
+  mcgpu_trace* trace = nullptr;
+  int trace_off = 0, trace_stride = 0, lanes_cap = 0;
+};
+__global__ void k_chain_steps(Pool P, ChainLaunch A);
+__global__ void k_chain_steps_wide(Pool P, ChainLaunch A);
 __global__ void k_chain_init(Pool P, const int* mol_chain, int m_begin, int m_end);
 __global__ void k_nl_config(Pool P, const NlCfg* cfg);
 cudaError_t launch_nl_rebuild(Pool P, const int* mol_chain, int n_mol, int max_cells,

@@ -14,6 +14,7 @@
 //                          Philox proposal, staging, screen, pairs, FP64
 //                          dE, decision and commit without leaving the GPU
 #include "chain.cuh"
+#include "host.h"
 #include "intra.h"
 #include "pairsum.cuh"
 
@@ -439,8 +440,68 @@ __global__ void k_chain_export(Pool P, const int* mol_chain, const int* atom_mol
   P.z[a] = x.z;
 }
 
-// Persistent kernel: groups of `gwarps` warps pull chain tasks from `queue`
-// (task k runs chain order[k]) and advance each by n_steps steps on the
+// The chain task with the most work left: warp 0 of a group looks through
+// sched (entry k: steps task k has taken, kChainBusy while a group runs it)
+// for the free task of the largest remaining steps x cost and claims it; -1
+// when every task is finished or running (each running task's group takes the
+// next one itself, so this group is not needed any more).  sizes: the tasks'
+// molecule counts, in one row so that a look through 512 tasks is 16
+// coalesced loads (from the chain headers it took 12 us).  Each group sees the
+// costs a few per cent apart from what the others see, or groups that look at
+// the same time would all reach for the same task.
+constexpr unsigned kChainBusy = 0x80000000u;
+
+__device__ __forceinline__ int claim_chain(const int* sizes, unsigned* sched, int n_tasks,
+                                           int n_steps, int group, bool start, int lane,
+                                           int* done) {
+  // at the start of a launch group k takes task k, so that the groups do not
+  // all reach for the same one
+  if (start && group < n_tasks) {
+    int won = 0;
+    if (lane == 0) won = atomicCAS(sched + group, 0u, kChainBusy) == 0u;
+    if (__shfl_sync(~0u, won, 0)) {
+      *done = 0;
+      return group;
+    }
+  }
+  for (;;) {
+    float best = 0.f;
+    int at = -1;
+    unsigned seen = 0;
+    for (int k = lane; k < n_tasks; k += 32) {
+      const unsigned v = *(volatile unsigned*)(sched + k);
+      if ((v & kChainBusy) || (int)v >= n_steps) continue;
+      // a step costs a fixed latency and its screen: about 4,096 molecules' worth
+      const unsigned mix = ((unsigned)k * 2654435761u) ^ ((unsigned)group * 2246822519u);
+      const float key = (float)(n_steps - (int)v) * (float)(4096 + sizes[k]) *
+                        (1.f + 1.4e-11f * (float)mix);
+      if (key > best) {
+        best = key;
+        at = k;
+        seen = v;
+      }
+    }
+    float top = best;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(~0u, top, off));
+    if (top == 0.f) return -1;
+    const int src = __ffs(__ballot_sync(~0u, best == top)) - 1;
+    int won = 0;
+    if (lane == src) won = atomicCAS(sched + at, seen, seen | kChainBusy) == seen;
+    if (__shfl_sync(~0u, won, src)) {
+      __threadfence();   // the rows the last group to run the task wrote
+      *done = (int)__shfl_sync(~0u, seen, src);
+      return __shfl_sync(~0u, at, src);
+    }
+  }
+}
+
+// Persistent kernel: groups of `gwarps` warps take chain tasks (task k runs
+// chain order[k]) for `seg` steps at a time, the one with the most work left
+// first, until each has taken n_steps; sched: n_tasks zeroed words.  With a
+// task per group for all its steps, 512 chains of uneven size on 456 groups
+// left the chip half idle in a second wave of 56 (SMs busy 77 % of a launch).
+// A task stays on one group at a time, and its steps on the
 // chain state.  A step: every warp screens its share of the candidates
 // against the move staged in FP32 during the previous step and evaluates
 // the in-range ones (FP32 pair terms, double-float sums); the last warp then
@@ -458,21 +519,31 @@ __global__ void k_chain_export(Pool P, const int* mol_chain, const int* atom_mol
 // shared memory; when a commit moves the molecule of the move staged next,
 // warp 0 stages it again (one more barrier).  lanes_cap > 0 caps the lanes
 // per neighbour molecule of every chain.
-__device__ __forceinline__ void chain_steps(Pool P, int n_steps, unsigned* queue,
-                                            const int* order, int n_tasks, int gwarps,
-                                            SmemShape shape, mcgpu_trace* trace, int trace_off,
-                                            int trace_stride, int lanes_cap, char* smem) {
+__device__ __forceinline__ void chain_steps(Pool P, const ChainLaunch& A, char* smem) {
+  const int n_steps = A.n_steps, seg = A.seg, n_tasks = A.n_tasks, gwarps = A.gwarps;
+  const SmemShape shape = A.shape;
+  mcgpu_trace* trace = A.trace;
   const int gsize = gwarps * 32;
   const int gid = threadIdx.x / gsize;
   Group g{(int)threadIdx.x - gid * gsize, gsize, 1 + gid};
   GroupSmem s = shape.carve(smem + gid * shape.bytes());
   const int lane = threadIdx.x & 31, w = g.warp(), nw = g.nwarps();
+  const int group = blockIdx.x * ((int)blockDim.x / gsize) + gid;
+  bool start = true;
   for (;;) {
-    if (g.tid == 0) s.misc[31] = (int)atomicAdd(queue, 1u);
+    if (w == 0) {
+      int taken = 0;
+      const int t = claim_chain(A.sizes, A.sched, n_tasks, n_steps, group, start, lane, &taken);
+      start = false;
+      if (lane == 0) {
+        s.misc[31] = t;
+        s.misc[30] = taken;
+      }
+    }
     g.sync();
-    const int task = s.misc[31];
-    if (task >= n_tasks) break;
-    const int c = order[task];
+    const int task = s.misc[31], base = s.misc[30];
+    if (task < 0) break;
+    const int c = A.order[task];
     ChainHdr* Hp = P.hdr + c;
     const ChainHdr& H = *Hp;
     float4* pcache = (s.pc && H.simple_prim && H.n_mol <= shape.cache_n) ? s.pc : nullptr;
@@ -498,12 +569,12 @@ __device__ __forceinline__ void chain_steps(Pool P, int n_steps, unsigned* queue
     // lanes per neighbour molecule: the cap, else one lane for a chain of
     // one species of at most 4 atoms (the single-lane pair batch), else the
     // power of two at or above its largest molecule
-    const int T = lanes_cap > 0 ? min(lanes_cap, H.tpm)
+    const int T = A.lanes_cap > 0 ? min(A.lanes_cap, H.tpm)
                                 : ((H.uniform && H.ulen <= 4 && !H.precise) ? 1 : H.tpm);
     MoveF* props = (MoveF*)s.props;
-    int my_steps = n_steps;
+    int my_steps = min(seg, n_steps - base);
     if (H.step_limit > 0)
-      my_steps = (int)max(0LL, min((long long)n_steps, H.step_limit - (long long)step0));
+      my_steps = (int)max(0LL, min((long long)my_steps, H.step_limit - (long long)step0));
     // step st's move is staged in slot st % 3 (the last warp stages step
     // st + 1 during step st; slot (st + 2) % 3 = (st - 1) % 3 is rewritten
     // only after every warp has passed step st's reduction barrier, so no
@@ -615,7 +686,7 @@ __device__ __forceinline__ void chain_steps(Pool P, int n_steps, unsigned* queue
           t.u = (double)u;
           t.fp64 = tie;
           t.pad0 = 0;
-          trace[(size_t)c * trace_stride + trace_off + st] = t;
+          trace[(size_t)c * A.trace_stride + A.trace_off + base + st] = t;
         }
       }
       // the next move was staged from rows this commit changes only if it
@@ -640,30 +711,24 @@ __device__ __forceinline__ void chain_steps(Pool P, int n_steps, unsigned* queue
       }
     }
     g.sync();
+    // give the task back: every thread's writes, then the steps taken
+    if (g.tid == 0) {
+      __threadfence();
+      atomicExch(A.sched + task, (unsigned)min(base + seg, n_steps));
+    }
   }
 }
 
-__global__ void __launch_bounds__(256, 2) k_chain_steps(Pool P, int n_steps, unsigned* queue,
-                                                     const int* order, int n_tasks, int gwarps,
-                                                     SmemShape shape, mcgpu_trace* trace,
-                                                     int trace_off, int trace_stride,
-                                                     int lanes_cap) {
+__global__ void __launch_bounds__(256, 2) k_chain_steps(Pool P, ChainLaunch A) {
   extern __shared__ __align__(16) char smem[];
-  chain_steps(P, n_steps, queue, order, n_tasks, gwarps, shape, trace, trace_off, trace_stride,
-              lanes_cap, smem);
+  chain_steps(P, A, smem);
 }
 
 // The same for one group of up to 16 warps per CTA (a single large chain:
 // more warps per step, one CTA per SM).
-__global__ void __launch_bounds__(512, 1) k_chain_steps_wide(Pool P, int n_steps,
-                                                          unsigned* queue, const int* order,
-                                                          int n_tasks, int gwarps,
-                                                          SmemShape shape, mcgpu_trace* trace,
-                                                          int trace_off, int trace_stride,
-                                                          int lanes_cap) {
+__global__ void __launch_bounds__(512, 1) k_chain_steps_wide(Pool P, ChainLaunch A) {
   extern __shared__ __align__(16) char smem[];
-  chain_steps(P, n_steps, queue, order, n_tasks, gwarps, shape, trace, trace_off, trace_stride,
-              lanes_cap, smem);
+  chain_steps(P, A, smem);
 }
 
 // ---- host launchers (template kernels are instantiated here) --------------

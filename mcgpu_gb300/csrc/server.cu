@@ -107,8 +107,9 @@ struct mcgpu_server {
   int gw = 8, grid = 1, smem = 0;
   SmemShape shape{};
   // device scratch
-  unsigned* qctr = nullptr;
-  int* dlist = nullptr;  // order [slots] | act_slot [slots] | act_m0 [slots] | act_pref [slots+1]
+  unsigned* sched = nullptr;   // steps each job has taken in a round (slots)
+  // order [slots] | act_slot [slots] | act_m0 [slots] | act_pref [slots+1] | sizes [slots]
+  int* dlist = nullptr;
   int* dinit = nullptr;  // per slot: (slot, m0, 0, n_mol) range of a job being initialised
   VolMove* vm = nullptr;
   double2* emol2 = nullptr;
@@ -159,8 +160,8 @@ int server_alloc(mcgpu_server* s) {
   dp.n_mol = (int)nm;
   dp.n_pidx = (int)np;
   dp.max_len = ml;
-  s->qctr = dalloc<unsigned>(1, &e);
-  s->dlist = dalloc<int>(4 * (size_t)nc + 1, &e);
+  s->sched = dalloc<unsigned>(nc, &e);
+  s->dlist = dalloc<int>(5 * (size_t)nc + 1, &e);
   s->dinit = dalloc<int>(4 * (size_t)nc, &e);
   s->vm = dalloc<VolMove>(nc, &e);
   s->emol2 = dalloc<double2>(nm, &e);
@@ -170,7 +171,7 @@ int server_alloc(mcgpu_server* s) {
   s->vlist = dalloc<int>(3 * (size_t)nc + 3, &e);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.hdr, 0, sizeof(ChainHdr) * nc, ctx->stream);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&s->hmirror, sizeof(ChainHdr) * nc);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&s->hlist, sizeof(int) * (4 * (size_t)nc + 1));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&s->hlist, sizeof(int) * (5 * (size_t)nc + 1));
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess)
     return set_err(ctx, MCGPU_ERR_NOMEM, "server arena allocation failed: %s", cudaGetErrorString(e));
@@ -179,7 +180,7 @@ int server_alloc(mcgpu_server* s) {
 
 void server_free(mcgpu_server* s) {
   s->pool.release();
-  void* d[] = {s->qctr, s->dlist, s->dinit, s->vm, s->emol2, s->eabs2, s->vsum, s->vsum_abs,
+  void* d[] = {s->sched, s->dlist, s->dinit, s->vm, s->emol2, s->eabs2, s->vsum, s->vsum_abs,
                s->vlist};
   for (void* p : d)
     if (p) cudaFree(p);
@@ -405,11 +406,13 @@ int launch_round(mcgpu_server* s) {
   int* aslot = s->hlist + nc;
   int* am0 = s->hlist + 2 * nc;
   int* apref = s->hlist + 3 * nc;
+  int* sizes = s->hlist + 4 * nc + 1;
   int n_npt = 0, total = 0;
   bool has64 = false, has32 = false;
   for (size_t i = 0; i < act.size(); i++) {
     order[i] = act[i];
     const Job* j = s->slot_job[act[i]];
+    sizes[i] = j->n_mol;
     if (!j->npt) continue;
     has64 = has64 || !j->vol_mixed;
     has32 = has32 || j->vol_mixed;
@@ -420,24 +423,25 @@ int launch_round(mcgpu_server* s) {
     n_npt++;
   }
   apref[n_npt] = total;
-  CK(ctx, cudaMemcpyAsync(s->dlist, s->hlist, sizeof(int) * (4 * (size_t)nc + 1),
+  CK(ctx, cudaMemcpyAsync(s->dlist, s->hlist, sizeof(int) * (5 * (size_t)nc + 1),
                           cudaMemcpyHostToDevice, st));
   if (s->copies_pending) {
     CK(ctx, cudaStreamWaitEvent(st, s->ev_copy, 0));
     s->copies_pending = false;
   }
   CK(ctx, cudaEventRecord(s->ev_t0, st));
-  CK(ctx, cudaMemsetAsync(s->qctr, 0, sizeof(unsigned), st));
+  CK(ctx, cudaMemsetAsync(s->sched, 0, sizeof(unsigned) * act.size(), st));
   const int need = ((int)act.size() + s->cfg.chains_per_cta - 1) / s->cfg.chains_per_cta;
   const int grid = std::max(1, std::min(need, s->grid));
+  // a job runs a whole round on one group: its energy sums must not depend on
+  // the other jobs
+  ChainLaunch A{s->cfg.round_steps, s->cfg.round_steps, (int)act.size(), s->gw, s->sched, s->dlist,
+                s->dlist + 4 * nc + 1, s->shape};
+  A.lanes_cap = s->cfg.lanes_per_molecule;
   if (s->cfg.threads > 256)
-    k_chain_steps_wide<<<grid, s->cfg.threads, s->smem, st>>>(s->pool.P, s->cfg.round_steps, s->qctr,
-                                                      s->dlist, (int)act.size(), s->gw, s->shape,
-                                                      nullptr, 0, 0, s->cfg.lanes_per_molecule);
+    k_chain_steps_wide<<<grid, s->cfg.threads, s->smem, st>>>(s->pool.P, A);
   else
-    k_chain_steps<<<grid, s->cfg.threads, s->smem, st>>>(s->pool.P, s->cfg.round_steps, s->qctr,
-                                                      s->dlist, (int)act.size(), s->gw, s->shape,
-                                                      nullptr, 0, 0, s->cfg.lanes_per_molecule);
+    k_chain_steps<<<grid, s->cfg.threads, s->smem, st>>>(s->pool.P, A);
   CK(ctx, cudaGetLastError());
   if (n_npt > 0) {
     MolRanges R;
