@@ -93,8 +93,6 @@ __device__ inline void stage_chain(const Pool& P, const ChainHdr& H, const MoveF
     const float3 on = mvec(R, t.x, t.y, t.z);
     s.o_old[i] = o;
     s.o_new[i] = make_float4(on.x, on.y, on.z, o.w);
-    s.l_old[i] = make_float4(0.f, 0.f, 0.f, 0.f);  // the chain state's offsets are exact
-    s.l_new[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     s.eq[i] = make_float4(qe.x, qe.y, fmaf(o.x, o.x, fmaf(o.y, o.y, o.z * o.z)),
                           fmaf(on.x, on.x, fmaf(on.y, on.y, on.z * on.z)));
     qsum += qe.y;
@@ -164,16 +162,6 @@ __device__ __forceinline__ int screen_chain(const Pool& P, const ChainHdr& H, co
   return f;
 }
 
-// The single-lane pair batch for the chain's molecule length.
-__device__ __forceinline__ void batch_u1_any(const Pool& P, const ChainHdr& H, const GroupSmem& s,
-                                             const MovedInfo& mi, const int* rj, int head,
-                                             int count, int w, int lane, AccFF& acc) {
-  if (H.ulen == 3)
-    batch_u3(P, H, s, mi, rj, head, count, lane, acc, H.ljmask);
-  else
-    batch_u1(P, H, s, mi, rj, head, count, w, lane, acc);
-}
-
 // Bits 4k + i: the LJ term between atoms i and k of a uniform chain's
 // molecules (at most 4 atoms) is not exactly zero (sigma and epsilon
 // products both nonzero in FP32).  The same for every lane.
@@ -189,14 +177,23 @@ __device__ __forceinline__ unsigned uniform_lj_mask(const Pool& P, const ChainHd
   return m;
 }
 
-// One warp screens chain candidates [c_begin, c_end) -- or, with a Verlet
-// list, the molecules cand[c_begin .. c_end) -- in warp-strided rounds of 32
-// (screen positions from the shared-memory cache when given) and evaluates
-// the in-range ones in batches of 32.
-__device__ inline void warp_eval_chain(const Pool& P, const ChainHdr& H, const GroupSmem& s,
-                                const MovedInfo& mi, const float4* pcache, int c_begin, int c_end,
-                                int w, int nw, int lane, int T, AccFF& acc,
-                                const int* cand = nullptr) {
+// The group evaluates both placements of the staged move over chain candidates
+// [c_begin, c_end) -- or, with a Verlet list, the molecules cand[c_begin ..
+// c_end).  Every warp screens its share in rounds of 32 (screen positions from
+// the shared-memory cache when given) into its ring.  A chain of one species
+// then shares the in-range neighbours of all warps out to the threads of the
+// first `workers` warps as items (one more barrier): every warp waited for the
+// one with most (4,000 16-atom molecules on 16 warps: 45 neighbours, 3 +- 2 a
+// warp, 29,000 cycles a step).  Other chains evaluate their own rings in
+// batches of 32, T lanes per neighbour molecule -- and so do chains of 3-site
+// molecules, a lane per placement: there the extra barrier costs what the
+// balance gains (512 water chains: 14.2 ms either way on 256 threads, 14.0
+// against 16.5 on 160).
+__device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const Group& g,
+                                        const GroupSmem& s, const MovedInfo& mi,
+                                        const float4* pcache, int c_begin, int c_end, int workers,
+                                        int T, AccFF& acc, const int* cand = nullptr) {
+  const int lane = g.tid & 31, w = g.warp(), nw = g.nwarps();
   int* rj = s.lj + w * kRing;
   int head = 0, tail = 0;
   const unsigned lt = lanemask_lt();
@@ -204,7 +201,9 @@ __device__ inline void warp_eval_chain(const Pool& P, const ChainHdr& H, const G
   // (short, in cell order): warp w takes every nw-th entry, so every warp
   // gets its share of the in-range neighbours
   const int rounds = cand ? (c_end - c_begin + 32 * nw - 1) / (32 * nw) : 0;
-  const bool u1 = H.uniform && T == 1 && H.ulen <= 4 && !H.precise;
+  const bool precise = H.precise != 0;
+  const bool u3 = H.uniform && H.ulen == 3 && !precise, shared = H.uniform && !u3;
+  const unsigned ljmask = H.ljmask;
   // one primary each (the common chain): the moved molecule's two placements
   // and the screen's constants in registers -- the header is global memory,
   // and the ring's stores would have it read again every round
@@ -212,61 +211,109 @@ __device__ inline void warp_eval_chain(const Pool& P, const ChainHdr& H, const G
   const float Lx = H.Lf[0], Ly = H.Lf[1], Lz = H.Lf[2], lo = H.cut2_lo, hi = H.cut2_hi;
   const float4 po = s.p_old[0], pn = s.p_new[0];
   const int mol0 = H.mol0, pidx0 = H.pidx0;
-  for (int it = 0;; it++) {
-    int idx;
-    if (cand) {
-      if (it >= rounds) break;
-      idx = c_begin + (it * 32 + lane) * nw + w;
-    } else {
-      const int base = c_begin + w * 32 + it * nw * 32;
-      if (base >= c_end) break;
-      idx = base + lane;
-    }
-    const int j = (cand && idx < c_end) ? cand[idx] : idx;
-    int f = 0;
-    if (idx < c_end && j != mi.mol) {
-      if (single) {
-        const float4 q0 = pcache ? pcache[j - mol0] : P.ppos[pidx0 + (j - mol0)];
-        const float ox = wrapf(q0.x - po.x, Lx), oy = wrapf(q0.y - po.y, Ly),
-                    oz = wrapf(q0.z - po.z, Lz);
-        const float nx = wrapf(q0.x - pn.x, Lx), ny = wrapf(q0.y - pn.y, Ly),
-                    nz = wrapf(q0.z - pn.z, Lz);
-        const float ro = fmaf(ox, ox, fmaf(oy, oy, oz * oz));
-        const float rn = fmaf(nx, nx, fmaf(ny, ny, nz * nz));
-        f = (ro <= lo ? kInOld : 0) | (rn <= lo ? kInNew : 0);
-        if ((ro > lo && ro <= hi) || (rn > lo && rn <= hi))
-          f = screen_chain(P, H, s, mi, j, q0);   // inside the guard band
+  for (int it = 0;;) {
+    // rounds of the screen until they end or the ring holds a batch (a shared
+    // one waits for the other warps' with up to 32 entries)
+    bool more = false;
+    for (;; it++) {
+      int idx;
+      if (cand) {
+        if (it >= rounds) break;
+        idx = c_begin + (it * 32 + lane) * nw + w;
       } else {
-        const float4 q0 = pcache ? pcache[j - mol0]
-                                 : P.ppos[H.simple_prim ? pidx0 + (j - mol0) : P.mpi[j].x];
-        f = screen_chain(P, H, s, mi, j, q0);
+        const int base = c_begin + w * 32 + it * nw * 32;
+        if (base >= c_end) break;
+        idx = base + lane;
       }
+      if (tail - head > (shared ? 32 : 31)) {
+        more = true;
+        break;
+      }
+      const int j = (cand && idx < c_end) ? cand[idx] : idx;
+      int f = 0;
+      if (idx < c_end && j != mi.mol) {
+        if (single) {
+          const float4 q0 = pcache ? pcache[j - mol0] : P.ppos[pidx0 + (j - mol0)];
+          const float ox = wrapf(q0.x - po.x, Lx), oy = wrapf(q0.y - po.y, Ly),
+                      oz = wrapf(q0.z - po.z, Lz);
+          const float nx = wrapf(q0.x - pn.x, Lx), ny = wrapf(q0.y - pn.y, Ly),
+                      nz = wrapf(q0.z - pn.z, Lz);
+          const float ro = fmaf(ox, ox, fmaf(oy, oy, oz * oz));
+          const float rn = fmaf(nx, nx, fmaf(ny, ny, nz * nz));
+          f = (ro <= lo ? kInOld : 0) | (rn <= lo ? kInNew : 0);
+          if ((ro > lo && ro <= hi) || (rn > lo && rn <= hi))
+            f = screen_chain(P, H, s, mi, j, q0);   // inside the guard band
+        } else {
+          const float4 q0 = pcache ? pcache[j - mol0]
+                                   : P.ppos[H.simple_prim ? pidx0 + (j - mol0) : P.mpi[j].x];
+          f = screen_chain(P, H, s, mi, j, q0);
+        }
+      }
+      const unsigned bal = __ballot_sync(~0u, f != 0);
+      if (f) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 4) | f;
+      tail += __popc(bal);
+      if (shared) acc.np += __popc(f);
     }
-    const unsigned bal = __ballot_sync(~0u, f != 0);
-    if (f) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 4) | f;
-    tail += __popc(bal);
-    if (tail - head >= 32) {
+    __syncwarp();
+    if (!shared) {
+      const int count = min(32, tail - head);
+      if (count > 0) {
+        if (u3)
+          batch_u3(P, H, s, mi, rj, head, count, lane, acc, ljmask);
+        else if (precise)
+          batch_ff<true, false>(P, H, s, mi, rj, head, count, lane, T, acc);
+        else
+          batch_ff<false, false>(P, H, s, mi, rj, head, count, lane, T, acc);
+        head += count;
+      }
       __syncwarp();
-      if (u1)
-        batch_u1_any(P, H, s, mi, rj, head, 32, w, lane, acc);
-      else if (H.precise)
-        batch_ff<true, false>(P, H, s, mi, rj, head, 32, lane, T, acc);
-      else
-        batch_ff<false, false>(P, H, s, mi, rj, head, 32, lane, T, acc);
-      head += 32;
-      __syncwarp();
+      if (!more && tail == head) return;
+      continue;
     }
-  }
-  __syncwarp();
-  if (tail > head) {
-    if (u1)
-      batch_u1_any(P, H, s, mi, rj, head, tail - head, w, lane, acc);
-    else if (H.precise)
-      batch_ff<true, false>(P, H, s, mi, rj, head, tail - head, lane, T, acc);
+    // entry e of the items: in the ring of the last warp q with pref <= e
+    // (lane q of every warp holds q's ring head and pref, the entries before)
+    int count = 32, tid = lane, threads = 32;
+    const int k = lane & 15;
+    int pref = k <= w ? 0 : 0x40000000, hd = head;   // this warp's own ring
+    if (!more) {
+      acc.np *= mi.act * H.uact;
+      if (lane == 0) {
+        s.hits[w] = tail - head;
+        s.hits[16 + w] = head;
+      }
+      g.sync();
+      if (w >= workers) return;
+      const int cnt = k < nw ? s.hits[k] : 0;
+      hd = s.hits[16 + k];
+      pref = cnt;
+#pragma unroll
+      for (int off = 1; off < 16; off <<= 1) {
+        const int v = __shfl_up_sync(~0u, pref, off, 16);
+        if (k >= off) pref += v;
+      }
+      count = __shfl_sync(~0u, pref, 15);
+      pref -= cnt;
+      tid = g.tid;
+      threads = 32 * workers;
+    }
+    auto entry = [&](int e) {
+      int q = 0;
+#pragma unroll
+      for (int step = 8; step > 0; step >>= 1) {
+        const int v = __shfl_sync(~0u, pref, q + step);
+        if (q + step < nw && v <= e) q += step;
+      }
+      const int at = __shfl_sync(~0u, hd, q) + e - __shfl_sync(~0u, pref, q);
+      return s.lj[q * kRing + (at & (kRing - 1))];
+    };
+    if (precise)
+      uniform_items<true>(P, H, s, mi, count, tid, threads, acc, entry);
     else
-      batch_ff<false, false>(P, H, s, mi, rj, head, tail - head, lane, T, acc);
+      uniform_items<false>(P, H, s, mi, count, tid, threads, acc, entry);
+    if (!more) return;
+    head += 32;
+    __syncwarp();
   }
-  __syncwarp();
 }
 
 // Group-wide deterministic double-float sum, the same in every thread.  After

@@ -442,37 +442,32 @@ struct GroupSmem {
   int* pa;                              // primary atom slots in the molecule [kMaxP]
   // per-warp neighbour rings [nwarps * kRing]
   int* lj;                              // (j << 4) | flags
-  float4* lA;                           // (Dold.xyz, Dnew.x)
-  float2* lB;                           // (Dnew.y, Dnew.z)
+  int* hits;                            // [2 * 16] per warp: entries left in its ring, their head
   double* red;                          // [2][3 * nwarps] reduction scratch (two buffers)
   long long* redl;                      // [2][nwarps]
   int* misc;                            // [32] broadcast ints
-  double* miscd;                        // [32] broadcast doubles
   float4* pc;                           // [cache_n] screen positions of the chain (or null)
   void* props;                          // [32] drawn moves of the next steps (chain kernel)
-  float4* nbuf;                         // [nwarps * 32 * 5] per-lane neighbour rows (async copies)
   float2* teq;                          // [maxA] pair factors per slot of a uniform chain
   char* ahead;                          // three more staging slots (the chain kernel's moves)
 };
 
 // The rows a staged move occupies: offsets, pair factors, primaries, the
-// broadcast ints and doubles: the ones inside GroupSmem, and three more the
+// broadcast ints: the ones inside GroupSmem, and three more the
 // chain kernel rotates through (a step's move, the next one staged ahead,
 // and the one before, which slower warps may still be committing).
 struct StageSlot {
   float4* o_old; float4* o_new;
-  float4* l_old; float4* l_new;
   float4* eq;
   float4* p_old; float4* p_new;
   int* pa;
   int* misc;
-  double* miscd;
 };
 
 // s with its staging rows replaced by slot t's.
 __device__ __forceinline__ GroupSmem with_slot(GroupSmem s, const StageSlot& t) {
-  s.o_old = t.o_old; s.o_new = t.o_new; s.l_old = t.l_old; s.l_new = t.l_new; s.eq = t.eq;
-  s.p_old = t.p_old; s.p_new = t.p_new; s.pa = t.pa; s.misc = t.misc; s.miscd = t.miscd;
+  s.o_old = t.o_old; s.o_new = t.o_new; s.eq = t.eq;
+  s.p_old = t.p_old; s.p_new = t.p_new; s.pa = t.pa; s.misc = t.misc;
   return s;
 }
 
@@ -487,32 +482,27 @@ struct SmemShape {
     b += align16(2 * kMaxP * 16);
     b += align16(kMaxP * 4);
     b += align16(nwarps * kRing * 4);
-    b += align16(nwarps * kRing * 16);
-    b += align16(nwarps * kRing * 8);
+    b += align16(2 * 16 * 4);
     b += align16(6 * nwarps * 8);
     b += align16(2 * nwarps * 8);
     b += align16(32 * 4);
-    b += align16(32 * 8);
     b += align16(cache_n * 16);
     b += align16(32 * kPropBytes);
-    b += align16(nwarps * 32 * 5 * 16);
     b += align16(maxA * 8);
     b += 3 * ahead_bytes();
     return b;
   }
-  // the second staging slot: offsets and factors, primaries, misc, miscd
+  // a staging slot: offsets and factors, primaries, misc
   __host__ __device__ int ahead_bytes() const {
-    return align16(5 * maxA * 16) + align16(2 * kMaxP * 16) + align16(kMaxP * 4) + align16(32 * 4) +
-           align16(32 * 8);
+    return align16(3 * maxA * 16) + align16(2 * kMaxP * 16) + align16(kMaxP * 4) + align16(32 * 4);
   }
   __device__ StageSlot ahead_slot(char* p) const {
     StageSlot t;
-    t.o_old = (float4*)p; t.o_new = t.o_old + maxA; t.l_old = t.o_new + maxA;
-    t.l_new = t.l_old + maxA; t.eq = t.l_new + maxA; p += align16(5 * maxA * 16);
+    t.o_old = (float4*)p; t.o_new = t.o_old + maxA; t.eq = t.o_new + maxA;
+    p += align16(3 * maxA * 16);
     t.p_old = (float4*)p; t.p_new = t.p_old + kMaxP; p += align16(2 * kMaxP * 16);
     t.pa = (int*)p; p += align16(kMaxP * 4);
-    t.misc = (int*)p; p += align16(32 * 4);
-    t.miscd = (double*)p;
+    t.misc = (int*)p;
     return t;
   }
   __device__ GroupSmem carve(char* base) const {
@@ -528,18 +518,14 @@ struct SmemShape {
     s.p_old = (float4*)p; s.p_new = s.p_old + kMaxP; p += align16(2 * kMaxP * 16);
     s.pa = (int*)p; p += align16(kMaxP * 4);
     s.lj = (int*)p; p += align16(nwarps * kRing * 4);
-    s.lA = (float4*)p; p += align16(nwarps * kRing * 16);
-    s.lB = (float2*)p; p += align16(nwarps * kRing * 8);
+    s.hits = (int*)p; p += align16(2 * 16 * 4);
     s.red = (double*)p; p += align16(6 * nwarps * 8);
     s.redl = (long long*)p; p += align16(2 * nwarps * 8);
     s.misc = (int*)p; p += align16(32 * 4);
-    s.miscd = (double*)p; p += align16(32 * 8);
     s.pc = cache_n > 0 ? (float4*)p : nullptr;
     p += align16(cache_n * 16);
     s.props = (void*)p;
     p += align16(32 * kPropBytes);
-    s.nbuf = (float4*)p;
-    p += align16(nwarps * 32 * 5 * 16);
     s.teq = (float2*)p;
     p += align16(maxA * 8);
     s.ahead = p;

@@ -588,6 +588,9 @@ __device__ __forceinline__ void chain_steps(Pool P, const ChainLaunch& A, char* 
                                     P.mlen + H.mol0, (float)H.max_t, (float)H.max_r, H.rot_mode);
       __syncwarp();
     };
+    // the last warp stages the next move while the others take the items (it
+    // takes its share of them in groups of fewer than four warps)
+    const int workers = nw >= 4 ? nw - 1 : nw;
     if (w == 0 && my_steps > 0) {
       draw32(0);
       stage_chain(P, H, props[0], slot(0), pcache, lane);
@@ -608,10 +611,10 @@ __device__ __forceinline__ void chain_steps(Pool P, const ChainLaunch& A, char* 
       const bool f64all = H.fp64_pairs != 0;
       if (f64all) {
       } else if (use_list)
-        warp_eval_chain(P, H, ss, mi, pcache, 0, P.nl_cnt[mi.mol], w, nw, lane, T, acc,
+        group_eval_chain(P, H, g, ss, mi, pcache, 0, P.nl_cnt[mi.mol], workers, T, acc,
                         P.nl + (size_t)mi.mol * P.nl_stride);
       else
-        warp_eval_chain(P, H, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, w, nw, lane, T, acc);
+        group_eval_chain(P, H, g, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, workers, T, acc);
       // the last warp (with the fewest screen blocks) stages the next move
       // while the others finish their share
       if (w == nw - 1 && st + 1 < my_steps) {

@@ -94,7 +94,7 @@ enum : int { kMiscRad = 21, kMiscQm = 22 };
 // non-vertex atom rotated about the vertex and translated, the vertex
 // translated, then the molecule wrapped by its first primary atom
 // (keepMoleculeInBox, :710-729).  Results go to shared memory; scalars to
-// misc/miscd.  The caller synchronises the group afterwards.
+// misc.  The caller synchronises the group afterwards.
 __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Proposal* p,
                       const GroupSmem& s, int lane) {
   const int a0 = P.mstart[m];
@@ -261,10 +261,15 @@ struct AccFF {
 
 // Displacement of a pair, atom b of the neighbour minus atom a of the moved
 // molecule, both anchor-relative to the moved molecule's anchor.  PRECISE
-// adds the low parts (bl: of b = D + o_b; la: of a's offset) so the only
-// rounding left is the final one at the displacement's own magnitude.
-template <bool PRECISE>
-__device__ __forceinline__ float3 pair_disp(float3 bh, float3 bl, float4 a, float4 la) {
+// adds the low parts (bl: of b = D + o_b; la, with LO: of a's offset -- the
+// chain state's offsets have none) so the only rounding left is the final
+// one at the displacement's own magnitude.
+template <bool PRECISE, bool LO>
+__device__ __forceinline__ float3 pair_disp(float3 bh, float3 bl, float4 a, const float4* lo,
+                                            int i) {
+  if (PRECISE && !LO)
+    return make_float3((bh.x - a.x) + bl.x, (bh.y - a.y) + bl.y, (bh.z - a.z) + bl.z);
+  const float4 la = PRECISE ? lo[i] : a;
   if (PRECISE)
     return make_float3((bh.x - a.x) + (bl.x - la.x), (bh.y - a.y) + (bl.y - la.y),
                        (bh.z - a.z) + (bl.z - la.z));
@@ -280,7 +285,7 @@ __device__ __forceinline__ float3 pair_disp(float3 bh, float3 bl, float4 a, floa
 // ljmask clear means the LJ term of moved atom i is exactly zero (a sigma or
 // epsilon product of zero) and is not evaluated.  NLEN == 0 (any length up
 // to 64) ignores ljmask.  Neither changes a bit of the sum.
-template <bool PRECISE, int NLEN = 0>
+template <bool PRECISE, bool LO, int NLEN = 0>
 __device__ __forceinline__ float sum_moved32_wrap(const float4* o, const float4* lo,
                                                   const float4* eq, int len, float3 bh, float3 bl,
                                                   float sb, float2 qb, const ChainHdr& H,
@@ -289,7 +294,7 @@ __device__ __forceinline__ float sum_moved32_wrap(const float4* o, const float4*
   auto term = [&](int i) {
     const float4 ea = eq[i];
     const float4 a = o[i];
-    const float3 d = pair_disp<PRECISE>(bh, bl, a, PRECISE ? lo[i] : a);
+    const float3 d = pair_disp<PRECISE, LO>(bh, bl, a, lo, i);
     const float dx = wrapf(d.x, H.Lf[0]);
     const float dy = wrapf(d.y, H.Lf[1]);
     const float dz = wrapf(d.z, H.Lf[2]);
@@ -319,7 +324,7 @@ __device__ __forceinline__ float sum_moved32_wrap(const float4* o, const float4*
 // proportionally less FP32 rounding.  A coincident pair (r = 0) is skipped
 // as the reference skips it (BruteForceStep.cpp:68-69).  use_new selects the
 // |o_a|^2 of the placement (eq.z old, eq.w new).
-template <bool PRECISE, int NLEN = 0>
+template <bool PRECISE, bool LO, int NLEN = 0>
 __device__ __forceinline__ float sum_moved32_cf(const float4* o, const float4* lo,
                                                 const float4* eq, int len, bool use_new,
                                                 float3 bh, float3 bl, float sb, float2 qb,
@@ -332,7 +337,7 @@ __device__ __forceinline__ float sum_moved32_cf(const float4* o, const float4* l
   auto term = [&](int i) {
     const float4 a = o[i];
     const float4 ea = eq[i];
-    const float3 d = pair_disp<PRECISE>(bh, bl, a, PRECISE ? lo[i] : a);
+    const float3 d = pair_disp<PRECISE, LO>(bh, bl, a, lo, i);
     const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
     const float ir = rsqrt_nr(r2);
     const float lj = (NLEN == 0 || ((ljmask >> i) & 1u)) ? lj32(rcp_nr(r2), a.w, sb, ea.x, qb.x)
@@ -418,8 +423,8 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
           bl = make_float3(ex + (Dol.x + obl.x), ey + (Dol.y + obl.y), ez + (Dol.z + obl.z));
         }
         so += (f & kWrapOld)
-                  ? sum_moved32_wrap<PRECISE>(s.o_old, s.l_old, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
-                  : sum_moved32_cf<PRECISE>(s.o_old, s.l_old, s.eq, mi.len, false, bh, bl, ob.w, qb,
+                  ? sum_moved32_wrap<PRECISE, LO>(s.o_old, s.l_old, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
+                  : sum_moved32_cf<PRECISE, LO>(s.o_old, s.l_old, s.eq, mi.len, false, bh, bl, ob.w, qb,
                                             mi.qm, sa);
       }
       if (f & kInNew) {
@@ -431,8 +436,8 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
           bl = make_float3(ex + (Dnl.x + obl.x), ey + (Dnl.y + obl.y), ez + (Dnl.z + obl.z));
         }
         sn += (f & kWrapNew)
-                  ? sum_moved32_wrap<PRECISE>(s.o_new, s.l_new, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
-                  : sum_moved32_cf<PRECISE>(s.o_new, s.l_new, s.eq, mi.len, true, bh, bl, ob.w, qb,
+                  ? sum_moved32_wrap<PRECISE, LO>(s.o_new, s.l_new, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
+                  : sum_moved32_cf<PRECISE, LO>(s.o_new, s.l_new, s.eq, mi.len, true, bh, bl, ob.w, qb,
                                             mi.qm, sa);
       }
     }
@@ -455,75 +460,14 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
   }
 }
 
-// Asynchronous global -> shared copies (cp.async): the data lands in shared
-// memory without passing through registers; each thread waits for its own.
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// batch_ff with one lane per entry (T = 1) for a uniform chain of molecules
-// of at most 4 atoms: the entry's anchor and atom offsets follow from the
-// neighbour index, so each lane requests all of them at once with async
-// copies into its own shared-memory slot (one round trip to L2 instead of
-// one per atom, no registers held), and the pair factors come from the
-// chain's per-slot template.  Each placement's sum is batch_ff's bit for bit.
-// Both placements run through one copy of the pair code (a rolled loop),
-// which keeps the step loop's code small enough for the instruction cache.
-__device__ __forceinline__ void batch_u1(const Pool& P, const ChainHdr& H, const GroupSmem& s,
-                                         const MovedInfo& mi, const int* rj, int head, int count,
-                                         int w, int lane, AccFF& acc) {
-  if (lane >= count) return;  // lanes are independent: no shuffles below
-  const int jf = rj[(head + lane) & (kRing - 1)];
-  const int j = jf >> 4;
-  const int f = jf & 15;
-  const int lenj = H.ulen;
-  const int b0 = H.atom0 + (j - H.mol0) * lenj;
-  float4* nb = s.nbuf + (w * 32 + lane) * 5;
-  cp_async16(nb + 4, P.mfix + j);
-  for (int k = 0; k < lenj; k++) cp_async16(nb + k, P.aoff + b0 + k);
-  cp_async_wait_all();
-  const uint4 fj = *reinterpret_cast<const uint4*>(nb + 4);
-  const float rr = mi.rad + H.umrad;
-  const float3 z3 = make_float3(0.f, 0.f, 0.f);
-  float sa = 0.f;
-#pragma unroll 1
-  for (int p = 0; p < 2; p++) {
-    if (!(f & (p ? kInNew : kInOld))) continue;
-    const float3 D = fixdiff(fj, p ? mi.fx_new : mi.fx_old, H);
-    const bool wrap = needs_wrap(D, rr, H);
-    const float4* o = p ? s.o_new : s.o_old;
-    float sp = 0.f;
-#pragma unroll 1
-    for (int k = 0; k < lenj; k++) {
-      const float4 ob = nb[k];
-      const float2 qb = s.teq[k];
-      const float3 bh = make_float3(D.x + ob.x, D.y + ob.y, D.z + ob.z);
-      sp += wrap ? sum_moved32_wrap<false>(o, s.l_old, s.eq, mi.len, bh, z3, ob.w, qb, H, sa)
-                 : sum_moved32_cf<false>(o, s.l_old, s.eq, mi.len, p != 0, bh, z3, ob.w, qb,
-                                         mi.qm, sa);
-    }
-    if (p)
-      ff_add(acc.nh, acc.nl, sp);
-    else
-      ff_add(acc.oh, acc.ol, sp);
-    acc.np += (long long)mi.act * H.uact;
-  }
-  acc.ab += sa;
-}
-
-// batch_u1 for molecules of 3 atoms, one lane per (entry, placement): a batch
-// of at most 16 entries then takes one round of 9 pair terms instead of 18
-// (a warp's share of the in-range neighbours is about 15 to 20, so a lane per
-// entry left half the lanes idle for twice the time).  The header's scales
-// and the moved atoms go to registers once per round, the neighbour's rows
-// come with four independent loads (one round trip).  ljmask bits 4k + i: the
-// LJ term of neighbour atom k with moved atom i is not exactly zero (the same
-// in every lane: the chain is uniform).  Each placement's sum is batch_ff's
-// bit for bit.
+// batch_ff for a uniform chain of molecules of 3 atoms, one lane per (entry,
+// placement): a batch of at most 16 entries takes one round of 9 pair terms (a
+// warp's share of the in-range neighbours is about 15 to 20, so a lane per
+// entry left half the lanes idle for twice the time).  Rows and factors follow
+// from the neighbour's index, and the four rows are requested together (one
+// round trip to L2).  ljmask bits 4k + i: the LJ term of neighbour atom k with
+// moved atom i is not exactly zero (the same in every lane).  Each placement's
+// sum is batch_ff's bit for bit.
 __device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                          const MovedInfo& mi, const int* rj, int head, int count,
                                          int lane, AccFF& acc, unsigned ljmask) {
@@ -557,19 +501,19 @@ __device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const
 #pragma unroll 1
       for (int k = 0; k < 3; k++) {
         const float4 b = k == 0 ? ob[0] : k == 1 ? ob[1] : ob[2];
-        sp += sum_moved32_wrap<false, 3>(o, s.l_old, s.eq, 3,
-                                         make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
-                                         make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], H, sa,
-                                         (ljmask >> (4 * k)) & 15u);
+        sp += sum_moved32_wrap<false, false, 3>(o, nullptr, s.eq, 3,
+                                                make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
+                                                make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], H, sa,
+                                                (ljmask >> (4 * k)) & 15u);
       }
     } else {
 #pragma unroll 1
       for (int k = 0; k < 3; k++) {
         const float4 b = k == 0 ? ob[0] : k == 1 ? ob[1] : ob[2];
-        sp += sum_moved32_cf<false, 3>(o, s.l_old, s.eq, 3, p,
-                                       make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
-                                       make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], mi.qm, sa,
-                                       (ljmask >> (4 * k)) & 15u);
+        sp += sum_moved32_cf<false, false, 3>(o, nullptr, s.eq, 3, p,
+                                              make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
+                                              make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], mi.qm,
+                                              sa, (ljmask >> (4 * k)) & 15u);
       }
     }
     if (p)
@@ -578,6 +522,52 @@ __device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const
       ff_add(acc.oh, acc.ol, sp);
     acc.ab += sa;
     acc.np += pairs;
+  }
+}
+
+// This thread's items (tid, tid + nthreads, ...) of a uniform chain's `count`
+// entries that entry(e) gives (called by every lane of the warp): one atom of
+// the neighbour against one placement of the moved molecule.  Items run atom
+// by atom and placement by placement; rows and factors follow from the
+// neighbour's index.
+template <bool PRECISE, class Entry>
+__device__ __forceinline__ void uniform_items(const Pool& P, const ChainHdr& H, const GroupSmem& s,
+                                              const MovedInfo& mi, int count, int tid,
+                                              int nthreads, AccFF& acc, Entry entry) {
+  const int ulen = H.ulen, units = 2 * count, items = units * ulen;
+  const float rr = mi.rad + H.umrad;
+  for (int base = tid & ~31; base < items; base += nthreads) {
+    const int it = base + (tid & 31);
+    const int k = it / units, u = it - k * units;
+    const bool p = u >= count;
+    const int jf = entry(p ? u - count : u);
+    if (it >= items || !(jf & (p ? kInNew : kInOld))) continue;
+    const int j = jf >> 4;
+    const uint4 fj = P.mfix[j];
+    const float4 b = P.aoff[H.atom0 + (j - H.mol0) * ulen + k];
+    const float2 qb = s.teq[k];
+    const uint4 fm = p ? mi.fx_new : mi.fx_old;
+    float3 D, bl = make_float3(0.f, 0.f, 0.f);
+    if (PRECISE) fixdiff_ff(fj, fm, H, D, bl); else D = fixdiff(fj, fm, H);
+    const float3 bh = make_float3(D.x + b.x, D.y + b.y, D.z + b.z);
+    if (PRECISE) {
+      // two-sum of D + o_b per axis, then the low part
+      bl.x += (D.x - (bh.x - (bh.x - D.x))) + (b.x - (bh.x - D.x));
+      bl.y += (D.y - (bh.y - (bh.y - D.y))) + (b.y - (bh.y - D.y));
+      bl.z += (D.z - (bh.z - (bh.z - D.z))) + (b.z - (bh.z - D.z));
+    }
+    const float4* o = p ? s.o_new : s.o_old;
+    float sa = 0.f;
+    const float sp =
+        needs_wrap(D, rr, H)
+            ? sum_moved32_wrap<PRECISE, false>(o, nullptr, s.eq, mi.len, bh, bl, b.w, qb, H, sa)
+            : sum_moved32_cf<PRECISE, false>(o, nullptr, s.eq, mi.len, p, bh, bl, b.w, qb, mi.qm,
+                                             sa);
+    if (p)
+      ff_add(acc.nh, acc.nl, sp);
+    else
+      ff_add(acc.oh, acc.ol, sp);
+    acc.ab += sa;
   }
 }
 

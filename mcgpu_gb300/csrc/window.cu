@@ -211,10 +211,10 @@ __device__ void window_eval(const Pool& P, const ChainHdr& H, const Group& g, co
   const bool f64all = H.fp64_pairs != 0;
   if (f64all) {
   } else if (use_list) {
-    warp_eval_chain(P, H, ss, mi, pcache, 0, P.nl_cnt[mi.mol], w, nw, lane, T, acc,
-                    P.nl + (size_t)mi.mol * P.nl_stride);
+    group_eval_chain(P, H, g, ss, mi, pcache, 0, P.nl_cnt[mi.mol], nw, T, acc,
+                     P.nl + (size_t)mi.mol * P.nl_stride);
   } else {
-    warp_eval_chain(P, H, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, w, nw, lane, T, acc);
+    group_eval_chain(P, H, g, ss, mi, pcache, H.mol0, H.mol0 + H.n_mol, nw, T, acc);
   }
   group_reduce_ff(g, ss, acc, nred++ & 1);
   const float de_f = __fadd_rn(__fsub_rn(acc.nh, acc.oh), __fsub_rn(acc.nl, acc.ol));
