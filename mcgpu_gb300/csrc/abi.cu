@@ -439,7 +439,7 @@ int pool_set_verlet(mcgpu_ctx* ctx, DevPool& dp, double skin, cudaStream_t st) {
 
 int pool_nl_rebuild(mcgpu_ctx* ctx, DevPool& dp, cudaStream_t st) {
   if (!dp.nl_on) return MCGPU_OK;
-  CK(ctx, launch_nl_rebuild(dp.P, dp.mol_chain, dp.n_mol, dp.nl_max_cells, st));
+  CK(ctx, launch_nl_rebuild(dp.P, dp.nl_max_cells, st));
   return MCGPU_OK;
 }
 
@@ -1432,7 +1432,7 @@ extern "C" int mcgpu_chain_run(mcgpu_box* b, uint64_t seed, uint32_t chain_id, i
     const int k = std::min(seg, n_steps - done);
     int rc = pool_nl_rebuild(ctx, dp, st);
     if (rc) return rc;
-    CK(ctx, cudaMemsetAsync(b->queue, 0, sizeof(unsigned), st));
+    if (K == 1) CK(ctx, cudaMemsetAsync(b->queue, 0, sizeof(unsigned), st));
     Pool P = dp.P;
     P.trace = nullptr;
     if (K > 1)

@@ -95,7 +95,7 @@ struct __align__(16) ChainHdr {
   int vol_mixed;        // volume moves with FP32 pairs (FP64 re-take near threshold)
   int vol_fp64;         // volume decisions re-taken with FP64 pairs
   int vncell[3];        // cells per edge of the volume move in flight
-  int pad8;
+  int nl_done;          // CTAs of a list build that are done (0 between builds)
   // uniform chain: one species (every molecule ulen atoms, uact active, the
   // same parameters slot by slot) laid out contiguously from atom0, one
   // primary at slot uprim, radius <= umrad: atom and primary indexes and

@@ -39,8 +39,7 @@ __global__ void k_chain_steps(Pool P, ChainLaunch A);
 __global__ void k_chain_steps_wide(Pool P, ChainLaunch A);
 __global__ void k_chain_init(Pool P, const int* mol_chain, int m_begin, int m_end);
 __global__ void k_nl_config(Pool P, const NlCfg* cfg);
-cudaError_t launch_nl_rebuild(Pool P, const int* mol_chain, int n_mol, int max_cells,
-                              cudaStream_t st);
+cudaError_t launch_nl_rebuild(Pool P, int max_cells, cudaStream_t st);
 __global__ void k_chain_export(Pool P, const int* mol_chain, const int* atom_mol, int a_begin,
                                int a_end);
 cudaError_t launch_mol_energy(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,

@@ -18,18 +18,36 @@
 // members are sorted by index and each list is written cell by cell in a
 // fixed stencil order, so the lists (and the pair summation order that
 // follows them) are deterministic.
+//
+// Two launches: the cells of a chain by one CTA, the lists by CTAs of a cell's
+// members.  They run before every step launch and find nothing to do nine
+// times in ten, and then they are two empty launches (as seven kernels they
+// cost 18 us beside the 120 us of a 64-step launch).
 #include "chain.cuh"
 
 namespace mcgpu {
 
 __device__ __forceinline__ bool nl_rebuilding(const ChainHdr& H) { return H.nl_on && !H.nl_valid; }
 
-// Cell grid of every stale chain from its current box; zero the counters.
-__global__ void k_nl_reset(Pool P) {
+__device__ __forceinline__ int cell_of(unsigned a, int n) {
+  return (int)(((unsigned long long)a * (unsigned)n) >> 32);
+}
+
+constexpr int kNlCellThreads = 1024;
+constexpr int kNlSortMax = 256;   // members of a cell sorted in shared memory
+
+// The cells of a stale chain (blockIdx.x): grid from its current box, members
+// counted, scanned, scattered, and each cell's sorted by index -- a warp per
+// cell writes each member at its rank.  One CTA: 32,768 waters in 343 cells
+// take the time of a few step launches, once per rebuild.
+__global__ void __launch_bounds__(kNlCellThreads) k_nl_cells(Pool P) {
   ChainHdr& H = P.hdr[blockIdx.x];
   if (!nl_rebuilding(H)) return;
   __shared__ int nc[3];
-  if (threadIdx.x == 0) {
+  __shared__ int tot[kNlCellThreads / 32];
+  __shared__ int buf[kNlCellThreads / 32][kNlSortMax];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (tid == 0) {
     for (int k = 0; k < 3; k++) nc[k] = max(1, (int)floor(H.L[k] / (double)H.nl_rlist));
     // fewer, larger cells if the grid outgrew its allocation (box growth)
     while (nc[0] * nc[1] * nc[2] > H.cell_cap) {
@@ -41,69 +59,79 @@ __global__ void k_nl_reset(Pool P) {
     for (int k = 0; k < 3; k++) H.ncell[k] = nc[k];
   }
   __syncthreads();
-  const int n = nc[0] * nc[1] * nc[2];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) P.cell_cnt[H.cell0 + i] = 0;
-}
-
-__device__ __forceinline__ int cell_of(unsigned a, int n) {
-  return (int)(((unsigned long long)a * (unsigned)n) >> 32);
-}
-
-__global__ void k_nl_count(Pool P, const int* mol_chain, int n_mol) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n_mol) return;
-  const ChainHdr& H = P.hdr[mol_chain[m]];
-  if (!nl_rebuilding(H)) return;
-  const uint4 A = P.mfix[m];
-  const int cx = cell_of(A.x, H.ncell[0]), cy = cell_of(A.y, H.ncell[1]), cz = cell_of(A.z, H.ncell[2]);
-  const int cell = H.cell0 + (cx * H.ncell[1] + cy) * H.ncell[2] + cz;
-  P.mcell[m] = cell;
-  atomicAdd(&P.cell_cnt[cell], 1);
-}
-
-// Exclusive scan of a stale chain's cell counts into cell_start (pool
-// positions from the chain's first molecule); counters reset for the fill.
-__global__ void k_nl_scan(Pool P) {
-  const ChainHdr& H = P.hdr[blockIdx.x];
-  if (!nl_rebuilding(H) || threadIdx.x != 0) return;
-  const int n = H.ncell[0] * H.ncell[1] * H.ncell[2];
-  int run = H.mol0;
-  for (int i = 0; i < n; i++) {
-    const int c = H.cell0 + i;
-    P.cell_start[c] = run;
-    run += P.cell_cnt[c];
-    P.cell_cnt[c] = 0;
+  const int n0 = nc[0], n1 = nc[1], n2 = nc[2], n = n0 * n1 * n2;
+  const int m0 = H.mol0, m1 = H.mol0 + H.n_mol, c0 = H.cell0;
+  for (int i = tid; i < n; i += kNlCellThreads) P.cell_cnt[c0 + i] = 0;
+  __syncthreads();
+  for (int m = m0 + tid; m < m1; m += kNlCellThreads) {
+    const uint4 A = P.mfix[m];
+    const int cell = c0 + (cell_of(A.x, n0) * n1 + cell_of(A.y, n1)) * n2 + cell_of(A.z, n2);
+    P.mcell[m] = cell;
+    atomicAdd(&P.cell_cnt[cell], 1);
   }
-}
-
-__global__ void k_nl_scatter(Pool P, const int* mol_chain, int n_mol) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n_mol) return;
-  const ChainHdr& H = P.hdr[mol_chain[m]];
-  if (!nl_rebuilding(H)) return;
-  const int cell = P.mcell[m];
-  const int pos = atomicAdd(&P.cell_cnt[cell], 1);
-  P.cell_mol[P.cell_start[cell] + pos] = m;
-}
-
-// Sorts each cell's members by index (insertion sort; cells hold tens of
-// molecules).  One thread per cell; blockIdx.y is the chain.
-__global__ void k_nl_sort(Pool P) {
-  const ChainHdr& H = P.hdr[blockIdx.y];
-  if (!nl_rebuilding(H)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= H.ncell[0] * H.ncell[1] * H.ncell[2]) return;
-  const int c = H.cell0 + i;
-  int* v = P.cell_mol + P.cell_start[c];
-  const int n = P.cell_cnt[c];
-  for (int a = 1; a < n; a++) {
-    const int key = v[a];
-    int b = a - 1;
-    while (b >= 0 && v[b] > key) {
-      v[b + 1] = v[b];
-      b--;
+  __syncthreads();
+  // exclusive scan into cell_start (pool positions from the chain's first
+  // molecule), 1,024 cells a pass; the counters are reset for the scatter
+  int run = m0;
+  for (int i0 = 0; i0 < n; i0 += kNlCellThreads) {
+    const int i = i0 + tid;
+    const int v = i < n ? __ldcg(P.cell_cnt + c0 + i) : 0;
+    int incl = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(~0u, incl, off);
+      if (lane >= off) incl += u;
     }
-    v[b + 1] = key;
+    if (lane == 31) tot[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+      int t = tot[lane];
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int u = __shfl_up_sync(~0u, t, off);
+        if (lane >= off) t += u;
+      }
+      tot[lane] = t;
+    }
+    __syncthreads();
+    if (i < n) {
+      P.cell_start[c0 + i] = run + (w > 0 ? tot[w - 1] : 0) + incl - v;
+      P.cell_cnt[c0 + i] = 0;
+    }
+    run += tot[kNlCellThreads / 32 - 1];
+    __syncthreads();
+  }
+  for (int m = m0 + tid; m < m1; m += kNlCellThreads) {
+    const int cell = P.mcell[m];
+    const int pos = atomicAdd(&P.cell_cnt[cell], 1);
+    P.cell_mol[P.cell_start[cell] + pos] = m;
+  }
+  __syncthreads();
+  for (int i = w; i < n; i += kNlCellThreads / 32) {
+    int* v = P.cell_mol + P.cell_start[c0 + i];
+    const int cnt = __ldcg(P.cell_cnt + c0 + i);
+    if (cnt <= kNlSortMax) {
+      for (int k = lane; k < cnt; k += 32) buf[w][k] = v[k];
+      __syncwarp();
+      for (int k = lane; k < cnt; k += 32) {
+        const int key = buf[w][k];
+        int rank = 0;
+        for (int q = 0; q < cnt; q++) rank += buf[w][q] < key;
+        v[rank] = key;
+      }
+      __syncwarp();
+    } else if (lane == 0) {
+      // a cell of a box of few cells: in place
+      for (int a = 1; a < cnt; a++) {
+        const int key = v[a];
+        int b = a - 1;
+        while (b >= 0 && v[b] > key) {
+          v[b + 1] = v[b];
+          b--;
+        }
+        v[b + 1] = key;
+      }
+    }
   }
 }
 
@@ -120,69 +148,129 @@ __device__ __forceinline__ int stencil(int c, int n, int* out) {
   return n;
 }
 
-// One warp per molecule of a stale chain: its list from the stencil cells,
-// appended in cell order and member order; the build positions of its
-// primaries.
-__global__ void k_nl_build(Pool P, const int* mol_chain, int n_mol) {
-  const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (m >= n_mol) return;
-  ChainHdr& H = P.hdr[mol_chain[m]];
+// The lists of a stale chain (blockIdx.y), a quarter of a cell's members at a
+// time (gridDim.x CTAs stride over the quarters): the screen positions of the stencil cells' members
+// go to shared memory in chunks, in cell and member order, and each warp
+// appends the near ones to its molecules' lists in that order (a warp per
+// molecule that followed cell_mol -> mpi -> ppos for each of its 2,200
+// candidates took 440 us for 32,768 waters).  Also the build positions of the
+// members' primaries.  The last CTA of the chain marks its lists valid; a
+// chain with a list beyond its row drops its lists (full scans stay exact).
+constexpr int kNlThreads = 256;
+constexpr int kNlChunk = 1536;
+constexpr int kNlSlices = 4;
+
+__global__ void __launch_bounds__(kNlThreads) k_nl_build(Pool P) {
+  ChainHdr& H = P.hdr[blockIdx.y];
   if (!nl_rebuilding(H)) return;
-  const int2 pi = P.mpi[m];
-  for (int k = lane; k < pi.y; k += 32) P.pbuild[pi.x + k] = P.ppos[pi.x + k];
-  const float4 am = P.ppos[pi.x];
-  const int local = P.mcell[m] - H.cell0;
-  const int n1 = H.ncell[1], n2 = H.ncell[2];
-  const int cz = local % n2, cy = (local / n2) % n1, cx = local / (n1 * n2);
-  int sx[3], sy[3], sz[3];
-  const int nx = stencil(cx, H.ncell[0], sx), ny = stencil(cy, n1, sy), nz = stencil(cz, n2, sz);
-  int* out = P.nl + (size_t)m * P.nl_stride;
-  int cnt = 0;
-  bool over = false;
-  const unsigned lt = lanemask_lt();
-  for (int a = 0; a < nx; a++)
-    for (int b = 0; b < ny; b++)
-      for (int c = 0; c < nz; c++) {
-        const int cell = H.cell0 + (sx[a] * n1 + sy[b]) * n2 + sz[c];
-        const int s0 = P.cell_start[cell], n = P.cell_cnt[cell];
-        for (int base = 0; base < n; base += 32) {
-          const int t = base + lane;
-          bool in = false;
-          int j = -1;
-          if (t < n) {
-            j = P.cell_mol[s0 + t];
-            if (j != m) in = r2_screen(am, P.ppos[P.mpi[j].x], H) <= H.nl_r2;
-          }
-          const unsigned bal = __ballot_sync(~0u, in);
-          const int at = cnt + __popc(bal & lt);
-          if (in) {
-            if (at < P.nl_stride) out[at] = j;
-            else over = true;
-          }
-          cnt += __popc(bal);
+  __shared__ float4 pos[kNlChunk];
+  __shared__ int mol[kNlChunk];
+  __shared__ int start[27], pref[28];
+  __shared__ int n_cells;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int n0 = H.ncell[0], n1 = H.ncell[1], n2 = H.ncell[2];
+  for (int item = blockIdx.x; item < n0 * n1 * n2 * kNlSlices; item += gridDim.x) {
+    const int local = item / kNlSlices, slice = item - local * kNlSlices;
+    const int cell = H.cell0 + local;
+    const int cnt = P.cell_cnt[cell], first = P.cell_start[cell];
+    const int per = (cnt + kNlSlices - 1) / kNlSlices;
+    const int i0 = min(cnt, slice * per), i1 = min(cnt, i0 + per);
+    if (i0 < i1) {
+      __syncthreads();   // the last item's stencil is read no more
+      if (w == 0) {
+        const int cz = local % n2, cy = (local / n2) % n1, cx = local / (n1 * n2);
+        int sx[3], sy[3], sz[3];
+        const int nx = stencil(cx, n0, sx), ny = stencil(cy, n1, sy), nz = stencil(cz, n2, sz);
+        const int n = nx * ny * nz;
+        int st = 0, c = 0;
+        if (lane < n) {
+          const int a = lane / (ny * nz), b = (lane / nz) % ny, d = lane % nz;
+          const int q = H.cell0 + (sx[a] * n1 + sy[b]) * n2 + sz[d];
+          st = P.cell_start[q];
+          c = P.cell_cnt[q];
+        }
+        int incl = c;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const int u = __shfl_up_sync(~0u, incl, off);
+          if (lane >= off) incl += u;
+        }
+        if (lane < n) {
+          start[lane] = st;
+          pref[lane] = incl - c;
+        }
+        if (lane == n - 1) {
+          pref[n] = incl;
+          n_cells = n;
         }
       }
-  over = __any_sync(~0u, over);
-  if (lane == 0) {
-    P.nl_cnt[m] = min(cnt, P.nl_stride);
-    if (over) atomicAdd(&H.nl_overflow, 1);
+      __syncthreads();
+      const int total = pref[n_cells];
+      const bool simple = H.simple_prim != 0;
+      const float Lx = H.Lf[0], Ly = H.Lf[1], Lz = H.Lf[2], nl_r2 = H.nl_r2;
+      const unsigned lt = lanemask_lt();
+      bool over = false;
+      for (int c0 = 0; c0 < total; c0 += kNlChunk) {
+        const int c1 = min(total, c0 + kNlChunk);
+        int k = 0;
+        for (int t = c0 + tid; t < c1; t += kNlThreads) {
+          while (pref[k + 1] <= t) k++;
+          const int j = P.cell_mol[start[k] + (t - pref[k])];
+          mol[t - c0] = j;
+          pos[t - c0] = P.ppos[simple ? H.pidx0 + (j - H.mol0) : P.mpi[j].x];
+        }
+        __syncthreads();
+        for (int i = i0 + w; i < i1; i += kNlThreads / 32) {
+          const int m = P.cell_mol[first + i];
+          const int2 pi = P.mpi[m];
+          if (c0 == 0)
+            for (int q = lane; q < pi.y; q += 32) P.pbuild[pi.x + q] = P.ppos[pi.x + q];
+          const float4 am = P.ppos[pi.x];
+          int* out = P.nl + (size_t)m * P.nl_stride;
+          int cnt_m = c0 == 0 ? 0 : P.nl_cnt[m];
+          for (int base = 0; base < c1 - c0; base += 32) {
+            const int t = base + lane;
+            bool in = false;
+            int j = -1;
+            if (t < c1 - c0) {
+              j = mol[t];
+              const float4 q = pos[t];
+              const float dx = wrapf(q.x - am.x, Lx), dy = wrapf(q.y - am.y, Ly),
+                          dz = wrapf(q.z - am.z, Lz);
+              in = j != m && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= nl_r2;
+            }
+            const unsigned bal = __ballot_sync(~0u, in);
+            if (in) {
+              const int at = cnt_m + __popc(bal & lt);
+              if (at < P.nl_stride) out[at] = j;
+              else over = true;
+            }
+            cnt_m += __popc(bal);
+          }
+          __syncwarp();
+          if (lane == 0) P.nl_cnt[m] = min(cnt_m, P.nl_stride);
+          __syncwarp();
+        }
+        __syncthreads();
+      }
+      if (__any_sync(~0u, over) && lane == 0) atomicAdd(&H.nl_overflow, 1);
+    }
   }
-}
-
-// Marks rebuilt lists valid (an overflowing chain drops its list: full
-// scans stay exact).
-__global__ void k_nl_finish(Pool P) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= P.n_chains) return;
-  ChainHdr& H = P.hdr[c];
-  if (!nl_rebuilding(H)) return;
-  if (H.nl_overflow) {
-    H.nl_on = 0;
-    return;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    // nl_done counts the chain's CTAs of this launch
+    if (atomicAdd(&H.nl_done, 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      H.nl_done = 0;
+      if (*(volatile int*)&H.nl_overflow) {
+        H.nl_on = 0;
+      } else {
+        H.nl_builds++;
+        H.nl_valid = 1;
+      }
+    }
   }
-  H.nl_valid = 1;
-  H.nl_builds++;
 }
 
 // Per-chain list configuration (host-computed), applied to the headers.
@@ -201,16 +289,18 @@ __global__ void k_nl_config(Pool P, const NlCfg* cfg) {
   H.nl_rlist = f.rlist;
 }
 
-cudaError_t launch_nl_rebuild(Pool P, const int* mol_chain, int n_mol, int max_cells,
-                              cudaStream_t st) {
+cudaError_t launch_nl_rebuild(Pool P, int max_cells, cudaStream_t st) {
   const int nc = P.n_chains;
-  k_nl_reset<<<nc, 256, 0, st>>>(P);
-  k_nl_count<<<(n_mol + 255) / 256, 256, 0, st>>>(P, mol_chain, n_mol);
-  k_nl_scan<<<nc, 32, 0, st>>>(P);
-  k_nl_scatter<<<(n_mol + 255) / 256, 256, 0, st>>>(P, mol_chain, n_mol);
-  k_nl_sort<<<dim3((max_cells + 127) / 128, nc), 128, 0, st>>>(P);
-  k_nl_build<<<(n_mol + 7) / 8, 256, 0, st>>>(P, mol_chain, n_mol);
-  k_nl_finish<<<(nc + 127) / 128, 128, 0, st>>>(P);
+  k_nl_cells<<<nc, kNlCellThreads, 0, st>>>(P);
+  // six CTAs an SM in all, no more than a chain has work for
+  int gx = 152 * 6 / nc;
+  gx = gx < 1 ? 1 : gx > max_cells * kNlSlices ? max_cells * kNlSlices : gx;
+  // grid.y holds at most 65,535 chains
+  for (int c0 = 0; c0 < nc; c0 += 65535) {
+    Pool Q = P;
+    Q.hdr += c0;
+    k_nl_build<<<dim3(gx, nc - c0 < 65535 ? nc - c0 : 65535), kNlThreads, 0, st>>>(Q);
+  }
   return cudaGetLastError();
 }
 

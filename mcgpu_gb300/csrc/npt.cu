@@ -295,11 +295,10 @@ struct VcStencil {
 // each pair of molecules is met once, from the molecule whose cell comes
 // first, or within a cell from the lower index.  Otherwise every cell once
 // (c-1, c, c+1 per edge with at least 3 cells, else all) with pairs j > m.
-// Warp 0 builds it: one cell per lane, so the counts and starts arrive in
+// One warp builds it: one cell per lane, so the counts and starts arrive in
 // one round trip.
-__device__ inline void vc_stencil(const Pool& P, const ChainHdr& H, int m, VcStencil& S) {
-  if (threadIdx.x >= 32) return;
-  const int lane = threadIdx.x;
+__device__ inline void vc_stencil(const Pool& P, const ChainHdr& H, int m, VcStencil& S,
+                                  int lane) {
   const int local = P.vc_of[m] - H.mol0;
   const int n0 = H.vncell[0], n1 = H.vncell[1], n2 = H.vncell[2];
   const int cz = local % n2, cy = (local / n2) % n1, cx = local / (n1 * n2);
@@ -541,7 +540,7 @@ __device__ __forceinline__ void vol_f64_mol(const Pool& P, const int* mol_chain,
   const ChainHdr& H = P.hdr[c];
   if (!vol_take64(v, H, pass)) return;
   const int nvol = pass == 2 ? 1 : 2;
-  vc_stencil(P, H, m, S);
+  if (threadIdx.x < 32) vc_stencil(P, H, m, S, threadIdx.x);
   if (threadIdx.x < 2) vb[threadIdx.x] = v.box[threadIdx.x];
   const int a0 = P.mstart[m], len = P.mlen[m] & 255;
   const int2 pi = P.mpi[m];
@@ -701,7 +700,7 @@ __device__ __forceinline__ void vol_df_mol(const Pool& P, const int* mol_chain,
   if (v.state != 4 && v.state != 6) return;
   // state 6 re-takes U(V') only (.x stays 0)
   const int w0 = v.state == 6 ? 1 : 0, nvol = v.state == 6 ? 1 : 2;
-  vc_stencil(P, H, m, S);
+  if (threadIdx.x < 32) vc_stencil(P, H, m, S, threadIdx.x);
   const int a0 = P.mstart[m], len = P.mlen[m] & 255;
   const int2 pi = P.mpi[m];
   const uint4 Am = P.mfix[m];
@@ -933,83 +932,97 @@ __device__ __forceinline__ void vol_atoms_delta(const float4* so, const float2* 
 // gets the sums of the magnitudes that bound their rounding.  The in-range
 // test is the FP32 screen with the FP64 re-test inside its guard band: the
 // FP64 test's set exactly.
-__global__ void __launch_bounds__(kVolThreads, 8) k_vol_pair_sums32(Pool P, const int* mol_chain,
-                                                                 const VolMove* vm, int m_begin,
-                                                                 MolRanges R, double2* emol2,
-                                                                 double2* eabs2, int init) {
-  __shared__ float4 so[kMaxA];
-  __shared__ float2 sq[kMaxA];
-  __shared__ int spa[kMaxP];
-  __shared__ VolBox vb[2];
-  __shared__ float wred[kVolWarps][6];
-  __shared__ VcStencil S;
-  __shared__ int ent[kVolChunk];
-  __shared__ int wcnt[kVolWarps], woff[kVolWarps + 1];
-  const int m = range_mol(R, m_begin, blockIdx.x);
+//
+// One warp per molecule: it screens its stencil's candidates 32 at a time into
+// a ring and evaluates full rings as (neighbour, atom) items, an atom at a time
+// over the neighbours, with no block barrier and one reduction.  Where each
+// molecule has one primary, its anchor, the screen is one distance: every
+// edge scales alike, so r' = s r, and both cutoffs are tested on it; before, each
+// candidate took two double-float differences.  A CTA of four warps per
+// molecule, its chunks between barriers, took 622 us a move on 32,768 waters
+// (rc 12 A) and 3.6 ms a round of 160 served jobs (214,016 molecules).
+constexpr int kVolWarpThreads = 256;
+
+__global__ void __launch_bounds__(kVolWarpThreads, 3)
+    k_vol_pair_sums32(Pool P, const int* mol_chain, const VolMove* vm, int m_begin, int n_items,
+                      MolRanges R, double2* emol2, double2* eabs2, int init) {
+  constexpr int kWarps = kVolWarpThreads / 32;
+  __shared__ float4 so_[kWarps][kMaxA];
+  __shared__ float2 sq_[kWarps][kMaxA];
+  __shared__ int spa_[kWarps][kMaxP];
+  __shared__ VcStencil S_[kWarps];
+  __shared__ int ring_[kWarps][kRing];
+  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int item = blockIdx.x * kWarps + wi;
+  if (item >= n_items) return;
+  const int m = range_mol(R, m_begin, item);
   const int c = mol_chain[m];
   const VolMove& v = vm[c];
   const ChainHdr& H = P.hdr[c];
   // init: a chain's energy at its current box; else dU of a mixed move
   if (!(v.state == 1 && (H.vol_mixed || init))) return;
   const bool delta = !init;
-  __shared__ float sm1[3];   // s - 1 per edge, s = L'/L
-  if (delta && threadIdx.x < 3)
-    sm1[threadIdx.x] = (float)(v.box[1].L[threadIdx.x] / v.box[0].L[threadIdx.x] - 1.0);
-  vc_stencil(P, H, m, S);
+  float4* so = so_[wi];
+  float2* sq = sq_[wi];
+  int* spa = spa_[wi];
+  VcStencil& S = S_[wi];
+  int* ring = ring_[wi];
+  vc_stencil(P, H, m, S, lane);
   const int a0 = P.mstart[m], len = P.mlen[m] & 255;
   const int2 pi = P.mpi[m];
   const uint4 Am = P.mfix[m];
-  for (int i = threadIdx.x; i < len; i += blockDim.x) {
+  for (int i = lane; i < len; i += 32) {
     so[i] = P.aoff[a0 + i];
     sq[i] = P.aeq[a0 + i];
   }
-  for (int k = threadIdx.x; k < pi.y; k += blockDim.x) spa[k] = P.pidx[pi.x + k] - a0;
-  if (threadIdx.x < 2) vb[threadIdx.x] = v.box[threadIdx.x];
-  __syncthreads();
+  for (int k = lane; k < pi.y; k += 32) spa[k] = P.pidx[pi.x + k] - a0;
+  __syncwarp();
   const float reach2 = v.reach * v.reach;
-  const float sf = v.sf;
+  const float sf = v.sf, sf2 = sf * sf;
   const float rad_m = P.mrad[m];
-  float eh[2] = {0.f, 0.f}, el[2] = {0.f, 0.f}, ab[2] = {0.f, 0.f};
+  const float fx0 = H.fxs[0], fx1 = H.fxs[1], fx2 = H.fxs[2];
+  // s - 1 per edge, s = L'/L
+  float sm1[3] = {0.f, 0.f, 0.f};
+  if (delta)
+    for (int k = 0; k < 3; k++) sm1[k] = (float)(v.box[1].L[k] / v.box[0].L[k] - 1.0);
+  const bool simple = H.simple_prim != 0, uniform = H.uniform != 0;
+  const float lo0 = v.box[0].cut2_lo, hi0 = v.box[0].cut2_hi;
+  const float lo1 = v.box[1].cut2_lo, hi1 = v.box[1].cut2_hi;
+  const VolBox B0 = v.box[0];   // (the fields the pairs read, in registers)
   const int maxlen = H.max_len;
-  const int n_cand = S.pref[S.n];
-  int kc = 0;
-  for (int c0 = 0; c0 < n_cand; c0 += kVolChunk) {
-    for (int r = 0; r < kVolChunk / kVolThreads; r++) {
-      const int t = c0 + r * kVolThreads + (int)threadIdx.x;
-      int f = 0, j = 0;
-      if (t < n_cand) {
-        j = vc_candidate(P, S, t, kc);
-        if (vc_takes(S, kc, j, m))
-          f = vol_screen(P, H, vb, so, spa, pi.y, Am, j, reach2, sf, 0, delta ? 2 : 1);
+  float eh = 0.f, el = 0.f, ab = 0.f;
+  auto add = [&](float e, float a) {
+    ff_add(eh, el, e);
+    ab += a;
+  };
+  auto pairs = [&](int head, int count) {
+    const int items = count * maxlen;
+    for (int it = lane; it < items; it += 32) {
+      const int bi = it / count, e = it - bi * count;
+      const int jf = ring[(head + e) & (kRing - 1)];
+      const int j = jf & kVolJMask, f = (jf >> kVolFShift) & 3;
+      int bb;
+      float rad_j;
+      if (uniform) {
+        bb = H.atom0 + (j - H.mol0) * maxlen + bi;
+        rad_j = H.umrad;
+      } else {
+        if (bi >= (P.mlen[j] & 255)) continue;
+        bb = P.mstart[j] + bi;
+        rad_j = P.mrad[j];
       }
-      vol_append(ent, wcnt, j, f, r);
-    }
-    __syncthreads();
-    vol_offsets(wcnt, woff);
-    __syncthreads();
-    const int items = woff[kVolWarps] * maxlen;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int e = it / maxlen, bi = it - e * maxlen;
-      const int jf = vol_entry(ent, woff, e);
-      const int j = jf & kVolJMask, f = jf >> kVolFShift;
-      const int lenj = P.mlen[j] & 255;
-      if (bi >= lenj) continue;
-      const int bb = P.mstart[j] + bi;
+      const uint4 Aj = P.mfix[j];
       const float4 ob = P.aoff[bb];
       const float2 qb = P.aeq[bb];
-      const uint4 Aj = P.mfix[j];
-      const float rad_j = P.mrad[j];
       const float rr = rad_m + rad_j;
+      float3 Dh, Dl;
+      vol_fixdiff(Aj, Am, B0, Dh, Dl);
       if (delta && f == 3) {
-        float3 Dh, Dl, Dh1, Dl1;
-        vol_fixdiff(Aj, Am, vb[0], Dh, Dl);
-        vol_fixdiff(Aj, Am, vb[1], Dh1, Dl1);
-        const bool wrap = fabsf(Dh.x) + rr > 0.5f * vb[0].Lf[0] - 1e-3f ||
-                          fabsf(Dh.y) + rr > 0.5f * vb[0].Lf[1] - 1e-3f ||
-                          fabsf(Dh.z) + rr > 0.5f * vb[0].Lf[2] - 1e-3f ||
-                          fabsf(Dh1.x) + rr > 0.5f * vb[1].Lf[0] - 1e-3f ||
-                          fabsf(Dh1.y) + rr > 0.5f * vb[1].Lf[1] - 1e-3f ||
-                          fabsf(Dh1.z) + rr > 0.5f * vb[1].Lf[2] - 1e-3f;
+        // the larger of the two volumes' reaches, against the smaller half edge
+        const float g = fmaxf(1.f, sf), h = fminf(1.f, sf);
+        const bool wrap = fabsf(Dh.x) * g + rr > 0.5f * B0.Lf[0] * h - 2e-3f ||
+                          fabsf(Dh.y) * g + rr > 0.5f * B0.Lf[1] * h - 2e-3f ||
+                          fabsf(Dh.z) * g + rr > 0.5f * B0.Lf[2] * h - 2e-3f;
         if (!wrap) {
           const float bx = Dh.x + ob.x, by = Dh.y + ob.y, bz = Dh.z + ob.z;
           const float lx = ((Dh.x - (bx - (bx - Dh.x))) + (ob.x - (bx - Dh.x))) + Dl.x;
@@ -1018,17 +1031,15 @@ __global__ void __launch_bounds__(kVolThreads, 8) k_vol_pair_sums32(Pool P, cons
           float e32 = 0.f, a32 = 0.f;
           vol_atoms_delta(so, sq, len, bx, by, bz, lx, ly, lz, Dh.x * sm1[0], Dh.y * sm1[1],
                           Dh.z * sm1[2], ob.w, qb, e32, a32);
-          ff_add(eh[1], el[1], e32);
-          ab[1] += a32;
+          add(e32, a32);
           continue;
         }
       }
-#pragma unroll
+#pragma unroll 1
       for (int w = 0; w < 2; w++) {
         if (!(f & (1 << w))) continue;
-        const VolBox& B = vb[w];
-        float3 Dh, Dl;
-        vol_fixdiff(Aj, Am, B, Dh, Dl);
+        const VolBox& B = v.box[w];
+        if (w == 1) vol_fixdiff(Aj, Am, B, Dh, Dl);
         // b relative to m's anchor as a double-float: two-sum of D + o_b
         const float bx = Dh.x + ob.x, by = Dh.y + ob.y, bz = Dh.z + ob.z;
         const float lx = ((Dh.x - (bx - (bx - Dh.x))) + (ob.x - (bx - Dh.x))) + Dl.x;
@@ -1040,39 +1051,64 @@ __global__ void __launch_bounds__(kVolThreads, 8) k_vol_pair_sums32(Pool P, cons
           vol_atoms32<true>(so, sq, len, bx, by, bz, lx, ly, lz, ob.w, qb, B, e32, a32);
         else
           vol_atoms32<false>(so, sq, len, bx, by, bz, lx, ly, lz, ob.w, qb, B, e32, a32);
-        // the change of a volume move: +E(V') - E(V), both into .y
-        const int wo = delta ? 1 : w;
-        ff_add(eh[wo], el[wo], (delta && w == 0) ? -e32 : e32);
-        ab[wo] += a32;
+        // the change of a volume move: E(V') - E(V)
+        add((delta && w == 0) ? -e32 : e32, a32);
       }
     }
-    __syncthreads();
+  };
+  const unsigned lt = lanemask_lt();
+  const int n_cand = S.pref[S.n];
+  int head = 0, tail = 0, kc = 0;
+  for (int base = 0; base < n_cand; base += 32) {
+    const int t = base + lane;
+    int f = 0, j = 0;
+    if (t < n_cand) {
+      j = vc_candidate(P, S, t, kc);
+      if (vc_takes(S, kc, j, m)) {
+        if (simple) {
+          const uint4 Aj = P.mfix[j];
+          const float dx = (float)(int)(Aj.x - Am.x) * fx0, dy = (float)(int)(Aj.y - Am.y) * fx1,
+                      dz = (float)(int)(Aj.z - Am.z) * fx2;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r2p = r2 * sf2;
+          f = (r2 <= lo0 ? 1 : 0) | (delta && r2p <= lo1 ? 2 : 0);
+          if ((r2 > lo0 && r2 <= hi0) || (delta && r2p > lo1 && r2p <= hi1)) {
+            // inside the guard band: the reference's FP64 test
+            const float4 oj = P.aoff[P.pidx[P.mpi[j].x]], om = so[spa[0]];
+            f = 0;
+            for (int w = 0; w < (delta ? 2 : 1); w++) {
+              const double* L = v.box[w].L;
+              if (dist2_at(pos_at(Am, om, L), pos_at(Aj, oj, L), L) <= __dmul_rn(H.cutoff, H.cutoff))
+                f |= 1 << w;
+            }
+          }
+        } else {
+          f = vol_screen(P, H, v.box, so, spa, pi.y, Am, j, reach2, sf, 0, delta ? 2 : 1);
+        }
+      }
+    }
+    const unsigned bal = __ballot_sync(~0u, f != 0);
+    if (f) ring[(tail + __popc(bal & lt)) & (kRing - 1)] = j | (f << kVolFShift);
+    tail += __popc(bal);
+    if (tail - head >= 32) {
+      __syncwarp();
+      pairs(head, 32);
+      head += 32;
+      __syncwarp();
+    }
   }
-  // double-float reduction (warp butterflies, then the warps in order); one
-  // conversion to FP64 per molecule
+  __syncwarp();
+  if (tail > head) pairs(head, tail - head);
+  __syncwarp();
+#pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-    for (int w = 0; w < 2; w++) {
-      const float h = __shfl_xor_sync(~0u, eh[w], off), l = __shfl_xor_sync(~0u, el[w], off);
-      ff_add2(eh[w], el[w], h, l);
-      ab[w] += __shfl_xor_sync(~0u, ab[w], off);
-    }
+    const float h = __shfl_xor_sync(~0u, eh, off), l = __shfl_xor_sync(~0u, el, off);
+    ff_add2(eh, el, h, l);
+    ab += __shfl_xor_sync(~0u, ab, off);
   }
-  if ((threadIdx.x & 31) == 0) {
-    const int wi = threadIdx.x >> 5;
-    wred[wi][0] = eh[0]; wred[wi][1] = el[0]; wred[wi][2] = eh[1];
-    wred[wi][3] = el[1]; wred[wi][4] = ab[0]; wred[wi][5] = ab[1];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float h0 = 0.f, l0 = 0.f, h1 = 0.f, l1 = 0.f, a0 = 0.f, a1 = 0.f;
-    for (int wi = 0; wi < kVolWarps; wi++) {
-      ff_add2(h0, l0, wred[wi][0], wred[wi][1]);
-      ff_add2(h1, l1, wred[wi][2], wred[wi][3]);
-      a0 += wred[wi][4];
-      a1 += wred[wi][5];
-    }
-    emol2[m] = make_double2((double)h0 + (double)l0, (double)h1 + (double)l1);
-    eabs2[m] = make_double2((double)a0, (double)a1);
+  if (lane == 0) {
+    const double e = (double)eh + (double)el, a = (double)ab;
+    emol2[m] = delta ? make_double2(0.0, e) : make_double2(e, 0.0);
+    eabs2[m] = delta ? make_double2(0.0, a) : make_double2(a, 0.0);
   }
 }
 
@@ -1258,6 +1294,10 @@ __global__ void k_vol_self_energy(Pool P, const VolMove* vm, const double2* esum
   P.hdr[c].run_err = f64 ? 0.0 : kTieRel * esum_abs[c].x;
 }
 
+static int vol_warp_grid(int n) {
+  return (n + kVolWarpThreads / 32 - 1) / (kVolWarpThreads / 32);
+}
+
 // Sets the running energy of the chains in act (all when act has no
 // ranges) to their system energy, FP64 or FP32 pair terms (double-float
 // sums), through the volume machinery; vm, emol2, eabs2, esum, esum_abs are
@@ -1282,7 +1322,8 @@ cudaError_t launch_chain_energy(Pool P, const int* mol_chain, int n_mol_total, V
     if (f64)
       k_vol_pair_sums<<<n, kVolThreads, 0, st>>>(P, mol_chain, vm, m0, act, emol2, 2);
     else
-      k_vol_pair_sums32<<<n, kVolThreads, 0, st>>>(P, mol_chain, vm, m0, act, emol2, eabs2, 1);
+      k_vol_pair_sums32<<<vol_warp_grid(n), kVolWarpThreads, 0, st>>>(P, mol_chain, vm, m0, n, act,
+                                                                     emol2, eabs2, 1);
   }
   k_vol_sums<<<nc, kVolSumThreads, 0, st>>>(P, vm, emol2, eabs2, esum, esum_abs, act, 1);
   k_vol_self_energy<<<(nc + 127) / 128, 128, 0, st>>>(P, vm, esum, esum_abs, act, nc, f64 ? 1 : 0);
@@ -1317,7 +1358,8 @@ cudaError_t launch_volume_phase(Pool P, const int* mol_chain, int n_mol_total, V
       if (f64)
         k_vol_pair_sums<<<items, kVolThreads, 0, st>>>(P, mol_chain, vm, 0, act, emol2, pass);
       else
-        k_vol_pair_sums32<<<items, kVolThreads, 0, st>>>(P, mol_chain, vm, 0, act, emol2, eabs2, 0);
+        k_vol_pair_sums32<<<vol_warp_grid(items), kVolWarpThreads, 0, st>>>(
+            P, mol_chain, vm, 0, items, act, emol2, eabs2, 0);
       return;
     }
     const int chunk = 1 << 20;
@@ -1326,7 +1368,8 @@ cudaError_t launch_volume_phase(Pool P, const int* mol_chain, int n_mol_total, V
       if (f64)
         k_vol_pair_sums<<<n, kVolThreads, 0, st>>>(P, mol_chain, vm, m0, act, emol2, pass);
       else
-        k_vol_pair_sums32<<<n, kVolThreads, 0, st>>>(P, mol_chain, vm, m0, act, emol2, eabs2, 0);
+        k_vol_pair_sums32<<<vol_warp_grid(n), kVolWarpThreads, 0, st>>>(
+            P, mol_chain, vm, m0, n, act, emol2, eabs2, 0);
     }
   };
   if (has64) pairs(true, 0);
