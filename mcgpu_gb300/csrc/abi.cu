@@ -1618,6 +1618,7 @@ extern "C" int mcgpu_batch_create(mcgpu_ctx* ctx, int n_chains, const mcgpu_box_
     P.vc_start = dalloc<int>(nm, &e2);
     P.vc_mol = dalloc<int>(nm, &e2);
     P.vc_of = dalloc<int>(nm, &e2);
+    P.vc_fix = dalloc<uint4>(nm, &e2);
     if (e2 == cudaSuccess)
       e2 = launch_chain_energy(P, bt->pool.mol_chain, bt->pool.n_mol, bt->vm, bt->emol2, bt->eabs2,
                                bt->vsum, bt->vsum_abs, ctx->stream, MolRanges(), false);
@@ -1976,6 +1977,7 @@ extern "C" int mcgpu_batch_set_npt(mcgpu_batch* bt, int interval, const double* 
       P.vc_start = dalloc<int>(nm, &e);
       P.vc_mol = dalloc<int>(nm, &e);
       P.vc_of = dalloc<int>(nm, &e);
+      P.vc_fix = dalloc<uint4>(nm, &e);
     }
     if (e != cudaSuccess) return set_err(ctx, MCGPU_ERR_NOMEM, "NPT buffers: %s", cudaGetErrorString(e));
   }

@@ -156,6 +156,7 @@ struct VolBox {
 struct VolMove {
   VolBox box[2];
   float reach, sf;   // rc + 2 prad + 0.01; edge ratio L'/L
+  float sm1[3], pad;   // L'/L - 1 per edge
   double L[3];
   double dlnv, u;
   int state;   // 0 not due, 1 evaluate, 2 rejected outright, 3 accepted;
@@ -210,6 +211,7 @@ struct Pool {
   int* vc_start;       // [n_mol] first slot in vc_mol
   int* vc_mol;         // [n_mol] molecules grouped by cell
   int* vc_of;          // [n_mol] cell of each molecule
+  uint4* vc_fix;       // [n_mol] anchors in the order of vc_mol, the molecule in .w
 };
 
 // ---- Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11), from the published
@@ -554,7 +556,10 @@ __device__ __forceinline__ float wrapf(float d, float L) {
 // step y' = y + (y/2)(1 - r2 y^2): the estimate is good to about 2^-23
 // relative, the refined value to about one ulp.
 __device__ __forceinline__ float rsqrt_nr(float r2) {
-  float ir = rsqrtf(r2);
+  // the estimate without the library function's scaling of subnormal
+  // arguments (a distance below 1e-19 A), three instructions of every term
+  float ir;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ir) : "f"(r2));
   const float t0 = r2 * ir;
   const float h = fmaf(-t0, ir, 1.0f);
   return fmaf(0.5f * ir, h, ir);

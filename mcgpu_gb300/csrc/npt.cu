@@ -100,6 +100,7 @@ __global__ void k_vol_propose(Pool P, VolMove* vm, MolRanges R, int n_items) {
     volbox_set(v.box[1], v.L, H.cutoff);
     v.reach = vol_reach(H);
     v.sf = (float)(v.L[0] / H.L[0]);
+    for (int k = 0; k < 3; k++) v.sm1[k] = (float)(v.box[1].L[k] / v.box[0].L[k] - 1.0);
     // molecules must stay within a quarter of an edge (the chain state's
     // anchor-image rule); the cutoff may exceed half an edge, as in the
     // reference's single-image minimum convention
@@ -238,8 +239,16 @@ __global__ void k_vc_scatter(Pool P, const int* mol_chain, const VolMove* vm, Mo
 // and each is written at its rank (the number of smaller members: the
 // indexes are distinct).  A cell of more than kVcSortMax members (a box of
 // fewer than three cells per edge) is sorted by lane 0 in place.
+// Beside its index each member's anchor goes to vc_fix: the pair sums then read
+// a candidate with one load instead of two that follow one another.
 constexpr int kVcSortWarps = 8;
 constexpr int kVcSortMax = 384;
+
+__device__ __forceinline__ uint4 vc_entry(const Pool& P, int m) {
+  uint4 A = P.mfix[m];
+  A.w = (unsigned)m;
+  return A;
+}
 
 __global__ void __launch_bounds__(32 * kVcSortWarps) k_vc_sort(Pool P, const int* mol_chain,
                                                                const VolMove* vm, MolRanges R,
@@ -254,6 +263,7 @@ __global__ void __launch_bounds__(32 * kVcSortWarps) k_vc_sort(Pool P, const int
   const ChainHdr& H = P.hdr[c];
   if (m - H.mol0 >= H.vncell[0] * H.vncell[1] * H.vncell[2]) return;
   int* v = P.vc_mol + P.vc_start[m];
+  uint4* fix = P.vc_fix + P.vc_start[m];
   const int n = P.vc_cnt[m];
   if (n <= kVcSortMax) {
     int* sb = buf[wi];
@@ -264,6 +274,7 @@ __global__ void __launch_bounds__(32 * kVcSortWarps) k_vc_sort(Pool P, const int
       int rank = 0;
       for (int k = 0; k < n; k++) rank += sb[k] < key;
       v[rank] = key;
+      fix[rank] = vc_entry(P, key);
     }
     return;
   }
@@ -277,15 +288,16 @@ __global__ void __launch_bounds__(32 * kVcSortWarps) k_vc_sort(Pool P, const int
     }
     v[k + 1] = key;
   }
+  for (int k = 0; k < n; k++) fix[k] = vc_entry(P, v[k]);
 }
 
 // The cells around molecule m's (27, or every cell once along an edge of
-// fewer than 3): first slot and member count of each, and prefix sums, in
-// shared memory; threads then take flat candidate indices.
+// fewer than 3) as runs of consecutive members: first slot of each and prefix
+// sums, in shared memory; threads then take flat candidate indices.
 struct VcStencil {
-  int start[27], cnt[27], pref[28];
+  int start[27], pref[28];
   int n;
-  int half;   // cell 0 is the molecule's own (pairs j > m), cells 1.. the
+  int half;   // run 0 is the molecule's own cell (pairs j > m), runs 1.. the
               // forward half of the neighbours (every pair): each pair once
 };
 
@@ -329,14 +341,19 @@ __device__ inline void vc_stencil(const Pool& P, const ChainHdr& H, int m, VcSte
     const int v = __shfl_up_sync(~0u, incl, off);
     if (lane >= off) incl += v;
   }
-  if (lane < n) {
-    S.start[lane] = start;
-    S.cnt[lane] = cnt;
-    S.pref[lane] = incl - cnt;
+  // cells next to each other in memory become one run (the z neighbours of a
+  // column are); the first stays alone
+  const int end_before = __shfl_up_sync(~0u, start + cnt, 1);
+  const unsigned runs = __ballot_sync(~0u, lane < n && (lane < 2 || start != end_before));
+  if ((runs >> lane) & 1u) {
+    const int r = __popc(runs & lanemask_lt());
+    S.start[r] = start;
+    S.pref[r] = incl - cnt;
   }
-  if (lane == n - 1) S.pref[n] = incl;
+  const int nr = __popc(runs);
+  if (lane == n - 1) S.pref[nr] = incl;
   if (lane == 0) {
-    S.n = n;
+    S.n = nr;
     S.half = half ? 1 : 0;
   }
 }
@@ -346,8 +363,13 @@ __device__ __forceinline__ bool vc_takes(const VcStencil& S, int k, int j, int m
   return S.half ? (k > 0 || j > m) : j > m;
 }
 
-// Candidate t of the stencil (t < S.pref[S.n]); k is the thread's cursor
-// over the cells (t only grows).
+// Candidate t of the stencil (t < S.pref[S.n]), its anchor and (.w) index; k is
+// the thread's cursor over the runs (t only grows).
+__device__ __forceinline__ uint4 vc_candidate_fix(const Pool& P, const VcStencil& S, int t,
+                                                  int& k) {
+  while (S.pref[k + 1] <= t) k++;
+  return P.vc_fix[S.start[k] + (t - S.pref[k])];
+}
 __device__ __forceinline__ int vc_candidate(const Pool& P, const VcStencil& S, int t, int& k) {
   while (S.pref[k + 1] <= t) k++;
   return P.vc_mol[S.start[k] + (t - S.pref[k])];
@@ -355,22 +377,22 @@ __device__ __forceinline__ int vc_candidate(const Pool& P, const VcStencil& S, i
 
 
 // Anchor difference b - a at box B as a double-float (fixdiff_ff's split).
+__device__ __forceinline__ void vol_fixdiff1(unsigned b, unsigned a, float fxs, float fxs_lo,
+                                             float& hi, float& lo) {
+  // d = (d >> 9) 2^9 + (d & 511): both parts exact in FP32
+  const int d = (int)(b - a);
+  const float fh = small_i2f(d >> 9) * 512.0f, fl = small_i2f(d & 511);
+  const float p = fh * fxs;
+  const float e = fmaf(fh, fxs, -p);
+  const float t = fmaf(fh, fxs_lo, fmaf(fl, fxs, e));
+  hi = p + t;
+  lo = t - (hi - p);
+}
 __device__ __forceinline__ void vol_fixdiff(uint4 b, uint4 a, const VolBox& B, float3& hi,
                                             float3& lo) {
-  const int d[3] = {(int)(b.x - a.x), (int)(b.y - a.y), (int)(b.z - a.z)};
-  float h[3], l[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    // d = (d >> 9) 2^9 + (d & 511): both parts exact in FP32
-    const float fh = small_i2f(d[k] >> 9) * 512.0f, fl = small_i2f(d[k] & 511);
-    const float p = fh * B.fxs[k];
-    const float e = fmaf(fh, B.fxs[k], -p);
-    const float t = fmaf(fh, B.fxs_lo[k], fmaf(fl, B.fxs[k], e));
-    h[k] = p + t;
-    l[k] = t - (h[k] - p);
-  }
-  hi = make_float3(h[0], h[1], h[2]);
-  lo = make_float3(l[0], l[1], l[2]);
+  vol_fixdiff1(b.x, a.x, B.fxs[0], B.fxs_lo[0], hi.x, lo.x);
+  vol_fixdiff1(b.y, a.y, B.fxs[1], B.fxs_lo[1], hi.y, lo.y);
+  vol_fixdiff1(b.z, a.z, B.fxs[2], B.fxs_lo[2], hi.z, lo.z);
 }
 
 // ---- chunked candidate screening shared by the pair kernels -------------
@@ -859,8 +881,9 @@ __device__ __forceinline__ void vol_atoms32(const float4* so, const float2* sq, 
     }
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     if (!(r2 > 0.f)) continue;
-    const float lj = lj32(rcp_nr(r2), a4.w, sig_b, ea.x, qb.x);
     const float cl = (ea.y * qb.y) * rsqrt_nr(r2);
+    float lj = 0.f;
+    if ((ea.x * qb.x) * (a4.w * sig_b) != 0.f) lj = lj32(rcp_nr(r2), a4.w, sig_b, ea.x, qb.x);
     e32 += lj + cl;
     a32 += fabsf(lj) + fabsf(cl);
   }
@@ -909,18 +932,22 @@ __device__ __forceinline__ void vol_atoms_delta(const float4* so, const float2* 
     const float qa = fabsf(2.f * dx * ex) + fabsf(2.f * dy * ey) + fabsf(2.f * dz * ez) +
                      fmaf(ex, ex, fmaf(ey, ey, ez * ez));
     const float ir = rsqrt_nr(r2), irp = rsqrt_nr(r2p);
-    const float ir2 = rcp_nr(r2), ir2p = rcp_nr(r2p);
     const float w = ir * irp * rcp_approx(fmaf(r2, ir, r2p * irp));  // 1 / (r r' (r + r'))
     const float dcl = cq * (-q * w);
-    const float t = s2 * ir2;
-    const float g = s2 * ir2 * ir2p;                                  // sigma^2 / (r^2 r'^2)
-    const float tp = fmaf(-q, g, t);
-    const float t3 = t * t * t, tp3 = tp * tp * tp;
-    const float d3 = (-q * g) * fmaf(tp, tp, fmaf(tp, t, t * t));
-    const float dlj = ee * (d3 * (tp3 + t3) - d3);
+    float dlj = 0.f, alj = 0.f;
+    if (ee * s2 != 0.f) {   // (water: one pair of nine; zero exactly otherwise)
+      const float ir2 = rcp_nr(r2), ir2p = rcp_nr(r2p);
+      const float t = s2 * ir2;
+      const float g = s2 * ir2 * ir2p;                                // sigma^2 / (r^2 r'^2)
+      const float tp = fmaf(-q, g, t);
+      const float t3 = t * t * t, tp3 = tp * tp * tp;
+      const float d3 = (-q * g) * fmaf(tp, tp, fmaf(tp, t, t * t));
+      dlj = ee * (d3 * (tp3 + t3) - d3);
+      const float tm = fmaxf(t, tp), tm2 = tm * tm;
+      alj = fabsf(ee) * g * tm2 * (6.f * tm2 * tm + 3.f);
+    }
     e32 += dlj + dcl;
-    const float tm = fmaxf(t, tp), tm2 = tm * tm;
-    a32 += qa * (fabsf(cq) * w + fabsf(ee) * g * tm2 * (6.f * tm2 * tm + 3.f));
+    a32 += qa * (fabsf(cq) * w + alj);
   }
 }
 
@@ -981,14 +1008,17 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
   const float sf = v.sf, sf2 = sf * sf;
   const float rad_m = P.mrad[m];
   const float fx0 = H.fxs[0], fx1 = H.fxs[1], fx2 = H.fxs[2];
-  // s - 1 per edge, s = L'/L
-  float sm1[3] = {0.f, 0.f, 0.f};
-  if (delta)
-    for (int k = 0; k < 3; k++) sm1[k] = (float)(v.box[1].L[k] / v.box[0].L[k] - 1.0);
+  const float sm1x = v.sm1[0], sm1y = v.sm1[1], sm1z = v.sm1[2];
   const bool simple = H.simple_prim != 0, uniform = H.uniform != 0;
   const float lo0 = v.box[0].cut2_lo, hi0 = v.box[0].cut2_hi;
   const float lo1 = v.box[1].cut2_lo, hi1 = v.box[1].cut2_hi;
-  const VolBox B0 = v.box[0];   // (the fields the pairs read, in registers)
+  // what every pair reads of the first box, in registers
+  const float sx = v.box[0].fxs[0], sy = v.box[0].fxs[1], sz = v.box[0].fxs[2];
+  const float tx = v.box[0].fxs_lo[0], ty = v.box[0].fxs_lo[1], tz = v.box[0].fxs_lo[2];
+  // the larger of the two volumes' reaches, against the smaller half edge
+  const float grow = fmaxf(1.f, sf), shrink = 0.5f * fminf(1.f, sf);
+  const float wx = v.box[0].Lf[0] * shrink - 2e-3f, wy = v.box[0].Lf[1] * shrink - 2e-3f,
+              wz = v.box[0].Lf[2] * shrink - 2e-3f;
   const int maxlen = H.max_len;
   float eh = 0.f, el = 0.f, ab = 0.f;
   auto add = [&](float e, float a) {
@@ -996,9 +1026,13 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
     ab += a;
   };
   auto pairs = [&](int head, int count) {
-    const int items = count * maxlen;
-    for (int it = lane; it < items; it += 32) {
-      const int bi = it / count, e = it - bi * count;
+    int bi = 0, e = lane;
+    for (;; e += 32) {
+      while (e >= count) {
+        e -= count;
+        bi++;
+      }
+      if (bi >= maxlen) break;
       const int jf = ring[(head + e) & (kRing - 1)];
       const int j = jf & kVolJMask, f = (jf >> kVolFShift) & 3;
       int bb;
@@ -1016,21 +1050,20 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
       const float2 qb = P.aeq[bb];
       const float rr = rad_m + rad_j;
       float3 Dh, Dl;
-      vol_fixdiff(Aj, Am, B0, Dh, Dl);
+      vol_fixdiff1(Aj.x, Am.x, sx, tx, Dh.x, Dl.x);
+      vol_fixdiff1(Aj.y, Am.y, sy, ty, Dh.y, Dl.y);
+      vol_fixdiff1(Aj.z, Am.z, sz, tz, Dh.z, Dl.z);
       if (delta && f == 3) {
-        // the larger of the two volumes' reaches, against the smaller half edge
-        const float g = fmaxf(1.f, sf), h = fminf(1.f, sf);
-        const bool wrap = fabsf(Dh.x) * g + rr > 0.5f * B0.Lf[0] * h - 2e-3f ||
-                          fabsf(Dh.y) * g + rr > 0.5f * B0.Lf[1] * h - 2e-3f ||
-                          fabsf(Dh.z) * g + rr > 0.5f * B0.Lf[2] * h - 2e-3f;
+        const bool wrap = fabsf(Dh.x) * grow + rr > wx || fabsf(Dh.y) * grow + rr > wy ||
+                          fabsf(Dh.z) * grow + rr > wz;
         if (!wrap) {
           const float bx = Dh.x + ob.x, by = Dh.y + ob.y, bz = Dh.z + ob.z;
           const float lx = ((Dh.x - (bx - (bx - Dh.x))) + (ob.x - (bx - Dh.x))) + Dl.x;
           const float ly = ((Dh.y - (by - (by - Dh.y))) + (ob.y - (by - Dh.y))) + Dl.y;
           const float lz = ((Dh.z - (bz - (bz - Dh.z))) + (ob.z - (bz - Dh.z))) + Dl.z;
           float e32 = 0.f, a32 = 0.f;
-          vol_atoms_delta(so, sq, len, bx, by, bz, lx, ly, lz, Dh.x * sm1[0], Dh.y * sm1[1],
-                          Dh.z * sm1[2], ob.w, qb, e32, a32);
+          vol_atoms_delta(so, sq, len, bx, by, bz, lx, ly, lz, Dh.x * sm1x, Dh.y * sm1y,
+                          Dh.z * sm1z, ob.w, qb, e32, a32);
           add(e32, a32);
           continue;
         }
@@ -1063,10 +1096,10 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
     const int t = base + lane;
     int f = 0, j = 0;
     if (t < n_cand) {
-      j = vc_candidate(P, S, t, kc);
+      const uint4 Aj = vc_candidate_fix(P, S, t, kc);
+      j = (int)Aj.w;
       if (vc_takes(S, kc, j, m)) {
         if (simple) {
-          const uint4 Aj = P.mfix[j];
           const float dx = (float)(int)(Aj.x - Am.x) * fx0, dy = (float)(int)(Aj.y - Am.y) * fx1,
                       dz = (float)(int)(Aj.z - Am.z) * fx2;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r2p = r2 * sf2;
@@ -1277,6 +1310,7 @@ __global__ void k_vol_self(Pool P, VolMove* vm, MolRanges R, int n_items) {
   v.box[1] = v.box[0];
   v.reach = vol_reach(H);
   v.sf = 1.0f;
+  for (int k = 0; k < 3; k++) v.sm1[k] = 0.f;
   v.dlnv = 0.0;
   v.u = 0.0;
   v.fp64 = 0;

@@ -147,13 +147,13 @@ int server_alloc(mcgpu_server* s) {
   P.pidx = dalloc<int>(np, &e); P.ppos = dalloc<float4>(np, &e);
   P.vc_cnt = dalloc<int>(nm, &e); P.vc_start = dalloc<int>(nm, &e);
   P.vc_mol = dalloc<int>(nm, &e); P.vc_of = dalloc<int>(nm, &e);
+  P.vc_fix = dalloc<uint4>(nm, &e);
   P.hdr = dalloc<ChainHdr>(nc, &e);
   P.rb = dalloc<double>((size_t)nc * 3 * ml, &e);
   P.trace = nullptr;
   P.n_chains = nc;
   dp.mol_chain = dalloc<int>(nm, &e);
   dp.atom_mol = dalloc<int>(na, &e);
-  dp.emol = dalloc<double>(nm, &e);
   dp.esum = dalloc<double>(nc, &e);
   dp.n_chains = nc;
   dp.n_atom = (int)na;
