@@ -576,7 +576,6 @@ static Proposal host_proposal(const mcgpu_move* mv) {
   Proposal p;
   std::memset(&p, 0, sizeof(p));
   p.vertex = mv->vertex;
-  p.mode = MCGPU_ROT_EULER;
   p.dx = mv->dx; p.dy = mv->dy; p.dz = mv->dz;
   p.r0 = mv->rx; p.r1 = mv->ry; p.r2 = mv->rz;
   const double deg[3] = {mv->rx, mv->ry, mv->rz};

@@ -12,6 +12,7 @@
 // b = 0 and discards the first 310 outputs.
 #pragma once
 
+#include <math.h>
 #include <stdint.h>
 
 #ifdef __CUDACC__
@@ -37,6 +38,23 @@ MCGPU_HD int32_t crand_next(CRand& g) {
     g.b = 0;
   }
   return (int32_t)(v >> 1);
+}
+
+// rand() / RAND_MAX of a number v of the stream (MathLibrary.cpp:31-33), the
+// correctly rounded quotient: the correctly rounded reciprocal and one
+// residual step (Markstein 1990), which gives the division's value for each of
+// the 2^31 numerators.  Three dependent FP64 instructions on the device, where
+// the division is a dozen and a flexible step waits on some thirty draws one
+// after another.
+MCGPU_HD double crand_unit(int32_t v) {
+  const double kInv = 1.0 / 2147483647.0;
+  const double x = (double)v;
+#ifdef __CUDA_ARCH__
+  const double q = __dmul_rn(x, kInv);
+#else
+  const double q = x * kInv;
+#endif
+  return fma(fma(-q, 2147483647.0, x), kInv, q);
 }
 
 inline void crand_seed(CRand& g, unsigned int seed) {

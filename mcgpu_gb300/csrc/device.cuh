@@ -234,102 +234,33 @@ __device__ __forceinline__ int uidx(unsigned r, int n) {
   return (int)(((unsigned long long)r * (unsigned long long)n) >> 32);
 }
 
-// A trial move: vertex, translation, rotation (Euler degrees or axis+angle).
+// A trial move of the plain path: vertex, translation, Euler angles in degrees.
 struct Proposal {
-  int mol, vertex, mode, trig;   // trig: cos/sin below hold the Euler angles' values
-  double dx, dy, dz, r0, r1, r2, r3, u;
-  double cs[3], sn[3];           // host-drawn Euler moves: cos, sin of each angle
+  int mol, vertex, trig, pad;    // trig: cos/sin below hold the angles' values
+  double dx, dy, dz, r0, r1, r2;
+  double cs[3], sn[3];           // host-drawn moves: cos, sin of each angle
 };
 
-// Draws the proposal of (seed, chain, step): the counter layout and the
-// uniform/index mappings are fixed so a CPU replay gets the same values.
-__device__ inline Proposal draw_proposal(unsigned long long seed, unsigned chain,
-                                         unsigned long long step, int n_mol,
-                                         const int* mlen_chain, double max_t,
-                                         double max_r, int mode) {
-  uint2 key = make_uint2((unsigned)seed, (unsigned)(seed >> 32));
-  uint4 a = philox4x32_10(make_uint4((unsigned)step, (unsigned)(step >> 32), chain, 0u), key);
-  uint4 c = philox4x32_10(make_uint4((unsigned)step, (unsigned)(step >> 32), chain, 1u), key);
-  uint4 d = philox4x32_10(make_uint4((unsigned)step, (unsigned)(step >> 32), chain, 2u), key);
-  Proposal p;
-  p.mol = uidx(a.x, n_mol);
-  p.vertex = uidx(a.y, mlen_chain[p.mol] & 255);
-  p.mode = mode;
-  p.trig = 0;
-  p.dx = __dadd_rn(__dmul_rn(2.0 * max_t, u01(a.z)), -max_t);
-  p.dy = __dadd_rn(__dmul_rn(2.0 * max_t, u01(a.w)), -max_t);
-  p.dz = __dadd_rn(__dmul_rn(2.0 * max_t, u01(c.x)), -max_t);
-  if (mode == MCGPU_ROT_EULER) {
-    p.r0 = __dadd_rn(__dmul_rn(2.0 * max_r, u01(c.y)), -max_r);
-    p.r1 = __dadd_rn(__dmul_rn(2.0 * max_r, u01(c.z)), -max_r);
-    p.r2 = __dadd_rn(__dmul_rn(2.0 * max_r, u01(c.w)), -max_r);
-    p.r3 = 0.0;
-  } else {
-    double zc = __dadd_rn(__dmul_rn(2.0, u01(c.y)), -1.0);
-    double phi = __dmul_rn(6.283185307179586, u01(c.z));
-    double s = sqrt(__dadd_rn(1.0, -__dmul_rn(zc, zc)));
-    double sp, cp;
-    sincos(phi, &sp, &cp);
-    p.r0 = __dmul_rn(s, cp);
-    p.r1 = __dmul_rn(s, sp);
-    p.r2 = zc;
-    p.r3 = __dadd_rn(__dmul_rn(2.0 * max_r, u01(c.w)), -max_r);
-  }
-  p.u = u01(d.x);
-  return p;
-}
-
-// Rotation matrix of a proposal, applied to v = atom - pivot:
-// Euler: rotateX, then rotateY, then rotateZ (SimulationStep.cpp:400-422),
-// composed as separate rounded steps exactly like the reference.
+// The cosines and sines of a move's rotation, applied to v = atom - pivot:
+// rotateX, then rotateY, then rotateZ (SimulationStep.cpp:400-422), composed
+// as separate rounded steps exactly like the reference.
 struct Rot {
-  double cx, sx, cy, sy, cz, sz;   // Euler; axis form: cx=cos, sx=sin, cy=1-cos
-  double kx, ky, kz;               // axis form: unit axis
-  int mode;
+  double cx, sx, cy, sy, cz, sz;
 };
-
-__device__ inline Rot make_rot(const Proposal& p) {
-  Rot R;
-  R.mode = p.mode;
-  if (p.mode == MCGPU_ROT_EULER && p.trig) {
-    R.cx = p.cs[0]; R.sx = p.sn[0];
-    R.cy = p.cs[1]; R.sy = p.sn[1];
-    R.cz = p.cs[2]; R.sz = p.sn[2];
-  } else if (p.mode == MCGPU_ROT_EULER) {
-    sincos(__dmul_rn(p.r0, 3.14159265358979) / 180.0, &R.sx, &R.cx);
-    sincos(__dmul_rn(p.r1, 3.14159265358979) / 180.0, &R.sy, &R.cy);
-    sincos(__dmul_rn(p.r2, 3.14159265358979) / 180.0, &R.sz, &R.cz);
-  } else {
-    sincos(__dmul_rn(p.r3, 3.14159265358979) / 180.0, &R.sx, &R.cx);
-    R.cy = __dadd_rn(1.0, -R.cx);
-    R.kx = p.r0; R.ky = p.r1; R.kz = p.r2;
-  }
-  return R;
-}
 
 // Applies the rotation to v (in place).
 __device__ __forceinline__ void rot_apply(const Rot& R, double& vx, double& vy, double& vz) {
-  if (R.mode == MCGPU_ROT_EULER) {
-    double oy = vy, oz = vz;   // rotateX
-    vy = __dadd_rn(__dmul_rn(oy, R.cx), __dmul_rn(oz, R.sx));
-    vz = __dadd_rn(__dmul_rn(oz, R.cx), -__dmul_rn(oy, R.sx));
-    oz = vz;
-    double ox = vx;            // rotateY
-    vz = __dadd_rn(__dmul_rn(oz, R.cy), __dmul_rn(ox, R.sy));
-    vx = __dadd_rn(__dmul_rn(ox, R.cy), -__dmul_rn(oz, R.sy));
-    ox = vx;
-    oy = vy;                   // rotateZ
-    vx = __dadd_rn(__dmul_rn(ox, R.cz), __dmul_rn(oy, R.sz));
-    vy = __dadd_rn(__dmul_rn(oy, R.cz), -__dmul_rn(ox, R.sz));
-  } else {
-    // Rodrigues: v' = v c + (k x v) s + k (k.v)(1-c)
-    double kv = R.kx * vx + R.ky * vy + R.kz * vz;
-    double qx = R.ky * vz - R.kz * vy, qy = R.kz * vx - R.kx * vz, qz = R.kx * vy - R.ky * vx;
-    double x = vx * R.cx + qx * R.sx + R.kx * kv * R.cy;
-    double y = vy * R.cx + qy * R.sx + R.ky * kv * R.cy;
-    double z = vz * R.cx + qz * R.sx + R.kz * kv * R.cy;
-    vx = x; vy = y; vz = z;
-  }
+  double oy = vy, oz = vz;   // rotateX
+  vy = __dadd_rn(__dmul_rn(oy, R.cx), __dmul_rn(oz, R.sx));
+  vz = __dadd_rn(__dmul_rn(oz, R.cx), -__dmul_rn(oy, R.sx));
+  oz = vz;
+  double ox = vx;            // rotateY
+  vz = __dadd_rn(__dmul_rn(oz, R.cy), __dmul_rn(ox, R.sy));
+  vx = __dadd_rn(__dmul_rn(ox, R.cy), -__dmul_rn(oz, R.sy));
+  ox = vx;
+  oy = vy;                   // rotateZ
+  vx = __dadd_rn(__dmul_rn(ox, R.cz), __dmul_rn(oy, R.sz));
+  vy = __dadd_rn(__dmul_rn(oy, R.cz), -__dmul_rn(ox, R.sz));
 }
 
 // SimCalcs::makePeriodic (SimulationStep.cpp:377-385), FP64.

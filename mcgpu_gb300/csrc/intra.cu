@@ -47,27 +47,23 @@ __device__ __forceinline__ double intra_pair(const Pool& P, int i, int j, const 
   return lj + P.q[i] * P.q[j] * 332.06 * ri;
 }
 
-// Block-wide deterministic sum of three values (every thread gets them).
-__device__ __forceinline__ void block_sum3(double& a, double& b, double& c, double* red) {
-  for (int off = 16; off > 0; off >>= 1) {
-    a += __shfl_xor_sync(~0u, a, off);
-    b += __shfl_xor_sync(~0u, b, off);
-    c += __shfl_xor_sync(~0u, c, off);
-  }
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Block-wide deterministic sum (every thread gets it; at most 32 warps).  Warps
+// from `active` on hold zeros and add nothing.  FP64 issues once in 16 cycles
+// per SM, so the instructions of idle warps count: three values summed in every
+// lane of eight warps took 312 of them, this takes 5 per active warp and 5 per
+// warp.
+__device__ __forceinline__ double block_sum(double a, int active, double* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (w < active)
+    for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(~0u, a, off);
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) {
-    red[w] = a;
-    red[nw + w] = b;
-    red[2 * nw + w] = c;
-  }
+  if (lane == 0) red[w] = a;
   __syncthreads();
-  a = b = c = 0.0;
-  for (int k = 0; k < nw; k++) {
-    a += red[k];
-    b += red[nw + k];
-    c += red[2 * nw + k];
-  }
+  const int n = min(active, nw);
+  a = lane < n ? red[lane] : 0.0;
+  for (int off = 16; off > 0; off >>= 1)
+    if (off < n) a += __shfl_xor_sync(~0u, a, off);
+  return __shfl_sync(~0u, a, 0);
 }
 
 // SimCalcs::calcIntraMolecularEnergy (SimulationStep.cpp:80-129) of box
@@ -76,41 +72,41 @@ __device__ double intra_energy(const Pool& P, const IntraRows& R, const ChainHdr
                                double* red) {
   const int m = H.mol0 + mol;
   const int tid = threadIdx.x, nt = blockDim.x;
-  double ea = 0.0, eb = 0.0, ep = 0.0;
+  double sum = 0.0;
+  int items = 0;
   if (R.flex_angles) {
     const int s = R.m_astart[mol], e = s + R.m_acount[mol];
+    items = max(items, e - s);
     for (int k = s + tid; k < e; k += nt)
       if (R.a_var[k]) {
         const double d = R.a_eq[k] - R.a_size[k];
-        ea += R.a_k[k] * d * d;
+        sum += R.a_k[k] * d * d;
       }
   }
   if (R.flex_bonds) {
     const int s = R.m_bstart[mol], e = s + R.m_bcount[mol];
+    items = max(items, e - s);
     for (int k = s + tid; k < e; k += nt)
       if (R.b_var[k]) {
         const double d = R.b_eq[k] - R.b_len[k];
-        eb += R.b_k[k] * d * d;
+        sum += R.b_k[k] * d * d;
       }
   }
   if (R.flex_bonds || R.flex_angles) {
     const int a0 = P.mstart[m], len = P.mlen[m] & 255;
     const int ty = R.m_type[mol], n = R.t_natom[ty];
     const unsigned char* code = R.code + R.t_off[ty];
+    items = max(items, len * len);
     for (int q = tid; q < len * len; q += nt) {
       const int i = q / len, j = q - i * len;
       if (j <= i) continue;
       const int c = (i < n && j < n) ? code[i * n + j] : 2;
       if (c == 0) continue;
       const double e = intra_pair(P, a0 + i, a0 + j, H);
-      ep += c == 1 ? 0.5 * e : e;
+      sum += c == 1 ? 0.5 * e : e;
     }
   }
-  block_sum3(ea, eb, ep, red);
-  double out = 0.0;
-  if (R.flex_angles) out += ea;
-  if (R.flex_bonds) out += eb;
-  return out + ep;
+  return block_sum(sum, (items + 31) / 32, red);
 }
 
 // The molecule's mirrors after its atoms moved, and its radius (max
@@ -126,10 +122,12 @@ __device__ void refresh_flexible(const Pool& P, const ChainHdr& H, int m, double
                  dz = P.z[a0 + i] - P.z[an];
     r = fmax(r, sqrt(dx * dx + dy * dy + dz * dz));
   }
-  for (int off = 16; off > 0; off >>= 1) r = fmax(r, __shfl_xor_sync(~0u, r, off));
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // (only the warps that hold atoms)
+  const int w = threadIdx.x >> 5, nw = min((int)blockDim.x >> 5, (len + 31) / 32);
+  if (w < nw)
+    for (int off = 16; off > 0; off >>= 1) r = fmax(r, __shfl_xor_sync(~0u, r, off));
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[w] = r;
+  if ((threadIdx.x & 31) == 0 && w < nw) red[w] = r;
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int k = 0; k < nw; k++) r = fmax(r, red[k]);
@@ -338,11 +336,13 @@ __global__ void __launch_bounds__(kIntraThreads) k_intra_rollback(Pool P, IntraR
 constexpr int kLoopThreads = 256;
 constexpr int kLoopDrawCap = 1 << 20;
 
-// randomReal (MathLibrary.cpp:31-33) on the restated C-library stream,
-// operation by operation.
+// randomReal (MathLibrary.cpp:31-33) of a number of the restated C-library
+// stream, operation by operation.
+__device__ __forceinline__ double real_of(int32_t v, double start, double end) {
+  return __dadd_rn(__dmul_rn(__dsub_rn(end, start), crand_unit(v)), start);
+}
 __device__ __forceinline__ double loop_real(CRand& g, double start, double end) {
-  const double r = __ddiv_rn((double)crand_next(g), 2147483647.0);
-  return __dadd_rn(__dmul_rn(__dsub_rn(end, start), r), start);
+  return real_of(crand_next(g), start, end);
 }
 
 // acceptMove (SimulationStep.cpp:794-803): no draw for a decrease.
@@ -402,6 +402,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
   PlainLoop* L = task.L;
   __shared__ PlainLoop st;
   __shared__ Proposal prop;
+  __shared__ int32_t raw[8];
   __shared__ double red[3 * (kLoopThreads / 32)];
   __shared__ double sv[9];
   __shared__ int sel[kLoopSel];
@@ -420,22 +421,29 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
   }
   __syncthreads();
   for (int k = 0; k < n_steps; k++) {
-    if (tid == 0) {
+    if (w == 0) {
       // chooseMolecule and the seven intermolecularMove draws
-      // (SimulationStep.cpp:25-27, 527-535), clamped as the host loop clamps
-      CRand& g = st.rng;
-      const int mol = min((int)loop_real(g, 0, n), n - 1);
+      // (SimulationStep.cpp:25-27, 527-535), clamped as the host loop clamps:
+      // lane 0 takes the numbers, lane k forms the k-th real
+      if (lane == 0)
+        for (int q = 0; q < 8; q++) raw[q] = crand_next(st.rng);
+      __syncwarp();
+      const int32_t v = raw[lane & 7];
+      const int mol = min((int)real_of(raw[0], 0, n), n - 1);
       const int len = P.mlen[H.mol0 + mol] & 255;
-      memset(&prop, 0, sizeof(prop));
-      prop.mol = mol;
-      prop.mode = MCGPU_ROT_EULER;
-      prop.vertex = min((int)loop_real(g, 0, len), len - 1);
-      prop.dx = loop_real(g, -max_t, max_t);
-      prop.dy = loop_real(g, -max_t, max_t);
-      prop.dz = loop_real(g, -max_t, max_t);
-      prop.r0 = loop_real(g, -max_r, max_r);
-      prop.r1 = loop_real(g, -max_r, max_r);
-      prop.r2 = loop_real(g, -max_r, max_r);
+      const double top = lane < 5 ? max_t : max_r;
+      const double x = lane == 1 ? real_of(v, 0, len) : real_of(v, -top, top);
+      if (lane == 0) {
+        prop.mol = mol;
+        prop.trig = 0;
+      }
+      if (lane == 1) prop.vertex = min((int)x, len - 1);
+      if (lane == 2) prop.dx = x;
+      if (lane == 3) prop.dy = x;
+      if (lane == 4) prop.dz = x;
+      if (lane == 5) prop.r0 = x;
+      if (lane == 6) prop.r1 = x;
+      if (lane == 7) prop.r2 = x;
     }
     __syncthreads();
     const int mol = prop.mol, m = H.mol0 + mol;

@@ -16,9 +16,12 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 
 // Primary position wrapped into [0, L) (FP32), for the screen.
 __device__ __forceinline__ float4 wrap_pos(double x, double y, double z, const ChainHdr& H) {
-  double wx = x - H.L[0] * floor(x / H.L[0]);
-  double wy = y - H.L[1] * floor(y / H.L[1]);
-  double wz = z - H.L[2] * floor(z / H.L[2]);
+  // x / L through the header's 2^32 / L (FP64 divisions are slow; a quotient at
+  // an integer may round to either side of it, which moves the position by an
+  // edge: the screen's minimum image does not see it)
+  double wx = x - H.L[0] * floor(x * (H.fxinv[0] * 0x1p-32));
+  double wy = y - H.L[1] * floor(y * (H.fxinv[1] * 0x1p-32));
+  double wz = z - H.L[2] * floor(z * (H.fxinv[2] * 0x1p-32));
   return make_float4((float)wx, (float)wy, (float)wz, 0.f);
 }
 
@@ -129,14 +132,19 @@ __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Prop
     s.misc[kMiscQm] = __float_as_int(qsum);
   }
   if (!p) return;
+  // lane k forms the cosine and sine of the k-th Euler angle
+  double rc = 1.0, rs = 0.0;
+  if (p->trig) {
+    rc = lane == 0 ? p->cs[0] : lane == 1 ? p->cs[1] : p->cs[2];
+    rs = lane == 0 ? p->sn[0] : lane == 1 ? p->sn[1] : p->sn[2];
+  } else if (lane < 3) {
+    sincos(__dmul_rn(lane == 0 ? p->r0 : lane == 1 ? p->r1 : p->r2, 3.14159265358979) / 180.0, &rs,
+           &rc);
+  }
   Rot R;
-  if (lane == 0) R = make_rot(*p);
-  R.mode = p->mode;
-  R.cx = __shfl_sync(~0u, R.cx, 0); R.sx = __shfl_sync(~0u, R.sx, 0);
-  R.cy = __shfl_sync(~0u, R.cy, 0); R.sy = __shfl_sync(~0u, R.sy, 0);
-  R.cz = __shfl_sync(~0u, R.cz, 0); R.sz = __shfl_sync(~0u, R.sz, 0);
-  R.kx = __shfl_sync(~0u, R.kx, 0); R.ky = __shfl_sync(~0u, R.ky, 0);
-  R.kz = __shfl_sync(~0u, R.kz, 0);
+  R.cx = __shfl_sync(~0u, rc, 0); R.sx = __shfl_sync(~0u, rs, 0);
+  R.cy = __shfl_sync(~0u, rc, 1); R.sy = __shfl_sync(~0u, rs, 1);
+  R.cz = __shfl_sync(~0u, rc, 2); R.sz = __shfl_sync(~0u, rs, 2);
   __syncwarp();
   const int v = p->vertex;
   const double px = s.ox[v], py = s.oy[v], pz = s.oz[v];
