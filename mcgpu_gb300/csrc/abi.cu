@@ -529,7 +529,8 @@ struct mcgpu_box {
   double* partials = nullptr;
   unsigned* counter = nullptr;
   double* dout = nullptr;
-  double* hout = nullptr;  // pinned
+  double* hout = nullptr;  // pinned [4]; hout[3] holds the last finished call's number
+  unsigned call = 0;       // number of the last call whose results go to hout
   long long* dpairs = nullptr;  // atom pairs the plain energy kernels evaluated
   bool energy_ready = false;
   mcgpu_trace* dtrace = nullptr;
@@ -549,6 +550,36 @@ static int box_rows(mcgpu_box* b) {
   int rc = pool_chain_export(b->ctx, b->pool, b->ctx->stream);
   if (rc) return rc;
   b->rows_stale = false;
+  return MCGPU_OK;
+}
+
+// The word of b->hout that a plain kernel sets to its call's number.
+static unsigned* box_done(mcgpu_box* b) { return (unsigned*)(b->hout + 3); }
+
+// Waits for call number b->call by polling its word in pinned memory: the
+// results are there a few microseconds before a stream synchronisation returns
+// (and with no copy launched behind the kernel).  The stream is asked now and
+// then, so a launch that failed ends the wait with its error.
+static int box_wait(mcgpu_box* b) {
+  mcgpu_ctx* ctx = b->ctx;
+  const volatile unsigned* done = box_done(b);
+  for (unsigned spin = 1;; spin++) {
+    if (*done == b->call) break;
+    if ((spin & 0x3fff) == 0) {
+      const cudaError_t e = cudaStreamQuery(ctx->stream);
+      if (e == cudaErrorNotReady) {
+        cudaGetLastError();   // not an error: clear it
+        continue;
+      }
+      if (e != cudaSuccess)
+        return set_err(ctx, MCGPU_ERR_CUDA, "plain energy kernel failed: %s",
+                       cudaGetErrorString(e));
+      if (*done != b->call)
+        return set_err(ctx, MCGPU_ERR_DEVICE, "a plain energy kernel left no result");
+      break;
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
   return MCGPU_OK;
 }
 
@@ -614,6 +645,7 @@ extern "C" int mcgpu_box_upload(mcgpu_ctx* ctx, const mcgpu_box_desc* desc, int 
   b->queue = dalloc<unsigned>(1, &e);
   b->order = dalloc<int>(2, &e);   // chain 0, and a zero for its size
   if (e == cudaSuccess) e = cudaMallocHost((void**)&b->hout, 4 * sizeof(double));
+  if (e == cudaSuccess) b->hout[3] = 0.0;   // no call finished yet
   if (e == cudaSuccess) e = cudaMemsetAsync(b->counter, 0, 2 * sizeof(unsigned), ctx->stream);
   if (e == cudaSuccess) b->dpairs = dalloc<long long>(1, &e);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->dpairs, 0, sizeof(long long), ctx->stream);
@@ -674,11 +706,11 @@ extern "C" int mcgpu_mol_energy(mcgpu_box* b, int curr, int start, double* out) 
   const int nw = 4;
   SmemShape sh = shape_for(b->pool.max_len, nw);
   const int grid = box_grid(b, n - start);
-  CK(ctx, launch_mol_energy(b->precision == MCGPU_PREC_FP64, grid, nw * 32, sh, ctx->stream,
-                            b->pool.P, 0, curr, start, b->partials, b->counter, b->dout,
-                            b->dpairs));
+  const bool f64 = b->precision == MCGPU_PREC_FP64;
   if (b->intra_on) {
     // SimulationStep::calcMoleculeEnergy with ENABLE_INTRA (SimulationStep.cpp:15-18)
+    CK(ctx, launch_mol_energy(f64, grid, nw * 32, sh, ctx->stream, b->pool.P, 0, curr, start,
+                              b->partials, b->counter, b->dout, b->dpairs));
     CK(ctx, launch_intra_energy(b->pool.P, b->intra->R, 0, curr, b->dout + 1, ctx->stream));
     CK(ctx, cudaMemcpyAsync(b->hout, b->dout, 2 * sizeof(double), cudaMemcpyDeviceToHost,
                             ctx->stream));
@@ -686,8 +718,10 @@ extern "C" int mcgpu_mol_energy(mcgpu_box* b, int curr, int start, double* out) 
     *out = b->hout[0] + b->hout[1];
     return MCGPU_OK;
   }
-  CK(ctx, cudaMemcpyAsync(b->hout, b->dout, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
+  CK(ctx, launch_mol_energy(f64, grid, nw * 32, sh, ctx->stream, b->pool.P, 0, curr, start,
+                            b->partials, b->counter, b->hout, b->dpairs, box_done(b), ++b->call));
+  rc = box_wait(b);
+  if (rc) return rc;
   *out = b->hout[0];
   return MCGPU_OK;
 }
@@ -759,9 +793,9 @@ extern "C" int mcgpu_move_energies(mcgpu_box* b, int mol, const mcgpu_move* mv, 
   const int grid = box_grid(b, b->pool.n_mol);
   CK(ctx, launch_move_energies(b->precision == MCGPU_PREC_FP64, grid, nw * 32, sh, ctx->stream,
                                b->pool.P, 0, mol, host_proposal(mv), b->partials, b->counter,
-                               b->dout, b->dpairs));
-  CK(ctx, cudaMemcpyAsync(b->hout, b->dout, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
+                               b->hout, b->dpairs, box_done(b), ++b->call));
+  rc = box_wait(b);
+  if (rc) return rc;
   *e_old = b->hout[0];
   *e_new = b->hout[1];
   return MCGPU_OK;
@@ -811,6 +845,10 @@ static int run_plain_rigid(mcgpu_box* b, int n_steps, int fused, mcgpu_plain_sta
   const ChainHdr& h = b->pool.hdr[0];
   const int n = b->pool.n_mol;
   const double kT = h.kT, max_t = h.max_t, max_r = h.max_r;
+  const bool f64 = b->precision == MCGPU_PREC_FP64;
+  const int nw = 4, grid = box_grid(b, n);
+  const SmemShape sh = shape_for(b->pool.max_len, nw);
+  if (int rc = box_rows(b)) return rc;
   for (int step = 0; step < n_steps; step++) {
     // chooseMolecule (SimulationStep.cpp:25-27); rand() == RAND_MAX gives n,
     // clamped to n - 1 (the reference would read past its rows)
@@ -831,9 +869,18 @@ static int run_plain_rigid(mcgpu_box* b, int n_steps, int fused, mcgpu_plain_sta
     if (fused) {
       rc = mcgpu_move_energies(b, mol, &mv, &e_old, &e_new);
     } else {
-      rc = mcgpu_mol_energy(b, mol, 0, &e_old);
-      if (!rc) rc = mcgpu_change_molecule(b, mol, &mv);
-      if (!rc) rc = mcgpu_mol_energy(b, mol, 0, &e_new);
+      // the contract calls, launched one behind another with one wait: the
+      // old energy is not needed before the move
+      CK(b->ctx, launch_mol_energy(f64, grid, nw * 32, sh, b->ctx->stream, b->pool.P, 0, mol, 0,
+                                   b->partials, b->counter, b->hout, b->dpairs));
+      rc = mcgpu_change_molecule(b, mol, &mv);
+      if (rc) return rc;
+      CK(b->ctx, launch_mol_energy(f64, grid, nw * 32, sh, b->ctx->stream, b->pool.P, 0, mol, 0,
+                                   b->partials, b->counter, b->hout + 1, b->dpairs, box_done(b),
+                                   ++b->call));
+      rc = box_wait(b);
+      e_old = b->hout[0];
+      e_new = b->hout[1];
     }
     if (rc) return rc;
     // acceptMove (SimulationStep.cpp:794-803)

@@ -42,12 +42,16 @@ __global__ void k_nl_config(Pool P, const NlCfg* cfg);
 cudaError_t launch_nl_rebuild(Pool P, int max_cells, cudaStream_t st);
 __global__ void k_chain_export(Pool P, const int* mol_chain, const int* atom_mol, int a_begin,
                                int a_end);
+// out (and done, if any) may lie in pinned host memory: *done becomes `call`
+// once the results are there.
 cudaError_t launch_mol_energy(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
                               Pool P, int chain, int curr, int start, double* partials,
-                              unsigned* counter, double* out, long long* pairs = nullptr);
+                              unsigned* counter, double* out, long long* pairs = nullptr,
+                              unsigned* done = nullptr, unsigned call = 0);
 cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
                                  Pool P, int chain, int mol, Proposal prop, double* partials,
-                                 unsigned* counter, double* out, long long* pairs = nullptr);
+                                 unsigned* counter, double* out, long long* pairs = nullptr,
+                                 unsigned* done = nullptr, unsigned call = 0);
 // emol[m] with the sum over the chains' molecules of E(m, j > m).
 cudaError_t launch_mol_pair_sums(bool f64, int n_mol, SmemShape sh, cudaStream_t st,
                                  const Pool& P, const int* mol_chain, double* emol);

@@ -46,6 +46,15 @@ __device__ bool arrive_last(unsigned* counter) {
 
 // ---- plain contract ---------------------------------------------------------
 
+// Publishes a plain kernel's results to the host: `out` and `done` lie in pinned
+// host memory, and the host polls `done` for the call's number.
+__device__ __forceinline__ void host_done(unsigned* done, unsigned call) {
+  if (done) {
+    __threadfence_system();
+    *(volatile unsigned*)done = call;
+  }
+}
+
 // Energy of molecule `curr` against chain-local candidates [start, n_mol)
 // (BruteForceCalcs::calcMolecularEnergyContribution, BruteForceStep.cpp:
 // 15-46).  Each CTA takes an equal slice of the candidates.
@@ -53,7 +62,8 @@ template <bool F64>
 __global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr, int start,
                                                     SmemShape shape, double* partials,
                                                     unsigned* counter, double* out,
-                                                    long long* pairs) {
+                                                    long long* pairs, unsigned* done,
+                                                    unsigned call) {
   extern __shared__ __align__(16) char smem[];
   const ChainHdr& H = P.hdr[chain];
   Group g{(int)threadIdx.x, (int)blockDim.x, 1};
@@ -80,6 +90,7 @@ __global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr,
       for (unsigned b = 0; b < gridDim.x; b++) sum += ((volatile double*)partials)[b];
       out[0] = sum;
       *counter = 0;
+      host_done(done, call);
     }
   }
 }
@@ -91,7 +102,8 @@ template <bool F64>
 __global__ void __launch_bounds__(256) k_move_energies(Pool P, int chain, int mol, Proposal prop,
                                                        SmemShape shape, double* partials,
                                                        unsigned* counter, double* out,
-                                                       long long* pairs) {
+                                                       long long* pairs, unsigned* done,
+                                                       unsigned call) {
   extern __shared__ __align__(16) char smem[];
   const ChainHdr& H = P.hdr[chain];
   Group g{(int)threadIdx.x, (int)blockDim.x, 1};
@@ -135,6 +147,7 @@ __global__ void __launch_bounds__(256) k_move_energies(Pool P, int chain, int mo
       out[0] = so;
       out[1] = sn;
       *counter = 0;
+      host_done(done, call);
     }
   }
 }
@@ -738,25 +751,27 @@ __global__ void __launch_bounds__(512, 1) k_chain_steps_wide(Pool P, ChainLaunch
 
 cudaError_t launch_mol_energy(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
                               Pool P, int chain, int curr, int start, double* partials,
-                              unsigned* counter, double* out, long long* pairs) {
+                              unsigned* counter, double* out, long long* pairs, unsigned* done,
+                              unsigned call) {
   if (f64)
     k_mol_energy<true><<<grid, threads, sh.bytes(), st>>>(P, chain, curr, start, sh, partials,
-                                                          counter, out, pairs);
+                                                          counter, out, pairs, done, call);
   else
     k_mol_energy<false><<<grid, threads, sh.bytes(), st>>>(P, chain, curr, start, sh, partials,
-                                                           counter, out, pairs);
+                                                           counter, out, pairs, done, call);
   return cudaGetLastError();
 }
 
 cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
                                  Pool P, int chain, int mol, Proposal prop, double* partials,
-                                 unsigned* counter, double* out, long long* pairs) {
+                                 unsigned* counter, double* out, long long* pairs, unsigned* done,
+                                 unsigned call) {
   if (f64)
     k_move_energies<true><<<grid, threads, sh.bytes(), st>>>(P, chain, mol, prop, sh, partials,
-                                                             counter, out, pairs);
+                                                             counter, out, pairs, done, call);
   else
     k_move_energies<false><<<grid, threads, sh.bytes(), st>>>(P, chain, mol, prop, sh, partials,
-                                                              counter, out, pairs);
+                                                              counter, out, pairs, done, call);
   return cudaGetLastError();
 }
 
