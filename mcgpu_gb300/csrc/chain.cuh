@@ -261,9 +261,9 @@ __device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const 
         if (u3)
           batch_u3(P, H, s, mi, rj, head, count, lane, acc, ljmask);
         else if (precise)
-          batch_ff<true, false>(P, H, s, mi, rj, head, count, lane, T, acc);
+          batch_ff<true>(P, H, s, mi, rj, head, count, lane, T, acc);
         else
-          batch_ff<false, false>(P, H, s, mi, rj, head, count, lane, T, acc);
+          batch_ff<false>(P, H, s, mi, rj, head, count, lane, T, acc);
         head += count;
       }
       __syncwarp();

@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
       if (w == 0) stage(P, H, m, &prop, s, lane);
       grp.sync();
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, np);
+      warp_eval<F64, false>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, s.lj + w * kRing, lane, eo, en, np);
       group_reduce(grp, s, eo, en, np);
       if (tid == 0) {
         const double de = en - eo;
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     grp.sync();
     {
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, np);
+      warp_eval<F64, false>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, s.lj + w * kRing, lane, eo, en, np);
       group_reduce(grp, s, eo, en, np);
     }
     const double e_old = eo + ei_old;
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     np = 0;
     {
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, lane, H.tpm, eo, en, np);
+      warp_eval<F64, false>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, s.lj + w * kRing, lane, eo, en, np);
       group_reduce(grp, s, eo, en, np);
     }
     if (tid == 0) {

@@ -55,9 +55,20 @@ __device__ __forceinline__ void host_done(unsigned* done, unsigned call) {
   }
 }
 
+// Sum of the grid's partials p[0], p[stride], ... by one warp, every lane: lane
+// l adds every 32nd, then a butterfly (one after another by one thread, each an
+// L2 round trip, they took 22 of the 39 us of a 32-CTA launch).
+__device__ __forceinline__ double sum_partials(const double* p, int stride, int lane) {
+  double v = 0.0;
+  for (unsigned b = lane; b < gridDim.x; b += 32) v += __ldcg(p + (size_t)b * stride);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(~0u, v, off);
+  return v;
+}
+
 // Energy of molecule `curr` against chain-local candidates [start, n_mol)
 // (BruteForceCalcs::calcMolecularEnergyContribution, BruteForceStep.cpp:
-// 15-46).  Each CTA takes an equal slice of the candidates.
+// 15-46).  The candidates are dealt over the warps of the grid.
 template <bool F64>
 __global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr, int start,
                                                     SmemShape shape, double* partials,
@@ -73,25 +84,25 @@ __global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr,
   if (w == 0) stage(P, H, m, nullptr, s, lane);
   g.sync();
   const MovedInfo mi = load_moved(s);
-  const int n_cand = H.n_mol - start;
-  const int chunk = ((n_cand + gridDim.x - 1) / gridDim.x + 31) & ~31;
-  const int cb = H.mol0 + start + blockIdx.x * chunk;
-  const int ce = min(cb + chunk, H.mol0 + H.n_mol);
   double eo = 0.0, en = 0.0;
   long long np = 0;
-  if (cb < ce) warp_eval<F64>(P, H, s, mi, cb, ce, w, nw, lane, H.tpm, eo, en, np);
+  warp_eval<F64, true>(P, H, s, mi, H.mol0 + start, H.mol0 + H.n_mol, (int)blockIdx.x * nw + w,
+                 (int)gridDim.x * nw, s.lj + w * kRing, lane, eo, en, np);
   group_reduce(g, s, eo, en, np);
+  __shared__ int last;
   if (threadIdx.x == 0) {
     if (pairs) atomicAdd((unsigned long long*)pairs, (unsigned long long)np);
     partials[blockIdx.x] = eo;
-    if (arrive_last(counter)) {
-      __threadfence();
-      double sum = 0.0;
-      for (unsigned b = 0; b < gridDim.x; b++) sum += ((volatile double*)partials)[b];
-      out[0] = sum;
-      *counter = 0;
-      host_done(done, call);
-    }
+    last = arrive_last(counter) ? 1 : 0;
+  }
+  __syncthreads();
+  if (!last || w != 0) return;
+  __threadfence();
+  const double sum = sum_partials(partials, 1, lane);
+  if (lane == 0) {
+    out[0] = sum;
+    *counter = 0;
+    host_done(done, call);
   }
 }
 
@@ -113,12 +124,10 @@ __global__ void __launch_bounds__(256) k_move_energies(Pool P, int chain, int mo
   if (w == 0) stage(P, H, m, &prop, s, lane);
   g.sync();
   const MovedInfo mi = load_moved(s);
-  const int chunk = ((H.n_mol + gridDim.x - 1) / gridDim.x + 31) & ~31;
-  const int cb = H.mol0 + blockIdx.x * chunk;
-  const int ce = min(cb + chunk, H.mol0 + H.n_mol);
   double eo = 0.0, en = 0.0;
   long long np = 0;
-  if (cb < ce) warp_eval<F64>(P, H, s, mi, cb, ce, w, nw, lane, H.tpm, eo, en, np);
+  warp_eval<F64, true>(P, H, s, mi, H.mol0, H.mol0 + H.n_mol, (int)blockIdx.x * nw + w,
+                 (int)gridDim.x * nw, s.lj + w * kRing, lane, eo, en, np);
   group_reduce(g, s, eo, en, np);
   __shared__ int last;
   if (threadIdx.x == 0) {
@@ -138,12 +147,8 @@ __global__ void __launch_bounds__(256) k_move_energies(Pool P, int chain, int mo
       rb[2 * H.max_len + i] = s.oz[i];
     }
     commit(P, s, mi, lane);
+    const double so = sum_partials(partials, 2, lane), sn = sum_partials(partials + 1, 2, lane);
     if (lane == 0) {
-      double so = 0.0, sn = 0.0;
-      for (unsigned b = 0; b < gridDim.x; b++) {
-        so += ((volatile double*)partials)[2 * b];
-        sn += ((volatile double*)partials)[2 * b + 1];
-      }
       out[0] = so;
       out[1] = sn;
       *counter = 0;
@@ -349,7 +354,8 @@ __global__ void __launch_bounds__(256) k_pair_sums32(Pool P0, const LoopTask* ta
   const MovedInfo mi = load_moved(s);
   double eo = 0.0, en = 0.0;
   long long np = 0;
-  warp_eval<false>(P, H, s, mi, m + 1, H.mol0 + H.n_mol, w, nw, lane, H.tpm, eo, en, np);
+  warp_eval<false, false>(P, H, s, mi, m + 1, H.mol0 + H.n_mol, w, nw, s.lj + w * kRing, lane, eo, en,
+                   np);
   group_reduce(g, s, eo, en, np);
   if (threadIdx.x == 0) emol[m] = eo;
 }

@@ -375,9 +375,8 @@ __device__ __forceinline__ float sum_moved32_cf(const float4* o, const float4* l
 // (fixed point -> FP32, or double-float when PRECISE) and image flags, lane
 // tl takes neighbour atoms tl, tl+T, ... against every atom of the moved
 // molecule, and the team's FP32 partial of the entry is added in
-// double-float to the team leader's accumulators.  LO: the plain path, whose
-// FP32 offsets carry low parts (aofl, l_old/l_new).
-template <bool PRECISE, bool LO>
+// double-float to the team leader's accumulators.  (Chains of several species.)
+template <bool PRECISE>
 __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                          const MovedInfo& mi, const int* rj, int head, int count,
                                          int lane, int T, AccFF& acc) {
@@ -391,19 +390,11 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
       const int j = jf >> 4;
       f = jf & 15;
       float mrj;
-      if (!LO && H.uniform) {
-        // uniform chain: the neighbour's rows follow from its index
-        b0 = H.atom0 + (j - H.mol0) * H.ulen;
-        lenj = H.ulen;
-        actj = H.uact;
-        mrj = H.umrad;
-      } else {
-        b0 = P.mstart[j];
-        const int lw = P.mlen[j];
-        lenj = lw & 255;
-        actj = lw >> 8;
-        mrj = P.mrad[j];
-      }
+      b0 = P.mstart[j];
+      const int lw = P.mlen[j];
+      lenj = lw & 255;
+      actj = lw >> 8;
+      mrj = P.mrad[j];
       const uint4 fj = P.mfix[j];
       const float rr = mi.rad + mrj;
       if (f & kInOld) {
@@ -419,8 +410,6 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
     for (int b = b0 + tl; b < b0 + lenj; b += T) {
       const float4 ob = P.aoff[b];
       const float2 qb = P.aeq[b];
-      float4 obl = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (LO && PRECISE) obl = P.aofl[b];
       if (f & kInOld) {
         float3 bh = make_float3(Do.x + ob.x, Do.y + ob.y, Do.z + ob.z), bl = Dol;
         if (PRECISE) {
@@ -428,11 +417,11 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
           const float ex = (Do.x - (bh.x - (bh.x - Do.x))) + (ob.x - (bh.x - Do.x));
           const float ey = (Do.y - (bh.y - (bh.y - Do.y))) + (ob.y - (bh.y - Do.y));
           const float ez = (Do.z - (bh.z - (bh.z - Do.z))) + (ob.z - (bh.z - Do.z));
-          bl = make_float3(ex + (Dol.x + obl.x), ey + (Dol.y + obl.y), ez + (Dol.z + obl.z));
+          bl = make_float3(ex + Dol.x, ey + Dol.y, ez + Dol.z);
         }
         so += (f & kWrapOld)
-                  ? sum_moved32_wrap<PRECISE, LO>(s.o_old, s.l_old, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
-                  : sum_moved32_cf<PRECISE, LO>(s.o_old, s.l_old, s.eq, mi.len, false, bh, bl, ob.w, qb,
+                  ? sum_moved32_wrap<PRECISE, false>(s.o_old, nullptr, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
+                  : sum_moved32_cf<PRECISE, false>(s.o_old, nullptr, s.eq, mi.len, false, bh, bl, ob.w, qb,
                                             mi.qm, sa);
       }
       if (f & kInNew) {
@@ -441,11 +430,11 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
           const float ex = (Dn.x - (bh.x - (bh.x - Dn.x))) + (ob.x - (bh.x - Dn.x));
           const float ey = (Dn.y - (bh.y - (bh.y - Dn.y))) + (ob.y - (bh.y - Dn.y));
           const float ez = (Dn.z - (bh.z - (bh.z - Dn.z))) + (ob.z - (bh.z - Dn.z));
-          bl = make_float3(ex + (Dnl.x + obl.x), ey + (Dnl.y + obl.y), ez + (Dnl.z + obl.z));
+          bl = make_float3(ex + Dnl.x, ey + Dnl.y, ez + Dnl.z);
         }
         sn += (f & kWrapNew)
-                  ? sum_moved32_wrap<PRECISE, LO>(s.o_new, s.l_new, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
-                  : sum_moved32_cf<PRECISE, LO>(s.o_new, s.l_new, s.eq, mi.len, true, bh, bl, ob.w, qb,
+                  ? sum_moved32_wrap<PRECISE, false>(s.o_new, nullptr, s.eq, mi.len, bh, bl, ob.w, qb, H, sa)
+                  : sum_moved32_cf<PRECISE, false>(s.o_new, nullptr, s.eq, mi.len, true, bh, bl, ob.w, qb,
                                             mi.qm, sa);
       }
     }
@@ -761,20 +750,112 @@ __device__ __forceinline__ void batch_f64(const Pool& P, const ChainHdr& H, cons
                 });
 }
 
-// One warp screens candidates [c_begin, c_end) in warp-strided rounds of 32
-// (round r of warp w covers c_begin + (r*nw + w)*32 + lane), appends hits to
-// its ring and evaluates them in batches of 32.  FP32 pairs accumulate in
-// double-float and are added to the FP64 sums at the end.
-template <bool F64>
-__device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSmem& s, const MovedInfo& mi,
-                          int c_begin, int c_end, int w, int nw, int lane, int T, double& eo,
-                          double& en, long long& np) {
-  int* rj = s.lj + w * kRing;
+// FP32 pair batch of `count` (1..32) ring entries from `head` on the plain path
+// (offsets with their low parts), the items (placement, entry, neighbour atom)
+// dealt to the lanes as batch_items64 deals them; each item's sum over the
+// moved molecule's atoms is added in double-float.
+template <bool PRECISE>
+__device__ __forceinline__ void batch_items32(const Pool& P, const ChainHdr& H,
+                                              const GroupSmem& s, const MovedInfo& mi,
+                                              const int* rj, int head, int count, int lane,
+                                              AccFF& acc) {
+  const int two = mi.states == 3 ? 2 : 1;
+  int pref = 0, total;
+  const bool uni = H.uniform != 0;
+  if (uni) {
+    total = count * H.ulen;
+    if (lane < count)
+      acc.np += (long long)__popc(rj[(head + lane) & (kRing - 1)] & (kInOld | kInNew)) *
+                (mi.act * H.uact);
+  } else {
+    int len = 0;
+    if (lane < count) {
+      const int jf = rj[(head + lane) & (kRing - 1)];
+      const int lw = P.mlen[jf >> 4];
+      len = lw & 255;
+      acc.np += (long long)__popc(jf & (kInOld | kInNew)) * (mi.act * (lw >> 8));
+    }
+    pref = len;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(~0u, pref, off);
+      if (lane >= off) pref += v;
+    }
+    total = __shfl_sync(~0u, pref, 31);
+    pref -= len;
+  }
+  const int items = total * two;
+  for (int base = 0; base < items; base += 32) {
+    const int it = base + lane;
+    const bool p = it >= total || mi.states == 2;
+    const int local = it >= total ? it - total : it;
+    int e, k;
+    if (uni) {
+      k = local / count;
+      e = local - k * count;
+    } else {
+      e = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int at = e + step;
+        const int v = __shfl_sync(~0u, pref, at & 31);
+        if (at < count && v <= local) e = at;
+      }
+      k = local - __shfl_sync(~0u, pref, e);
+    }
+    if (it >= items) continue;
+    const int jf = rj[(head + e) & (kRing - 1)];
+    if (!(jf & (p ? kInNew : kInOld))) continue;
+    const int j = jf >> 4;
+    const int b = (uni ? H.atom0 + (j - H.mol0) * H.ulen : P.mstart[j]) + k;
+    const uint4 fj = P.mfix[j];
+    const float4 ob = P.aoff[b];
+    const float2 qb = P.aeq[b];
+    float4 obl = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (PRECISE) obl = P.aofl[b];
+    // mrad, not the header's radius: a flexible molecule's changes
+    const float rr = mi.rad + P.mrad[j];
+    const uint4 fm = p ? mi.fx_new : mi.fx_old;
+    float3 D, bl = make_float3(0.f, 0.f, 0.f);
+    if (PRECISE) fixdiff_ff(fj, fm, H, D, bl); else D = fixdiff(fj, fm, H);
+    const float3 bh = make_float3(D.x + ob.x, D.y + ob.y, D.z + ob.z);
+    if (PRECISE) {
+      // two-sum of D + o_b per axis, then the low parts
+      const float ex = (D.x - (bh.x - (bh.x - D.x))) + (ob.x - (bh.x - D.x));
+      const float ey = (D.y - (bh.y - (bh.y - D.y))) + (ob.y - (bh.y - D.y));
+      const float ez = (D.z - (bh.z - (bh.z - D.z))) + (ob.z - (bh.z - D.z));
+      bl = make_float3(ex + (bl.x + obl.x), ey + (bl.y + obl.y), ez + (bl.z + obl.z));
+    }
+    float sa = 0.f;
+    const float sp =
+        needs_wrap(D, rr, H)
+            ? sum_moved32_wrap<PRECISE, true>(p ? s.o_new : s.o_old, p ? s.l_new : s.l_old, s.eq,
+                                              mi.len, bh, bl, ob.w, qb, H, sa)
+            : sum_moved32_cf<PRECISE, true>(p ? s.o_new : s.o_old, p ? s.l_new : s.l_old, s.eq,
+                                            mi.len, p, bh, bl, ob.w, qb, mi.qm, sa);
+    if (p)
+      ff_add(acc.nh, acc.nl, sp);
+    else
+      ff_add(acc.oh, acc.ol, sp);
+  }
+}
+
+// Warp w of nw screens its share of candidates [c_begin, c_end) in rounds of 32,
+// appends hits to its ring rj and evaluates them in batches of 32.  DEALT: the
+// warps of a whole grid, each with every nw-th candidate (neighbours in space
+// are neighbours in index on a lattice start or in a file: of 128 warps with
+// 32 consecutive candidates a few had all of a molecule's neighbours); the warps
+// of one CTA take 32 consecutive ones in turn, one load each.  FP32 pairs
+// accumulate in double-float and are added to the FP64 sums at the end.
+template <bool F64, bool DEALT>
+__device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSmem& s,
+                                 const MovedInfo& mi, int c_begin, int c_end, int w, int nw,
+                                 int* rj, int lane, double& eo, double& en, long long& np) {
   int head = 0, tail = 0;
   const unsigned lt = lanemask_lt();
   AccFF acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0};
-  for (int base = c_begin + w * 32; base < c_end; base += nw * 32) {
-    const int j = base + lane;
+  for (int base = c_begin + (DEALT ? w : w * 32); base < c_end; base += nw * 32) {
+    const int j = base + (DEALT ? lane * nw : lane);
     int f = 0;
     // the FP32 screen with the FP64 re-test inside its guard band gives the
     // FP64 test's in-range set exactly, for FP64 and FP32 pair terms alike
@@ -782,28 +863,20 @@ __device__ inline void warp_eval(const Pool& P, const ChainHdr& H, const GroupSm
     const unsigned bal = __ballot_sync(~0u, f != 0);
     if (f) rj[(tail + __popc(bal & lt)) & (kRing - 1)] = (j << 4) | f;
     tail += __popc(bal);
-    if (tail - head >= 32) {
+    const bool last = base + nw * 32 >= c_end;
+    while (tail - head >= 32 || (last && tail > head)) {
+      const int count = min(32, tail - head);
       __syncwarp();
       if (F64)
-        batch_f64(P, H, s, mi, rj, head, 32, lane, eo, en, np);
+        batch_f64(P, H, s, mi, rj, head, count, lane, eo, en, np);
       else if (H.precise)
-        batch_ff<true, true>(P, H, s, mi, rj, head, 32, lane, T, acc);
+        batch_items32<true>(P, H, s, mi, rj, head, count, lane, acc);
       else
-        batch_ff<false, true>(P, H, s, mi, rj, head, 32, lane, T, acc);
-      head += 32;
+        batch_items32<false>(P, H, s, mi, rj, head, count, lane, acc);
+      head += count;
       __syncwarp();
     }
   }
-  __syncwarp();
-  if (tail > head) {
-    if (F64)
-      batch_f64(P, H, s, mi, rj, head, tail - head, lane, eo, en, np);
-    else if (H.precise)
-      batch_ff<true, true>(P, H, s, mi, rj, head, tail - head, lane, T, acc);
-    else
-      batch_ff<false, true>(P, H, s, mi, rj, head, tail - head, lane, T, acc);
-  }
-  __syncwarp();
   if (!F64) {
     eo += (double)acc.oh + (double)acc.ol;
     en += (double)acc.nh + (double)acc.nl;
