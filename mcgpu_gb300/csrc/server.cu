@@ -67,6 +67,9 @@ constexpr long long kBytesAtom = 6 * 8 + 16 + 16 + 8 + 16 + 4;          // 108
 constexpr long long kBytesMol = 4 + 4 + 8 + 16 + 4 + 16 + 4 + 8 + 8 + 16;  // 88
 constexpr long long kBytesPidx = 4 + 16;                                  // 20
 
+// Warps of a group for jobs of molecules of more than kWideAtoms atoms.
+constexpr int kWideWarps = 16, kWideAtoms = 4;
+
 struct Job {
   int64_t id = 0;
   HostPool hp;  // the job's rows as chain 0 at offset 0
@@ -96,8 +99,8 @@ struct mcgpu_server {
   std::deque<mcgpu_job_result> done;
   long long in_use = 0;
   int64_t next_id = 1, finished = 0;
-  cudaStream_t copy = nullptr;
-  cudaEvent_t ev_round = nullptr, ev_copy = nullptr;
+  cudaStream_t copy = nullptr, side = nullptr;   // uploads; the second kind's round
+  cudaEvent_t ev_round = nullptr, ev_copy = nullptr, ev_fork = nullptr, ev_join = nullptr;
   // GPU time of the rounds (chain kernel + volume phase), and the atom pairs
   // the retired jobs evaluated (device-counted)
   cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
@@ -106,9 +109,14 @@ struct mcgpu_server {
   bool round_in_flight = false, copies_pending = false;
   int gw = 8, grid = 1, smem = 0;
   SmemShape shape{};
+  // groups of kWideWarps for jobs of larger molecules (wide_grid 0: the tile's
+  // own groups for every job)
+  int wide_grid = 0, wide_smem = 0;
+  SmemShape wide{};
   // device scratch
-  unsigned* sched = nullptr;   // steps each job has taken in a round (slots)
-  // order [slots] | act_slot [slots] | act_m0 [slots] | act_pref [slots+1] | sizes [slots]
+  unsigned* sched = nullptr;   // steps each job has taken in a round (slots, per kind)
+  // per kind (see launch_round): order [slots] | act_slot [slots] | act_m0 [slots] |
+  // act_pref [slots+1] | sizes [slots]
   int* dlist = nullptr;
   int* dinit = nullptr;  // per slot: (slot, m0, 0, n_mol) range of a job being initialised
   VolMove* vm = nullptr;
@@ -116,7 +124,7 @@ struct mcgpu_server {
   double2* eabs2 = nullptr;
   double2* vsum = nullptr;
   double2* vsum_abs = nullptr;
-  int* vlist = nullptr;        // chains of a re-take (3 * slots + 3)
+  int* vlist = nullptr;        // chains of a re-take (3 * slots + 3, per kind)
   // pinned host buffers
   ChainHdr* hmirror = nullptr;
   int* hlist = nullptr;
@@ -160,18 +168,18 @@ int server_alloc(mcgpu_server* s) {
   dp.n_mol = (int)nm;
   dp.n_pidx = (int)np;
   dp.max_len = ml;
-  s->sched = dalloc<unsigned>(nc, &e);
-  s->dlist = dalloc<int>(5 * (size_t)nc + 1, &e);
+  s->sched = dalloc<unsigned>(2 * (size_t)nc, &e);
+  s->dlist = dalloc<int>(2 * (5 * (size_t)nc + 1), &e);
   s->dinit = dalloc<int>(4 * (size_t)nc, &e);
   s->vm = dalloc<VolMove>(nc, &e);
   s->emol2 = dalloc<double2>(nm, &e);
   s->eabs2 = dalloc<double2>(nm, &e);
   s->vsum = dalloc<double2>(nc, &e);
   s->vsum_abs = dalloc<double2>(nc, &e);
-  s->vlist = dalloc<int>(3 * (size_t)nc + 3, &e);
+  s->vlist = dalloc<int>(2 * (3 * (size_t)nc + 3), &e);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.hdr, 0, sizeof(ChainHdr) * nc, ctx->stream);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&s->hmirror, sizeof(ChainHdr) * nc);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&s->hlist, sizeof(int) * (5 * (size_t)nc + 1));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&s->hlist, sizeof(int) * 2 * (5 * (size_t)nc + 1));
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess)
     return set_err(ctx, MCGPU_ERR_NOMEM, "server arena allocation failed: %s", cudaGetErrorString(e));
@@ -191,7 +199,10 @@ void server_free(mcgpu_server* s) {
   if (s->ev_t0) cudaEventDestroy(s->ev_t0);
   if (s->ev_t1) cudaEventDestroy(s->ev_t1);
   if (s->ev_copy) cudaEventDestroy(s->ev_copy);
+  if (s->ev_fork) cudaEventDestroy(s->ev_fork);
+  if (s->ev_join) cudaEventDestroy(s->ev_join);
   if (s->copy) cudaStreamDestroy(s->copy);
+  if (s->side) cudaStreamDestroy(s->side);
   for (Job* j : s->slot_job) delete j;
   for (Job* j : s->queue) delete j;
 }
@@ -390,69 +401,97 @@ int launch_round(mcgpu_server* s) {
   mcgpu_ctx* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   const int nc = s->cfg.max_slots;
-  std::vector<int> act;
+  // kind 0: the tile's groups; kind 1: wide groups (the rule is the job's own,
+  // as its energies' last bits depend on the width)
+  std::vector<int> act[2];
   for (int slot = 0; slot < nc; slot++) {
-    s->in_round[slot] = s->slot_job[slot] != nullptr;
-    if (s->slot_job[slot]) act.push_back(slot);
+    const Job* j = s->slot_job[slot];
+    s->in_round[slot] = j != nullptr;
+    if (j) act[s->wide_grid > 0 && j->hp.max_len > kWideAtoms ? 1 : 0].push_back(slot);
   }
-  if (act.empty()) return MCGPU_OK;
-  // cost-descending order: screen ~ n_mol, pairs ~ max_len^2
-  std::stable_sort(act.begin(), act.end(), [&](int a, int b) {
-    const Job* ja = s->slot_job[a];
-    const Job* jb = s->slot_job[b];
-    return (double)ja->n_mol * (1 + ja->hp.max_len) > (double)jb->n_mol * (1 + jb->hp.max_len);
-  });
-  int* order = s->hlist;
-  int* aslot = s->hlist + nc;
-  int* am0 = s->hlist + 2 * nc;
-  int* apref = s->hlist + 3 * nc;
-  int* sizes = s->hlist + 4 * nc + 1;
-  int n_npt = 0, total = 0;
-  bool has64 = false, has32 = false;
-  for (size_t i = 0; i < act.size(); i++) {
-    order[i] = act[i];
-    const Job* j = s->slot_job[act[i]];
-    sizes[i] = j->n_mol;
-    if (!j->npt) continue;
-    has64 = has64 || !j->vol_mixed;
-    has32 = has32 || j->vol_mixed;
-    aslot[n_npt] = act[i];
-    am0[n_npt] = (int)j->m0;
-    apref[n_npt] = total;
-    total += j->n_mol;
-    n_npt++;
+  if (act[0].empty() && act[1].empty()) return MCGPU_OK;
+  struct Kind {
+    int n_npt = 0, total = 0;
+    bool has64 = false, has32 = false;
+  } kind[2];
+  for (int q = 0; q < 2; q++) {
+    // cost-descending order: screen ~ n_mol, pairs ~ max_len^2
+    std::stable_sort(act[q].begin(), act[q].end(), [&](int a, int b) {
+      const Job* ja = s->slot_job[a];
+      const Job* jb = s->slot_job[b];
+      return (double)ja->n_mol * (1 + ja->hp.max_len) > (double)jb->n_mol * (1 + jb->hp.max_len);
+    });
+    int* order = s->hlist + q * (5 * nc + 1);
+    int* aslot = order + nc;
+    int* am0 = order + 2 * nc;
+    int* apref = order + 3 * nc;
+    int* sizes = order + 4 * nc + 1;
+    Kind& k = kind[q];
+    for (size_t i = 0; i < act[q].size(); i++) {
+      order[i] = act[q][i];
+      const Job* j = s->slot_job[act[q][i]];
+      sizes[i] = j->n_mol;
+      if (!j->npt) continue;
+      k.has64 = k.has64 || !j->vol_mixed;
+      k.has32 = k.has32 || j->vol_mixed;
+      aslot[k.n_npt] = act[q][i];
+      am0[k.n_npt] = (int)j->m0;
+      apref[k.n_npt] = k.total;
+      k.total += j->n_mol;
+      k.n_npt++;
+    }
+    apref[k.n_npt] = k.total;
   }
-  apref[n_npt] = total;
-  CK(ctx, cudaMemcpyAsync(s->dlist, s->hlist, sizeof(int) * (5 * (size_t)nc + 1),
+  CK(ctx, cudaMemcpyAsync(s->dlist, s->hlist, sizeof(int) * 2 * (5 * (size_t)nc + 1),
                           cudaMemcpyHostToDevice, st));
   if (s->copies_pending) {
     CK(ctx, cudaStreamWaitEvent(st, s->ev_copy, 0));
     s->copies_pending = false;
   }
   CK(ctx, cudaEventRecord(s->ev_t0, st));
-  CK(ctx, cudaMemsetAsync(s->sched, 0, sizeof(unsigned) * act.size(), st));
-  const int need = ((int)act.size() + s->cfg.chains_per_cta - 1) / s->cfg.chains_per_cta;
-  const int grid = std::max(1, std::min(need, s->grid));
-  // a job runs a whole round on one group: its energy sums must not depend on
-  // the other jobs
-  ChainLaunch A{s->cfg.round_steps, s->cfg.round_steps, (int)act.size(), s->gw, s->sched, s->dlist,
-                s->dlist + 4 * nc + 1, s->shape};
-  A.lanes_cap = s->cfg.lanes_per_molecule;
-  if (s->cfg.threads > 256)
-    k_chain_steps_wide<<<grid, s->cfg.threads, s->smem, st>>>(s->pool.P, A);
-  else
-    k_chain_steps<<<grid, s->cfg.threads, s->smem, st>>>(s->pool.P, A);
-  CK(ctx, cudaGetLastError());
-  if (n_npt > 0) {
-    MolRanges R;
-    R.act_slot = s->dlist + nc;
-    R.act_m0 = s->dlist + 2 * nc;
-    R.act_pref = s->dlist + 3 * nc;
-    R.n_act = n_npt;
-    R.total = total;
-    CK(ctx, launch_volume_phase(s->pool.P, s->pool.mol_chain, 0, s->vm, s->emol2, s->eabs2,
-                                s->vsum, s->vsum_abs, s->vlist, nullptr, 0, 0, st, R, has64,
-                                has32));
+  CK(ctx, cudaMemsetAsync(s->sched, 0, sizeof(unsigned) * 2 * nc, st));
+  const bool both = !act[0].empty() && !act[1].empty();
+  if (both) {
+    CK(ctx, cudaEventRecord(s->ev_fork, st));
+    CK(ctx, cudaStreamWaitEvent(s->side, s->ev_fork, 0));
+  }
+  // the slower kind's launches go first
+  for (int q = 1; q >= 0; q--) {
+    if (act[q].empty()) continue;
+    cudaStream_t sq = both && q == 0 ? s->side : st;
+    const int* dl = s->dlist + q * (5 * nc + 1);
+    const int n = (int)act[q].size();
+    ChainLaunch A{s->cfg.round_steps, s->cfg.round_steps, n, q ? kWideWarps : s->gw,
+                  s->sched + q * nc, dl, dl + 4 * nc + 1, q ? s->wide : s->shape};
+    A.lanes_cap = s->cfg.lanes_per_molecule;
+    if (q == 1) {
+      k_chain_steps_wide<<<std::min(n, s->wide_grid), kWideWarps * 32, s->wide_smem, sq>>>(
+          s->pool.P, A);
+    } else {
+      const int need = (n + s->cfg.chains_per_cta - 1) / s->cfg.chains_per_cta;
+      const int grid = std::max(1, std::min(need, s->grid));
+      if (s->cfg.threads > 256)
+        k_chain_steps_wide<<<grid, s->cfg.threads, s->smem, sq>>>(s->pool.P, A);
+      else
+        k_chain_steps<<<grid, s->cfg.threads, s->smem, sq>>>(s->pool.P, A);
+    }
+    CK(ctx, cudaGetLastError());
+    const Kind& k = kind[q];
+    if (k.n_npt > 0) {
+      MolRanges R;
+      R.act_slot = dl + nc;
+      R.act_m0 = dl + 2 * nc;
+      R.act_pref = dl + 3 * nc;
+      R.n_act = k.n_npt;
+      R.total = k.total;
+      CK(ctx, launch_volume_phase(s->pool.P, s->pool.mol_chain, 0, s->vm, s->emol2, s->eabs2,
+                                  s->vsum, s->vsum_abs, s->vlist + q * (3 * nc + 3), nullptr, 0,
+                                  0, sq, R, k.has64, k.has32));
+    }
+  }
+  if (both) {
+    CK(ctx, cudaEventRecord(s->ev_join, s->side));
+    CK(ctx, cudaStreamWaitEvent(st, s->ev_join, 0));
   }
   CK(ctx, cudaEventRecord(s->ev_t1, st));
   CK(ctx, cudaMemcpyAsync(s->hmirror, s->pool.P.hdr, sizeof(ChainHdr) * nc, cudaMemcpyDeviceToHost, st));
@@ -504,6 +543,9 @@ extern "C" int mcgpu_server_create(mcgpu_ctx* ctx, const mcgpu_server_config* cf
   int rc = server_alloc(s);
   cudaError_t e = cudaSuccess;
   if (rc == MCGPU_OK) e = cudaStreamCreateWithFlags(&s->copy, cudaStreamNonBlocking);
+  if (rc == MCGPU_OK && e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
+  if (rc == MCGPU_OK && e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming);
+  if (rc == MCGPU_OK && e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming);
   if (rc == MCGPU_OK && e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_round, cudaEventDisableTiming);
   if (rc == MCGPU_OK && e == cudaSuccess) e = cudaEventCreate(&s->ev_t0);
   if (rc == MCGPU_OK && e == cudaSuccess) e = cudaEventCreate(&s->ev_t1);
@@ -527,6 +569,16 @@ extern "C" int mcgpu_server_create(mcgpu_ctx* ctx, const mcgpu_server_config* cf
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &per_sm, c.threads > 256 ? k_chain_steps_wide : k_chain_steps, c.threads, s->smem);
   s->grid = std::max(1, per_sm) * ctx->sm_count;
+  // one chain per CTA of at most 8 warps leaves room for wider groups
+  if (c.chains_per_cta == 1 && c.threads < kWideWarps * 32 && c.max_mol_atoms > kWideAtoms) {
+    s->wide = shape_for(c.max_mol_atoms, kWideWarps, 2048);
+    s->wide_smem = s->wide.bytes();
+    per_sm = 0;
+    if (s->wide_smem <= 200 * 1024)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chain_steps_wide, kWideWarps * 32,
+                                                    s->wide_smem);
+    s->wide_grid = per_sm * ctx->sm_count;
+  }
   *out = s;
   return MCGPU_OK;
 }
@@ -535,6 +587,7 @@ extern "C" int mcgpu_server_destroy(mcgpu_server* s) {
   if (!s) return MCGPU_OK;
   cudaSetDevice(s->ctx->device);
   cudaStreamSynchronize(s->ctx->stream);
+  if (s->side) cudaStreamSynchronize(s->side);
   if (s->copy) cudaStreamSynchronize(s->copy);
   server_free(s);
   delete s;
