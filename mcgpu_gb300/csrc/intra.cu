@@ -31,7 +31,8 @@ constexpr int kIntraThreads = 128;
 // 344-375): blending by sqrt|a b| (sites with negative sigma or epsilon take
 // part), no cutoff, zero at r = 0.  1/r from one FP64 rsqrt (a few ulps from
 // the reference's sqrt and divisions, which cost many FP64 passes on this
-// part); sigma^2 = |s_i s_j| and 4 eps = 4 sqrt|e_i e_j|.
+// part); sigma^2 = |s_i s_j| and 4 eps = 4 sqrt|e_i e_j|, the root as the
+// product of the atoms' own (the blending rows) where neither is negative.
 __device__ __forceinline__ double intra_pair(const Pool& P, int i, int j, const ChainHdr& H) {
   const double dx = make_periodic(__dsub_rn(P.x[j], P.x[i]), H.L[0]);
   const double dy = make_periodic(__dsub_rn(P.y[j], P.y[i]), H.L[1]);
@@ -40,10 +41,12 @@ __device__ __forceinline__ double intra_pair(const Pool& P, int i, int j, const 
   if (r2 == 0.0) return 0.0;
   const double ri = rsqrt(r2);
   const double ss = fabs(P.sig[i] * P.sig[j]);
-  const double ee = P.eps[i] * P.eps[j];
+  const double2 bi = P.blend[i], bj = P.blend[j];
+  double ee = bi.y * bj.y;
+  if (blend_skipped(bi.x) || blend_skipped(bj.x)) ee = sqrt(fabs(P.eps[i] * P.eps[j]));
   const double s2 = ss * (ri * ri);
   const double s6 = s2 * s2 * s2;
-  const double lj = 4.0 * sqrt(fabs(ee)) * (s6 * s6 - s6);
+  const double lj = 4.0 * ee * (s6 * s6 - s6);
   return lj + P.q[i] * P.q[j] * 332.06 * ri;
 }
 
@@ -162,107 +165,153 @@ __global__ void __launch_bounds__(32) k_intra_add_boxes(const LoopTask* tasks) {
   if (threadIdx.x == 0) T.emol[mol] += e;
 }
 
-// One SimCalcs::stretchBond (kind 0, SimulationStep.cpp:257-315) or
-// SimCalcs::expandAngle (kind 1, :148-239) of entry i of box molecule mol,
-// every thread of the block; c1, s1 / c2, s2: the cosine and sine of the
-// first / second group's angle.  Returns false when the call changes nothing
-// (a bond in a ring, an angle whose ends share a component).
-__device__ bool apply_op(const Pool& P, const IntraRows& R, const ChainHdr& H, int mol, int kind,
-                         int i, double amt, double c1, double s1, double c2, double s2,
-                         double* sv) {
-  const int m = H.mol0 + mol;
-  const int a0 = P.mstart[m], len = P.mlen[m] & 255;
+// Rows of one stage's ops in shared memory.
+struct OpRows {
+  double x[kMaxA], y[kMaxA], z[kMaxA];   // the molecule's coordinates
+  double mx[kLoopSel], my[kLoopSel], mz[kLoopSel];  // a middle atom of another molecule
+  int part[kLoopSel], e1[kLoopSel], e2[kLoopSel], mid[kLoopSel];  // local atoms; mid -1: mx..mz
+  double v[9];
+  int moved;
+};
+
+// n ops of one stage in order, SimCalcs::stretchBond (kind 0,
+// SimulationStep.cpp:257-315) or SimCalcs::expandAngle (kind 1, :148-239) of
+// entries idx[] of box molecule mol; trig[4 q ..]: the cosine and sine of the
+// first and of the second group's angle.  Every thread of the block calls it;
+// the first warp works, with the ops' rows and the coordinates in shared memory
+// (an op is a chain of FP64 steps, and each followed three dependent loads and
+// stood between two block barriers).  Returns whether any op changed anything
+// (a bond in a ring, an angle whose ends share a component do not).
+__device__ bool apply_ops(const Pool& P, const IntraRows& R, const ChainHdr& H, int mol, int kind,
+                          int n, const int* idx, const double* amt, const double* trig,
+                          OpRows& W) {
+  const int a0 = P.mstart[H.mol0 + mol], len = P.mlen[H.mol0 + mol] & 255;
   const int tid = threadIdx.x;
-  if (kind == 0) {
-    const int b = R.m_bstart[mol] + i;
-    const int off = R.b_part[b];
-    if (off < 0) return false;  // a ring: the reference returns before moving
-    if (tid < 3) {
-      // lanes 0-2 each form the whole vector and its length (same values)
-      // and divide their own component: one division's latency, not three.
-      // (v / d) / 2 == (v / d) * 0.5 exactly.
-      const int e1 = H.atom0 + R.b_a1[b], e2 = H.atom0 + R.b_a2[b];
-      const double vx = __dsub_rn(P.x[e2], P.x[e1]);
-      const double vy = __dsub_rn(P.y[e2], P.y[e1]);
-      const double vz = __dsub_rn(P.z[e2], P.z[e1]);
-      double d = __dadd_rn(0.0, __dmul_rn(vx, vx));
-      d = __dadd_rn(d, __dmul_rn(vy, vy));
-      d = __dadd_rn(d, __dmul_rn(vz, vz));
-      d = __dsqrt_rn(d);
-      const double vc = tid == 0 ? vx : (tid == 1 ? vy : vz);
-      sv[tid] = __dmul_rn(__ddiv_rn(vc, d), 0.5);
-      if (tid == 0) R.b_len[b] = __dadd_rn(R.b_len[b], amt);
-    }
-    __syncthreads();
-    if (tid < len) {
-      const int a = a0 + tid;
-      const double sx = __dmul_rn(sv[0], amt), sy = __dmul_rn(sv[1], amt),
-                   sz = __dmul_rn(sv[2], amt);
-      if (R.part[off + tid] == 1) {
-        P.x[a] = __dadd_rn(P.x[a], sx);
-        P.y[a] = __dadd_rn(P.y[a], sy);
-        P.z[a] = __dadd_rn(P.z[a], sz);
-      } else {
-        P.x[a] = __dsub_rn(P.x[a], sx);
-        P.y[a] = __dsub_rn(P.y[a], sy);
-        P.z[a] = __dsub_rn(P.z[a], sz);
+  if (tid < 32) {
+    bool any = false;
+    for (int q = tid; q < n; q += 32) {
+      const int k = (kind == 0 ? R.m_bstart : R.m_astart)[mol] + idx[q];
+      const int off = (kind == 0 ? R.b_part : R.a_part)[k];
+      W.part[q] = off;
+      any = any || off >= 0;
+      const int base = a0 - H.atom0;
+      W.e1[q] = (kind == 0 ? R.b_a1 : R.a_a1)[k] - base;
+      W.e2[q] = (kind == 0 ? R.b_a2 : R.a_a2)[k] - base;
+      if (kind == 1) {
+        const int md = R.a_mid[k] - base;
+        const bool in = md >= 0 && md < len;
+        W.mid[q] = in ? md : -1;
+        if (!in) {
+          W.mx[q] = P.x[a0 + md];
+          W.my[q] = P.y[a0 + md];
+          W.mz[q] = P.z[a0 + md];
+        }
       }
+      // lengths and sizes: exact sums of the drawn amounts
+      double* row = (kind == 0 ? R.b_len : R.a_size) + k;
+      if (off >= 0) *row = __dadd_rn(*row, amt[q]);
     }
-    __syncthreads();
-    return true;
-  }
-  const int g = R.m_astart[mol] + i;
-  const int off = R.a_part[g];
-  if (off < 0) return false;  // both ends in one component
-  if (tid < 3) {
-    // lanes 0-2: the same normal and length, one component's division each
-    const int e1 = H.atom0 + R.a_a1[g], e2 = H.atom0 + R.a_a2[g], md = H.atom0 + R.a_mid[g];
-    const double m0 = P.x[md], m1 = P.y[md], m2 = P.z[md];
-    const double p0 = __dsub_rn(m0, P.x[e1]), p1 = __dsub_rn(m1, P.y[e1]),
-                 p2 = __dsub_rn(m2, P.z[e1]);
-    const double q0 = __dsub_rn(m0, P.x[e2]), q1 = __dsub_rn(m1, P.y[e2]),
-                 q2 = __dsub_rn(m2, P.z[e2]);
-    const double n0 = __dsub_rn(__dmul_rn(p1, q2), __dmul_rn(q1, p2));
-    const double n1 = __dsub_rn(__dmul_rn(q0, p2), __dmul_rn(p0, q2));
-    const double n2 = __dsub_rn(__dmul_rn(p0, q1), __dmul_rn(q0, p1));
-    double nl = __dadd_rn(0.0, __dmul_rn(n0, n0));
-    nl = __dadd_rn(nl, __dmul_rn(n1, n1));
-    nl = __dadd_rn(nl, __dmul_rn(n2, n2));
-    nl = __dsqrt_rn(nl);
-    const double nc = tid == 0 ? n0 : (tid == 1 ? n1 : n2);
-    sv[tid] = __ddiv_rn(nc, nl);
-    sv[3 + tid] = tid == 0 ? m0 : (tid == 1 ? m1 : m2);
-    if (tid == 0) R.a_size[g] = __dadd_rn(R.a_size[g], amt);
+    for (int i = tid; i < len; i += 32) {
+      W.x[i] = P.x[a0 + i];
+      W.y[i] = P.y[a0 + i];
+      W.z[i] = P.z[a0 + i];
+    }
+    any = __any_sync(~0u, any);
+    if (tid == 0) W.moved = any;
+    __syncwarp();
+    for (int q = 0; q < n; q++) {
+      const int off = W.part[q];
+      if (off < 0) continue;   // the reference returns before moving
+      const int e1 = W.e1[q], e2 = W.e2[q];
+      if (kind == 0) {
+        if (tid < 3) {
+          // lanes 0-2 each form the whole vector and its length (same values)
+          // and divide their own component: one division's latency, not
+          // three.  (v / d) / 2 == (v / d) * 0.5 exactly.
+          const double vx = __dsub_rn(W.x[e2], W.x[e1]);
+          const double vy = __dsub_rn(W.y[e2], W.y[e1]);
+          const double vz = __dsub_rn(W.z[e2], W.z[e1]);
+          double d = __dadd_rn(0.0, __dmul_rn(vx, vx));
+          d = __dadd_rn(d, __dmul_rn(vy, vy));
+          d = __dadd_rn(d, __dmul_rn(vz, vz));
+          d = __dsqrt_rn(d);
+          const double vc = tid == 0 ? vx : (tid == 1 ? vy : vz);
+          W.v[tid] = __dmul_rn(__dmul_rn(__ddiv_rn(vc, d), 0.5), amt[q]);
+        }
+        __syncwarp();
+        for (int i = tid; i < len; i += 32) {
+          const double sx = W.v[0], sy = W.v[1], sz = W.v[2];
+          if (R.part[off + i] == 1) {
+            W.x[i] = __dadd_rn(W.x[i], sx);
+            W.y[i] = __dadd_rn(W.y[i], sy);
+            W.z[i] = __dadd_rn(W.z[i], sz);
+          } else {
+            W.x[i] = __dsub_rn(W.x[i], sx);
+            W.y[i] = __dsub_rn(W.y[i], sy);
+            W.z[i] = __dsub_rn(W.z[i], sz);
+          }
+        }
+        __syncwarp();
+        continue;
+      }
+      if (tid < 3) {
+        // lanes 0-2: the same normal and length, one component's division each
+        const int md = W.mid[q];
+        const double m0 = md >= 0 ? W.x[md] : W.mx[q], m1 = md >= 0 ? W.y[md] : W.my[q],
+                     m2 = md >= 0 ? W.z[md] : W.mz[q];
+        const double p0 = __dsub_rn(m0, W.x[e1]), p1 = __dsub_rn(m1, W.y[e1]),
+                     p2 = __dsub_rn(m2, W.z[e1]);
+        const double q0 = __dsub_rn(m0, W.x[e2]), q1 = __dsub_rn(m1, W.y[e2]),
+                     q2 = __dsub_rn(m2, W.z[e2]);
+        const double n0 = __dsub_rn(__dmul_rn(p1, q2), __dmul_rn(q1, p2));
+        const double n1 = __dsub_rn(__dmul_rn(q0, p2), __dmul_rn(p0, q2));
+        const double n2 = __dsub_rn(__dmul_rn(p0, q1), __dmul_rn(q0, p1));
+        double nl = __dadd_rn(0.0, __dmul_rn(n0, n0));
+        nl = __dadd_rn(nl, __dmul_rn(n1, n1));
+        nl = __dadd_rn(nl, __dmul_rn(n2, n2));
+        nl = __dsqrt_rn(nl);
+        const double nc = tid == 0 ? n0 : (tid == 1 ? n1 : n2);
+        W.v[tid] = __ddiv_rn(nc, nl);
+        W.v[3 + tid] = tid == 0 ? m0 : (tid == 1 ? m1 : m2);
+      }
+      __syncwarp();
+      for (int i = tid; i < len; i += 32) {
+        const int lab = R.part[off + i];
+        if (lab) {
+          const double cs = trig[4 * q + (lab == 1 ? 0 : 2)];
+          const double sn = trig[4 * q + (lab == 1 ? 1 : 3)];
+          const double omc = __dsub_rn(1.0, cs);
+          const double u0 = W.v[0], u1 = W.v[1], u2 = W.v[2];
+          const double t0 = __dsub_rn(W.x[i], W.v[3]), t1 = __dsub_rn(W.y[i], W.v[4]),
+                       t2 = __dsub_rn(W.z[i], W.v[5]);
+          double dot = __dadd_rn(0.0, __dmul_rn(t0, u0));
+          dot = __dadd_rn(dot, __dmul_rn(t1, u1));
+          dot = __dadd_rn(dot, __dmul_rn(t2, u2));
+          const double k0 = __dsub_rn(__dmul_rn(u1, t2), __dmul_rn(t1, u2));
+          const double k1 = __dsub_rn(__dmul_rn(t0, u2), __dmul_rn(u0, t2));
+          const double k2 = __dsub_rn(__dmul_rn(u0, t1), __dmul_rn(t0, u1));
+          const double r0 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(u0, dot), omc),
+                                                __dmul_rn(t0, cs)), __dmul_rn(k0, sn));
+          const double r1 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(u1, dot), omc),
+                                                __dmul_rn(t1, cs)), __dmul_rn(k1, sn));
+          const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(u2, dot), omc),
+                                                __dmul_rn(t2, cs)), __dmul_rn(k2, sn));
+          W.x[i] = __dadd_rn(r0, W.v[3]);
+          W.y[i] = __dadd_rn(r1, W.v[4]);
+          W.z[i] = __dadd_rn(r2, W.v[5]);
+        }
+      }
+      __syncwarp();
+    }
+    if (any)
+      for (int i = tid; i < len; i += 32) {
+        P.x[a0 + i] = W.x[i];
+        P.y[a0 + i] = W.y[i];
+        P.z[a0 + i] = W.z[i];
+      }
   }
   __syncthreads();
-  if (tid < len) {
-    const int lab = R.part[off + tid];
-    if (lab) {
-      const double cs = lab == 1 ? c1 : c2;
-      const double sn = lab == 1 ? s1 : s2;
-      const double omc = __dsub_rn(1.0, cs);
-      const int a = a0 + tid;
-      const double t0 = __dsub_rn(P.x[a], sv[3]), t1 = __dsub_rn(P.y[a], sv[4]),
-                   t2 = __dsub_rn(P.z[a], sv[5]);
-      double dot = __dadd_rn(0.0, __dmul_rn(t0, sv[0]));
-      dot = __dadd_rn(dot, __dmul_rn(t1, sv[1]));
-      dot = __dadd_rn(dot, __dmul_rn(t2, sv[2]));
-      const double k0 = __dsub_rn(__dmul_rn(sv[1], t2), __dmul_rn(t1, sv[2]));
-      const double k1 = __dsub_rn(__dmul_rn(t0, sv[2]), __dmul_rn(sv[0], t2));
-      const double k2 = __dsub_rn(__dmul_rn(sv[0], t1), __dmul_rn(t0, sv[1]));
-      const double u0 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(sv[0], dot), omc),
-                                            __dmul_rn(t0, cs)), __dmul_rn(k0, sn));
-      const double u1 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(sv[1], dot), omc),
-                                            __dmul_rn(t1, cs)), __dmul_rn(k1, sn));
-      const double u2 = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(sv[2], dot), omc),
-                                            __dmul_rn(t2, cs)), __dmul_rn(k2, sn));
-      P.x[a] = __dadd_rn(u0, sv[3]);
-      P.y[a] = __dadd_rn(u1, sv[4]);
-      P.z[a] = __dadd_rn(u2, sv[5]);
-    }
-  }
-  __syncthreads();
-  return true;
+  return W.moved != 0;
 }
 
 // SimCalcs::saveBonds / saveAngles (SimulationStep.cpp:678-701), all threads.
@@ -301,7 +350,9 @@ __device__ void rollback_rows(const Pool& P, const IntraRows& R, const ChainHdr&
 __global__ void __launch_bounds__(kIntraThreads) k_intra_ops(Pool P, IntraRows R, int chain,
                                                              IntraOps ops, double* out) {
   __shared__ double red[3 * (kIntraThreads / 32)];
-  __shared__ double sv[9];
+  __shared__ OpRows W;
+  __shared__ int idx[kIntraOps];
+  __shared__ double amt[kIntraOps], trig[4 * kIntraOps];
   const ChainHdr& H = P.hdr[chain];
   const int mol = ops.mol, m = H.mol0 + mol;
   const int tid = threadIdx.x;
@@ -311,11 +362,16 @@ __global__ void __launch_bounds__(kIntraThreads) k_intra_ops(Pool P, IntraRows R
     const double e = intra_energy(P, R, H, mol, red);
     if (tid == 0) out[0] = e;
   }
-  bool moved = false;
-  for (int k = 0; k < ops.n; k++)
-    moved |= apply_op(P, R, H, mol, ops.kind, ops.idx[k], ops.amt[k], ops.c1[k], ops.s1[k],
-                      ops.c2[k], ops.s2[k], sv);
-  if (moved) {
+  if (tid < ops.n) {
+    idx[tid] = ops.idx[tid];
+    amt[tid] = ops.amt[tid];
+    trig[4 * tid] = ops.c1[tid];
+    trig[4 * tid + 1] = ops.s1[tid];
+    trig[4 * tid + 2] = ops.c2[tid];
+    trig[4 * tid + 3] = ops.s2[tid];
+  }
+  __syncthreads();
+  if (apply_ops(P, R, H, mol, ops.kind, ops.n, idx, amt, trig, W)) {
     refresh_flexible(P, H, m, red);
     __syncthreads();
   }
@@ -351,41 +407,75 @@ __device__ __forceinline__ bool loop_accept(CRand& g, double de, double kT) {
   return exp(-(de) / kT) >= loop_real(g, 0.0, 1.0);
 }
 
-// Thread 0: the draws of one stage of intramolecularMove (kind 0 bonds,
+// The first warp: the draws of one stage of intramolecularMove (kind 0 bonds,
 // :589-609; kind 1 angles, :621-640): how many, which (a std::set's distinct
 // draws in ascending order), an amount each; the variable entries go to
-// sel / amt.  Returns the count the counters take, or -1 when the set did
-// not fill within the draw cap.
+// sel / amt, and for angles the cosines and sines of their two groups to trig.
+// Lane 0 takes the numbers; the amounts, variable flags and sines are formed
+// side by side (one after another in lane 0 they took 15,000 cycles a stage,
+// most of them sines).  Returns the count the counters take, or -1 when the set
+// did not fill within the draw cap; every lane gets it and *n_sel.
 __device__ int loop_draw_stage(CRand& g, const IntraRows& R, int mol, int kind, double delta,
-                               int max_moves, int* sel, double* amt, int* n_sel) {
+                               int max_moves, int* sel, double* amt, double* trig, int32_t* raw,
+                               int* n_sel) {
+  const int lane = threadIdx.x & 31;
   const int count = kind == 0 ? R.m_bcount[mol] : R.m_acount[mol];
   const int start = kind == 0 ? R.m_bstart[mol] : R.m_astart[mol];
   const int* var = kind == 0 ? R.b_var : R.a_var;
   int n = count;
-  if (n > 3) n = min((int)loop_real(g, 2, count), max_moves);
+  if (lane == 0) {
+    if (n > 3) n = min((int)loop_real(g, 2, count), max_moves);
+    int have = 0, draws = 0;
+    while (have < n) {
+      if (++draws > kLoopDrawCap) {
+        n = -1;
+        break;
+      }
+      const int v = min((int)loop_real(g, 0, count), count - 1);
+      int pos = 0;
+      while (pos < have && sel[pos] < v) pos++;
+      if (pos < have && sel[pos] == v) continue;
+      for (int k = have; k > pos; k--) sel[k] = sel[k - 1];
+      sel[pos] = v;
+      have++;
+    }
+    for (int k = 0; k < n; k++) raw[k] = crand_next(g);
+  }
+  n = __shfl_sync(~0u, n, 0);
+  __syncwarp();
+  if (n < 0) return n;
   // 0.25 + (0.75 / n) * intraScaleFactor, rounded step by step as the host does
   const double scale = __dadd_rn(0.25, __dmul_rn(__ddiv_rn(0.75, (double)n), 0.625));
-  int have = 0, draws = 0;
-  while (have < n) {
-    if (++draws > kLoopDrawCap) return -1;
-    const int v = min((int)loop_real(g, 0, count), count - 1);
-    int pos = 0;
-    while (pos < have && sel[pos] < v) pos++;
-    if (pos < have && sel[pos] == v) continue;
-    for (int k = have; k > pos; k--) sel[k] = sel[k - 1];
-    sel[pos] = v;
-    have++;
-  }
   int ns = 0;
-  for (int k = 0; k < have; k++) {
-    const double d = __dmul_rn(scale, loop_real(g, -delta, delta));
-    if (var[start + sel[k]]) {
-      sel[ns] = sel[k];
-      amt[ns] = d;
-      ns++;
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    const int k = k0 + lane;
+    int e = 0;
+    bool on = false;
+    double d = 0.0;
+    if (k < n) {
+      e = sel[k];
+      on = var[start + e] != 0;
+      d = __dmul_rn(scale, real_of(raw[k], -delta, delta));
+    }
+    const unsigned bal = __ballot_sync(~0u, on);
+    __syncwarp();
+    if (on) {
+      const int at = ns + __popc(bal & lanemask_lt());   // at <= k: entries not read yet
+      sel[at] = e;
+      amt[at] = d;
+    }
+    ns += __popc(bal);
+    __syncwarp();
+  }
+  if (kind == 1) {
+    const double deg2rad = 3.14159256358979323846264 / 180.0;   // expandAngle's constant
+    for (int q = lane; q < 2 * ns; q += 32) {
+      const double a = amt[q >> 1];
+      sincos(__dmul_rn(a, (q & 1) ? deg2rad : -deg2rad), &trig[2 * q + 1], &trig[2 * q]);
     }
   }
   *n_sel = ns;
+  __syncwarp();
   return n;
 }
 
@@ -402,9 +492,9 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
   PlainLoop* L = task.L;
   __shared__ PlainLoop st;
   __shared__ Proposal prop;
-  __shared__ int32_t raw[8];
+  __shared__ int32_t raw[kLoopSel];
   __shared__ double red[3 * (kLoopThreads / 32)];
-  __shared__ double sv[9];
+  __shared__ OpRows W;
   __shared__ int sel[kLoopSel];
   __shared__ double amt[kLoopSel], trig[4 * kLoopSel];
   __shared__ int n_sel, flag, stop;
@@ -414,7 +504,6 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
   const int tid = threadIdx.x, lane = tid & 31, w = grp.warp(), nw = grp.nwarps();
   const int n = H.n_mol;
   const double kT = H.kT, max_t = H.max_t, max_r = H.max_r;
-  const double deg2rad = 3.14159256358979323846264 / 180.0;   // expandAngle's constant
   if (tid == 0) {
     st = *L;
     stop = 0;
@@ -506,32 +595,28 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     bool have_cur = false;
     for (int kind = 0; kind < 2; kind++) {
       if (kind == 0 ? !R.flex_bonds : !R.flex_angles) continue;
-      if (tid == 0) {
+      if (w == 0) {
+        int ns = 0;
         const int cnt = loop_draw_stage(st.rng, R, mol, kind, kind == 0 ? bond_delta : angle_delta,
-                                        st.max_intra_moves, sel, amt, &n_sel);
-        if (cnt < 0) {
-          st.error = 1;
-          stop = 1;
-        } else if (kind == 0) {
-          st.bond_moves += cnt;
-        } else {
-          st.angle_moves += cnt;
-        }
-        flag = cnt;
-        for (int q = 0; kind == 1 && q < n_sel; q++) {
-          sincos(__dmul_rn(amt[q], -deg2rad), &trig[4 * q + 1], &trig[4 * q]);
-          sincos(__dmul_rn(amt[q], deg2rad), &trig[4 * q + 3], &trig[4 * q + 2]);
+                                        st.max_intra_moves, sel, amt, trig, raw, &ns);
+        if (lane == 0) {
+          if (cnt < 0) {
+            st.error = 1;
+            stop = 1;
+          } else if (kind == 0) {
+            st.bond_moves += cnt;
+          } else {
+            st.angle_moves += cnt;
+          }
+          flag = cnt;
+          n_sel = ns;
         }
       }
       __syncthreads();
       if (stop) break;
       const int cnt = flag;
       const double e0 = have_cur ? cur : intra_energy(P, R, H, mol, red);
-      bool moved = false;
-      for (int q = 0; q < n_sel; q++)
-        moved |= apply_op(P, R, H, mol, kind, sel[q], amt[q], trig[4 * q], trig[4 * q + 1],
-                          trig[4 * q + 2], trig[4 * q + 3], sv);
-      if (moved) {
+      if (apply_ops(P, R, H, mol, kind, n_sel, sel, amt, trig, W)) {
         refresh_flexible(P, H, m, red);
         __syncthreads();
       }
