@@ -407,6 +407,136 @@ __device__ __forceinline__ bool loop_accept(CRand& g, double de, double kT) {
   return exp(-(de) / kT) >= loop_real(g, 0.0, 1.0);
 }
 
+// Scratch of cta_eval: per warp the in-range candidates of a segment, their atoms'
+// items, and (mixed lengths) each entry's first item.
+constexpr int kLoopWarps = kLoopThreads / 32;
+struct EvalRows {
+  int ent[kLoopWarps], tot[kLoopWarps];
+  int first[kLoopWarps * kRing];
+};
+
+// The staged molecule's pair energies with all others, one share per thread of
+// the kLoopThreads of grp (group_reduce adds them).  The warps screen 64
+// candidates each, then all items (placement, entry, neighbour atom) of the
+// segment are dealt over the CTA's lanes: with each warp evaluating its own hits
+// a warp's last round was part full and the warps' counts differed (FP64 issues a
+// warp instruction in 16 cycles however few lanes work).  Where the items leave
+// warps idle the moved molecule's atoms are dealt too (FP64 pairs; the FP32 items
+// factor the whole molecule's charge).
+template <bool F64>
+__device__ void cta_eval(const Pool& P, const ChainHdr& H, const Group& grp, const GroupSmem& s,
+                         const MovedInfo& mi, EvalRows& E, double& eo, double& en,
+                         long long& np) {
+  const int lane = grp.tid & 31, w = grp.warp();
+  const unsigned lt = lanemask_lt();
+  const bool uni = H.uniform != 0;
+  const int two = mi.states == 3 ? 2 : 1;
+  const int c_end = H.mol0 + H.n_mol;
+  int* rj = s.lj + w * kRing;
+  AccFF acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0};
+  for (int base = H.mol0; base < c_end; base += kLoopWarps * kRing) {
+    if (base > H.mol0) grp.sync();   // the last segment's entries are read
+    int cnt = 0, tot = 0;
+#pragma unroll
+    for (int r = 0; r < kRing / 32; r++) {
+      const int j0 = base + (r * kLoopWarps + w) * 32;
+      if (j0 >= c_end) break;
+      const int j = j0 + lane;
+      int f = 0;
+      // the FP32 screen with the FP64 re-test inside its guard band gives the
+      // FP64 test's in-range set exactly, for FP64 and FP32 pair terms alike
+      if (j < c_end && j != mi.mol) f = screen_mixed(P, H, s, mi, j);
+      const unsigned bal = __ballot_sync(~0u, f != 0);
+      const int at = cnt + __popc(bal & lt);
+      if (f) rj[at] = (j << 4) | f;
+      cnt += __popc(bal);
+      const int hits = __popc(f & (kInOld | kInNew));
+      if (uni) {
+        np += (long long)hits * (mi.act * H.uact);
+        continue;
+      }
+      const int lw = f ? P.mlen[j] : 0;
+      np += (long long)hits * (mi.act * (lw >> 8));
+      int pre = lw & 255;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(~0u, pre, off);
+        if (lane >= off) pre += v;
+      }
+      if (f) E.first[w * kRing + at] = tot + pre - (lw & 255);
+      tot += __shfl_sync(~0u, pre, 31);
+    }
+    if (lane == 0) {
+      E.ent[w] = cnt;
+      E.tot[w] = tot;
+    }
+    grp.sync();
+    int entries = 0, total = 0;
+#pragma unroll
+    for (int v = 0; v < kLoopWarps; v++) {
+      entries += E.ent[v];
+      total += E.tot[v];
+    }
+    if (uni) total = entries * H.ulen;
+    const int items = total * two;
+    // a part takes whole warps: pair_sum64's votes need the lanes of a warp on the
+    // same atoms
+    const int span = (items + 31) & ~31;
+    const int parts = F64 && items > 0 ? max(1, min(mi.len, kLoopThreads / span)) : 1;
+    for (int it = grp.tid; it < span * parts; it += kLoopThreads) {
+      const int part = it / span;
+      int local = it - part * span;
+      if (local >= items) continue;
+      const bool use_new = local >= total || mi.states == 2;
+      if (local >= total) local -= total;
+      // item -> (warp's ring, entry, atom): all entries' first atoms, then their
+      // second ones in a uniform box; entry by entry with mixed lengths
+      int k = 0, at = local, v = 0;
+      if (uni) {
+        k = local / entries;
+        at = local - k * entries;
+      }
+      while (v < kLoopWarps - 1 && at >= (uni ? E.ent[v] : E.tot[v])) {
+        at -= uni ? E.ent[v] : E.tot[v];
+        v++;
+      }
+      if (!uni) {
+        const int n_e = E.ent[v];
+        int e = 0;
+#pragma unroll
+        for (int step = kRing / 2; step > 0; step >>= 1)
+          if (e + step < n_e && E.first[v * kRing + e + step] <= at) e += step;
+        k = at - E.first[v * kRing + e];
+        at = e;
+      }
+      const int jf = s.lj[v * kRing + at];
+      if (!(jf & (use_new ? kInNew : kInOld))) continue;
+      const int j = jf >> 4;
+      const int b = (uni ? H.atom0 + (j - H.mol0) * H.ulen : P.mstart[j]) + k;
+      if (F64) {
+        const int i0 = part * mi.len / parts, n_i = (part + 1) * mi.len / parts - i0;
+        const double2 bl = P.blend[b];
+        const double e = pair_sum64<true>(
+            (use_new ? s.nx : s.ox) + i0, (use_new ? s.ny : s.oy) + i0,
+            (use_new ? s.nz : s.oz) + i0, s.sd + i0, s.ed + i0, s.qd + i0, n_i, P.x[b], P.y[b],
+            P.z[b], bl.x, bl.y, P.q[b], H.L[0], H.L[1], H.L[2]);
+        if (use_new) en += e; else eo += e;
+      } else {
+        const float e = H.precise ? pair_item32<true>(P, H, s, mi, j, b, use_new)
+                                  : pair_item32<false>(P, H, s, mi, j, b, use_new);
+        if (use_new)
+          ff_add(acc.nh, acc.nl, e);
+        else
+          ff_add(acc.oh, acc.ol, e);
+      }
+    }
+  }
+  if (!F64) {
+    eo += (double)acc.oh + (double)acc.ol;
+    en += (double)acc.nh + (double)acc.nl;
+  }
+}
+
 // The first warp: the draws of one stage of intramolecularMove (kind 0 bonds,
 // :589-609; kind 1 angles, :621-640): how many, which (a std::set's distinct
 // draws in ascending order), an amount each; the variable entries go to
@@ -495,13 +625,14 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
   __shared__ int32_t raw[kLoopSel];
   __shared__ double red[3 * (kLoopThreads / 32)];
   __shared__ OpRows W;
+  __shared__ EvalRows E;
   __shared__ int sel[kLoopSel];
   __shared__ double amt[kLoopSel], trig[4 * kLoopSel];
   __shared__ int n_sel, flag, stop;
   const ChainHdr& H = P.hdr[0];
   Group grp{(int)threadIdx.x, (int)blockDim.x, 1};
   GroupSmem s = shape.carve(smem);
-  const int tid = threadIdx.x, lane = tid & 31, w = grp.warp(), nw = grp.nwarps();
+  const int tid = threadIdx.x, lane = tid & 31, w = grp.warp();
   const int n = H.n_mol;
   const double kT = H.kT, max_t = H.max_t, max_r = H.max_r;
   if (tid == 0) {
@@ -543,7 +674,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
       if (w == 0) stage(P, H, m, &prop, s, lane);
       grp.sync();
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64, false>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, s.lj + w * kRing, lane, eo, en, np);
+      cta_eval<F64>(P, H, grp, s, mi, E, eo, en, np);
       group_reduce(grp, s, eo, en, np);
       if (tid == 0) {
         const double de = en - eo;
@@ -567,7 +698,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     grp.sync();
     {
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64, false>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, s.lj + w * kRing, lane, eo, en, np);
+      cta_eval<F64>(P, H, grp, s, mi, E, eo, en, np);
       group_reduce(grp, s, eo, en, np);
     }
     const double e_old = eo + ei_old;
@@ -654,7 +785,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     np = 0;
     {
       const MovedInfo mi = load_moved(s);
-      warp_eval<F64, false>(P, H, s, mi, H.mol0, H.mol0 + n, w, nw, s.lj + w * kRing, lane, eo, en, np);
+      cta_eval<F64>(P, H, grp, s, mi, E, eo, en, np);
       group_reduce(grp, s, eo, en, np);
     }
     if (tid == 0) {

@@ -750,6 +750,38 @@ __device__ __forceinline__ void batch_f64(const Pool& P, const ChainHdr& H, cons
                 });
 }
 
+// FP32 pair terms of atom b of molecule j with the moved molecule's old (p false)
+// or new placement (offsets with their low parts).
+template <bool PRECISE>
+__device__ __forceinline__ float pair_item32(const Pool& P, const ChainHdr& H,
+                                             const GroupSmem& s, const MovedInfo& mi, int j,
+                                             int b, bool p) {
+  const uint4 fj = P.mfix[j];
+  const float4 ob = P.aoff[b];
+  const float2 qb = P.aeq[b];
+  float4 obl = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (PRECISE) obl = P.aofl[b];
+  // mrad, not the header's radius: a flexible molecule's changes
+  const float rr = mi.rad + P.mrad[j];
+  const uint4 fm = p ? mi.fx_new : mi.fx_old;
+  float3 D, bl = make_float3(0.f, 0.f, 0.f);
+  if (PRECISE) fixdiff_ff(fj, fm, H, D, bl); else D = fixdiff(fj, fm, H);
+  const float3 bh = make_float3(D.x + ob.x, D.y + ob.y, D.z + ob.z);
+  if (PRECISE) {
+    // two-sum of D + o_b per axis, then the low parts
+    const float ex = (D.x - (bh.x - (bh.x - D.x))) + (ob.x - (bh.x - D.x));
+    const float ey = (D.y - (bh.y - (bh.y - D.y))) + (ob.y - (bh.y - D.y));
+    const float ez = (D.z - (bh.z - (bh.z - D.z))) + (ob.z - (bh.z - D.z));
+    bl = make_float3(ex + (bl.x + obl.x), ey + (bl.y + obl.y), ez + (bl.z + obl.z));
+  }
+  float sa = 0.f;
+  return needs_wrap(D, rr, H)
+          ? sum_moved32_wrap<PRECISE, true>(p ? s.o_new : s.o_old, p ? s.l_new : s.l_old, s.eq,
+                                            mi.len, bh, bl, ob.w, qb, H, sa)
+          : sum_moved32_cf<PRECISE, true>(p ? s.o_new : s.o_old, p ? s.l_new : s.l_old, s.eq,
+                                          mi.len, p, bh, bl, ob.w, qb, mi.qm, sa);
+}
+
 // FP32 pair batch of `count` (1..32) ring entries from `head` on the plain path
 // (offsets with their low parts), the items (placement, entry, neighbour atom)
 // dealt to the lanes as batch_items64 deals them; each item's sum over the
@@ -808,31 +840,7 @@ __device__ __forceinline__ void batch_items32(const Pool& P, const ChainHdr& H,
     if (!(jf & (p ? kInNew : kInOld))) continue;
     const int j = jf >> 4;
     const int b = (uni ? H.atom0 + (j - H.mol0) * H.ulen : P.mstart[j]) + k;
-    const uint4 fj = P.mfix[j];
-    const float4 ob = P.aoff[b];
-    const float2 qb = P.aeq[b];
-    float4 obl = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (PRECISE) obl = P.aofl[b];
-    // mrad, not the header's radius: a flexible molecule's changes
-    const float rr = mi.rad + P.mrad[j];
-    const uint4 fm = p ? mi.fx_new : mi.fx_old;
-    float3 D, bl = make_float3(0.f, 0.f, 0.f);
-    if (PRECISE) fixdiff_ff(fj, fm, H, D, bl); else D = fixdiff(fj, fm, H);
-    const float3 bh = make_float3(D.x + ob.x, D.y + ob.y, D.z + ob.z);
-    if (PRECISE) {
-      // two-sum of D + o_b per axis, then the low parts
-      const float ex = (D.x - (bh.x - (bh.x - D.x))) + (ob.x - (bh.x - D.x));
-      const float ey = (D.y - (bh.y - (bh.y - D.y))) + (ob.y - (bh.y - D.y));
-      const float ez = (D.z - (bh.z - (bh.z - D.z))) + (ob.z - (bh.z - D.z));
-      bl = make_float3(ex + (bl.x + obl.x), ey + (bl.y + obl.y), ez + (bl.z + obl.z));
-    }
-    float sa = 0.f;
-    const float sp =
-        needs_wrap(D, rr, H)
-            ? sum_moved32_wrap<PRECISE, true>(p ? s.o_new : s.o_old, p ? s.l_new : s.l_old, s.eq,
-                                              mi.len, bh, bl, ob.w, qb, H, sa)
-            : sum_moved32_cf<PRECISE, true>(p ? s.o_new : s.o_old, p ? s.l_new : s.l_old, s.eq,
-                                            mi.len, p, bh, bl, ob.w, qb, mi.qm, sa);
+    const float sp = pair_item32<PRECISE>(P, H, s, mi, j, b, p);
     if (p)
       ff_add(acc.nh, acc.nl, sp);
     else
