@@ -935,7 +935,7 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
   mcgpu_ctx* ctx = b0->ctx;
   if (n_steps < 0) return set_err(ctx, MCGPU_ERR_INVALID, "negative step count");
   int max_len = 0, max_mol = 0, max_groups = 0;
-  bool intra = false;
+  bool intra = false, rigid = false;
   for (int i = 0; i < n_boxes; i++) {
     mcgpu_box* b = boxes[i];
     if (!b) return set_err(ctx, MCGPU_ERR_INVALID, "null box %d", i);
@@ -948,7 +948,7 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
     max_len = std::max(max_len, b->pool.max_len);
     max_mol = std::max(max_mol, b->pool.n_mol);
     max_groups = std::max(max_groups, pair_sum_groups(b->pool.n_mol));
-    intra = intra || b->intra_on;
+    (b->intra_on ? intra : rigid) = true;
   }
   {
     std::vector<mcgpu_box*> sorted(boxes, boxes + n_boxes);
@@ -1010,9 +1010,28 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
     e = launch_box_energies(f64, dt, n_boxes, max_mol, max_groups, intra,
                             shape_for(max_len, kEnergyWarps), ctx->stream);
   SmemShape sh = shape_for(max_len, 8);
-  for (int done = 0; e == cudaSuccess && done < n_steps; done += kDeviceLoopSteps)
-    e = launch_plain_steps(f64, dt, n_boxes, std::min(kDeviceLoopSteps, n_steps - done), sh,
-                           ctx->stream);
+  // boxes of both kinds: two kernels, side by side on two streams
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr;
+  if (e == cudaSuccess && intra && rigid) {
+    e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(fork, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+  }
+  for (int done = 0; e == cudaSuccess && done < n_steps; done += kDeviceLoopSteps) {
+    const int n = std::min(kDeviceLoopSteps, n_steps - done);
+    if (rigid) e = launch_plain_steps(f64, false, dt, n_boxes, n, sh, ctx->stream);
+    if (e == cudaSuccess && intra)
+      e = launch_plain_steps(f64, true, dt, n_boxes, n, sh, side ? side : ctx->stream);
+  }
+  if (side) {
+    // joined whatever happened: the buffers below are freed
+    const cudaError_t js = cudaStreamSynchronize(side);
+    if (e == cudaSuccess) e = js;
+    if (fork) cudaEventDestroy(fork);
+    cudaStreamDestroy(side);
+  }
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(loops.data(), dl, sizeof(PlainLoop) * n_boxes, cudaMemcpyDeviceToHost,
                         ctx->stream);

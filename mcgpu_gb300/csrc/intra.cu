@@ -609,6 +609,7 @@ __device__ int loop_draw_stage(CRand& g, const IntraRows& R, int mol, int kind, 
   return n;
 }
 
+// The loop of a box with the intramolecular term and moves, one CTA a box.
 template <bool F64>
 __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* tasks, int n_steps,
                                                               SmemShape shape) {
@@ -616,9 +617,9 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
   __shared__ LoopTask task;
   if (threadIdx.x == 0) task = tasks[blockIdx.x];
   __syncthreads();
+  if (!task.intra) return;   // k_plain_rigid's
   const Pool& P = task.P;
   const IntraRows& R = task.R;
-  const int intra = task.intra;
   PlainLoop* L = task.L;
   __shared__ PlainLoop st;
   __shared__ Proposal prop;
@@ -669,30 +670,6 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     const int mol = prop.mol, m = H.mol0 + mol;
     double eo = 0.0, en = 0.0;
     long long np = 0;
-    if (!intra) {
-      // old and new placement in one pass (k_move_energies on one CTA)
-      if (w == 0) stage(P, H, m, &prop, s, lane);
-      grp.sync();
-      const MovedInfo mi = load_moved(s);
-      cta_eval<F64>(P, H, grp, s, mi, E, eo, en, np);
-      group_reduce(grp, s, eo, en, np);
-      if (tid == 0) {
-        const double de = en - eo;
-        flag = loop_accept(st.rng, de, kT);
-        st.pairs += np;
-        if (flag) {
-          st.energy += de;
-          st.accepted++;
-        } else {
-          st.rejected++;
-        }
-      }
-      __syncthreads();
-      if (flag && w == 0) commit(P, s, mi, lane);
-      __syncthreads();
-      continue;
-    }
-    // ---- with the intramolecular term and move ----
     const double ei_old = intra_energy(P, R, H, mol, red);
     if (w == 0) stage(P, H, m, nullptr, s, lane);
     grp.sync();
@@ -805,6 +782,151 @@ __global__ void __launch_bounds__(kLoopThreads) k_plain_steps(const LoopTask* ta
     __syncthreads();
   }
   if (tid == 0) *L = st;
+}
+
+// chooseMolecule and the seven intermolecularMove draws (SimulationStep.cpp:25-27,
+// 527-535) of words v0 (the first) and v (word lane & 7), clamped as the host loop
+// clamps; lane k of NL forms the k-th real.
+__device__ __forceinline__ void loop_propose(const Pool& P, const ChainHdr& H, int32_t v0,
+                                             int32_t v, int lane, Proposal& prop) {
+  const int n = H.n_mol;
+  const int mol = min((int)real_of(v0, 0, n), n - 1);
+  const int len = P.mlen[H.mol0 + mol] & 255;
+  const double top = lane < 5 ? H.max_t : H.max_r;
+  const double x = lane == 1 ? real_of(v, 0, len) : real_of(v, -top, top);
+  if (lane == 0) {
+    prop.mol = mol;
+    prop.trig = 0;
+  }
+  if (lane == 1) prop.vertex = min((int)x, len - 1);
+  if (lane == 2) prop.dx = x;
+  if (lane == 3) prop.dy = x;
+  if (lane == 4) prop.dz = x;
+  if (lane == 5) prop.r0 = x;
+  if (lane == 6) prop.r1 = x;
+  if (lane == 7) prop.r2 = x;
+}
+
+// The generator as its last words: word k of the stream (the state's own 31
+// first) in slot k mod 64.  One warp makes nine words at a time:
+// x[k] = x[k-3] + x[k-31] is three interleaved running sums.
+constexpr int kWords = 64;
+__device__ __forceinline__ void words_next(uint32_t* ring, int& made, int lane) {
+  uint32_t v = ring[(made + lane - 31) & (kWords - 1)];
+  if (lane < 3) v += ring[(made + lane - 3) & (kWords - 1)];
+  const uint32_t a = __shfl_up_sync(~0u, v, 3);
+  if (lane >= 3) v += a;
+  const uint32_t b = __shfl_up_sync(~0u, v, 6);
+  if (lane >= 6) v += b;
+  __syncwarp();
+  if (lane < 9) ring[(made + lane) & (kWords - 1)] = v;
+  made += 9;
+  __syncwarp();
+}
+
+// The loop of a rigid box, one CTA a box: eight warps evaluate the staged move,
+// and a ninth meanwhile draws and stages the next one.  Whether the acceptance
+// takes a number is not known yet, so its halves stage the two moves that can
+// follow, from the next word and the one after it; the step's end picks one.
+// (A move of the molecule that was just moved is staged again.)  Draws and staging
+// are FP64 chains of one warp: with the other warps waiting for them a step of
+// 256 waters took 22.8 us, this way 16.9.
+constexpr int kRigidThreads = kLoopThreads + 32;
+
+template <bool F64>
+__global__ void __launch_bounds__(kRigidThreads, 2) k_plain_rigid(const LoopTask* tasks, int n_steps,
+                                                               SmemShape shape) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ LoopTask task;
+  __shared__ Proposal prop[2];
+  __shared__ EvalRows E;
+  __shared__ uint32_t ring[kWords];
+  __shared__ int dec[2];   // of even and odd steps; bit 0: accepted, bit 1: a word taken
+  if (threadIdx.x == 0) task = tasks[blockIdx.x];
+  __syncthreads();
+  if (task.intra) return;   // k_plain_steps'
+  const Pool& P = task.P;
+  PlainLoop* L = task.L;
+  const ChainHdr& H = P.hdr[0];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int half = lane >> 4, hl = lane & 15;
+  const bool helper = w == kLoopWarps;
+  Group grp{tid, kLoopThreads, 1};
+  const int slot_bytes = shape.bytes();
+  const double kT = H.kT;
+  double energy = L->energy;
+  long long accepted = 0, pairs = 0;
+  if (tid < 31) ring[tid] = (uint32_t)L->rng.r[(L->rng.f + tid) % 31];
+  __syncthreads();
+  // pos: the words consumed up to the step's own draws; made: the words there are
+  int pos = 31, made = 31, cur = 0;
+  // the moves drawn from word `from` (first half) and the one after it into slots
+  // s0 and s0 + 1 mod 3
+  auto prepare = [&](int from, int s0) {
+    while (made < from + 10) words_next(ring, made, lane);
+    const int at = from + half;
+    loop_propose(P, H, (int32_t)(ring[at & (kWords - 1)] >> 1),
+                 (int32_t)(ring[(at + (hl & 7)) & (kWords - 1)] >> 1), hl, prop[half]);
+    __syncwarp();
+    const GroupSmem t = shape.carve(smem + ((s0 + half) % 3) * slot_bytes);
+    stage<16>(P, H, H.mol0 + prop[half].mol, &prop[half], t, hl);
+  };
+  if (helper) prepare(pos, 0);
+  pos += 8;
+  __syncthreads();
+  for (int k = 0; k < n_steps; k++) {
+    const GroupSmem s = shape.carve(smem + cur * slot_bytes);
+    const MovedInfo mi = load_moved(s);
+    const int ahead = (cur + 1) % 3;
+    if (helper) {
+      if (k + 1 < n_steps) prepare(pos, ahead);
+    } else {
+      double eo = 0.0, en = 0.0;
+      long long np = 0;
+      cta_eval<F64>(P, H, grp, s, mi, E, eo, en, np);
+      group_reduce(grp, s, eo, en, np);
+      if (tid == 0) {
+        // acceptMove (SimulationStep.cpp:794-803): no draw for a decrease
+        const double de = en - eo;
+        const bool draw = !(de < 0);
+        const bool acc =
+            !draw || exp(-(de) / kT) >= real_of((int32_t)(ring[pos & (kWords - 1)] >> 1), 0.0, 1.0);
+        pairs += np;
+        if (acc) {
+          energy += de;
+          accepted++;
+        }
+        dec[k & 1] = (acc ? 1 : 0) | (draw ? 2 : 0);
+      }
+    }
+    __syncthreads();
+    const int d = dec[k & 1], took = d >> 1;
+    pos += took;
+    cur = (ahead + took) % 3;
+    if (d & 1) {
+      // (read before the barrier: the helper's next draws come after it)
+      const bool again = k + 1 < n_steps && H.mol0 + prop[took].mol == mi.mol;
+      if (w == 0) commit(P, s, mi, lane);
+      __syncthreads();
+      if (again) {
+        if (helper)
+          stage<16>(P, H, mi.mol, &prop[took], shape.carve(smem + ((ahead + half) % 3) * slot_bytes),
+                    hl);
+        __syncthreads();
+      }
+    }
+    if (k + 1 < n_steps) pos += 8;
+  }
+  // the generator's state after pos words: its last 31, the oldest next
+  if (tid < 31) L->rng.r[tid] = (int32_t)ring[(pos - 31 + tid) & (kWords - 1)];
+  if (tid == 0) {
+    L->rng.f = 0;
+    L->rng.b = 28;
+    L->energy = energy;
+    L->accepted += accepted;
+    L->rejected += n_steps - accepted;
+    L->pairs += pairs;
+  }
 }
 
 // Union-find over local atom indexes (the partition is all that is used).
@@ -986,17 +1108,17 @@ cudaError_t launch_intra_rollback(const Pool& P, const IntraRows& R, int chain, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_plain_steps(bool f64, const LoopTask* tasks, int n_tasks, int n_steps,
-                               SmemShape sh, cudaStream_t st) {
+cudaError_t launch_plain_steps(bool f64, bool flexible, const LoopTask* tasks, int n_tasks,
+                               int n_steps, SmemShape sh, cudaStream_t st) {
   if (n_tasks <= 0) return cudaSuccess;
-  const int bytes = sh.bytes();
-  if (f64) {
-    cudaFuncSetAttribute(k_plain_steps<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    k_plain_steps<true><<<n_tasks, kLoopThreads, bytes, st>>>(tasks, n_steps, sh);
-  } else {
-    cudaFuncSetAttribute(k_plain_steps<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    k_plain_steps<false><<<n_tasks, kLoopThreads, bytes, st>>>(tasks, n_steps, sh);
-  }
+  // three staged moves in the rigid loop
+  const int bytes = flexible ? sh.bytes() : 3 * sh.bytes();
+  const int threads = flexible ? kLoopThreads : kRigidThreads;
+  const auto kernel = flexible ? (f64 ? k_plain_steps<true> : k_plain_steps<false>)
+                               : (f64 ? k_plain_rigid<true> : k_plain_rigid<false>);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  kernel<<<n_tasks, threads, bytes, st>>>(tasks, n_steps, sh);
   return cudaGetLastError();
 }
 

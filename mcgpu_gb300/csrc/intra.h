@@ -127,11 +127,11 @@ int pair_sum_groups(int n_mol);
 cudaError_t launch_intra_add_boxes(const LoopTask* tasks, int n_tasks, int max_mol,
                                    cudaStream_t st);
 
-// n_steps of Simulation::run's loop for each of n_tasks boxes, one CTA per
-// box, the draws from each L->rng; intra != 0: with the intramolecular term
-// and move.  f64: FP64 intermolecular pair terms, else FP32.  tasks is a
-// device array.
-cudaError_t launch_plain_steps(bool f64, const LoopTask* tasks, int n_tasks, int n_steps,
-                               SmemShape sh, cudaStream_t st);
+// n_steps of Simulation::run's loop for each of the n_tasks boxes with intra != 0
+// (flexible: with the intramolecular term and move) or with intra == 0, one CTA
+// per box, the draws from each L->rng.  f64: FP64 intermolecular pair terms, else
+// FP32.  tasks is a device array.
+cudaError_t launch_plain_steps(bool f64, bool flexible, const LoopTask* tasks, int n_tasks,
+                               int n_steps, SmemShape sh, cudaStream_t st);
 
 }  // namespace mcgpu

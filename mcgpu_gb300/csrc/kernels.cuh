@@ -97,14 +97,17 @@ enum : int { kMiscRad = 21, kMiscQm = 22 };
 // non-vertex atom rotated about the vertex and translated, the vertex
 // translated, then the molecule wrapped by its first primary atom
 // (keepMoleculeInBox, :710-729).  Results go to shared memory; scalars to
-// misc.  The caller synchronises the group afterwards.
+// misc.  The caller synchronises the group afterwards.  NL 16: each half of the
+// warp stages a molecule of its own (m, p, s and lane 0-15 are the half's; both
+// or neither have a move).
+template <int NL = 32>
 __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Proposal* p,
                       const GroupSmem& s, int lane) {
   const int a0 = P.mstart[m];
   const int lw = P.mlen[m];
   const int len = lw & 255;
   const int2 pi = P.mpi[m];
-  for (int i = lane; i < len; i += 32) {
+  for (int i = lane; i < len; i += NL) {
     int a = a0 + i;
     s.ox[i] = P.x[a]; s.oy[i] = P.y[a]; s.oz[i] = P.z[a];
     const double2 bl = P.blend ? P.blend[a] : blend64(P.sig[a], P.eps[a]);
@@ -117,9 +120,9 @@ __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Prop
   }
   // net FP32 charge factor of the molecule (sum over lanes, fixed order)
   float qsum = 0.f;
-  for (int i = lane; i < len; i += 32) qsum += P.aeq[a0 + i].y;
-  for (int off = 16; off > 0; off >>= 1) qsum += __shfl_xor_sync(~0u, qsum, off);
-  for (int k = lane; k < pi.y; k += 32) {
+  for (int i = lane; i < len; i += NL) qsum += P.aeq[a0 + i].y;
+  for (int off = NL / 2; off > 0; off >>= 1) qsum += __shfl_xor_sync(~0u, qsum, off);
+  for (int k = lane; k < pi.y; k += NL) {
     s.p_old[k] = P.ppos[pi.x + k];
     s.pa[k] = P.pidx[pi.x + k] - a0;
   }
@@ -142,13 +145,13 @@ __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Prop
            &rc);
   }
   Rot R;
-  R.cx = __shfl_sync(~0u, rc, 0); R.sx = __shfl_sync(~0u, rs, 0);
-  R.cy = __shfl_sync(~0u, rc, 1); R.sy = __shfl_sync(~0u, rs, 1);
-  R.cz = __shfl_sync(~0u, rc, 2); R.sz = __shfl_sync(~0u, rs, 2);
+  R.cx = __shfl_sync(~0u, rc, 0, NL); R.sx = __shfl_sync(~0u, rs, 0, NL);
+  R.cy = __shfl_sync(~0u, rc, 1, NL); R.sy = __shfl_sync(~0u, rs, 1, NL);
+  R.cz = __shfl_sync(~0u, rc, 2, NL); R.sz = __shfl_sync(~0u, rs, 2, NL);
   __syncwarp();
   const int v = p->vertex;
   const double px = s.ox[v], py = s.oy[v], pz = s.oz[v];
-  for (int i = lane; i < len; i += 32) {
+  for (int i = lane; i < len; i += NL) {
     double x, y, z;
     if (i == v) {
       x = __dadd_rn(px, p->dx); y = __dadd_rn(py, p->dy); z = __dadd_rn(pz, p->dz);
@@ -172,7 +175,7 @@ __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Prop
   if (shy != 0) ay = __dadd_rn(ay, shy);
   if (shz != 0) az = __dadd_rn(az, shz);
   __syncwarp();
-  for (int i = lane; i < len; i += 32) {
+  for (int i = lane; i < len; i += NL) {
     double x = s.nx[i], y = s.ny[i], z = s.nz[i];
     if (shx != 0) x = __dadd_rn(x, shx);
     if (shy != 0) y = __dadd_rn(y, shy);
@@ -186,7 +189,7 @@ __device__ inline void stage(const Pool& P, const ChainHdr& H, int m, const Prop
     s.eq[i].w = fmaf(o.x, o.x, fmaf(o.y, o.y, o.z * o.z));
   }
   __syncwarp();
-  for (int k = lane; k < pi.y; k += 32) {
+  for (int k = lane; k < pi.y; k += NL) {
     int q = s.pa[k];
     s.p_new[k] = wrap_pos(s.nx[q], s.ny[q], s.nz[q], H);
   }
