@@ -307,9 +307,9 @@ __device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const 
       return s.lj[q * kRing + (at & (kRing - 1))];
     };
     if (precise)
-      uniform_items<true>(P, H, s, mi, count, tid, threads, acc, entry);
+      uniform_items<true>(P, H, s, mi, count, tid, threads, T, acc, entry);
     else
-      uniform_items<false>(P, H, s, mi, count, tid, threads, acc, entry);
+      uniform_items<false>(P, H, s, mi, count, tid, threads, T, acc, entry);
     if (!more) return;
     head += 32;
     __syncwarp();
