@@ -56,11 +56,10 @@ FP32_FLOPS_PER_PAIR = 38   # per atom pair, fixed by convention from the referen
 # only for its own tile and kernel version; otherwise the line's traffic is
 # null and says why (a launch reads the chains' rows about once whatever the
 # tile, ~34 MB, but a figure from another tile or kernel is not this run's).
-CHAIN_KERNEL_VERSION = ("pair code shared by both placements, LJ mask in the header, FP32-only "
-                        "step, FP64 re-takes from per-atom blending rows and one rsqrt")
-# (the re-take's screen reusing the step's FP32 screen changed no row a launch
-# reads outside the rare re-takes; the capture above stands for it)
-CHAIN_TRAFFIC_BYTES = {(160, 1, 64, 1): (33.97e6, CHAIN_KERNEL_VERSION)}
+CHAIN_KERNEL_VERSION = ("chains handed between groups each segment, a lane per (entry, placement) "
+                        "of a 3-site pair batch, two-sum reduction over the lanes")
+CHAIN_TRAFFIC_BYTES = {(160, 1, 64, 1): (33.97e6, "pair code shared by both placements, LJ mask in "
+                                         "the header, FP64 re-takes from blending rows")}
 
 
 def chain_traffic(tile):
@@ -779,7 +778,8 @@ def main():
     else:
         tile = bt.autotune(128) if not args.no_autotune else bt.tile
     threads, cpc, spl, lanes = tile
-    launches_per_step = math.ceil(STEPS_PER_BENCH / spl)
+    # one launch takes up to 32 segments of spl steps
+    launches_per_step = math.ceil(STEPS_PER_BENCH / (32 * spl))
 
     # The library launches on a torch stream, so CUDA events recorded on that
     # stream bracket exactly the chain kernels of each bench step.

@@ -343,24 +343,28 @@ int mcgpu_chain_set_window(mcgpu_box* box, int k);
 int mcgpu_batch_create(mcgpu_ctx* ctx, int n_chains, const mcgpu_box_desc* descs,
                        const uint64_t* seeds, int rotation, mcgpu_batch** out);
 int mcgpu_batch_destroy(mcgpu_batch* batch);
-/* Advances every chain by n_steps steps (launches of steps_per_launch steps,
- * replayed from a captured CUDA graph).  Asynchronous on the batch stream
- * unless sync != 0. */
+/* Advances every chain by n_steps steps.  Without lists, windows and volume
+ * moves one launch takes up to 32 * steps_per_launch steps, its groups passing
+ * the chains on every steps_per_launch steps; otherwise launches of
+ * steps_per_launch steps, replayed from a captured CUDA graph.  Asynchronous on
+ * the batch stream unless sync != 0. */
 int mcgpu_batch_run(mcgpu_batch* batch, int n_steps, int sync);
 /* Chooses threads per CTA, chains per CTA, lanes per neighbour molecule and
- * steps per launch by timing candidate tiles on this batch, trial_steps
- * steps each, every timed launch starting from a cleared L2 (the rows are
+ * steps per launch by timing candidate tiles on this batch (runs of at least
+ * trial_steps steps and four segments), every timed launch starting from a cleared L2 (the rows are
  * saved first and restored after every trial and at the end, so the batch
  * continues from where it was).  Allocates a scratch buffer of twice the L2
  * size for the duration of the call. */
 int mcgpu_batch_autotune(mcgpu_batch* batch, int trial_steps);
 /* Sets the tile explicitly: threads per CTA (32..512, a multiple of 32),
- * chains per CTA (dividing its warps), steps per launch (>= 1), and lanes
- * per neighbour molecule (a power of two <= 32 capping every chain's
+ * chains per CTA (dividing its warps), steps a chain takes on a group before it
+ * is passed on (steps_per_launch >= 1; also the steps of one launch of a batch
+ * with lists, windows or volume moves), and lanes per neighbour molecule (a power of two <= 32 capping every chain's
  * default; 0 keeps the defaults: one lane for a chain of one species of at
  * most 4 atoms, else the power of two at or above its largest molecule).
  * Results do not depend on the first three; the lanes change the FP32
- * summation order and so the last bits of the energies. */
+ * summation order and so the last bits of the energies.  Few chains with FP64 pairs and no window set run windows of
+ * 4 or 2 steps on CTAs of their own; the tile then sets steps_per_launch. */
 int mcgpu_batch_set_tile(mcgpu_batch* batch, int threads, int chains_per_cta,
                          int steps_per_launch, int lanes_per_molecule);
 int mcgpu_batch_get_tile(mcgpu_batch* batch, int* threads, int* chains_per_cta,

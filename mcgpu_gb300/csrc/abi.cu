@@ -1502,7 +1502,7 @@ extern "C" int mcgpu_chain_run(mcgpu_box* b, uint64_t seed, uint32_t chain_id, i
     P.trace = nullptr;
     if (K > 1)
       CK(ctx, launch_chain_window(K, 1, nw * 32, wsmem, st, P, k, b->order, 1, sh,
-                                  trace ? b->dtrace : nullptr, done, 0, 0));
+                                  trace ? b->dtrace : nullptr, done, 0, 0, true));
     else {
       ChainLaunch A{k, k, 1, nw, b->queue, b->order, b->order + 1, sh};
       A.trace = trace ? b->dtrace : nullptr;
@@ -1555,6 +1555,8 @@ struct mcgpu_batch {
   int graph_launches = 0, graph_spl = 0, graph_threads = 0, graph_cpc = 0, graph_lanes = 0;
   int graph_interval = 0;                 // NPT interval the graph covers (0 = NVT graph)
   int window = 1;                         // steps per window (clusters of `window` CTAs)
+  int idle_window = 1;                    // the same where none is set (batch_idle_window)
+  bool tuning = false;                    // the tile search: one-step kernels
   int graph_window = 0;
   // NPT: steps every chain has taken (all chains advance together), the
   // volume interval, and the volume phase's device buffers
@@ -1586,27 +1588,66 @@ static int batch_grid(mcgpu_batch* bt, int* smem_out) {
   return std::max(1, std::min(need, per_sm * bt->ctx->sm_count));
 }
 
+// Few chains with FP64 pairs leave most SMs idle, while each chain's step is bound by
+// the FP64 pipe of its SM (a warp instruction in 16 cycles).  Where no window is set
+// such a batch runs windows of 4 or 2 steps over clusters of as many CTAs, if all
+// chains' clusters are resident at once: the decisions and coordinates are the
+// one-step kernel's.  Not 8: in boxes of some hundred molecules most steps of a
+// window depend on an earlier one and are evaluated again.  37 chains of 64 to 700
+// waters, 96 steps: 2.80 ms one step at a time, 1.81 in windows of 4.
+constexpr int kIdleWindowThreads = 256;
+
+static int batch_idle_window(mcgpu_batch* bt, int* out) {
+  mcgpu_ctx* ctx = bt->ctx;
+  const int nc = bt->pool.n_chains;
+  std::vector<int> f64(nc);
+  CK(ctx, cudaMemcpy2DAsync(f64.data(), sizeof(int), &bt->pool.P.hdr->fp64_pairs, sizeof(ChainHdr),
+                            sizeof(int), nc, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(ctx, cudaStreamSynchronize(ctx->stream));
+  *out = 1;
+  for (int v : f64)
+    if (!v) return MCGPU_OK;
+  const SmemShape sh = shape_for(bt->pool.max_len, kIdleWindowThreads / 32, bt->cache_n);
+  for (int k : {4, 2}) {
+    const int smem = window_smem_bytes(sh, k);
+    if (nc * k > ctx->sm_count || smem > kWindowSmemMax) continue;
+    if (window_max_clusters(k, kIdleWindowThreads, smem) < nc) continue;
+    *out = k;
+    break;
+  }
+  return MCGPU_OK;
+}
+
+// Steps per window a launch of the batch takes, and the threads of its CTAs.
+static int batch_window(const mcgpu_batch* bt) {
+  return bt->window > 1 || bt->tuning ? bt->window : bt->idle_window;
+}
+
 // One launch of `steps` steps of every chain, each chain spl steps at a time on
 // a group (the running energy takes a chain's dE sum once per spl steps, so a
 // batch's energies do not depend on how its steps are split into launches).
 static int batch_launch(mcgpu_batch* bt, int steps, cudaStream_t st,
                         mcgpu_trace* trace = nullptr, int trace_off = 0, int trace_stride = 0) {
   mcgpu_ctx* ctx = bt->ctx;
+  bt->rows_stale = true;
+  int rc = pool_nl_rebuild(ctx, bt->pool, st);
+  if (rc) return rc;
+  if (batch_window(bt) > 1) {
+    const bool set = bt->window > 1;
+    const int K = batch_window(bt), threads = set ? bt->threads : kIdleWindowThreads;
+    const SmemShape sh = shape_for(bt->pool.max_len, threads / 32, bt->cache_n);
+    const int wsmem = window_smem_bytes(sh, K);
+    const int n_cl = std::max(1, std::min(bt->pool.n_chains,
+                                          window_max_clusters(K, threads, wsmem)));
+    CK(ctx, launch_chain_window(K, n_cl, threads, wsmem, st, bt->pool.P, steps, bt->order,
+                                bt->pool.n_chains, sh, trace, trace_off, trace_stride, bt->lanes,
+                                set));
+    return MCGPU_OK;
+  }
   int smem = 0;
   const int grid = batch_grid(bt, &smem);
   const int gw = batch_gwarps(bt);
   SmemShape sh = shape_for(bt->pool.max_len, gw, bt->cache_n);
-  bt->rows_stale = true;
-  int rc = pool_nl_rebuild(ctx, bt->pool, st);
-  if (rc) return rc;
-  if (bt->window > 1) {
-    const int K = bt->window, wsmem = window_smem_bytes(sh, K);
-    const int n_cl = std::max(1, std::min(bt->pool.n_chains,
-                                          window_max_clusters(K, bt->threads, wsmem)));
-    CK(ctx, launch_chain_window(K, n_cl, bt->threads, wsmem, st, bt->pool.P, steps, bt->order,
-                                bt->pool.n_chains, sh, trace, trace_off, trace_stride, bt->lanes));
-    return MCGPU_OK;
-  }
   const int seg = std::min(steps, bt->spl);
   CK(ctx, cudaMemsetAsync(bt->sched, 0, sizeof(unsigned) * bt->pool.n_chains, st));
   const int n = bt->pool.n_chains;
@@ -1849,7 +1890,7 @@ static int batch_build_graph(mcgpu_batch* bt, int launches, int interval) {
   bt->graph_cpc = bt->cpc;
   bt->graph_lanes = bt->lanes;
   bt->graph_interval = interval;
-  bt->graph_window = bt->window;
+  bt->graph_window = batch_window(bt);
   return MCGPU_OK;
 }
 
@@ -1857,7 +1898,7 @@ static bool batch_graph_matches(const mcgpu_batch* bt, int launches, int interva
   return bt->graph && bt->graph_spl == bt->spl && bt->graph_launches == launches &&
          bt->graph_threads == bt->threads && bt->graph_cpc == bt->cpc &&
          bt->graph_lanes == bt->lanes && bt->graph_interval == interval &&
-         bt->graph_window == bt->window;
+         bt->graph_window == batch_window(bt);
 }
 
 // Steps n_steps with direct launches of at most `most` steps (recording steps
@@ -1890,7 +1931,7 @@ static int batch_advance(mcgpu_batch* bt, int n_steps, mcgpu_trace* trace, int t
     int done = 0;
     // nothing to do between the launches of a one-step NVT batch without
     // lists: one launch takes the steps of 32, the chains spl steps at a time
-    const bool merged = bt->window == 1 && !bt->pool.nl_on;
+    const bool merged = batch_window(bt) == 1 && !bt->pool.nl_on;
     const int most = merged ? (int)std::min(32LL * spl, 1LL << 30) : spl;
     if (!merged && !trace && full >= per_graph) {
       if (!batch_graph_matches(bt, per_graph, 0)) {
@@ -2074,7 +2115,7 @@ extern "C" int mcgpu_batch_set_precision(mcgpu_batch* bt, int precision) {
   CK(ctx, cudaMemcpy2DAsync(&bt->pool.P.hdr->fp64_pairs, sizeof(ChainHdr), v.data(), sizeof(int),
                             sizeof(int), nc, cudaMemcpyHostToDevice, ctx->stream));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return MCGPU_OK;
+  return batch_idle_window(bt, &bt->idle_window);
 }
 
 extern "C" int mcgpu_batch_sync(mcgpu_batch* bt) {
@@ -2289,7 +2330,7 @@ extern "C" int mcgpu_batch_restore(mcgpu_batch* bt, const void* buf, size_t len)
   CK(ctx, cudaStreamSynchronize(ctx->stream));
   bt->steps_done = h.steps_done;
   bt->rows_stale = false;
-  return MCGPU_OK;
+  return batch_idle_window(bt, &bt->idle_window);
 }
 
 // ---- autotuner ---------------------------------------------------------------------
@@ -2325,6 +2366,11 @@ extern "C" int mcgpu_batch_autotune(mcgpu_batch* bt, int trial_steps) {
     return set_err(ctx, MCGPU_ERR_INVALID, "the tile search times one-step kernels: set the window to 1 first");
   int rc = batch_snapshot(bt, false);
   if (rc) return rc;
+  struct Tuning {
+    mcgpu_batch* bt;
+    explicit Tuning(mcgpu_batch* b) : bt(b) { bt->tuning = true; }
+    ~Tuning() { bt->tuning = false; }
+  } tuning(bt);
   const long long steps0 = bt->steps_done;
   struct Tile { int threads, cpc, spl, lanes; };
   cudaEvent_t e0, e1;

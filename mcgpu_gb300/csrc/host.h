@@ -220,10 +220,11 @@ cudaError_t window_init();
 // once (0 if none).
 int window_max_clusters(int K, int threads, int smem);
 // n_clusters clusters of K CTAs of `threads` threads, chain tasks order[0
-// .. n_tasks) advanced n_steps steps each in windows of K steps.
+// .. n_tasks) advanced n_steps steps each in windows of K steps; count_redo: the
+// chains' headers count the steps evaluated again.
 cudaError_t launch_chain_window(int K, int n_clusters, int threads, int smem, cudaStream_t st,
                                 const Pool& P, int n_steps, const int* order, int n_tasks,
                                 SmemShape sh, mcgpu_trace* trace, int trace_off, int trace_stride,
-                                int lanes_cap);
+                                int lanes_cap, bool count_redo);
 
 }  // namespace mcgpu

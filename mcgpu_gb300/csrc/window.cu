@@ -23,10 +23,12 @@
 // depends on an accepted one is a vote away.  The steps before it stand and
 // are committed by one warp each.  Walking the steps one by one, every warp
 // committing each, took 2 to 2.5 us a step and most of a window: 28 us per
-// window of 8 on 32,768 waters where a step's evaluation takes 10.  Decisions, coordinates and counters are therefore those of
-// the one-group kernel on the same draws; the FP32 pair sums are the
-// one-group kernel's too when the CTA has as many warps (same split of the
-// candidates over the warps).
+// window of 8 on 32,768 waters where a step's evaluation takes 10.
+//
+// Decisions, coordinates and counters are therefore those of the one-group
+// kernel on the same draws; the FP32 pair sums are its own up to their order (it
+// evaluates with one warp less on chains whose items the warps share, the last
+// one staging the next move).
 //
 // Memory: every CTA writes every accepted placement (the same values), and
 // a CTA reads the pool only after its own writes of every earlier step.  A
@@ -255,7 +257,8 @@ __device__ void window_eval(const Pool& P, const ChainHdr& H, const Group& g, co
 // trace_stride and lanes_cap as in chain_steps.
 __global__ void __launch_bounds__(512, 1)
     k_chain_window(Pool P, int n_steps, const int* order, int n_tasks, SmemShape shape,
-                   mcgpu_trace* trace, int trace_off, int trace_stride, int lanes_cap) {
+                   mcgpu_trace* trace, int trace_off, int trace_stride, int lanes_cap,
+                   bool count_redo) {
   extern __shared__ __align__(16) char smem[];
   const unsigned K = cluster_size(), rank = cluster_rank();
   const int n_cl = (int)(gridDim.x / K), cid = (int)(blockIdx.x / K);
@@ -479,7 +482,7 @@ __global__ void __launch_bounds__(512, 1)
       Hp->accepted += acc_n;
       Hp->pairs += npairs;
       Hp->ties += ties;
-      Hp->win_redo += redo;
+      if (count_redo) Hp->win_redo += redo;
       if (H.nl_on) {
         Hp->nl_valid = nl_ok ? 1 : 0;
         Hp->nl_full += full_scans;
@@ -528,7 +531,7 @@ int window_max_clusters(int K, int threads, int smem) {
 cudaError_t launch_chain_window(int K, int n_clusters, int threads, int smem, cudaStream_t st,
                                 const Pool& P, int n_steps, const int* order, int n_tasks,
                                 SmemShape sh, mcgpu_trace* trace, int trace_off, int trace_stride,
-                                int lanes_cap) {
+                                int lanes_cap, bool count_redo) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(K * n_clusters, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
@@ -542,7 +545,7 @@ cudaError_t launch_chain_window(int K, int n_clusters, int threads, int smem, cu
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k_chain_window, P, n_steps, order, n_tasks, sh, trace, trace_off,
-                            trace_stride, lanes_cap);
+                            trace_stride, lanes_cap, count_redo);
 }
 
 }  // namespace mcgpu

@@ -14,7 +14,7 @@ import numpy as np
 import pytest
 
 from helpers import tol_mixed
-from mcgpu_gb300 import PREC_MIXED, ROT_AXIS, ChainBatch, Context, GpuBox
+from mcgpu_gb300 import PREC_FP64, PREC_MIXED, ROT_AXIS, ChainBatch, Context, GpuBox
 from mcgpu_gb300 import workloads as W
 from oracle.pyoracle import OracleBox, OracleChain
 from test_gpu_chain import check_energies, replay
@@ -162,3 +162,40 @@ def test_more_chains_than_groups(ctx, tile):
         assert stats[c].accepted == acc
         assert np.array_equal(np.stack(bt.download(int(c)), 1), oc.coords()), c
     bt.close()
+
+
+@pytest.mark.parametrize("n,skin,interval", [(37, 0.0, 0), (60, 0.0, 0), (3, 1.0, 0),
+                                             (20, 0.0, 15), (4, 1.0, 15)])
+def test_few_fp64_chains_equal_many(ctx, n, skin, interval):
+    """Few FP64-pair chains run in windows over clusters, many one step at a time:
+    the same chains, decisions and coordinates (FP64 sums in another order), also
+    from a checkpoint restored into a batch whose precision was not set."""
+    boxes, seeds = W.water_chains(80, n_min=300 if skin else 40, n_max=400, seed=23)
+    def batch(k, f64=True):
+        bt = ChainBatch(ctx, boxes[:k], seeds[:k], rotation=ROT_AXIS)
+        bt.set_tile(128, 1, 16)
+        if f64:
+            bt.set_precision(PREC_FP64)
+        if interval:
+            bt.set_npt(interval, 1.0, 0.02)
+        if skin:
+            bt.set_verlet(skin)
+        return bt
+    many, few = batch(80), batch(n)
+    for bt in (many, few):
+        bt.run(40)
+    ck = few.checkpoint()
+    again = batch(n, False)
+    again.restore(ck)
+    for bt in (many, few, again):
+        bt.run(33)
+    sm = many.stats()
+    for bt in (few, again):
+        for c, s in enumerate(bt.stats()):
+            assert (s.accepted, s.steps, s.error) == (sm[c].accepted, 73, 0), c
+            assert (s.ties, s.pairs) == (sm[c].ties, sm[c].pairs), c
+            assert s.window_redo == 0 and s.vol_accepted == sm[c].vol_accepted
+            assert abs(s.energy - sm[c].energy) <= 1e-9 * max(1.0, abs(sm[c].energy)), c
+            assert np.array_equal(np.stack(bt.download(c)), np.stack(many.download(c))), c
+    for bt in (many, few, again):
+        bt.close()
