@@ -1,6 +1,6 @@
 """Batched device-resident chains: many independent Metropolis chains of
-uneven size and temperature advanced by one persistent kernel, replayed as a
-captured CUDA graph, with autotuned tiles (mcgpu_batch_* in the C ABI)."""
+uneven size and temperature advanced by one persistent kernel (replayed as a
+captured CUDA graph with lists, windows or volume moves), with autotuned tiles (mcgpu_batch_* in the C ABI)."""
 from __future__ import annotations
 
 import ctypes as C

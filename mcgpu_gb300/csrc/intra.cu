@@ -4,7 +4,7 @@
 // only with ENABLE_INTRA true (SimulationStep.h:15).
 //
 // A stage is one CTA on one molecule (a molecule has at most 64 atoms): the
-// ops of the stage run in order, each as a scalar set-up by thread 0 (the
+// ops of the stage run in order in the first warp, each as a scalar set-up (the
 // bond's unit vector or the plane normal) and one update per atom; then the
 // molecule's mirrors and radius, and the intramolecular energy.  The union-
 // find the reference runs on every call depends only on the bonds, so its
@@ -180,7 +180,8 @@ struct OpRows {
 // first and of the second group's angle.  Every thread of the block calls it;
 // the first warp works, with the ops' rows and the coordinates in shared memory
 // (an op is a chain of FP64 steps, and each followed three dependent loads and
-// stood between two block barriers).  Returns whether any op changed anything
+// stood between two block barriers; 304 flexible boxes, 192 steps: 44.9 ms then,
+// 42.4 this way).  Returns whether any op changed anything
 // (a bond in a ring, an angle whose ends share a component do not).
 __device__ bool apply_ops(const Pool& P, const IntraRows& R, const ChainHdr& H, int mol, int kind,
                           int n, const int* idx, const double* amt, const double* trig,
@@ -422,7 +423,8 @@ struct EvalRows {
 // a warp's last round was part full and the warps' counts differed (FP64 issues a
 // warp instruction in 16 cycles however few lanes work).  Where the items leave
 // warps idle the moved molecule's atoms are dealt too (FP64 pairs; the FP32 items
-// factor the whole molecule's charge).
+// factor the whole molecule's charge).  256 waters, FP64: 24.4 us a step with the
+// warps' own hits, 22.8 pooled; 304 flexible boxes (192 steps) 42.4 and 40.7 ms.
 template <bool F64>
 __device__ void cta_eval(const Pool& P, const ChainHdr& H, const Group& grp, const GroupSmem& s,
                          const MovedInfo& mi, EvalRows& E, double& eo, double& en,
