@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
       }
     }
     __syncthreads();
+    const bool alike = ps_alike(G, n);
     int* rj = G.ring[w];
     int head = 0, tail = 0;
     double acc = 0.0;
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
         tail += __popc(bal);
         if (tail - head >= 32) {
           __syncwarp();
-          acc += ps_items<true>(G, PoolRows{P}, rj, head, 32, lane, H.L[0], H.L[1], H.L[2]);
+          acc += ps_items<true>(G, PoolRows{P}, rj, head, 32, lane, alike, H.L[0], H.L[1], H.L[2]);
           head += 32;
           __syncwarp();
         }
@@ -324,7 +325,8 @@ __global__ void __launch_bounds__(kPsThreads, 4)
     }
     __syncwarp();
     if (tail > head)
-      acc += ps_items<true>(G, PoolRows{P}, rj, head, tail - head, lane, H.L[0], H.L[1], H.L[2]);
+      acc += ps_items<true>(G, PoolRows{P}, rj, head, tail - head, lane, alike, H.L[0], H.L[1],
+                            H.L[2]);
     const double sum = ps_block_sum(G, acc);
     if ((int)threadIdx.x < n) emol[m0 + threadIdx.x] = threadIdx.x == 0 ? sum : 0.0;
     m0 = m1;

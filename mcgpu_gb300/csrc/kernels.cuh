@@ -646,7 +646,13 @@ __device__ __forceinline__ double image64(double d, double L, int half) {
 // reference's own image from the unshifted rows.
 // (sb, eb): b's factors, qb its charge; sd, ed, qd the molecule's: sqrt(eps)
 // and, with ROOT, sqrt(sigma), else sigma itself (sigma_ab^2 = s_a s_b).
-template <bool ROOT>
+//
+// With VOTE the rare image and the LJ term stand behind votes of the lanes that
+// enter together, so those lanes must hold rows of the same length with the same
+// sites skipped: a lane that leaves the loop, or passes over a site, is waited for
+// by the others.  Lanes on unlike molecules take VOTE false, the same terms in the
+// same order behind branches of their own.
+template <bool ROOT, bool VOTE = true>
 __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys, const double* zs,
                                              const double* sd, const double* ed, const double* qd,
                                              int len, double xb, double yb, double zb, double sb,
@@ -661,7 +667,7 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
   const double bz = hi_abs(tz) >= hz ? zb - copysign(Lz, tz) : zb;
   const bool lj_b = bits_nonzero(sb) && bits_nonzero(eb);
   const double qk = qb * kCoulomb, e4 = 4.0 * eb;
-  const unsigned am = __activemask();
+  const unsigned am = VOTE ? __activemask() : 0u;
   double acc = 0.0;
 #pragma unroll 3
   for (int i = 0; i < len; i++) {
@@ -669,14 +675,14 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
     if (blend_skipped(sa)) continue;
     double dx = bx - xs[i], dy = by - ys[i], dz = bz - zs[i];
     const bool far = hi_abs(dx) >= hx || hi_abs(dy) >= hy || hi_abs(dz) >= hz;
-    if (__any_sync(am, far)) {
-      __syncwarp(am);
+    if (VOTE ? __any_sync(am, far) != 0 : far) {
+      if (VOTE) __syncwarp(am);
       if (far) {
         dx = image64(xb - xs[i], Lx, hx);
         dy = image64(yb - ys[i], Ly, hy);
         dz = image64(zb - zs[i], Lz, hz);
       }
-      __syncwarp(am);
+      if (VOTE) __syncwarp(am);
     }
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
     const bool apart = bits_nonzero(r2);  // coincident: skipped (BruteForceStep.cpp:68-69)
@@ -684,8 +690,8 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
     const double q = qd[i] * qk;
     acc = fma(apart ? q : 0.0, apart ? ri : 0.0, acc);
     const bool lj = apart && lj_b && bits_nonzero(sa) && bits_nonzero(ea);
-    if (__any_sync(am, lj)) {
-      __syncwarp(am);
+    if (VOTE ? __any_sync(am, lj) != 0 : lj) {
+      if (VOTE) __syncwarp(am);
       double t2;
       if (ROOT) {
         const double t = (sa * sb) * ri;
@@ -696,7 +702,7 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
       const double s6 = t2 * t2 * t2;
       const double e = ea * e4;
       if (lj) acc = fma(s6, fma(e, s6, -e), acc);
-      __syncwarp(am);
+      if (VOTE) __syncwarp(am);
     }
   }
   return acc;

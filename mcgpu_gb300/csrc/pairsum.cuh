@@ -30,13 +30,27 @@ struct PsGroup {
   double red[kPsWarps];
 };
 
+// Whether the group's n staged molecules have one length and the same skipped
+// sites, as the lanes of ps_items must for pair_sum64's votes.  Every thread of the
+// CTA calls it once the rows are staged, and gets the same answer.
+__device__ __forceinline__ bool ps_alike(const PsGroup& G, int n) {
+  if (n == 1) return true;
+  bool differ = false;
+  for (int g = 1; g < n; g++) {
+    differ = differ || G.len[g] != G.len[0];
+    for (int i = threadIdx.x; i < min(G.len[0], G.len[g]); i += kPsThreads)
+      differ = differ || blend_skipped(G.sd[g * kPsPitch + i]) != blend_skipped(G.sd[i]);
+  }
+  return !__syncthreads_or(differ);
+}
+
 // Evaluates `count` (1..32) ring entries (j << 3 | group molecule) from
 // `head`: this lane's share of the sum.  rows: len(j), start(j) of molecule
-// j and its atoms' position and factors.
+// j and its atoms' position and factors.  alike: ps_alike's answer.
 template <bool ROOT, class Rows>
 __device__ __forceinline__ double ps_items(const PsGroup& G, const Rows& rows, const int* rj,
-                                           int head, int count, int lane, double Lx, double Ly,
-                                           double Lz) {
+                                           int head, int count, int lane, bool alike, double Lx,
+                                           double Ly, double Lz) {
   int len = 0;
   if (lane < count) len = rows.len(rj[(head + lane) & (kRing - 1)] >> 3);
   const int len0 = __shfl_sync(~0u, len, 0);
@@ -76,8 +90,12 @@ __device__ __forceinline__ double ps_items(const PsGroup& G, const Rows& rows, c
     const int o = (jm & 7) * kPsPitch;
     double xb, yb, zb, sb, eb, qb;
     rows.atom(rows.start(jm >> 3) + k, xb, yb, zb, sb, eb, qb);
-    acc += pair_sum64<ROOT>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o,
-                            G.len[jm & 7], xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
+    if (alike)
+      acc += pair_sum64<ROOT>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o, G.len[0],
+                              xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
+    else
+      acc += pair_sum64<ROOT, false>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o,
+                                     G.len[jm & 7], xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
   }
   return acc;
 }

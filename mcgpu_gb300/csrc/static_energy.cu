@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
       if (threadIdx.x == 0) G.len[g] = len;
     }
     __syncthreads();
+    const bool alike = ps_alike(G, n);
     int head = 0, tail = 0;
     for (int base = m0 + 1 + w * 32; base < r.n_mol; base += kPsThreads) {
       const int j = base + lane;
@@ -204,7 +205,8 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
         tail += __popc(bal);
         if (tail - head >= 32) {
           __syncwarp();
-          acc += ps_items<false>(G, StaticRows{r}, rj, head, 32, lane, r.L[0], r.L[1], r.L[2]);
+          acc += ps_items<false>(G, StaticRows{r}, rj, head, 32, lane, alike, r.L[0], r.L[1],
+                                 r.L[2]);
           head += 32;
           __syncwarp();
         }
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
     }
     __syncwarp();
     if (tail > head)
-      acc += ps_items<false>(G, StaticRows{r}, rj, head, tail - head, lane, r.L[0], r.L[1],
+      acc += ps_items<false>(G, StaticRows{r}, rj, head, tail - head, lane, alike, r.L[0], r.L[1],
                              r.L[2]);
     __syncthreads();   // the next atoms overwrite the stage
   }
