@@ -335,6 +335,8 @@ int upload_pool(mcgpu_ctx* ctx, HostPool& hp, DevPool& dp) {
   CK(ctx, cudaGetLastError());
   CK(ctx, cudaStreamSynchronize(st));
   dp.hdr.assign(hp.hdr.begin(), hp.hdr.end());
+  dp.min_chain = dp.n_mol;
+  for (const ChainHdr& h : dp.hdr) dp.min_chain = std::min(dp.min_chain, h.n_mol);
   dp.mstart.assign(hp.mstart.begin(), hp.mstart.end());
   dp.mlen.assign(hp.mlen.begin(), hp.mlen.end());
   return MCGPU_OK;
@@ -445,8 +447,8 @@ int pool_nl_rebuild(mcgpu_ctx* ctx, DevPool& dp, cudaStream_t st) {
 
 // Full system energy of every chain of the pool into dp.esum (device).
 int pool_system_energy(mcgpu_ctx* ctx, DevPool& dp, bool f64, cudaStream_t st) {
-  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, shape_for(dp.max_len, kEnergyWarps), st, dp.P,
-                               dp.mol_chain, dp.emol));
+  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, dp.min_chain, shape_for(dp.max_len, kEnergyWarps),
+                               st, dp.P, dp.mol_chain, dp.emol));
   k_chain_sums<<<dp.n_chains, 256, 0, st>>>(dp.P, dp.emol, dp.esum);
   CK(ctx, cudaGetLastError());
   return MCGPU_OK;
@@ -810,7 +812,7 @@ extern "C" int mcgpu_system_energy(mcgpu_box* b, double* out) {
     // calcSystemEnergy with ENABLE_INTRA: molecule m adds E(m, j > m) and its
     // intramolecular energy (SimulationStep.cpp:40-71 over :15-18)
     DevPool& dp = b->pool;
-    CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64, dp.n_mol,
+    CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64, dp.n_mol, dp.min_chain,
                                  shape_for(dp.max_len, kEnergyWarps), ctx->stream, dp.P,
                                  dp.mol_chain, dp.emol));
     CK(ctx, launch_intra_add(dp.P, b->intra->R, dp.n_mol, dp.emol, ctx->stream));

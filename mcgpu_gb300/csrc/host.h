@@ -52,9 +52,11 @@ cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, 
                                  Pool P, int chain, int mol, Proposal prop, double* partials,
                                  unsigned* counter, double* out, long long* pairs = nullptr,
                                  unsigned* done = nullptr, unsigned call = 0);
-// emol[m] with the sum over the chains' molecules of E(m, j > m).
-cudaError_t launch_mol_pair_sums(bool f64, int n_mol, SmemShape sh, cudaStream_t st,
-                                 const Pool& P, const int* mol_chain, double* emol);
+// emol[m], summed over a chain's molecules, with E(m, j > m); min_chain: the
+// molecules of the smallest chain.  A chain's rows depend on the chain alone.
+cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, SmemShape sh,
+                                 cudaStream_t st, const Pool& P, const int* mol_chain,
+                                 double* emol);
 // One volume phase of the chains in act (all when act has no ranges) on
 // stream st: proposals, cell grids, FP32 / FP64 totals, decisions, the
 // double-float and FP64 re-takes; vlist holds 3 * (chains) + 3 ints.
@@ -167,6 +169,7 @@ int build_pool(mcgpu_ctx* ctx, HostPool& hp, const mcgpu_box_desc* descs, int n,
 struct DevPool {
   Pool P{};
   int n_chains = 0, n_mol = 0, n_atom = 0, n_pidx = 0, max_len = 0;
+  int min_chain = 0;              // molecules of the smallest chain
   int* mol_chain = nullptr;
   int* atom_mol = nullptr;
   double* emol = nullptr;

@@ -222,14 +222,16 @@ struct PoolRows {
 };
 
 // E(m, j > m) of SimulationStep::calcSystemEnergy (SimulationStep.cpp:47-48)
-// with FP64 pairs, ps_group consecutive molecules per CTA (a group that spans
-// chains is taken chain by chain): emol[first molecule] holds the sum over
-// the group's molecules of the chain, the others 0.  The in-range set is the
+// with FP64 pairs, groups of ps_group consecutive molecules of a chain:
+// emol[first molecule] holds the sum over the group's molecules, the others 0.
+// A CTA takes the groups that start among its `span` molecules (at most the
+// smallest chain's group, so that a CTA has one to take or, in a larger chain,
+// none).  The in-range set is the
 // FP64 test's (the FP32 screen decides outside its guard band).  32,768
 // waters (rc 12 A, 35.6 M pairs): 1.84 ms, bound by the issue of the N^2 / 2
 // screen beside the FP64 pipe (58 % busy); 5.84 ms with a CTA per molecule.
 __global__ void __launch_bounds__(kPsThreads, 4)
-    k_pair_sums64(Pool P0, const LoopTask* tasks, const int* mol_chain, int m_begin, int m_end,
+    k_pair_sums64(Pool P0, const LoopTask* tasks, const int* mol_chain, int n_mol, int span,
                   double* emol) {
   __shared__ Pool SP;
   __shared__ PsGroup G;
@@ -238,18 +240,23 @@ __global__ void __launch_bounds__(kPsThreads, 4)
   load_pool(SP, P0, tasks);
   const Pool& P = SP;
   if (tasks) {
-    m_end = tasks[blockIdx.y].n_mol;
+    n_mol = tasks[blockIdx.y].n_mol;
+    span = ps_group(n_mol);
     emol = tasks[blockIdx.y].emol;
   }
-  const int group = ps_group(m_end - m_begin);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = lanemask_lt();
-  int m0 = m_begin + (int)blockIdx.x * group;
-  const int mg = min(m0 + group, m_end);
+  int m0 = (int)blockIdx.x * span;
+  const int mg = min(m0 + span, n_mol);
   while (m0 < mg) {
     const int c = tasks ? 0 : mol_chain[m0];
     const ChainHdr& H = P.hdr[c];
-    const int m1 = min(mg, H.mol0 + H.n_mol), n = m1 - m0;
+    const int group = ps_group(H.n_mol), off = (m0 - H.mol0) % group;
+    const int m1 = min(m0 - off + group, H.mol0 + H.n_mol), n = m1 - m0;
+    if (off > 0) {   // inside a group that starts before this CTA's molecules
+      m0 = m1;
+      continue;
+    }
     for (int g = 0; g < n; g++) {
       const int m = m0 + g, a0 = P.mstart[m], len = P.mlen[m] & 255;
       const int2 pi = P.mpi[m];
@@ -785,11 +792,13 @@ cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, 
 
 int pair_sum_groups(int n_mol) { return (n_mol + ps_group(n_mol) - 1) / ps_group(n_mol); }
 
-cudaError_t launch_mol_pair_sums(bool f64, int n_mol, SmemShape sh, cudaStream_t st,
-                                 const Pool& P, const int* mol_chain, double* emol) {
+cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, SmemShape sh,
+                                 cudaStream_t st, const Pool& P, const int* mol_chain,
+                                 double* emol) {
   if (f64) {
-    k_pair_sums64<<<pair_sum_groups(n_mol), kPsThreads, 0, st>>>(P, nullptr, mol_chain, 0, n_mol,
-                                                             emol);
+    const int span = ps_group(min_chain);
+    k_pair_sums64<<<(n_mol + span - 1) / span, kPsThreads, 0, st>>>(P, nullptr, mol_chain, n_mol,
+                                                                    span, emol);
   } else {
     k_pair_sums32<<<n_mol, sh.nwarps * 32, sh.bytes(), st>>>(P, nullptr, mol_chain, 0, sh, emol);
   }
