@@ -353,8 +353,9 @@ int mcgpu_batch_run(mcgpu_batch* batch, int n_steps, int sync);
  * steps per launch by timing candidate tiles on this batch (runs of at least
  * trial_steps steps and four segments), every timed launch starting from a cleared L2 (the rows are
  * saved first and restored after every trial and at the end, so the batch
- * continues from where it was).  Allocates a scratch buffer of twice the L2
- * size for the duration of the call. */
+ * continues from where it was).  A batch that runs windows unasked
+ * (mcgpu_batch_set_tile) has its steps per launch alone searched.  Allocates a
+ * scratch buffer of twice the L2 size for the duration of the call. */
 int mcgpu_batch_autotune(mcgpu_batch* batch, int trial_steps);
 /* Sets the tile explicitly: threads per CTA (32..512, a multiple of 32),
  * chains per CTA (dividing its warps), steps a chain takes on a group before it
@@ -363,8 +364,11 @@ int mcgpu_batch_autotune(mcgpu_batch* batch, int trial_steps);
  * default; 0 keeps the defaults: one lane for a chain of one species of at
  * most 4 atoms, else the power of two at or above its largest molecule).
  * Results do not depend on the first three; the lanes change the FP32
- * summation order and so the last bits of the energies.  Few chains with FP64 pairs and no window set run windows of
- * 4 or 2 steps on CTAs of their own; the tile then sets steps_per_launch. */
+ * summation order and so the last bits of the energies.  Few chains with FP64
+ * pairs run windows of 4 or 2 steps on CTAs of 256 threads, and the tile then
+ * sets steps_per_launch alone, unless a window has been set:
+ * mcgpu_batch_set_window(batch, 1) keeps them on the one-step kernel and the
+ * tile's threads. */
 int mcgpu_batch_set_tile(mcgpu_batch* batch, int threads, int chains_per_cta,
                          int steps_per_launch, int lanes_per_molecule);
 int mcgpu_batch_get_tile(mcgpu_batch* batch, int* threads, int* chains_per_cta,
@@ -373,7 +377,8 @@ int mcgpu_batch_get_tile(mcgpu_batch* batch, int* threads, int* chains_per_cta,
  * mcgpu_chain_set_window: one cluster of k CTAs per chain, each CTA one
  * group of the tile's threads (the tile must have one chain per CTA and at
  * least k warps).  For a few large chains; a batch of many chains already
- * fills the device one chain per group. */
+ * fills the device one chain per group.  k = 1: one step at a time, whatever
+ * the batch would choose by itself (mcgpu_batch_set_tile). */
 int mcgpu_batch_set_window(mcgpu_batch* batch, int k);
 /* Like mcgpu_batch_run (synchronous, no graph) and records every step:
  * out[c * n_steps + s] is step s of chain c.  If vol_out is non-NULL it

@@ -162,7 +162,8 @@ class ChainBatch:
     def set_window(self, k: int) -> None:
         """Windows of k steps (1, 2, 4, 8): one cluster of k CTAs per chain,
         the window's moves evaluated at once and decided in step order
-        (mcgpu_batch_set_window); results equal k = 1."""
+        (mcgpu_batch_set_window); results equal k = 1, one step at a time
+        (which a batch of few FP64-pair chains takes only when it is set)."""
         self._check(_abi.lib().mcgpu_batch_set_window(self._h, int(k)))
 
     @property

@@ -1556,9 +1556,8 @@ struct mcgpu_batch {
   cudaGraphExec_t graph = nullptr;
   int graph_launches = 0, graph_spl = 0, graph_threads = 0, graph_cpc = 0, graph_lanes = 0;
   int graph_interval = 0;                 // NPT interval the graph covers (0 = NVT graph)
-  int window = 1;                         // steps per window (clusters of `window` CTAs)
+  int window = 0;                         // steps per window (clusters of `window` CTAs); 0: not set
   int idle_window = 1;                    // the same where none is set (batch_idle_window)
-  bool tuning = false;                    // the tile search: one-step kernels
   int graph_window = 0;
   // NPT: steps every chain has taken (all chains advance together), the
   // volume interval, and the volume phase's device buffers
@@ -1620,9 +1619,9 @@ static int batch_idle_window(mcgpu_batch* bt, int* out) {
   return MCGPU_OK;
 }
 
-// Steps per window a launch of the batch takes, and the threads of its CTAs.
+// Steps per window a launch of the batch takes: the caller's choice, 1 included.
 static int batch_window(const mcgpu_batch* bt) {
-  return bt->window > 1 || bt->tuning ? bt->window : bt->idle_window;
+  return bt->window > 0 ? bt->window : bt->idle_window;
 }
 
 // One launch of `steps` steps of every chain, each chain spl steps at a time on
@@ -2366,13 +2365,11 @@ extern "C" int mcgpu_batch_autotune(mcgpu_batch* bt, int trial_steps) {
   if (trial_steps < 1) trial_steps = 64;
   if (bt->window > 1)
     return set_err(ctx, MCGPU_ERR_INVALID, "the tile search times one-step kernels: set the window to 1 first");
+  // a batch that runs windows unasked takes CTAs of their size whatever the tile:
+  // only the steps of a launch are searched, on the kernel that will run
+  const bool windows = batch_window(bt) > 1;
   int rc = batch_snapshot(bt, false);
   if (rc) return rc;
-  struct Tuning {
-    mcgpu_batch* bt;
-    explicit Tuning(mcgpu_batch* b) : bt(b) { bt->tuning = true; }
-    ~Tuning() { bt->tuning = false; }
-  } tuning(bt);
   const long long steps0 = bt->steps_done;
   struct Tile { int threads, cpc, spl, lanes; };
   cudaEvent_t e0, e1;
@@ -2424,7 +2421,8 @@ extern "C" int mcgpu_batch_autotune(mcgpu_batch* bt, int trial_steps) {
   // search settles)
   std::vector<Tile> shapes;
   const int tw[] = {64, 128, 256, 512};
-  for (int t : tw)
+  for (int t : tw) {
+    if (windows) break;
     for (int gw = 1; gw <= t / 32; gw *= 2) {
       const int cpc = (t / 32) / gw;
       if (gw > 1 && cpc > 15) continue;
@@ -2433,9 +2431,11 @@ extern "C" int mcgpu_batch_autotune(mcgpu_batch* bt, int trial_steps) {
       if (t == 512 && cpc != 1) continue;
       shapes.push_back({t, cpc, 64, 0});
     }
+  }
   // one group of 3, 5, 6 or 7 warps per CTA (at 128 registers a thread,
   // 5-warp CTAs fit three to an SM: three chains in flight instead of two)
-  for (int t : {96, 160, 192, 224}) shapes.push_back({t, 1, 64, 0});
+  for (int t : {96, 160, 192, 224})
+    if (!windows) shapes.push_back({t, 1, 64, 0});
   int max_tpm = 1;
   for (const ChainHdr& h : bt->pool.hdr) max_tpm = std::max(max_tpm, h.tpm);
   for (const Tile& S : shapes)
