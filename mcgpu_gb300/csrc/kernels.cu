@@ -675,6 +675,7 @@ __device__ __forceinline__ void chain_steps(Pool P, const ChainLaunch& A, char* 
         group_reduce(g, ss, eo, en, np2, st & 1);
         e_old = eo;
         e_new = en;
+        if (f64all) acc.np = np2;   // (a re-take's pairs are counted already)
         const double d64 = e_new - e_old;
         ok = (d64 < 0) || (exp(-d64 / H.kT) >= (double)u);
       } else {

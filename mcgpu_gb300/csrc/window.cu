@@ -246,6 +246,7 @@ __device__ void window_eval(const Pool& P, const ChainHdr& H, const Group& g, co
     group_reduce(g, ss, eo, en, np2, nred++ & 1);
     x.eo = eo;
     x.en = en;
+    if (f64all) x.np = np2;   // (a re-take's pairs are counted already)
   }
 }
 
