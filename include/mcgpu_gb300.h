@@ -482,7 +482,10 @@ typedef struct {
   int32_t max_mol_atoms;      /* largest molecule a job may hold (<= 64)     */
   int32_t rotation;           /* MCGPU_ROT_EULER or MCGPU_ROT_AXIS          */
   int32_t threads, chains_per_cta, lanes_per_molecule; /* chain-kernel tile,
-                                 fixed for the server's life (0: defaults)   */
+                                 fixed for the server's life (0: defaults).  The
+                                 default, 256 threads with one chain, runs jobs
+                                 of molecules of more than 4 atoms on 512; any
+                                 other tile is every job's                   */
   int32_t pad0;
 } mcgpu_server_config;
 

@@ -69,11 +69,14 @@ constexpr long long kBytesAtom = 6 * 8 + 16 + 16 + 8 + 16 + 4;          // 108
 constexpr long long kBytesMol = 4 + 4 + 8 + 16 + 4 + 16 + 4 + 8 + 8 + 16;  // 88
 constexpr long long kBytesPidx = 4 + 16;                                  // 20
 
-// Warps of a group for jobs of molecules of more than kWideAtoms atoms.  A round
+// The default tile, and the warps of a group for jobs of molecules of more than
+// kWideAtoms atoms where the caller left the tile at it (any other tile is taken
+// as it is for every job).  A round
 // lasts as long as its largest job (4,096 16-atom molecules: 29 us a step on 8
 // warps, half the chip idle meanwhile).  160 jobs of both species: 238 ms with all
 // on 8 warps one kind after the other, 202 ms with the larger molecules on 16 and
 // the two kinds side by side.
+constexpr int kDefaultThreads = 256, kDefaultChains = 1;
 constexpr int kWideWarps = 16, kWideAtoms = 4;
 
 struct Job {
@@ -520,8 +523,8 @@ extern "C" int mcgpu_server_create(mcgpu_ctx* ctx, const mcgpu_server_config* cf
     return set_err(ctx, MCGPU_ERR_INVALID, "max_mol_atoms %d outside [1, %d]", c.max_mol_atoms, kMaxA);
   if (c.rotation != MCGPU_ROT_EULER && c.rotation != MCGPU_ROT_AXIS)
     return set_err(ctx, MCGPU_ERR_INVALID, "unknown rotation form %d", c.rotation);
-  if (c.threads == 0) c.threads = 256;
-  if (c.chains_per_cta == 0) c.chains_per_cta = 1;
+  if (c.threads == 0) c.threads = kDefaultThreads;
+  if (c.chains_per_cta == 0) c.chains_per_cta = kDefaultChains;
   if (c.threads < 32 || c.threads > 512 || c.threads % 32 || (c.threads / 32) % c.chains_per_cta)
     return set_err(ctx, MCGPU_ERR_INVALID, "tile %d threads / %d chains per CTA", c.threads,
                    c.chains_per_cta);
@@ -575,8 +578,8 @@ extern "C" int mcgpu_server_create(mcgpu_ctx* ctx, const mcgpu_server_config* cf
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &per_sm, c.threads > 256 ? k_chain_steps_wide : k_chain_steps, c.threads, s->smem);
   s->grid = std::max(1, per_sm) * ctx->sm_count;
-  // one chain per CTA of at most 8 warps leaves room for wider groups
-  if (c.chains_per_cta == 1 && c.threads < kWideWarps * 32 && c.max_mol_atoms > kWideAtoms) {
+  if (c.threads == kDefaultThreads && c.chains_per_cta == kDefaultChains &&
+      c.max_mol_atoms > kWideAtoms) {
     s->wide = shape_for(c.max_mol_atoms, kWideWarps, 2048);
     s->wide_smem = s->wide.bytes();
     per_sm = 0;
