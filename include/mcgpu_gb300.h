@@ -365,10 +365,10 @@ int mcgpu_batch_autotune(mcgpu_batch* batch, int trial_steps);
  * most 4 atoms, else the power of two at or above its largest molecule).
  * Results do not depend on the first three; the lanes change the FP32
  * summation order and so the last bits of the energies.  Few chains with FP64
- * pairs run windows of 4 or 2 steps on CTAs of 256 threads, and the tile then
- * sets steps_per_launch alone, unless a window has been set:
- * mcgpu_batch_set_window(batch, 1) keeps them on the one-step kernel and the
- * tile's threads. */
+ * pairs, the largest of at least 192 atoms, run windows of 4 or 2 steps on CTAs
+ * of 256 threads, and the tile then sets steps_per_launch alone, unless a window
+ * has been set: mcgpu_batch_set_window(batch, 1) keeps them on the one-step
+ * kernel and the tile's threads. */
 int mcgpu_batch_set_tile(mcgpu_batch* batch, int threads, int chains_per_cta,
                          int steps_per_launch, int lanes_per_molecule);
 int mcgpu_batch_get_tile(mcgpu_batch* batch, int* threads, int* chains_per_cta,

@@ -1595,8 +1595,11 @@ static int batch_grid(mcgpu_batch* bt, int* smem_out) {
 // chains' clusters are resident at once: the decisions and coordinates are the
 // one-step kernel's.  Not 8: in boxes of some hundred molecules most steps of a
 // window depend on an earlier one and are evaluated again.  37 chains of 64 to 700
-// waters, 96 steps: 2.80 ms one step at a time, 1.81 in windows of 4.
-constexpr int kIdleWindowThreads = 256;
+// waters, 96 steps: 2.80 ms one step at a time, 1.81 in windows of 4.  For the same
+// reason not where even the largest chain is small: 37 chains, 96 steps, one at a time
+// against windows: 32 waters 2.44 and 2.62 ms, 64 waters 2.42 and 2.43, 128 waters 1.76
+// and 1.52; 32 one-site molecules 1.10 and 1.35 ms.
+constexpr int kIdleWindowThreads = 256, kIdleWindowAtoms = 192;
 
 static int batch_idle_window(mcgpu_batch* bt, int* out) {
   mcgpu_ctx* ctx = bt->ctx;
@@ -1606,6 +1609,9 @@ static int batch_idle_window(mcgpu_batch* bt, int* out) {
                             sizeof(int), nc, cudaMemcpyDeviceToHost, ctx->stream));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
   *out = 1;
+  int largest = 0;
+  for (const ChainHdr& h : bt->pool.hdr) largest = std::max(largest, h.n_atom);
+  if (largest < kIdleWindowAtoms) return MCGPU_OK;
   for (int v : f64)
     if (!v) return MCGPU_OK;
   const SmemShape sh = shape_for(bt->pool.max_len, kIdleWindowThreads / 32, bt->cache_n);

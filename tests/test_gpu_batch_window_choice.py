@@ -17,12 +17,12 @@ def ctx():
     c.close()
 
 
-def boxes(n):
-    return [water_box(130 + 37 * (c % 6), cutoff=6.0, seed=c % 6) for c in range(n)]
+def boxes(n, waters=130):
+    return [water_box(waters + waters // 4 * (c % 6), cutoff=6.0, seed=c % 6) for c in range(n)]
 
 
-def run(ctx, n_chains, window, steps=600):
-    bt = ChainBatch(ctx, boxes(n_chains), list(range(n_chains)), rotation=ROT_AXIS)
+def run(ctx, n_chains, window, steps=600, waters=130):
+    bt = ChainBatch(ctx, boxes(n_chains, waters), list(range(n_chains)), rotation=ROT_AXIS)
     bt.set_precision(PREC_FP64)
     bt.set_tile(64, 1, 16)
     if window:
@@ -39,6 +39,15 @@ def test_window_of_one_is_the_one_step_kernel(ctx):
     (which never run windows) to the last bit."""
     st, xyz = run(ctx, 6, 1)
     ref, rxyz = run(ctx, 100, 0)
+    for a, b, x, y in zip(st, ref, xyz, rxyz):
+        assert a.energy == b.energy and a.accepted == b.accepted
+        assert np.array_equal(x, y)
+
+
+def test_few_small_chains_run_one_step_at_a_time(ctx):
+    """27 to 60 waters: most steps of a window would be evaluated twice."""
+    st, xyz = run(ctx, 6, 0, waters=27)
+    ref, rxyz = run(ctx, 100, 0, waters=27)
     for a, b, x, y in zip(st, ref, xyz, rxyz):
         assert a.energy == b.energy and a.accepted == b.accepted
         assert np.array_equal(x, y)
