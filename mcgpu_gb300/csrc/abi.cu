@@ -441,7 +441,7 @@ int pool_set_verlet(mcgpu_ctx* ctx, DevPool& dp, double skin, cudaStream_t st) {
 
 int pool_nl_rebuild(mcgpu_ctx* ctx, DevPool& dp, cudaStream_t st) {
   if (!dp.nl_on) return MCGPU_OK;
-  CK(ctx, launch_nl_rebuild(dp.P, dp.nl_max_cells, st));
+  CK(ctx, launch_nl_rebuild(dp.P, dp.nl_max_cells, ctx->sm_count, st));
   return MCGPU_OK;
 }
 

@@ -371,7 +371,7 @@ __device__ __forceinline__ void group_reduce_ff(const Group& g, const GroupSmem&
 }
 
 // FP64 re-take of a step near the decision threshold: FP64 pair terms
-// (pair64, BruteForceStep.cpp:48-79) on the FP64 positions of the chain
+// (pair_sum64, BruteForceStep.cpp:48-79) on the FP64 positions of the chain
 // state (anchor + offset).  Warp 0 first writes the moved molecule's old
 // and new FP64 coordinates and its FP64 parameters to shared memory; the
 // caller synchronises.
@@ -407,7 +407,7 @@ __device__ __forceinline__ void batch_chain64(const Pool& P, const ChainHdr& H, 
 // on the chain state's FP64 positions.
 //
 // With a Verlet list (cand non-null), the molecules cand[c_begin .. c_end),
-// every nw-th entry per warp as in warp_eval_chain.
+// every nw-th entry per warp as in group_eval_chain.
 __device__ inline void warp_eval_chain64(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                   const MovedInfo& mi, const float4* pcache, int c_begin,
                                   int c_end, int w, int nw, int lane, double& eo,

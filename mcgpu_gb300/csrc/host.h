@@ -39,7 +39,7 @@ __global__ void k_chain_steps(Pool P, ChainLaunch A);
 __global__ void k_chain_steps_wide(Pool P, ChainLaunch A);
 __global__ void k_chain_init(Pool P, const int* mol_chain, int m_begin, int m_end);
 __global__ void k_nl_config(Pool P, const NlCfg* cfg);
-cudaError_t launch_nl_rebuild(Pool P, int max_cells, cudaStream_t st);
+cudaError_t launch_nl_rebuild(Pool P, int max_cells, int sm_count, cudaStream_t st);
 __global__ void k_chain_export(Pool P, const int* mol_chain, const int* atom_mol, int a_begin,
                                int a_end);
 // out (and done, if any) may lie in pinned host memory: *done becomes `call`

@@ -244,24 +244,6 @@ __device__ __forceinline__ int screen_mixed(const Pool& P, const ChainHdr& H, co
   return f;
 }
 
-// FP64 screen: the reference's test for every primary pair.
-__device__ __forceinline__ int screen_f64(const Pool& P, const ChainHdr& H, const GroupSmem& s,
-                                          const MovedInfo& mi, int j) {
-  const int2 pj = P.mpi[j];
-  int f = 0;
-  for (int k2 = 0; k2 < pj.y; k2++) {
-    const int p2 = P.pidx[pj.x + k2];
-    for (int k1 = 0; k1 < mi.npidx; k1++) {
-      const int pa = s.pa[k1];
-      if ((mi.states & 1) && !(f & kInOld) && in_range64(s.ox[pa], s.oy[pa], s.oz[pa], p2, P, H))
-        f |= kInOld;
-      if ((mi.states & 2) && !(f & kInNew) && in_range64(s.nx[pa], s.ny[pa], s.nz[pa], p2, P, H))
-        f |= kInNew;
-    }
-  }
-  return f;
-}
-
 // ---- pair batches -----------------------------------------------------------
 
 // Per-thread double-float accumulators of one evaluation.

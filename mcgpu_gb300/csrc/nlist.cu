@@ -289,11 +289,11 @@ __global__ void k_nl_config(Pool P, const NlCfg* cfg) {
   H.nl_rlist = f.rlist;
 }
 
-cudaError_t launch_nl_rebuild(Pool P, int max_cells, cudaStream_t st) {
+cudaError_t launch_nl_rebuild(Pool P, int max_cells, int sm_count, cudaStream_t st) {
   const int nc = P.n_chains;
   k_nl_cells<<<nc, kNlCellThreads, 0, st>>>(P);
   // six CTAs an SM in all, no more than a chain has work for
-  int gx = 152 * 6 / nc;
+  int gx = sm_count * 6 / nc;
   gx = gx < 1 ? 1 : gx > max_cells * kNlSlices ? max_cells * kNlSlices : gx;
   // grid.y holds at most 65,535 chains
   for (int c0 = 0; c0 < nc; c0 += 65535) {

@@ -63,10 +63,9 @@ struct RangeAlloc {
 };
 
 // Device bytes per row element of the arena (see DevPool / server_alloc) a job is
-// charged; the volume moves' anchors in cell order (vc_fix, 16 B a molecule) are
-// scratch beside them.
+// charged: a molecule's rows and its places in the volume moves' cell grid (vc_*).
 constexpr long long kBytesAtom = 6 * 8 + 16 + 16 + 8 + 16 + 4;          // 108
-constexpr long long kBytesMol = 4 + 4 + 8 + 16 + 4 + 16 + 4 + 8 + 8 + 16;  // 88
+constexpr long long kBytesMol = 4 + 4 + 8 + 16 + 4 + 16 + 4 + 4 * 4 + 16;  // 88
 constexpr long long kBytesPidx = 4 + 16;                                  // 20
 
 // The default tile, and the warps of a group for jobs of molecules of more than

@@ -1,7 +1,7 @@
 // static_energy.cu -- mcgpu_system_energy_static: the FP64 system energy
-// (SimulationStep::calcSystemEnergy's sum, the reference's pair arithmetic)
-// over SimBox rows that the CALLER already holds in device memory, without
-// allocating anything.
+// (SimulationStep::calcSystemEnergy's pairs and in-range test; the pair terms
+// from per-atom roots and 1/r of an FP64 rsqrt, see pair_sum64) over SimBox rows
+// that the CALLER already holds in device memory, without allocating anything.
 //
 // Who needs it: programs that cannot call cudaMalloc for this library --
 // an OpenACC or OpenMP-offload build that keeps its SimBox rows in its own
@@ -9,7 +9,8 @@
 // application whose device memory is owned by another allocator (a
 // framework's caching allocator, a fixed arena of a long-running service)
 // and forbids allocations from third-party code.  They pass device pointers
-// to their rows and to one output double; the partial energies live in a fixed file-scope device array instead of a cudaMalloc'd buffer.
+// to their rows and to one output double; the partial energies live in a fixed
+// file-scope device array instead of a cudaMalloc'd buffer.
 //
 // Limits and sharing: at most kStaticMaxMol molecules per call (larger boxes
 // are rejected with MCGPU_ERR_UNSUPPORTED).  Every GPU that loads the
