@@ -342,9 +342,6 @@ int upload_pool(mcgpu_ctx* ctx, HostPool& hp, DevPool& dp) {
   return MCGPU_OK;
 }
 
-// Warps of a CTA of the FP32 system-energy kernel.
-static constexpr int kEnergyWarps = 4;
-
 SmemShape shape_for(int max_len, int nwarps, int cache_n) {
   SmemShape s;
   s.maxA = std::max(max_len, 1);
@@ -447,7 +444,7 @@ int pool_nl_rebuild(mcgpu_ctx* ctx, DevPool& dp, cudaStream_t st) {
 
 // Full system energy of every chain of the pool into dp.esum (device).
 int pool_system_energy(mcgpu_ctx* ctx, DevPool& dp, bool f64, cudaStream_t st) {
-  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, dp.min_chain, shape_for(dp.max_len, kEnergyWarps),
+  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, dp.min_chain, shape_for(dp.max_len, kPlainWarps),
                                st, dp.P, dp.mol_chain, dp.emol));
   k_chain_sums<<<dp.n_chains, 256, 0, st>>>(dp.P, dp.emol, dp.esum);
   CK(ctx, cudaGetLastError());
@@ -705,13 +702,12 @@ extern "C" int mcgpu_mol_energy(mcgpu_box* b, int curr, int start, double* out) 
   }
   int rc = box_rows(b);
   if (rc) return rc;
-  const int nw = 4;
-  SmemShape sh = shape_for(b->pool.max_len, nw);
+  SmemShape sh = shape_for(b->pool.max_len, kPlainWarps);
   const int grid = box_grid(b, n - start);
   const bool f64 = b->precision == MCGPU_PREC_FP64;
   if (b->intra_on) {
     // SimulationStep::calcMoleculeEnergy with ENABLE_INTRA (SimulationStep.cpp:15-18)
-    CK(ctx, launch_mol_energy(f64, grid, nw * 32, sh, ctx->stream, b->pool.P, 0, curr, start,
+    CK(ctx, launch_mol_energy(f64, grid, sh, ctx->stream, b->pool.P, 0, curr, start,
                               b->partials, b->counter, b->dout, b->dpairs));
     CK(ctx, launch_intra_energy(b->pool.P, b->intra->R, 0, curr, b->dout + 1, ctx->stream));
     CK(ctx, cudaMemcpyAsync(b->hout, b->dout, 2 * sizeof(double), cudaMemcpyDeviceToHost,
@@ -720,7 +716,7 @@ extern "C" int mcgpu_mol_energy(mcgpu_box* b, int curr, int start, double* out) 
     *out = b->hout[0] + b->hout[1];
     return MCGPU_OK;
   }
-  CK(ctx, launch_mol_energy(f64, grid, nw * 32, sh, ctx->stream, b->pool.P, 0, curr, start,
+  CK(ctx, launch_mol_energy(f64, grid, sh, ctx->stream, b->pool.P, 0, curr, start,
                             b->partials, b->counter, b->hout, b->dpairs, box_done(b), ++b->call));
   rc = box_wait(b);
   if (rc) return rc;
@@ -790,10 +786,9 @@ extern "C" int mcgpu_move_energies(mcgpu_box* b, int mol, const mcgpu_move* mv, 
   if (rc) return rc;
   box_plain_moved(b);
   mcgpu_ctx* ctx = b->ctx;
-  const int nw = 4;
-  SmemShape sh = shape_for(b->pool.max_len, nw);
+  SmemShape sh = shape_for(b->pool.max_len, kPlainWarps);
   const int grid = box_grid(b, b->pool.n_mol);
-  CK(ctx, launch_move_energies(b->precision == MCGPU_PREC_FP64, grid, nw * 32, sh, ctx->stream,
+  CK(ctx, launch_move_energies(b->precision == MCGPU_PREC_FP64, grid, sh, ctx->stream,
                                b->pool.P, 0, mol, host_proposal(mv), b->partials, b->counter,
                                b->hout, b->dpairs, box_done(b), ++b->call));
   rc = box_wait(b);
@@ -813,7 +808,7 @@ extern "C" int mcgpu_system_energy(mcgpu_box* b, double* out) {
     // intramolecular energy (SimulationStep.cpp:40-71 over :15-18)
     DevPool& dp = b->pool;
     CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64, dp.n_mol, dp.min_chain,
-                                 shape_for(dp.max_len, kEnergyWarps), ctx->stream, dp.P,
+                                 shape_for(dp.max_len, kPlainWarps), ctx->stream, dp.P,
                                  dp.mol_chain, dp.emol));
     CK(ctx, launch_intra_add(dp.P, b->intra->R, dp.n_mol, dp.emol, ctx->stream));
     k_chain_sums<<<dp.n_chains, 256, 0, ctx->stream>>>(dp.P, dp.emol, dp.esum);
@@ -848,8 +843,8 @@ static int run_plain_rigid(mcgpu_box* b, int n_steps, int fused, mcgpu_plain_sta
   const int n = b->pool.n_mol;
   const double kT = h.kT, max_t = h.max_t, max_r = h.max_r;
   const bool f64 = b->precision == MCGPU_PREC_FP64;
-  const int nw = 4, grid = box_grid(b, n);
-  const SmemShape sh = shape_for(b->pool.max_len, nw);
+  const int grid = box_grid(b, n);
+  const SmemShape sh = shape_for(b->pool.max_len, kPlainWarps);
   if (int rc = box_rows(b)) return rc;
   for (int step = 0; step < n_steps; step++) {
     // chooseMolecule (SimulationStep.cpp:25-27); rand() == RAND_MAX gives n,
@@ -873,11 +868,11 @@ static int run_plain_rigid(mcgpu_box* b, int n_steps, int fused, mcgpu_plain_sta
     } else {
       // the contract calls, launched one behind another with one wait: the
       // old energy is not needed before the move
-      CK(b->ctx, launch_mol_energy(f64, grid, nw * 32, sh, b->ctx->stream, b->pool.P, 0, mol, 0,
+      CK(b->ctx, launch_mol_energy(f64, grid, sh, b->ctx->stream, b->pool.P, 0, mol, 0,
                                    b->partials, b->counter, b->hout, b->dpairs));
       rc = mcgpu_change_molecule(b, mol, &mv);
       if (rc) return rc;
-      CK(b->ctx, launch_mol_energy(f64, grid, nw * 32, sh, b->ctx->stream, b->pool.P, 0, mol, 0,
+      CK(b->ctx, launch_mol_energy(f64, grid, sh, b->ctx->stream, b->pool.P, 0, mol, 0,
                                    b->partials, b->counter, b->hout + 1, b->dpairs, box_done(b),
                                    ++b->call));
       rc = box_wait(b);
@@ -1010,7 +1005,7 @@ extern "C" int mcgpu_boxes_run_plain_device(mcgpu_box* const* boxes, int n_boxes
                         ctx->stream);
   if (e == cudaSuccess)
     e = launch_box_energies(f64, dt, n_boxes, max_mol, max_groups, intra,
-                            shape_for(max_len, kEnergyWarps), ctx->stream);
+                            shape_for(max_len, kPlainWarps), ctx->stream);
   SmemShape sh = shape_for(max_len, 8);
   // boxes of both kinds: two kernels, side by side on two streams
   cudaStream_t side = nullptr;
@@ -1324,8 +1319,7 @@ static int run_plain_intra(mcgpu_box* b, int n_steps, mcgpu_plain_stats* out, do
   const int n = b->pool.n_mol;
   const double kT = h.kT, max_t = h.max_t, max_r = h.max_r;
   const bool f64 = b->precision == MCGPU_PREC_FP64;
-  const int nw = 4;
-  SmemShape sh = shape_for(b->pool.max_len, nw);
+  SmemShape sh = shape_for(b->pool.max_len, kPlainWarps);
   SmemShape sh1 = shape_for(b->pool.max_len, 1);
   const int grid = box_grid(b, n);
   const long long step0 = I.step;
@@ -1347,7 +1341,7 @@ static int run_plain_intra(mcgpu_box* b, int n_steps, mcgpu_plain_stats* out, do
     mv.rz = random_real(-max_r, max_r);
     const double bond_delta = I.max_bond_delta, angle_delta = I.max_angle_delta;
     // old energy (inter + intra), the rigid move, the bond stage
-    CK(ctx, launch_mol_energy(f64, grid, nw * 32, sh, ctx->stream, b->pool.P, 0, mol, 0,
+    CK(ctx, launch_mol_energy(f64, grid, sh, ctx->stream, b->pool.P, 0, mol, 0,
                               b->partials, b->counter, b->dout, b->dpairs));
     CK(ctx, launch_intra_energy(b->pool.P, I.R, 0, mol, b->dout + 1, ctx->stream));
     k_change_molecule<<<1, 32, sh1.bytes(), ctx->stream>>>(b->pool.P, 0, mol,
@@ -1382,7 +1376,7 @@ static int run_plain_intra(mcgpu_box* b, int n_steps, mcgpu_plain_stats* out, do
                                 I.flex_bonds ? 0 : (kIntraSave | kIntraEnergyBefore), true);
       if (rc) return rc;
     }
-    CK(ctx, launch_mol_energy(f64, grid, nw * 32, sh, ctx->stream, b->pool.P, 0, mol, 0,
+    CK(ctx, launch_mol_energy(f64, grid, sh, ctx->stream, b->pool.P, 0, mol, 0,
                               b->partials, b->counter, b->dout, b->dpairs));
     CK(ctx, launch_intra_energy(b->pool.P, I.R, 0, mol, b->dout + 1, ctx->stream));
     CK(ctx, cudaMemcpyAsync(hv, b->dout, 2 * sizeof(double), cudaMemcpyDeviceToHost,

@@ -42,13 +42,20 @@ __global__ void k_nl_config(Pool P, const NlCfg* cfg);
 cudaError_t launch_nl_rebuild(Pool P, int max_cells, int sm_count, cudaStream_t st);
 __global__ void k_chain_export(Pool P, const int* mol_chain, const int* atom_mol, int a_begin,
                                int a_end);
+// Threads of the plain energy kernels' CTAs.  The FP32 kernels' launch bound also
+// tells the compiler that one CTA an SM is enough: the move kernel then takes 148
+// registers instead of 80 and its loop over a molecule's atoms no longer waits on
+// itself (20 moves of 64-atom molecules, 500 in the box: 3.08 and 1.51 ms).  The FP64
+// kernels keep to 128 registers: they wait on the pipe, and at 148 a move among 32,768
+// waters took 36 us instead of 30.
+constexpr int kPlainWarps = 4, kPlainThreads = 32 * kPlainWarps;
 // out (and done, if any) may lie in pinned host memory: *done becomes `call`
 // once the results are there.
-cudaError_t launch_mol_energy(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
+cudaError_t launch_mol_energy(bool f64, int grid, SmemShape sh, cudaStream_t st,
                               Pool P, int chain, int curr, int start, double* partials,
                               unsigned* counter, double* out, long long* pairs = nullptr,
                               unsigned* done = nullptr, unsigned call = 0);
-cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
+cudaError_t launch_move_energies(bool f64, int grid, SmemShape sh, cudaStream_t st,
                                  Pool P, int chain, int mol, Proposal prop, double* partials,
                                  unsigned* counter, double* out, long long* pairs = nullptr,
                                  unsigned* done = nullptr, unsigned call = 0);

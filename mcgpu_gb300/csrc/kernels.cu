@@ -70,11 +70,9 @@ __device__ __forceinline__ double sum_partials(const double* p, int stride, int 
 // (BruteForceCalcs::calcMolecularEnergyContribution, BruteForceStep.cpp:
 // 15-46).  The candidates are dealt over the warps of the grid.
 template <bool F64>
-__global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr, int start,
-                                                    SmemShape shape, double* partials,
-                                                    unsigned* counter, double* out,
-                                                    long long* pairs, unsigned* done,
-                                                    unsigned call) {
+__global__ void __launch_bounds__(F64 ? 256 : kPlainThreads, F64 ? 0 : 1)
+    k_mol_energy(Pool P, int chain, int curr, int start, SmemShape shape, double* partials,
+                 unsigned* counter, double* out, long long* pairs, unsigned* done, unsigned call) {
   extern __shared__ __align__(16) char smem[];
   const ChainHdr& H = P.hdr[chain];
   Group g{(int)threadIdx.x, (int)blockDim.x, 1};
@@ -110,11 +108,10 @@ __global__ void __launch_bounds__(256) k_mol_energy(Pool P, int chain, int curr,
 // (Simulation.cpp:244-250).  Every CTA stages the same proposed placement;
 // the CTA that finishes last saves the rollback copy and commits.
 template <bool F64>
-__global__ void __launch_bounds__(256) k_move_energies(Pool P, int chain, int mol, Proposal prop,
-                                                       SmemShape shape, double* partials,
-                                                       unsigned* counter, double* out,
-                                                       long long* pairs, unsigned* done,
-                                                       unsigned call) {
+__global__ void __launch_bounds__(F64 ? 256 : kPlainThreads, F64 ? 0 : 1)
+    k_move_energies(Pool P, int chain, int mol, Proposal prop, SmemShape shape, double* partials,
+                    unsigned* counter, double* out, long long* pairs, unsigned* done,
+                    unsigned call) {
   extern __shared__ __align__(16) char smem[];
   const ChainHdr& H = P.hdr[chain];
   Group g{(int)threadIdx.x, (int)blockDim.x, 1};
@@ -342,9 +339,9 @@ __global__ void __launch_bounds__(kPsThreads, 4)
 }
 
 // The same with FP32 pairs, one molecule m = m_begin + blockIdx.x per CTA.
-__global__ void __launch_bounds__(256) k_pair_sums32(Pool P0, const LoopTask* tasks,
-                                                     const int* mol_chain, int m_begin,
-                                                     SmemShape shape, double* emol) {
+__global__ void __launch_bounds__(kPlainThreads, 1)
+    k_pair_sums32(Pool P0, const LoopTask* tasks, const int* mol_chain, int m_begin,
+                  SmemShape shape, double* emol) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Pool SP;
   load_pool(SP, P0, tasks);
@@ -765,28 +762,28 @@ __global__ void __launch_bounds__(512, 1) k_chain_steps_wide(Pool P, ChainLaunch
 
 // ---- host launchers (template kernels are instantiated here) --------------
 
-cudaError_t launch_mol_energy(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
+cudaError_t launch_mol_energy(bool f64, int grid, SmemShape sh, cudaStream_t st,
                               Pool P, int chain, int curr, int start, double* partials,
                               unsigned* counter, double* out, long long* pairs, unsigned* done,
                               unsigned call) {
   if (f64)
-    k_mol_energy<true><<<grid, threads, sh.bytes(), st>>>(P, chain, curr, start, sh, partials,
+    k_mol_energy<true><<<grid, kPlainThreads, sh.bytes(), st>>>(P, chain, curr, start, sh, partials,
                                                           counter, out, pairs, done, call);
   else
-    k_mol_energy<false><<<grid, threads, sh.bytes(), st>>>(P, chain, curr, start, sh, partials,
+    k_mol_energy<false><<<grid, kPlainThreads, sh.bytes(), st>>>(P, chain, curr, start, sh, partials,
                                                            counter, out, pairs, done, call);
   return cudaGetLastError();
 }
 
-cudaError_t launch_move_energies(bool f64, int grid, int threads, SmemShape sh, cudaStream_t st,
+cudaError_t launch_move_energies(bool f64, int grid, SmemShape sh, cudaStream_t st,
                                  Pool P, int chain, int mol, Proposal prop, double* partials,
                                  unsigned* counter, double* out, long long* pairs, unsigned* done,
                                  unsigned call) {
   if (f64)
-    k_move_energies<true><<<grid, threads, sh.bytes(), st>>>(P, chain, mol, prop, sh, partials,
+    k_move_energies<true><<<grid, kPlainThreads, sh.bytes(), st>>>(P, chain, mol, prop, sh, partials,
                                                              counter, out, pairs, done, call);
   else
-    k_move_energies<false><<<grid, threads, sh.bytes(), st>>>(P, chain, mol, prop, sh, partials,
+    k_move_energies<false><<<grid, kPlainThreads, sh.bytes(), st>>>(P, chain, mol, prop, sh, partials,
                                                               counter, out, pairs, done, call);
   return cudaGetLastError();
 }
@@ -801,7 +798,7 @@ cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, SmemShape s
     k_pair_sums64<<<(n_mol + span - 1) / span, kPsThreads, 0, st>>>(P, nullptr, mol_chain, n_mol,
                                                                     span, emol);
   } else {
-    k_pair_sums32<<<n_mol, sh.nwarps * 32, sh.bytes(), st>>>(P, nullptr, mol_chain, 0, sh, emol);
+    k_pair_sums32<<<n_mol, kPlainThreads, sh.bytes(), st>>>(P, nullptr, mol_chain, 0, sh, emol);
   }
   return cudaGetLastError();
 }
@@ -816,7 +813,7 @@ cudaError_t launch_box_energies(bool f64, const LoopTask* tasks, int n_tasks, in
       k_pair_sums64<<<dim3(max_groups, nt), kPsThreads, 0, st>>>(Pool{}, T, nullptr, 0, 0,
                                                                  nullptr);
     } else {
-      k_pair_sums32<<<dim3(max_mol, nt), sh.nwarps * 32, sh.bytes(), st>>>(Pool{}, T, nullptr, 0,
+      k_pair_sums32<<<dim3(max_mol, nt), kPlainThreads, sh.bytes(), st>>>(Pool{}, T, nullptr, 0,
                                                                            sh, nullptr);
     }
     cudaError_t e = cudaGetLastError();

@@ -811,7 +811,11 @@ __device__ __forceinline__ float pair_item32(const Pool& P, const ChainHdr& H,
 // FP32 pair batch of `count` (1..32) ring entries from `head` on the plain path
 // (offsets with their low parts), the items (placement, entry, neighbour atom)
 // dealt to the lanes as batch_items64 deals them; each item's sum over the
-// moved molecule's atoms is added in double-float.
+// moved molecule's atoms is added in double-float.  Molecules of many atoms go
+// entry by entry: the lanes of a round then agree on the per-pair image of an entry
+// (atom by atom they took both forms of the sum where some entries straddle half an
+// edge: the system energy of 16 molecules of 64 atoms 143 us, 83 entry by entry).
+constexpr int kItemsByEntry = 16;
 template <bool PRECISE>
 __device__ __forceinline__ void batch_items32(const Pool& P, const ChainHdr& H,
                                               const GroupSmem& s, const MovedInfo& mi,
@@ -848,7 +852,10 @@ __device__ __forceinline__ void batch_items32(const Pool& P, const ChainHdr& H,
     const bool p = it >= total || mi.states == 2;
     const int local = it >= total ? it - total : it;
     int e, k;
-    if (uni) {
+    if (uni && H.ulen >= kItemsByEntry) {
+      e = local / H.ulen;
+      k = local - e * H.ulen;
+    } else if (uni) {
       k = local / count;
       e = local - k * count;
     } else {
