@@ -181,7 +181,7 @@ struct Pool {
   double *x, *y, *z, *sig, *eps, *q;
   float4* aoff;
   float4* aofl;        // plain path: low part of the offsets (FP64 offset - aoff)
-  double2* blend;      // FP64 blending factors (sqrt sigma, sqrt eps; -1 for a skipped
+  double2* blend;      // FP64 blending factors (sigma, sqrt eps; -1 for a skipped
                        // site), or null (pools of the served form)
   float2* aeq;
   int *mstart, *mlen;
@@ -522,12 +522,12 @@ __device__ __forceinline__ float lj32(float ir2, float sa, float sb, float ea, f
   return (ea * eb) * fmaf(t3, t3, -t3);
 }
 
-// The blending factor rows of an atom for the FP64 pair terms: sqrt(sigma) and
+// The blending factor rows of an atom for the FP64 pair terms: sigma and
 // sqrt(eps); sigma = -1 marks a site the reference skips (a negative sigma
 // or epsilon, BruteForceStep.cpp:64-65).
 __device__ __forceinline__ double2 blend64(double sig, double eps) {
   if (!(sig >= 0 && eps >= 0)) return make_double2(-1.0, 0.0);
-  return make_double2(sqrt(sig), sqrt(eps));
+  return make_double2(sig, sqrt(eps));
 }
 
 }  // namespace mcgpu

@@ -518,7 +518,7 @@ __device__ void cta_eval(const Pool& P, const ChainHdr& H, const Group& grp, con
       if (F64) {
         const int i0 = part * mi.len / parts, n_i = (part + 1) * mi.len / parts - i0;
         const double2 bl = P.blend[b];
-        const double e = pair_sum64<true>(
+        const double e = pair_sum64(
             (use_new ? s.nx : s.ox) + i0, (use_new ? s.ny : s.oy) + i0,
             (use_new ? s.nz : s.oz) + i0, s.sd + i0, s.ed + i0, s.qd + i0, n_i, P.x[b], P.y[b],
             P.z[b], bl.x, bl.y, P.q[b], H.L[0], H.L[1], H.L[2]);

@@ -600,7 +600,7 @@ __device__ __forceinline__ void uniform_items(const Pool& P, const ChainHdr& H, 
 //     tests read the operands' high words on the integer pipe;
 //   * the LJ term is formed only where its sigma and epsilon products are not
 //     zero (water: 1 pair of 9), and r^2 by fused multiply-adds.
-// 17 FP64 instructions a Coulomb pair and 25 with LJ, 43 before.
+// 16 FP64 instructions a Coulomb pair and 25 with LJ.
 
 // sigma factor of a skipped site (blend64).
 __device__ __forceinline__ bool blend_skipped(double sa) {
@@ -626,15 +626,21 @@ __device__ __forceinline__ double image64(double d, double L, int half) {
 // its image nearest the molecule's first atom; a pair that still lies beyond
 // half an edge (molecules straddling it, or rows outside the box) takes the
 // reference's own image from the unshifted rows.
-// (sb, eb): b's factors, qb its charge; sd, ed, qd the molecule's: sqrt(eps)
-// and, with ROOT, sqrt(sigma), else sigma itself (sigma_ab^2 = s_a s_b).
+// (sb, eb): b's factors (blend64), qb its charge; sd, ed, qd the molecule's.
+//
+// sigma_ab^2 / r^2 = (s_a s_b) / r^2 with 1/r^2 = (1/r)^2 corrected once by its own
+// residual: the twelfth power multiplies a relative error of the distance by twelve,
+// and the square of the 1-ulp rsqrt alone, with sigma_ab^2 from the atoms' square
+// roots, left the LJ terms half again as far from their true values as the
+// reference's square root and division do (mean 1.4e-15 against 8.1e-16 over 1,000
+// close pairs; 5.3e-16 this way).
 //
 // With VOTE the rare image and the LJ term stand behind votes of the lanes that
 // enter together, so those lanes must hold rows of the same length with the same
 // sites skipped: a lane that leaves the loop, or passes over a site, is waited for
 // by the others.  Lanes on unlike molecules take VOTE false, the same terms in the
 // same order behind branches of their own.
-template <bool ROOT, bool VOTE = true>
+template <bool VOTE = true>
 __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys, const double* zs,
                                              const double* sd, const double* ed, const double* qd,
                                              int len, double xb, double yb, double zb, double sb,
@@ -648,9 +654,8 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
   const double by = hi_abs(ty) >= hy ? yb - copysign(Ly, ty) : yb;
   const double bz = hi_abs(tz) >= hz ? zb - copysign(Lz, tz) : zb;
   const bool lj_b = bits_nonzero(sb) && bits_nonzero(eb);
-  const double qk = qb * kCoulomb, e4 = 4.0 * eb;
   const unsigned am = VOTE ? __activemask() : 0u;
-  double acc = 0.0;
+  double cl = 0.0, lj = 0.0;   // sums without b's charge and epsilon, which come last
 #pragma unroll 3
   for (int i = 0; i < len; i++) {
     const double sa = sd[i], ea = ed[i];
@@ -669,25 +674,18 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
     const bool apart = bits_nonzero(r2);  // coincident: skipped (BruteForceStep.cpp:68-69)
     const double ri = rsqrt(r2);
-    const double q = qd[i] * qk;
-    acc = fma(apart ? q : 0.0, apart ? ri : 0.0, acc);
-    const bool lj = apart && lj_b && bits_nonzero(sa) && bits_nonzero(ea);
-    if (VOTE ? __any_sync(am, lj) != 0 : lj) {
+    cl = fma(apart ? qd[i] : 0.0, apart ? ri : 0.0, cl);
+    const bool near = apart && lj_b && bits_nonzero(sa) && bits_nonzero(ea);
+    if (VOTE ? __any_sync(am, near) != 0 : near) {
       if (VOTE) __syncwarp(am);
-      double t2;
-      if (ROOT) {
-        const double t = (sa * sb) * ri;
-        t2 = t * t;
-      } else {
-        t2 = (sa * sb) * (ri * ri);
-      }
+      const double i2 = ri * ri, u = (sa * sb) * i2;
+      const double t2 = fma(u, fma(-r2, i2, 1.0), u);
       const double s6 = t2 * t2 * t2;
-      const double e = ea * e4;
-      if (lj) acc = fma(s6, fma(e, s6, -e), acc);
+      if (near) lj = fma(ea, fma(s6, s6, -s6), lj);
       if (VOTE) __syncwarp(am);
     }
   }
-  return acc;
+  return fma(cl, qb * kCoulomb, lj * (4.0 * eb));
 }
 
 // FP64 pair batch of `count` (1..32) ring entries from `head`: the items
@@ -757,7 +755,7 @@ __device__ __forceinline__ void batch_items64(const Pool& P, const ChainHdr& H,
     double xb, yb, zb;
     atom(j, b, xb, yb, zb);
     const double2 bl = P.blend ? P.blend[b] : blend64(P.sig[b], P.eps[b]);
-    const double v = pair_sum64<true>(use_new ? s.nx : s.ox, use_new ? s.ny : s.oy,
+    const double v = pair_sum64(use_new ? s.nx : s.ox, use_new ? s.ny : s.oy,
                                       use_new ? s.nz : s.oz, s.sd, s.ed, s.qd, mi.len, xb, yb,
                                       zb, bl.x, bl.y, P.q[b], H.L[0], H.L[1], H.L[2]);
     if (use_new) en += v; else eo += v;

@@ -20,8 +20,7 @@ constexpr int kPsPitch = kMaxA + 1;  // odd pitch: lanes on different molecules 
                                      // the group read different banks
 static_assert(kPsGroup == 8, "ring entries hold the molecule in three bits");
 
-// The group's staged atoms: positions, (sigma or its root; -1 for a skipped
-// site), sqrt(eps), charge.
+// The group's staged atoms: positions, blending factors (blend64), charge.
 struct PsGroup {
   double x[kPsGroup * kPsPitch], y[kPsGroup * kPsPitch], z[kPsGroup * kPsPitch];
   double sd[kPsGroup * kPsPitch], ed[kPsGroup * kPsPitch], qd[kPsGroup * kPsPitch];
@@ -47,7 +46,7 @@ __device__ __forceinline__ bool ps_alike(const PsGroup& G, int n) {
 // Evaluates `count` (1..32) ring entries (j << 3 | group molecule) from
 // `head`: this lane's share of the sum.  rows: len(j), start(j) of molecule
 // j and its atoms' position and factors.  alike: ps_alike's answer.
-template <bool ROOT, class Rows>
+template <class Rows>
 __device__ __forceinline__ double ps_items(const PsGroup& G, const Rows& rows, const int* rj,
                                            int head, int count, int lane, bool alike, double Lx,
                                            double Ly, double Lz) {
@@ -91,11 +90,11 @@ __device__ __forceinline__ double ps_items(const PsGroup& G, const Rows& rows, c
     double xb, yb, zb, sb, eb, qb;
     rows.atom(rows.start(jm >> 3) + k, xb, yb, zb, sb, eb, qb);
     if (alike)
-      acc += pair_sum64<ROOT>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o, G.len[0],
-                              xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
+      acc += pair_sum64(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o, G.len[0],
+                        xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
     else
-      acc += pair_sum64<ROOT, false>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o,
-                                     G.len[jm & 7], xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
+      acc += pair_sum64<false>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o,
+                               G.len[jm & 7], xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
   }
   return acc;
 }

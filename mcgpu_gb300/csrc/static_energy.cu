@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
         tail += __popc(bal);
         if (tail - head >= 32) {
           __syncwarp();
-          acc += ps_items<false>(G, StaticRows{r}, rj, head, 32, lane, alike, r.L[0], r.L[1],
+          acc += ps_items(G, StaticRows{r}, rj, head, 32, lane, alike, r.L[0], r.L[1],
                                  r.L[2]);
           head += 32;
           __syncwarp();
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
     }
     __syncwarp();
     if (tail > head)
-      acc += ps_items<false>(G, StaticRows{r}, rj, head, tail - head, lane, alike, r.L[0], r.L[1],
+      acc += ps_items(G, StaticRows{r}, rj, head, tail - head, lane, alike, r.L[0], r.L[1],
                              r.L[2]);
     __syncthreads();   // the next atoms overwrite the stage
   }
