@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
         tail += __popc(bal);
         if (tail - head >= 32) {
           __syncwarp();
-          acc += ps_items(G, PoolRows{P}, rj, head, 32, lane, alike, H.L[0], H.L[1], H.L[2]);
+          acc += ps_items<false>(G, PoolRows{P}, rj, head, 32, lane, alike, H.L[0], H.L[1], H.L[2]);
           head += 32;
           __syncwarp();
         }
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
     }
     __syncwarp();
     if (tail > head)
-      acc += ps_items(G, PoolRows{P}, rj, head, tail - head, lane, alike, H.L[0], H.L[1],
+      acc += ps_items<false>(G, PoolRows{P}, rj, head, tail - head, lane, alike, H.L[0], H.L[1],
                             H.L[2]);
     const double sum = ps_block_sum(G, acc);
     if ((int)threadIdx.x < n) emol[m0 + threadIdx.x] = threadIdx.x == 0 ? sum : 0.0;

@@ -600,7 +600,7 @@ __device__ __forceinline__ void uniform_items(const Pool& P, const ChainHdr& H, 
 //     tests read the operands' high words on the integer pipe;
 //   * the LJ term is formed only where its sigma and epsilon products are not
 //     zero (water: 1 pair of 9), and r^2 by fused multiply-adds.
-// 16 FP64 instructions a Coulomb pair and 25 with LJ.
+// 16 FP64 instructions a Coulomb pair and 23 with LJ.
 
 // sigma factor of a skipped site (blend64).
 __device__ __forceinline__ bool blend_skipped(double sa) {
@@ -628,19 +628,19 @@ __device__ __forceinline__ double image64(double d, double L, int half) {
 // reference's own image from the unshifted rows.
 // (sb, eb): b's factors (blend64), qb its charge; sd, ed, qd the molecule's.
 //
-// sigma_ab^2 / r^2 = (s_a s_b) / r^2 with 1/r^2 = (1/r)^2 corrected once by its own
-// residual: the twelfth power multiplies a relative error of the distance by twelve,
-// and the square of the 1-ulp rsqrt alone, with sigma_ab^2 from the atoms' square
-// roots, left the LJ terms half again as far from their true values as the
-// reference's square root and division do (mean 1.4e-15 against 8.1e-16 over 1,000
-// close pairs; 5.3e-16 this way).
+// The twelfth power multiplies a relative error of sigma_ab / r by twelve, so
+// sigma_ab^2 is the product of the sigmas themselves (from the atoms' square roots the
+// terms were 1.0e-15 off on average over 1,000 close pairs; 7.1e-16 this way, and
+// 8.1e-16 by the reference's square root and division).  FINE corrects 1/r^2 = (1/r)^2
+// once by its own residual (5.3e-16): two more instructions on the longest chain, which
+// cost the chains' steps up to 17 % and the static sums, bound by the pipe, 5 %.
 //
 // With VOTE the rare image and the LJ term stand behind votes of the lanes that
 // enter together, so those lanes must hold rows of the same length with the same
 // sites skipped: a lane that leaves the loop, or passes over a site, is waited for
 // by the others.  Lanes on unlike molecules take VOTE false, the same terms in the
 // same order behind branches of their own.
-template <bool VOTE = true>
+template <bool VOTE = true, bool FINE = false>
 __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys, const double* zs,
                                              const double* sd, const double* ed, const double* qd,
                                              int len, double xb, double yb, double zb, double sb,
@@ -678,8 +678,9 @@ __device__ __forceinline__ double pair_sum64(const double* xs, const double* ys,
     const bool near = apart && lj_b && bits_nonzero(sa) && bits_nonzero(ea);
     if (VOTE ? __any_sync(am, near) != 0 : near) {
       if (VOTE) __syncwarp(am);
-      const double i2 = ri * ri, u = (sa * sb) * i2;
-      const double t2 = fma(u, fma(-r2, i2, 1.0), u);
+      const double i2 = ri * ri;
+      double t2 = (sa * sb) * i2;
+      if (FINE) t2 = fma(t2, fma(-r2, i2, 1.0), t2);
       const double s6 = t2 * t2 * t2;
       if (near) lj = fma(ea, fma(s6, s6, -s6), lj);
       if (VOTE) __syncwarp(am);

@@ -45,8 +45,8 @@ __device__ __forceinline__ bool ps_alike(const PsGroup& G, int n) {
 
 // Evaluates `count` (1..32) ring entries (j << 3 | group molecule) from
 // `head`: this lane's share of the sum.  rows: len(j), start(j) of molecule
-// j and its atoms' position and factors.  alike: ps_alike's answer.
-template <class Rows>
+// j and its atoms' position and factors.  alike: ps_alike's answer; FINE: pair_sum64's.
+template <bool FINE, class Rows>
 __device__ __forceinline__ double ps_items(const PsGroup& G, const Rows& rows, const int* rj,
                                            int head, int count, int lane, bool alike, double Lx,
                                            double Ly, double Lz) {
@@ -90,11 +90,11 @@ __device__ __forceinline__ double ps_items(const PsGroup& G, const Rows& rows, c
     double xb, yb, zb, sb, eb, qb;
     rows.atom(rows.start(jm >> 3) + k, xb, yb, zb, sb, eb, qb);
     if (alike)
-      acc += pair_sum64(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o, G.len[0],
-                        xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
+      acc += pair_sum64<true, FINE>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o, G.len[0],
+                                    xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
     else
-      acc += pair_sum64<false>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o,
-                               G.len[jm & 7], xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
+      acc += pair_sum64<false, FINE>(G.x + o, G.y + o, G.z + o, G.sd + o, G.ed + o, G.qd + o,
+                                     G.len[jm & 7], xb, yb, zb, sb, eb, qb, Lx, Ly, Lz);
   }
   return acc;
 }

@@ -1,6 +1,6 @@
 // static_energy.cu -- mcgpu_system_energy_static: the FP64 system energy
-// (SimulationStep::calcSystemEnergy's pairs and in-range test; the pair terms
-// from per-atom roots and 1/r of an FP64 rsqrt, see pair_sum64) over SimBox rows
+// (SimulationStep::calcSystemEnergy's pairs and in-range test; the pair terms, as
+// exact as the reference's, from 1/r of an FP64 rsqrt: pair_sum64) over SimBox rows
 // that the CALLER already holds in device memory, without allocating anything.
 //
 // Who needs it: programs that cannot call cudaMalloc for this library --
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
         tail += __popc(bal);
         if (tail - head >= 32) {
           __syncwarp();
-          acc += ps_items(G, StaticRows{r}, rj, head, 32, lane, alike, r.L[0], r.L[1],
+          acc += ps_items<true>(G, StaticRows{r}, rj, head, 32, lane, alike, r.L[0], r.L[1],
                                  r.L[2]);
           head += 32;
           __syncwarp();
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(mcgpu::kPsThreads, 4)
     }
     __syncwarp();
     if (tail > head)
-      acc += ps_items(G, StaticRows{r}, rj, head, tail - head, lane, alike, r.L[0], r.L[1],
+      acc += ps_items<true>(G, StaticRows{r}, rj, head, tail - head, lane, alike, r.L[0], r.L[1],
                              r.L[2]);
     __syncthreads();   // the next atoms overwrite the stage
   }

@@ -7,6 +7,7 @@ import pytest
 
 from mcgpu_gb300 import PREC_FP64, Context, GpuBox
 from mcgpu_gb300.workloads import BoxData
+from test_gpu_fp64_items import device_energy
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +63,21 @@ def test_lj_terms_are_as_exact_as_the_reference_s(ctx):
     print("mean relative error", err(got).mean(), "the reference's", ref.mean())
     assert err(got).mean() <= ref.mean()
     assert err(got).max() <= 60 * 2.0 ** -53      # 12 x (r2 3, 1/r2 1, sigma 1) roundings at most
+
+
+def test_static_lj_terms_are_as_exact_as_the_reference_s(ctx):
+    """The same for the energy over the caller's rows, pair by pair."""
+    box = pairs(6, 6)
+    true = lj(box, np.longdouble, False)
+    got = []
+    for i in range(box.n_mol // 2):
+        b = box.copy()
+        for k in ("x", "y", "z", "sigma", "epsilon", "charge"):
+            setattr(b, k, getattr(box, k)[2 * i:2 * i + 2].copy())
+        b.mol_start = b.mol_pidx_start = b.pidx = np.arange(2)
+        b.mol_len = b.mol_pidx_count = np.ones(2)
+        got.append(device_energy(b.normalise()))
+    err = lambda v: np.abs((v.astype(np.longdouble) - true) / true).astype(float)
+    ref = err(lj(box, np.float64, True))
+    print("mean relative error", err(np.array(got)).mean(), "the reference's", ref.mean())
+    assert err(np.array(got)).mean() <= ref.mean()
