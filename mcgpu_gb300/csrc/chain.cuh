@@ -202,7 +202,12 @@ __device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const 
   // gets its share of the in-range neighbours
   const int rounds = cand ? (c_end - c_begin + 32 * nw - 1) / (32 * nw) : 0;
   const bool precise = H.precise != 0;
-  const bool u3 = H.uniform && H.ulen == 3 && !precise, shared = H.uniform && !u3;
+  const bool u3 = H.uniform && H.ulen == 3 && !precise;
+  // (one warp has nobody to share with: where its teams would be batch_ff's it takes
+  // that, both placements of a neighbour at once: 200 steps of 64 64-atom molecules 66.8
+  // ms, 77.4 by items)
+  const bool teams = T > 1 && (H.ulen & (H.ulen - 1)) == 0;
+  const bool shared = H.uniform && !u3 && !(nw == 1 && teams);
   const unsigned ljmask = H.ljmask;
   // one primary each (the common chain): the moved molecule's two placements
   // and the screen's constants in registers -- the header is global memory,

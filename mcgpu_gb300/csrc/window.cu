@@ -256,7 +256,12 @@ __device__ void window_eval(const Pool& P, const ChainHdr& H, const Group& g, co
 // c takes tasks c, c + clusters, ...), one group of all the CTA's warps per
 // CTA; n_steps steps per chain in windows of K.  trace, trace_off,
 // trace_stride and lanes_cap as in chain_steps.
-__global__ void __launch_bounds__(512, 1)
+//
+// kMaxThreads 512 has 128 registers a thread and spills; 256, for CTAs of up to eight
+// warps, takes the 214 it wants: windows of 4 steps on 64 molecules of 3 and 64 atoms
+// 15.1 ms for 200 steps and 10.7, on 256 9-atom molecules 0.86 and 0.74.
+template <int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads, 1)
     k_chain_window(Pool P, int n_steps, const int* order, int n_tasks, SmemShape shape,
                    mcgpu_trace* trace, int trace_off, int trace_stride, int lanes_cap,
                    bool count_redo) {
@@ -497,56 +502,67 @@ __global__ void __launch_bounds__(512, 1)
 int window_smem_bytes(const SmemShape& sh, int K) { return sh.bytes() + win_extra_bytes(sh, K); }
 
 cudaError_t window_init() {
-  const cudaError_t e = cudaFuncSetAttribute(
-      k_chain_window, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindowSmemMax);
-  if (e != cudaSuccess) return e;
-  // clusters of 16 CTAs are beyond the portable size of 8; where the device
-  // refuses them, window_max_clusters reports none and the setters refuse
-  // the window
-  if (cudaFuncSetAttribute(k_chain_window, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-      cudaSuccess)
-    cudaGetLastError();
+  for (const auto kernel : {k_chain_window<512>, k_chain_window<256>}) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindowSmemMax);
+    if (e != cudaSuccess) return e;
+    // clusters of 16 CTAs are beyond the portable size of 8; where the device
+    // refuses them, window_max_clusters reports none and the setters refuse
+    // the window
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+        cudaSuccess)
+      cudaGetLastError();
+  }
   return cudaSuccess;
 }
 
-int window_max_clusters(int K, int threads, int smem) {
+using WindowKernel = decltype(&k_chain_window<512>);
+
+// Launch configuration of n_clusters clusters of K CTAs; at holds its one attribute.
+static cudaLaunchConfig_t window_config(int K, int n_clusters, int threads, int smem,
+                                        cudaLaunchAttribute* at) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(K, 1, 1);
+  cfg.gridDim = dim3(K * n_clusters, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = K;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = K;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  return cfg;
+}
+
+static int active_clusters(WindowKernel kernel, int K, int threads, int smem) {
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = window_config(K, 1, threads, smem, &at);
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_chain_window, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return n;
 }
 
+int window_max_clusters(int K, int threads, int smem) {
+  return active_clusters(k_chain_window<512>, K, threads, smem);
+}
+
 cudaError_t launch_chain_window(int K, int n_clusters, int threads, int smem, cudaStream_t st,
                                 const Pool& P, int n_steps, const int* order, int n_tasks,
                                 SmemShape sh, mcgpu_trace* trace, int trace_off, int trace_stride,
                                 int lanes_cap, bool count_redo) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(K * n_clusters, 1, 1);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t cfg = window_config(K, n_clusters, threads, smem, &at);
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = K;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_chain_window, P, n_steps, order, n_tasks, sh, trace, trace_off,
-                            trace_stride, lanes_cap, count_redo);
+  // the kernel of more registers where all clusters are resident with it too (37
+  // clusters of 4 are not: one more wave, 1.15 ms against 1.28)
+  const bool few = threads <= 256 &&
+                   active_clusters(k_chain_window<256>, K, threads, smem) >= n_clusters;
+  return cudaLaunchKernelEx(&cfg, few ? k_chain_window<256> : k_chain_window<512>, P, n_steps,
+                            order, n_tasks, sh, trace, trace_off, trace_stride, lanes_cap,
+                            count_redo);
 }
 
 }  // namespace mcgpu
