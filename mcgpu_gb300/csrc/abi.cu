@@ -1501,6 +1501,7 @@ extern "C" int mcgpu_chain_run(mcgpu_box* b, uint64_t seed, uint32_t chain_id, i
                                   trace ? b->dtrace : nullptr, done, 0, 0, true));
     else {
       ChainLaunch A{k, k, 1, nw, b->queue, b->order, b->order + 1, sh};
+      A.in_order = true;
       A.trace = trace ? b->dtrace : nullptr;
       A.trace_off = done;
       if (nw > 8)
@@ -1653,7 +1654,7 @@ static int batch_launch(mcgpu_batch* bt, int steps, cudaStream_t st,
   CK(ctx, cudaMemsetAsync(bt->sched, 0, sizeof(unsigned) * bt->pool.n_chains, st));
   const int n = bt->pool.n_chains;
   const ChainLaunch A{steps, seg, n, gw, bt->sched, bt->order, bt->order + n, sh, trace,
-                      trace_off, trace_stride, bt->lanes};
+                      trace_off, trace_stride, bt->lanes, chains_in_order(n, steps, seg)};
   if (bt->threads > 256)
     k_chain_steps_wide<<<grid, bt->threads, smem, st>>>(bt->pool.P, A);
   else

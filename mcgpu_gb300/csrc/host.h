@@ -25,7 +25,9 @@ __global__ void k_chain_sums(Pool P, const double* emol, double* out);
 __global__ void k_set_energy(Pool P, const double* e);
 // One launch of the one-step chain kernels: n_steps steps of each task (task k
 // runs chain order[k] of sizes[k] molecules), seg at a time on a group of
-// gwarps warps; sched: n_tasks zeroed words.  trace: as mcgpu_batch_run_traced;
+// gwarps warps; sched: n_tasks zeroed words.  in_order: a group takes the next
+// task of `order` and keeps it for all its steps, instead of the one with the most
+// work left for one segment.  trace: as mcgpu_batch_run_traced;
 // lanes_cap > 0 caps the lanes per neighbour molecule.
 struct ChainLaunch {
   int n_steps, seg, n_tasks, gwarps;
@@ -34,7 +36,18 @@ struct ChainLaunch {
   SmemShape shape;
   mcgpu_trace* trace = nullptr;
   int trace_off = 0, trace_stride = 0, lanes_cap = 0;
+  bool in_order = false;
 };
+
+// Whether the tasks are taken in order.  Looking for the one with the most work
+// left takes 2 ns a task (a look through all of them), worth it only beside a
+// segment's microseconds: 4,096 chains of 32 waters, 64-thread groups, 256 steps
+// 12.3 ms in order and 11.3 by work left in segments of 64, 12.7 and 13.4 in
+// segments of 16, 64 steps 3.8 and 5.1 in segments of 4; 16,384 chains of 16 waters 49
+// and 56 ms in segments of 16.  A launch of one segment has nothing to choose.
+inline bool chains_in_order(int n_tasks, int n_steps, int seg) {
+  return n_steps <= seg || n_tasks > 128LL * seg;
+}
 __global__ void k_chain_steps(Pool P, ChainLaunch A);
 __global__ void k_chain_steps_wide(Pool P, ChainLaunch A);
 __global__ void k_chain_init(Pool P, const int* mol_chain, int m_begin, int m_end);

@@ -523,7 +523,8 @@ __device__ __forceinline__ int claim_chain(const int* sizes, unsigned* sched, in
 
 // Persistent kernel: groups of `gwarps` warps take chain tasks (task k runs
 // chain order[k]) for `seg` steps at a time, the one with the most work left
-// first, until each has taken n_steps; sched: n_tasks zeroed words.  With a
+// first (or, in_order, the next one for all its steps), until each has taken
+// n_steps; sched: n_tasks zeroed words.  With a
 // task per group for all its steps, 512 chains of uneven size on 456 groups
 // left the chip half idle in a second wave of 56 (SMs busy 77 % of a launch).
 // A task stays on one group at a time, and its steps on the
@@ -555,19 +556,32 @@ __device__ __forceinline__ void chain_steps(Pool P, const ChainLaunch& A, char* 
   const int lane = threadIdx.x & 31, w = g.warp(), nw = g.nwarps();
   const int group = blockIdx.x * ((int)blockDim.x / gsize) + gid;
   bool start = true;
+  int task = -1, base = 0;
   for (;;) {
-    if (w == 0) {
-      int taken = 0;
-      const int t = claim_chain(A.sizes, A.sched, n_tasks, n_steps, group, start, lane, &taken);
-      start = false;
-      if (lane == 0) {
-        s.misc[31] = t;
-        s.misc[30] = taken;
+    if (A.in_order && task >= 0 && base + seg < n_steps) {
+      base += seg;
+    } else {
+      if (w == 0) {
+        int taken = 0, t = -1;
+        if (A.in_order) {
+          // sched's first word counts the tasks taken
+          if (lane == 0) t = (int)atomicAdd(A.sched, 1u);
+          t = __shfl_sync(~0u, t, 0);
+          if (t >= n_tasks) t = -1;
+        } else {
+          t = claim_chain(A.sizes, A.sched, n_tasks, n_steps, group, start, lane, &taken);
+          start = false;
+        }
+        if (lane == 0) {
+          s.misc[31] = t;
+          s.misc[30] = taken;
+        }
       }
+      g.sync();
+      task = s.misc[31];
+      base = s.misc[30];
+      if (task < 0) break;
     }
-    g.sync();
-    const int task = s.misc[31], base = s.misc[30];
-    if (task < 0) break;
     const int c = A.order[task];
     ChainHdr* Hp = P.hdr + c;
     const ChainHdr& H = *Hp;
@@ -741,7 +755,7 @@ __device__ __forceinline__ void chain_steps(Pool P, const ChainLaunch& A, char* 
     }
     g.sync();
     // give the task back: every thread's writes, then the steps taken
-    if (g.tid == 0) {
+    if (!A.in_order && g.tid == 0) {
       __threadfence();
       atomicExch(A.sched + task, (unsigned)min(base + seg, n_steps));
     }

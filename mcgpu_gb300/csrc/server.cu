@@ -472,6 +472,7 @@ int launch_round(mcgpu_server* s) {
     ChainLaunch A{s->cfg.round_steps, s->cfg.round_steps, n, q ? kWideWarps : s->gw,
                   s->sched + q * nc, dl, dl + 4 * nc + 1, q ? s->wide : s->shape};
     A.lanes_cap = s->cfg.lanes_per_molecule;
+    A.in_order = true;   // (a round is one segment)
     if (q == 1) {
       k_chain_steps_wide<<<std::min(n, s->wide_grid), kWideWarps * 32, s->wide_smem, sq>>>(
           s->pool.P, A);
