@@ -336,7 +336,11 @@ int upload_pool(mcgpu_ctx* ctx, HostPool& hp, DevPool& dp) {
   CK(ctx, cudaStreamSynchronize(st));
   dp.hdr.assign(hp.hdr.begin(), hp.hdr.end());
   dp.min_chain = dp.n_mol;
-  for (const ChainHdr& h : dp.hdr) dp.min_chain = std::min(dp.min_chain, h.n_mol);
+  dp.mixed = false;
+  for (const ChainHdr& h : dp.hdr) {
+    dp.min_chain = std::min(dp.min_chain, h.n_mol);
+    dp.mixed = dp.mixed || !h.uniform;
+  }
   dp.mstart.assign(hp.mstart.begin(), hp.mstart.end());
   dp.mlen.assign(hp.mlen.begin(), hp.mlen.end());
   return MCGPU_OK;
@@ -1584,6 +1588,13 @@ static int batch_grid(mcgpu_batch* bt, int* smem_out) {
   return std::max(1, std::min(need, per_sm * bt->ctx->sm_count));
 }
 
+// All chains of the batch.
+static MolRanges batch_ranges(const mcgpu_batch* bt) {
+  MolRanges r;
+  r.mixed = bt->pool.mixed;
+  return r;
+}
+
 // Few chains with FP64 pairs leave most SMs idle, while each chain's step is bound by
 // the FP64 pipe of its SM (a warp instruction in 16 cycles).  Where no window is set
 // such a batch runs windows of 4 or 2 steps over clusters of as many CTAs, if all
@@ -1729,7 +1740,7 @@ extern "C" int mcgpu_batch_create(mcgpu_ctx* ctx, int n_chains, const mcgpu_box_
     P.vc_fix = dalloc<uint4>(nm, &e2);
     if (e2 == cudaSuccess)
       e2 = launch_chain_energy(P, bt->pool.mol_chain, bt->pool.n_mol, bt->vm, bt->emol2, bt->eabs2,
-                               bt->vsum, bt->vsum_abs, ctx->stream, MolRanges(), false);
+                               bt->vsum, bt->vsum_abs, ctx->stream, batch_ranges(bt), false);
     if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(ctx->stream);
     if (e2 != cudaSuccess) {
       mcgpu_batch_destroy(bt);
@@ -1871,7 +1882,7 @@ static int batch_build_graph(mcgpu_batch* bt, int launches, int interval) {
       cudaError_t e = launch_volume_phase(bt->pool.P, bt->pool.mol_chain, bt->pool.n_mol, bt->vm,
                                           bt->emol2, bt->eabs2, bt->vsum, bt->vsum_abs, bt->vlist,
                                           nullptr, 0,
-                                          0, st, MolRanges(), bt->vol_has64, bt->vol_has32);
+                                          0, st, batch_ranges(bt), bt->vol_has64, bt->vol_has32);
       if (e != cudaSuccess) rc = set_err(ctx, MCGPU_ERR_CUDA, "volume phase launch: %s", cudaGetErrorString(e));
     }
   } else {
@@ -1973,7 +1984,7 @@ static int batch_advance(mcgpu_batch* bt, int n_steps, mcgpu_trace* trace, int t
     if (bt->steps_done % iv == 0) {
       CK(ctx, launch_volume_phase(bt->pool.P, bt->pool.mol_chain, bt->pool.n_mol, bt->vm, bt->emol2,
                                   bt->eabs2, bt->vsum, bt->vsum_abs, bt->vlist, vtrace, vk, vstride,
-                                  ctx->stream, MolRanges(), bt->vol_has64, bt->vol_has32));
+                                  ctx->stream, batch_ranges(bt), bt->vol_has64, bt->vol_has32));
       vk++;
     }
   }

@@ -175,6 +175,7 @@ struct MolRanges {
   const int* act_pref = nullptr;
   int n_act = 0;
   int total = 0;
+  bool mixed = true;   // host: some chain of the ranges is not of one species
 };
 
 struct Pool {

@@ -190,6 +190,7 @@ struct DevPool {
   Pool P{};
   int n_chains = 0, n_mol = 0, n_atom = 0, n_pidx = 0, max_len = 0;
   int min_chain = 0;              // molecules of the smallest chain
+  bool mixed = false;             // some chain is not of one species
   int* mol_chain = nullptr;
   int* atom_mol = nullptr;
   double* emol = nullptr;

@@ -975,6 +975,10 @@ __device__ __forceinline__ void vol_atoms_delta(const float4* so, const float2* 
 // (rc 12 A) and 3.6 ms a round of 160 served jobs (214,016 molecules); 439 us now.
 constexpr int kVolWarpThreads = 256;
 
+//
+// kMixed false: every chain is of one species (the form for mixed lengths costs registers
+// that the other spills: 3 % of an isobaric run of 32,768 waters).
+template <bool kMixed>
 __global__ void __launch_bounds__(kVolWarpThreads, 3)
     k_vol_pair_sums32(Pool P, const int* mol_chain, const VolMove* vm, int m_begin, int n_items,
                       MolRanges R, double2* emol2, double2* eabs2, int init) {
@@ -985,7 +989,7 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
   __shared__ VcStencil S_[kWarps];
   __shared__ int ring_[kWarps][kRing];
   const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = blockIdx.x * kWarps + wi;
+  const int item = blockIdx.x * ((int)blockDim.x >> 5) + wi;
   if (item >= n_items) return;
   const int m = range_mol(R, m_begin, item);
   const int c = mol_chain[m];
@@ -1014,7 +1018,7 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
   const float rad_m = P.mrad[m];
   const float fx0 = H.fxs[0], fx1 = H.fxs[1], fx2 = H.fxs[2];
   const float sm1x = v.sm1[0], sm1y = v.sm1[1], sm1z = v.sm1[2];
-  const bool simple = H.simple_prim != 0, uniform = H.uniform != 0;
+  const bool simple = H.simple_prim != 0, uniform = !kMixed || H.uniform != 0;
   const float lo0 = v.box[0].cut2_lo, hi0 = v.box[0].cut2_hi;
   const float lo1 = v.box[1].cut2_lo, hi1 = v.box[1].cut2_hi;
   // what every pair reads of the first box, in registers
@@ -1030,68 +1034,95 @@ __global__ void __launch_bounds__(kVolWarpThreads, 3)
     ff_add(eh, el, e);
     ab += a;
   };
-  auto pairs = [&](int head, int count) {
-    int bi = 0, e = lane;
-    for (;; e += 32) {
-      while (e >= count) {
-        e -= count;
-        bi++;
-      }
-      if (bi >= maxlen) break;
-      const int jf = ring[(head + e) & (kRing - 1)];
-      const int j = jf & kVolJMask, f = (jf >> kVolFShift) & 3;
-      int bb;
-      float rad_j;
-      if (uniform) {
-        bb = H.atom0 + (j - H.mol0) * maxlen + bi;
-        rad_j = H.umrad;
-      } else {
-        if (bi >= (P.mlen[j] & 255)) continue;
-        bb = P.mstart[j] + bi;
-        rad_j = P.mrad[j];
-      }
-      const uint4 Aj = P.mfix[j];
-      const float4 ob = P.aoff[bb];
-      const float2 qb = P.aeq[bb];
-      const float rr = rad_m + rad_j;
-      float3 Dh, Dl;
-      vol_fixdiff1(Aj.x, Am.x, sx, tx, Dh.x, Dl.x);
-      vol_fixdiff1(Aj.y, Am.y, sy, ty, Dh.y, Dl.y);
-      vol_fixdiff1(Aj.z, Am.z, sz, tz, Dh.z, Dl.z);
-      if (delta && f == 3) {
-        const bool wrap = fabsf(Dh.x) * grow + rr > wx || fabsf(Dh.y) * grow + rr > wy ||
-                          fabsf(Dh.z) * grow + rr > wz;
-        if (!wrap) {
-          const float bx = Dh.x + ob.x, by = Dh.y + ob.y, bz = Dh.z + ob.z;
-          const float lx = ((Dh.x - (bx - (bx - Dh.x))) + (ob.x - (bx - Dh.x))) + Dl.x;
-          const float ly = ((Dh.y - (by - (by - Dh.y))) + (ob.y - (by - Dh.y))) + Dl.y;
-          const float lz = ((Dh.z - (bz - (bz - Dh.z))) + (ob.z - (bz - Dh.z))) + Dl.z;
-          float e32 = 0.f, a32 = 0.f;
-          vol_atoms_delta(so, sq, len, bx, by, bz, lx, ly, lz, Dh.x * sm1x, Dh.y * sm1y,
-                          Dh.z * sm1z, ob.w, qb, e32, a32);
-          add(e32, a32);
-          continue;
-        }
-      }
-#pragma unroll 1
-      for (int w = 0; w < 2; w++) {
-        if (!(f & (1 << w))) continue;
-        const VolBox& B = v.box[w];
-        if (w == 1) vol_fixdiff(Aj, Am, B, Dh, Dl);
-        // b relative to m's anchor as a double-float: two-sum of D + o_b
+  // atom bi of ring entry `at` with the molecule
+  auto term = [&](int at, int bi) {
+    const int jf = ring[at & (kRing - 1)];
+    const int j = jf & kVolJMask, f = (jf >> kVolFShift) & 3;
+    int bb;
+    float rad_j;
+    if (uniform) {
+      bb = H.atom0 + (j - H.mol0) * maxlen + bi;
+      rad_j = H.umrad;
+    } else {
+      bb = P.mstart[j] + bi;
+      rad_j = P.mrad[j];
+    }
+    const uint4 Aj = P.mfix[j];
+    const float4 ob = P.aoff[bb];
+    const float2 qb = P.aeq[bb];
+    const float rr = rad_m + rad_j;
+    float3 Dh, Dl;
+    vol_fixdiff1(Aj.x, Am.x, sx, tx, Dh.x, Dl.x);
+    vol_fixdiff1(Aj.y, Am.y, sy, ty, Dh.y, Dl.y);
+    vol_fixdiff1(Aj.z, Am.z, sz, tz, Dh.z, Dl.z);
+    if (delta && f == 3) {
+      const bool wrap = fabsf(Dh.x) * grow + rr > wx || fabsf(Dh.y) * grow + rr > wy ||
+                        fabsf(Dh.z) * grow + rr > wz;
+      if (!wrap) {
         const float bx = Dh.x + ob.x, by = Dh.y + ob.y, bz = Dh.z + ob.z;
         const float lx = ((Dh.x - (bx - (bx - Dh.x))) + (ob.x - (bx - Dh.x))) + Dl.x;
         const float ly = ((Dh.y - (by - (by - Dh.y))) + (ob.y - (by - Dh.y))) + Dl.y;
         const float lz = ((Dh.z - (bz - (bz - Dh.z))) + (ob.z - (bz - Dh.z))) + Dl.z;
         float e32 = 0.f, a32 = 0.f;
-        if (fabsf(Dh.x) + rr > 0.5f * B.Lf[0] - 1e-3f || fabsf(Dh.y) + rr > 0.5f * B.Lf[1] - 1e-3f ||
-            fabsf(Dh.z) + rr > 0.5f * B.Lf[2] - 1e-3f)
-          vol_atoms32<true>(so, sq, len, bx, by, bz, lx, ly, lz, ob.w, qb, B, e32, a32);
-        else
-          vol_atoms32<false>(so, sq, len, bx, by, bz, lx, ly, lz, ob.w, qb, B, e32, a32);
-        // the change of a volume move: E(V') - E(V)
-        add((delta && w == 0) ? -e32 : e32, a32);
+        vol_atoms_delta(so, sq, len, bx, by, bz, lx, ly, lz, Dh.x * sm1x, Dh.y * sm1y,
+                        Dh.z * sm1z, ob.w, qb, e32, a32);
+        add(e32, a32);
+        return;
       }
+    }
+#pragma unroll 1
+    for (int w = 0; w < 2; w++) {
+      if (!(f & (1 << w))) continue;
+      const VolBox& B = v.box[w];
+      if (w == 1) vol_fixdiff(Aj, Am, B, Dh, Dl);
+      // b relative to m's anchor as a double-float: two-sum of D + o_b
+      const float bx = Dh.x + ob.x, by = Dh.y + ob.y, bz = Dh.z + ob.z;
+      const float lx = ((Dh.x - (bx - (bx - Dh.x))) + (ob.x - (bx - Dh.x))) + Dl.x;
+      const float ly = ((Dh.y - (by - (by - Dh.y))) + (ob.y - (by - Dh.y))) + Dl.y;
+      const float lz = ((Dh.z - (bz - (bz - Dh.z))) + (ob.z - (bz - Dh.z))) + Dl.z;
+      float e32 = 0.f, a32 = 0.f;
+      if (fabsf(Dh.x) + rr > 0.5f * B.Lf[0] - 1e-3f || fabsf(Dh.y) + rr > 0.5f * B.Lf[1] - 1e-3f ||
+          fabsf(Dh.z) + rr > 0.5f * B.Lf[2] - 1e-3f)
+        vol_atoms32<true>(so, sq, len, bx, by, bz, lx, ly, lz, ob.w, qb, B, e32, a32);
+      else
+        vol_atoms32<false>(so, sq, len, bx, by, bz, lx, ly, lz, ob.w, qb, B, e32, a32);
+      // the change of a volume move: E(V') - E(V)
+      add((delta && w == 0) ? -e32 : e32, a32);
+    }
+  };
+  auto pairs = [&](int head, int count) {
+    int bi = 0, e = lane;
+    if (uniform) {
+      // an atom at a time over the neighbours
+      for (;; e += 32) {
+        while (e >= count) {
+          e -= count;
+          bi++;
+        }
+        if (bi >= maxlen) break;
+        term(head + e, bi);
+      }
+      return;
+    }
+    // neighbour after neighbour, an item's found in the prefix sums of their lengths
+    const int l = lane < count ? P.mlen[ring[(head + lane) & (kRing - 1)] & kVolJMask] & 255 : 0;
+    int pref = l;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(~0u, pref, off);
+      if (lane >= off) pref += u;
+    }
+    const int total = __shfl_sync(~0u, pref, 31);
+    pref -= l;
+    for (int it = lane; it - lane < total; it += 32) {
+      e = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int u = __shfl_sync(~0u, pref, (e + step) & 31);
+        if (e + step < count && u <= it) e += step;
+      }
+      bi = it - __shfl_sync(~0u, pref, e);
+      if (it < total) term(head + e, bi);
     }
   };
   const unsigned lt = lanemask_lt();
@@ -1333,8 +1364,19 @@ __global__ void k_vol_self_energy(Pool P, const VolMove* vm, const double2* esum
   P.hdr[c].run_err = f64 ? 0.0 : kTieRel * esum_abs[c].x;
 }
 
-static int vol_warp_grid(int n) {
-  return (n + kVolWarpThreads / 32 - 1) / (kVolWarpThreads / 32);
+// Threads of a CTA of k_vol_pair_sums32 for n molecules: fewer warps where the CTAs
+// would not reach all 152 SMs (a move of 64 molecules on 8 SMs takes the time of eight
+// such molecules an SM).
+static int vol_warp_threads(int n) {
+  return 32 * std::max(1, std::min(kVolWarpThreads / 32, n / 152));
+}
+static void pair_sums32(const Pool& P, const int* mol_chain, const VolMove* vm, int m_begin, int n,
+                        const MolRanges& act, double2* emol2, double2* eabs2, int init,
+                        cudaStream_t st) {
+  const int threads = vol_warp_threads(n), warps = threads / 32;
+  const auto kernel = act.mixed ? k_vol_pair_sums32<true> : k_vol_pair_sums32<false>;
+  kernel<<<(n + warps - 1) / warps, threads, 0, st>>>(P, mol_chain, vm, m_begin, n, act, emol2,
+                                                      eabs2, init);
 }
 
 // Sets the running energy of the chains in act (all when act has no
@@ -1361,8 +1403,7 @@ cudaError_t launch_chain_energy(Pool P, const int* mol_chain, int n_mol_total, V
     if (f64)
       k_vol_pair_sums<<<n, kVolThreads, 0, st>>>(P, mol_chain, vm, m0, act, emol2, 2);
     else
-      k_vol_pair_sums32<<<vol_warp_grid(n), kVolWarpThreads, 0, st>>>(P, mol_chain, vm, m0, n, act,
-                                                                     emol2, eabs2, 1);
+      pair_sums32(P, mol_chain, vm, m0, n, act, emol2, eabs2, 1, st);
   }
   k_vol_sums<<<nc, kVolSumThreads, 0, st>>>(P, vm, emol2, eabs2, esum, esum_abs, act, 1);
   k_vol_self_energy<<<(nc + 127) / 128, 128, 0, st>>>(P, vm, esum, esum_abs, act, nc, f64 ? 1 : 0);
@@ -1397,8 +1438,7 @@ cudaError_t launch_volume_phase(Pool P, const int* mol_chain, int n_mol_total, V
       if (f64)
         k_vol_pair_sums<<<items, kVolThreads, 0, st>>>(P, mol_chain, vm, 0, act, emol2, pass);
       else
-        k_vol_pair_sums32<<<vol_warp_grid(items), kVolWarpThreads, 0, st>>>(
-            P, mol_chain, vm, 0, items, act, emol2, eabs2, 0);
+        pair_sums32(P, mol_chain, vm, 0, items, act, emol2, eabs2, 0, st);
       return;
     }
     const int chunk = 1 << 20;
@@ -1407,8 +1447,7 @@ cudaError_t launch_volume_phase(Pool P, const int* mol_chain, int n_mol_total, V
       if (f64)
         k_vol_pair_sums<<<n, kVolThreads, 0, st>>>(P, mol_chain, vm, m0, act, emol2, pass);
       else
-        k_vol_pair_sums32<<<vol_warp_grid(n), kVolWarpThreads, 0, st>>>(
-            P, mol_chain, vm, m0, n, act, emol2, eabs2, 0);
+        pair_sums32(P, mol_chain, vm, m0, n, act, emol2, eabs2, 0, st);
     }
   };
   if (has64) pairs(true, 0);

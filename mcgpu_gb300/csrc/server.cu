@@ -83,6 +83,7 @@ struct Job {
   HostPool hp;  // the job's rows as chain 0 at offset 0
   int64_t n_steps = 0;
   int npt = 0, vol_mixed = 0;
+  bool mixed = true;   // not of one species
   double pressure = 0, max_dlnv = 0, lrc_v = 0;
   double *x_out = nullptr, *y_out = nullptr, *z_out = nullptr;
   double t_submit = 0, t_admit = 0;
@@ -281,6 +282,7 @@ int upload_job(mcgpu_server* s, Job* j) {
   h.max_dlnv = j->max_dlnv;
   h.lrc_v = j->lrc_v;
   h.vol_mixed = j->vol_mixed;
+  j->mixed = !h.uniform;
   Pool& P = s->pool.P;
   int rc = MCGPU_OK;
 #define SC(dst, vec) \
@@ -309,6 +311,7 @@ int upload_job(mcgpu_server* s, Job* j) {
   R.act_pref = dr + 2;
   R.n_act = 1;
   R.total = n;
+  R.mixed = j->mixed;
   CK(ctx, launch_chain_energy(P, s->pool.mol_chain, 0, s->vm, s->emol2, s->eabs2, s->vsum,
                               s->vsum_abs, st, R, !(j->npt && j->vol_mixed)));
   return MCGPU_OK;
@@ -420,7 +423,7 @@ int launch_round(mcgpu_server* s) {
   if (act[0].empty() && act[1].empty()) return MCGPU_OK;
   struct Kind {
     int n_npt = 0, total = 0;
-    bool has64 = false, has32 = false;
+    bool has64 = false, has32 = false, mixed = false;
   } kind[2];
   for (int q = 0; q < 2; q++) {
     // cost-descending order: screen ~ n_mol, pairs ~ max_len^2
@@ -442,6 +445,7 @@ int launch_round(mcgpu_server* s) {
       if (!j->npt) continue;
       k.has64 = k.has64 || !j->vol_mixed;
       k.has32 = k.has32 || j->vol_mixed;
+      k.mixed = k.mixed || j->mixed;
       aslot[k.n_npt] = act[q][i];
       am0[k.n_npt] = (int)j->m0;
       apref[k.n_npt] = k.total;
@@ -493,6 +497,7 @@ int launch_round(mcgpu_server* s) {
       R.act_pref = dl + 3 * nc;
       R.n_act = k.n_npt;
       R.total = k.total;
+      R.mixed = k.mixed;
       CK(ctx, launch_volume_phase(s->pool.P, s->pool.mol_chain, 0, s->vm, s->emol2, s->eabs2,
                                   s->vsum, s->vsum_abs, s->vlist + q * (3 * nc + 3), nullptr, 0,
                                   0, sq, R, k.has64, k.has32));
