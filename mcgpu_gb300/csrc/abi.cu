@@ -448,8 +448,8 @@ int pool_nl_rebuild(mcgpu_ctx* ctx, DevPool& dp, cudaStream_t st) {
 
 // Full system energy of every chain of the pool into dp.esum (device).
 int pool_system_energy(mcgpu_ctx* ctx, DevPool& dp, bool f64, cudaStream_t st) {
-  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, dp.min_chain, shape_for(dp.max_len, kPlainWarps),
-                               st, dp.P, dp.mol_chain, dp.emol));
+  CK(ctx, launch_mol_pair_sums(f64, dp.n_mol, dp.min_chain, dp.batch,
+                               shape_for(dp.max_len, kPlainWarps), st, dp.P, dp.mol_chain, dp.emol));
   k_chain_sums<<<dp.n_chains, 256, 0, st>>>(dp.P, dp.emol, dp.esum);
   CK(ctx, cudaGetLastError());
   return MCGPU_OK;
@@ -811,7 +811,7 @@ extern "C" int mcgpu_system_energy(mcgpu_box* b, double* out) {
     // calcSystemEnergy with ENABLE_INTRA: molecule m adds E(m, j > m) and its
     // intramolecular energy (SimulationStep.cpp:40-71 over :15-18)
     DevPool& dp = b->pool;
-    CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64, dp.n_mol, dp.min_chain,
+    CK(ctx, launch_mol_pair_sums(b->precision == MCGPU_PREC_FP64, dp.n_mol, dp.min_chain, dp.batch,
                                  shape_for(dp.max_len, kPlainWarps), ctx->stream, dp.P,
                                  dp.mol_chain, dp.emol));
     CK(ctx, launch_intra_add(dp.P, b->intra->R, dp.n_mol, dp.emol, ctx->stream));
@@ -1686,6 +1686,7 @@ extern "C" int mcgpu_batch_create(mcgpu_ctx* ctx, int n_chains, const mcgpu_box_
   if (int rc = build_pool(ctx, hp, descs, n_chains, seeds, rotation)) return rc;
   mcgpu_batch* bt = new mcgpu_batch();
   bt->ctx = ctx;
+  bt->pool.batch = true;
   int rc = upload_pool(ctx, hp, bt->pool);
   if (rc) {
     delete bt;

@@ -73,8 +73,9 @@ cudaError_t launch_move_energies(bool f64, int grid, SmemShape sh, cudaStream_t 
                                  unsigned* counter, double* out, long long* pairs = nullptr,
                                  unsigned* done = nullptr, unsigned call = 0);
 // emol[m], summed over a chain's molecules, with E(m, j > m); min_chain: the
-// molecules of the smallest chain.  A chain's rows depend on the chain alone.
-cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, SmemShape sh,
+// molecules of the smallest chain; batch: the pool is a batch's, not a box's.  A
+// chain's rows depend on the chain alone.
+cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, bool batch, SmemShape sh,
                                  cudaStream_t st, const Pool& P, const int* mol_chain,
                                  double* emol);
 // One volume phase of the chains in act (all when act has no ranges) on
@@ -191,6 +192,7 @@ struct DevPool {
   int n_chains = 0, n_mol = 0, n_atom = 0, n_pidx = 0, max_len = 0;
   int min_chain = 0;              // molecules of the smallest chain
   bool mixed = false;             // some chain is not of one species
+  bool batch = false;             // a batch's pool (a box's holds one chain too)
   int* mol_chain = nullptr;
   int* atom_mol = nullptr;
   double* emol = nullptr;

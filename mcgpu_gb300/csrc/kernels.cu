@@ -228,7 +228,7 @@ struct PoolRows {
 // waters (rc 12 A, 35.6 M pairs): 1.84 ms, bound by the issue of the N^2 / 2
 // screen beside the FP64 pipe (58 % busy); 5.84 ms with a CTA per molecule.
 __global__ void __launch_bounds__(kPsThreads, 4)
-    k_pair_sums64(Pool P0, const LoopTask* tasks, const int* mol_chain, int n_mol, int span,
+    k_pair_sums64(Pool P0, const LoopTask* tasks, const int* mol_chain, int n_mol, int span, int per,
                   double* emol) {
   __shared__ Pool SP;
   __shared__ PsGroup G;
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
   const Pool& P = SP;
   if (tasks) {
     n_mol = tasks[blockIdx.y].n_mol;
-    span = ps_group(n_mol);
+    span = ps_group(n_mol, per);
     emol = tasks[blockIdx.y].emol;
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kPsThreads, 4)
   while (m0 < mg) {
     const int c = tasks ? 0 : mol_chain[m0];
     const ChainHdr& H = P.hdr[c];
-    const int group = ps_group(H.n_mol), off = (m0 - H.mol0) % group;
+    const int group = ps_group(H.n_mol, per), off = (m0 - H.mol0) % group;
     const int m1 = min(m0 - off + group, H.mol0 + H.n_mol), n = m1 - m0;
     if (off > 0) {   // inside a group that starts before this CTA's molecules
       m0 = m1;
@@ -802,15 +802,18 @@ cudaError_t launch_move_energies(bool f64, int grid, SmemShape sh, cudaStream_t 
   return cudaGetLastError();
 }
 
-int pair_sum_groups(int n_mol) { return (n_mol + ps_group(n_mol) - 1) / ps_group(n_mol); }
+int pair_sum_groups(int n_mol) {
+  const int group = ps_group(n_mol, kPsPerBox);
+  return (n_mol + group - 1) / group;
+}
 
-cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, SmemShape sh,
+cudaError_t launch_mol_pair_sums(bool f64, int n_mol, int min_chain, bool batch, SmemShape sh,
                                  cudaStream_t st, const Pool& P, const int* mol_chain,
                                  double* emol) {
   if (f64) {
-    const int span = ps_group(min_chain);
+    const int per = batch ? kPsPerBatch : kPsPerBox, span = ps_group(min_chain, per);
     k_pair_sums64<<<(n_mol + span - 1) / span, kPsThreads, 0, st>>>(P, nullptr, mol_chain, n_mol,
-                                                                    span, emol);
+                                                                    span, per, emol);
   } else {
     k_pair_sums32<<<n_mol, kPlainThreads, sh.bytes(), st>>>(P, nullptr, mol_chain, 0, sh, emol);
   }
@@ -825,7 +828,7 @@ cudaError_t launch_box_energies(bool f64, const LoopTask* tasks, int n_tasks, in
     const LoopTask* T = tasks + t0;
     if (f64) {
       k_pair_sums64<<<dim3(max_groups, nt), kPsThreads, 0, st>>>(Pool{}, T, nullptr, 0, 0,
-                                                                 nullptr);
+                                                                 kPsPerBox, nullptr);
     } else {
       k_pair_sums32<<<dim3(max_mol, nt), kPlainThreads, sh.bytes(), st>>>(Pool{}, T, nullptr, 0,
                                                                            sh, nullptr);

@@ -326,7 +326,7 @@ extern "C" int mcgpu_system_energy_static(const mcgpu_box_desc* rows, double* ou
   sc.lo = (float)(r.cutoff * r.cutoff - band);
   sc.hi = (float)(r.cutoff * r.cutoff + band);
   sc.far = (float)(2.0 * Lmax);
-  const int group = mcgpu::ps_group(r.n_mol), grid = (r.n_mol + group - 1) / group;
+  const int group = mcgpu::ps_group(r.n_mol, mcgpu::kPsPerBox), grid = (r.n_mol + group - 1) / group;
   k_static_pair_sums<<<grid, mcgpu::kPsThreads, 0, st>>>(r, sc, group, emol);
   cudaError_t e = launch_error();
   if (e == cudaSuccess) {
