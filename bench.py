@@ -51,15 +51,15 @@ FP32_FLOPS_PER_PAIR = 38   # per atom pair, fixed by convention from the referen
 # DRAM bytes (read + write) per launch of k_chain_steps on this workload,
 # measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum, mean of six
 # launches after the untimed steps, L2 flushed between bench steps), by tile
-# (threads, chains per CTA, steps per launch, lanes per molecule), each with
-# the version of the chain kernel it was captured on.  A capture is reported
-# only for its own tile and kernel version; otherwise the line's traffic is
-# null and says why (a launch reads the chains' rows about once whatever the
+# (threads, chains per CTA, steps per launch, lanes per molecule, which play no part on
+# 3-site chains), each with the version of the chain kernel it was captured on.  A
+# capture is reported only for its own tile and kernel version; otherwise the line's
+# traffic is null and says why (a launch reads the chains' rows about once whatever the
 # tile, ~34 MB, but a figure from another tile or kernel is not this run's).
-CHAIN_KERNEL_VERSION = ("chains handed between groups each segment, a lane per (entry, placement) "
-                        "of a 3-site pair batch, two-sum reduction over the lanes")
-CHAIN_TRAFFIC_BYTES = {(160, 1, 64, 1): (33.97e6, "pair code shared by both placements, LJ mask in "
-                                         "the header, FP64 re-takes from blending rows")}
+CHAIN_KERNEL_VERSION = ("one segment: chains in order of cost, a lane per (entry, placement) of a "
+                        "3-site pair batch, two-sum reduction over the lanes")
+CHAIN_TRAFFIC_BYTES = {(160, 1, 64, lanes): (33.85e6, CHAIN_KERNEL_VERSION)
+                       for lanes in (0, 1, 2, 4)}
 
 
 def chain_traffic(tile):

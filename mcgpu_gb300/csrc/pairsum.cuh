@@ -116,8 +116,9 @@ __device__ __forceinline__ double ps_block_sum(PsGroup& G, double acc) {
 // 152 SMs (their shares of the in-range pairs are uneven; 286 CTAs of 7 of
 // 1,999 16-atom molecules left the busiest SM 1.6 times the mean).  In a batch the
 // other chains fill the SMs, and a chain's groups are larger: 152 chains of 2,000
-// waters 3.05 ms, 6.6 by the boxes' rule (one chain of 700: 76 us, 54).  Either way the groups follow from the chain's own size -- the card's 152 SMs are a
-// constant here -- so its sum is the same alone and among others.
+// waters 3.05 ms, 6.6 by the boxes' rule (one chain of 700: 76 us, 54).  Either way
+// the groups follow from the chain's own size -- the card's 152 SMs are a constant
+// here -- so its sum is the same alone and among others.
 constexpr int kPsPerBox = 152 * 8, kPsPerBatch = 128;
 __host__ __device__ inline int ps_group(int n, int per) {
   const int g = n / per;
