@@ -185,10 +185,11 @@ __device__ __forceinline__ unsigned uniform_lj_mask(const Pool& P, const ChainHd
 // first `workers` warps as items (one more barrier): every warp waited for the
 // one with most (4,000 16-atom molecules on 16 warps: 45 neighbours, 3 +- 2 a
 // warp, 29,000 cycles a step).  Other chains evaluate their own rings in
-// batches of 32, T lanes per neighbour molecule -- and so do chains of 3-site
-// molecules, a lane per placement: there the extra barrier costs what the
-// balance gains (512 water chains: 14.2 ms either way on 256 threads, 14.0
-// against 16.5 on 160).
+// batches of 32, T lanes per neighbour molecule -- and so do chains of molecules of
+// up to 3 sites, a lane per placement: there the extra barrier costs what the
+// balance gains or more (512 water chains: 14.2 ms either way on 256 threads, 14.0
+// against 16.5 on 160; 1,024 chains of 32 atoms, 64 steps on 64 threads 0.41 and 0.55;
+// with lists on five warps the atoms would gain 6 % by sharing).
 __device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const Group& g,
                                         const GroupSmem& s, const MovedInfo& mi,
                                         const float4* pcache, int c_begin, int c_end, int workers,
@@ -202,12 +203,13 @@ __device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const 
   // gets its share of the in-range neighbours
   const int rounds = cand ? (c_end - c_begin + 32 * nw - 1) / (32 * nw) : 0;
   const bool precise = H.precise != 0;
-  const bool u3 = H.uniform && H.ulen == 3 && !precise;
-  // (one warp has nobody to share with: where its teams would be batch_ff's it takes
-  // that, both placements of a neighbour at once: 200 steps of 64 64-atom molecules 66.8
-  // ms, 77.4 by items)
-  const bool teams = T > 1 && (H.ulen & (H.ulen - 1)) == 0;
-  const bool shared = H.uniform && !u3 && !(nw == 1 && teams);
+  const bool own = H.uniform && !precise && H.ulen <= 3;
+  // (one warp has nobody to share with: where its teams, of one lane for 4 sites, would
+  // be batch_ff's it takes that, both placements of a neighbour at once: 200 steps of 64
+  // 64-atom molecules 66.8 ms, 77.4 by items; 256 chains of 64 4-site ones, 64 steps
+  // 0.82 and 0.98)
+  const bool teams = (H.ulen & (H.ulen - 1)) == 0;
+  const bool shared = H.uniform && !own && !(nw == 1 && teams);
   const unsigned ljmask = H.ljmask;
   // one primary each (the common chain): the moved molecule's two placements
   // and the screen's constants in registers -- the header is global memory,
@@ -263,8 +265,12 @@ __device__ inline void group_eval_chain(const Pool& P, const ChainHdr& H, const 
     if (!shared) {
       const int count = min(32, tail - head);
       if (count > 0) {
-        if (u3)
-          batch_u3(P, H, s, mi, rj, head, count, lane, acc, ljmask);
+        if (own && H.ulen == 3)
+          batch_un<3>(P, H, s, mi, rj, head, count, lane, acc, ljmask);
+        else if (own && H.ulen == 1)
+          batch_un<1>(P, H, s, mi, rj, head, count, lane, acc, ljmask);
+        else if (own && H.ulen == 2)
+          batch_un<2>(P, H, s, mi, rj, head, count, lane, acc, ljmask);
         else if (precise)
           batch_ff<true>(P, H, s, mi, rj, head, count, lane, T, acc);
         else

@@ -442,15 +442,16 @@ __device__ __forceinline__ void batch_ff(const Pool& P, const ChainHdr& H, const
   }
 }
 
-// batch_ff for a uniform chain of molecules of 3 atoms, one lane per (entry,
-// placement): a batch of at most 16 entries takes one round of 9 pair terms (a
+// batch_ff for a uniform chain of molecules of N (1 to 3) atoms, one lane per (entry,
+// placement): a batch of at most 16 entries takes one round of N^2 pair terms (a
 // warp's share of the in-range neighbours is about 15 to 20, so a lane per
 // entry left half the lanes idle for twice the time).  Rows and factors follow
-// from the neighbour's index, and the four rows are requested together (one
+// from the neighbour's index, and the rows are requested together (one
 // round trip to L2).  ljmask bits 4k + i: the LJ term of neighbour atom k with
 // moved atom i is not exactly zero (the same in every lane).  Each placement's
 // sum is batch_ff's bit for bit.
-__device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const GroupSmem& s,
+template <int N>
+__device__ __forceinline__ void batch_un(const Pool& P, const ChainHdr& H, const GroupSmem& s,
                                          const MovedInfo& mi, const int* rj, int head, int count,
                                          int lane, AccFF& acc, unsigned ljmask) {
   const int atom0 = H.atom0, mol0 = H.mol0;
@@ -466,11 +467,11 @@ __device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const
     const int jf = rj[(head + (p ? it - count : it)) & (kRing - 1)];
     if (!(jf & (p ? kInNew : kInOld))) continue;
     const int j = jf >> 4;
-    const int b0 = atom0 + (j - mol0) * 3;
+    const int b0 = atom0 + (j - mol0) * N;
     const uint4 fj = P.mfix[j];
-    float4 ob[3];
+    float4 ob[N];
 #pragma unroll
-    for (int k = 0; k < 3; k++) ob[k] = P.aoff[b0 + k];
+    for (int k = 0; k < N; k++) ob[k] = P.aoff[b0 + k];
     const float4* o = p ? s.o_new : s.o_old;
     const uint4 fm = p ? mi.fx_new : mi.fx_old;
     const float3 D = make_float3((float)(int)(fj.x - fm.x) * sx, (float)(int)(fj.y - fm.y) * sy,
@@ -481,18 +482,24 @@ __device__ __forceinline__ void batch_u3(const Pool& P, const ChainHdr& H, const
     float sp = 0.f, sa = 0.f;
     if (wrap) {
 #pragma unroll 1
-      for (int k = 0; k < 3; k++) {
-        const float4 b = k == 0 ? ob[0] : k == 1 ? ob[1] : ob[2];
-        sp += sum_moved32_wrap<false, false, 3>(o, nullptr, s.eq, 3,
+      for (int k = 0; k < N; k++) {
+        float4 b = ob[0];
+#pragma unroll
+        for (int c = 1; c < N; c++)
+          if (k == c) b = ob[c];
+        sp += sum_moved32_wrap<false, false, N>(o, nullptr, s.eq, N,
                                                 make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
                                                 make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], H, sa,
                                                 (ljmask >> (4 * k)) & 15u);
       }
     } else {
 #pragma unroll 1
-      for (int k = 0; k < 3; k++) {
-        const float4 b = k == 0 ? ob[0] : k == 1 ? ob[1] : ob[2];
-        sp += sum_moved32_cf<false, false, 3>(o, nullptr, s.eq, 3, p,
+      for (int k = 0; k < N; k++) {
+        float4 b = ob[0];
+#pragma unroll
+        for (int c = 1; c < N; c++)
+          if (k == c) b = ob[c];
+        sp += sum_moved32_cf<false, false, N>(o, nullptr, s.eq, N, p,
                                               make_float3(D.x + b.x, D.y + b.y, D.z + b.z),
                                               make_float3(0.f, 0.f, 0.f), b.w, s.teq[k], mi.qm,
                                               sa, (ljmask >> (4 * k)) & 15u);
